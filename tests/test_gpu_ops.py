@@ -1,5 +1,6 @@
 """Parity of the CUDA operators (through the C ABI) with the CPU oracle and the golden vectors."""
 import math
+import types
 
 import pytest
 import torch
@@ -992,3 +993,17 @@ def test_layer_norm_applied_by_the_epilogue_of_the_product(with_slopes, Do):
     with pytest.raises(_lib.FaithError):   # 64 output features: not a shape of the fused kernel
         ops.matmul_residual_ln(*x, W[:64].contiguous(), bias[:64].contiguous(), tuple(v[..., :64].contiguous() for v in res),
                                rs, gamma[:64].contiguous(), beta[:64].contiguous(), *extra)
+
+
+@pytest.mark.parametrize("B,L,Do,Dy", [(1, 1, 128, 17), (1, 8, 516, 33), (1, 9, 1030, 128), (5, 51, 37, 96), (1, 255, 128, 512)])
+def test_product_of_few_rows(B, L, Do, Dy):
+    """The kernel for a few output tiles (8 rows x 32 columns per block, K split over the warps): remainders of rows, columns
+    and K, K beyond one chunk, K not a multiple of four."""
+    import faith_b200
+    t = cases.rand_bounds(1301, B, L, 2, Do)
+    W, bias = cases.rand_weight(1302, Dy, Do)
+    x = faith_b200.BoundsLite(2.0, 0.1, *[v.to(DEV) for v in t])
+    got = x.dense(types.SimpleNamespace(weight=W.to(DEV), bias=bias.to(DEV)))
+    o = O.OBounds(2.0, 0.1, *t).dense(W, bias)
+    o64 = O.OBounds(2.0, 0.1, *[v.double() for v in t]).dense(W.double(), bias.double())
+    helpers.assert_bounds_arbitrated(got, o, o64, "product of few rows %d %d %d" % (B * L, Do, Dy))
