@@ -78,6 +78,9 @@ SIGNATURES = {
     "fb_layernorm_novar_f32": [_P] * 14 + [_L, _I, _I, _P],
     "fb_split_heads_f32": [_P] * 4 + [_I] * 6 + [_P],
     "fb_merge_heads_f32": [_P] * 4 + [_I] * 5 + [_P],
+    "fb_split_heads_bound_f32": [_P] * 8 + [_I] * 6 + [_P],
+    "fb_merge_heads_bound_f32": [_P] * 8 + [_I] * 5 + [_P],
+    "fb_layernorm_standard_f32": [_P] * 10 + [_L, _I, _I, _I, _I, _F, _P, _P],
     "fb_conv2d_f32": [_P] * 10 + [_I] * 10 + [_P],
     "fb_conv2d_identity_relax_f32": [_I, _P, _P, _P, _P, _F] + [_P] * 5 + [_L, _L] + [_I] * 9 + [_F, _P, _P],
     "fb_conv2d_windowed_f32": [_P] * 5 + [_L, _L, _I, _I, _P, _I] + [_I] * 8 + [_P],
@@ -135,6 +138,22 @@ def load():
         fn.restype = _OTHER_RESTYPE.get(name, _I)
     _lib = lib
     return lib
+
+
+_binding_module = None
+
+
+def binding():
+    """The extension module behind ops.py (argument checks, output allocation and the C call in one native function per
+    operator), loaded once and over the same library."""
+    global _binding_module
+    if _binding_module is None:
+        load()
+        import torch  # noqa: F401  (the module links against torch's libraries)
+        from . import _binding
+        _binding.setup(FaithError, check)
+        _binding_module = _binding
+    return _binding_module
 
 
 class FaithError(RuntimeError):

@@ -15,40 +15,57 @@ inline unsigned stream_blocks(int64_t work_items) {
   return (unsigned)(want < 1 ? 1 : (want < cap ? want : cap));
 }
 
-// z = x + y over two (pointer, count) segments per side: the weight tensors and the bias tensors.
+// The exact operators below walk the weight tensors and the bias tensors of a bound in one launch: items [0, nv) are
+// groups of VEC weight elements, items [nv, nv + nb) single bias elements (two launches for a [1, 32, 128, 128] bound cost
+// more than the work: 2.1 + 1.7 us and the gap between them against 2.4 us).
+struct Lines {   // lower and upper line of one tensor
+  const float *l, *u;
+};
+struct OutLines {
+  float *l, *u;
+};
+
+// z = x + y
 template <int VEC>
 __global__ void __launch_bounds__(kThreads)
-add_kernel(const float* __restrict__ xa, const float* __restrict__ ya, float* __restrict__ za,
-           const float* __restrict__ xb, const float* __restrict__ yb, float* __restrict__ zb,
-           int64_t n) {
+add_kernel(Lines xw, Lines yw, OutLines zw, Lines xb, Lines yb, OutLines zb, int64_t nv, int64_t nb) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i * VEC < n; i += stride) {
-    if (VEC == 4) {
-      const float4 a = reinterpret_cast<const float4*>(xa)[i], b = reinterpret_cast<const float4*>(ya)[i];
-      const float4 c = reinterpret_cast<const float4*>(xb)[i], d = reinterpret_cast<const float4*>(yb)[i];
-      reinterpret_cast<float4*>(za)[i] = make_float4(fadd(a.x, b.x), fadd(a.y, b.y), fadd(a.z, b.z), fadd(a.w, b.w));
-      reinterpret_cast<float4*>(zb)[i] = make_float4(fadd(c.x, d.x), fadd(c.y, d.y), fadd(c.z, d.z), fadd(c.w, d.w));
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv + nb; i += stride) {
+    if (i >= nv) {
+      const int64_t k = i - nv;
+      const float a = fadd(xb.l[k], yb.l[k]), b = fadd(xb.u[k], yb.u[k]);   // z may be x
+      zb.l[k] = a;
+      zb.u[k] = b;
+    } else if (VEC == 4) {
+      const float4 a = reinterpret_cast<const float4*>(xw.l)[i], b = reinterpret_cast<const float4*>(yw.l)[i];
+      const float4 c = reinterpret_cast<const float4*>(xw.u)[i], d = reinterpret_cast<const float4*>(yw.u)[i];
+      reinterpret_cast<float4*>(zw.l)[i] = make_float4(fadd(a.x, b.x), fadd(a.y, b.y), fadd(a.z, b.z), fadd(a.w, b.w));
+      reinterpret_cast<float4*>(zw.u)[i] = make_float4(fadd(c.x, d.x), fadd(c.y, d.y), fadd(c.z, d.z), fadd(c.w, d.w));
     } else {
-      za[i] = fadd(xa[i], ya[i]);
-      zb[i] = fadd(xb[i], yb[i]);
+      const float a = fadd(xw.l[i], yw.l[i]), b = fadd(xw.u[i], yw.u[i]);
+      zw.l[i] = a;
+      zw.u[i] = b;
     }
   }
 }
 
-// za = c * xa, zb = c * xb (the caller swaps the sides for c <= 0)
+// z = c * x (the caller swaps the sides for c <= 0)
 template <int VEC>
 __global__ void __launch_bounds__(kThreads)
-scale_kernel(const float* __restrict__ xa, float* __restrict__ za, const float* __restrict__ xb,
-             float* __restrict__ zb, float c, int64_t n) {
+scale_kernel(Lines xw, OutLines zw, Lines xb, OutLines zb, float c, int64_t nv, int64_t nb) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i * VEC < n; i += stride) {
-    if (VEC == 4) {
-      const float4 a = reinterpret_cast<const float4*>(xa)[i], b = reinterpret_cast<const float4*>(xb)[i];
-      reinterpret_cast<float4*>(za)[i] = make_float4(fmul(a.x, c), fmul(a.y, c), fmul(a.z, c), fmul(a.w, c));
-      reinterpret_cast<float4*>(zb)[i] = make_float4(fmul(b.x, c), fmul(b.y, c), fmul(b.z, c), fmul(b.w, c));
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv + nb; i += stride) {
+    if (i >= nv) {
+      const int64_t k = i - nv;
+      zb.l[k] = fmul(xb.l[k], c);
+      zb.u[k] = fmul(xb.u[k], c);
+    } else if (VEC == 4) {
+      const float4 a = reinterpret_cast<const float4*>(xw.l)[i], b = reinterpret_cast<const float4*>(xw.u)[i];
+      reinterpret_cast<float4*>(zw.l)[i] = make_float4(fmul(a.x, c), fmul(a.y, c), fmul(a.z, c), fmul(a.w, c));
+      reinterpret_cast<float4*>(zw.u)[i] = make_float4(fmul(b.x, c), fmul(b.y, c), fmul(b.z, c), fmul(b.w, c));
     } else {
-      za[i] = fmul(xa[i], c);
-      zb[i] = fmul(xb[i], c);
+      zw.l[i] = fmul(xw.l[i], c);
+      zw.u[i] = fmul(xw.u[i], c);
     }
   }
 }
@@ -216,27 +233,43 @@ layernorm_novar_row128_kernel(const float* __restrict__ x_lw, const float* __res
 }
 
 // Head split / merge: pure index permutations with the head dimension d contiguous on both
-// sides.  One thread per group of VEC consecutive features.
-//   split: src [B, L, M, H, d] -> dst [B, H, L, M, d]      (M = Di for weights, 1 for biases)
+// sides.  One thread per group of VEC consecutive features; the weights (M = Di) and the biases (M = 1) of a line in one
+// launch, blockIdx.y = line when both lines are given.  Index: 32-bit unless the tensor needs more (five 64-bit divisions
+// per thread cost more than the copy).
+//   split: src [B, L, M, H, d] -> dst [B, H, L, M, d]
 //   merge: the inverse.
-template <int VEC, bool SPLIT>
+template <typename Index, bool SPLIT>
+__device__ __forceinline__ void permute_item(Index i, Index M, Index L, Index H, Index dv, Index& s, Index& o) {
+  // i enumerates the [B, H, L, M, d/VEC] side
+  Index t = i;
+  const Index f = t % dv; t /= dv;
+  const Index m = t % M; t /= M;
+  const Index l = t % L; t /= L;
+  const Index h = t % H;
+  const Index b = t / H;
+  const Index packed = (((b * L + l) * M + m) * H + h) * dv + f;  // [B, L, M, H, d/VEC]
+  s = SPLIT ? packed : i;
+  o = SPLIT ? i : packed;
+}
+template <int VEC, bool SPLIT, typename Index>
 __global__ void __launch_bounds__(kThreads)
-heads_permute_kernel(const float* __restrict__ src, float* __restrict__ dst, int B, int L, int M, int H, int d) {
-  const int dv = d / VEC;
-  const int64_t total = (int64_t)B * L * M * H * dv;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    // i enumerates the [B, H, L, M, d/VEC] side
-    int64_t t = i;
-    const int f = (int)(t % dv); t /= dv;
-    const int m = (int)(t % M); t /= M;
-    const int l = (int)(t % L); t /= L;
-    const int h = (int)(t % H); t /= H;
-    const int b = (int)t;
-    const int64_t packed = ((((int64_t)b * L + l) * M + m) * H + h) * dv + f;  // [B, L, M, H, d/VEC]
-    const int64_t s = SPLIT ? packed : i, o = SPLIT ? i : packed;
-    if (VEC == 4) reinterpret_cast<float4*>(dst)[o] = reinterpret_cast<const float4*>(src)[s];
-    else dst[o] = src[s];
+heads_permute_kernel(Lines src_w, OutLines dst_w, Lines src_b, OutLines dst_b, Index n_w, Index n_b, int L, int M, int H, int d) {
+  const bool up = blockIdx.y != 0;
+  const float* const sw = up ? src_w.u : src_w.l;
+  const float* const sb = up ? src_b.u : src_b.l;
+  float* const ow = up ? dst_w.u : dst_w.l;
+  float* const ob = up ? dst_b.u : dst_b.l;
+  const Index dv = (Index)(d / VEC), stride = (Index)gridDim.x * blockDim.x;
+  for (Index i = (Index)blockIdx.x * blockDim.x + threadIdx.x; i < n_w + n_b; i += stride) {
+    Index s, o;
+    if (i >= n_w) {
+      permute_item<Index, SPLIT>(i - n_w, (Index)1, (Index)L, (Index)H, (Index)d, s, o);
+      ob[o] = sb[s];
+    } else {
+      permute_item<Index, SPLIT>(i, (Index)M, (Index)L, (Index)H, dv, s, o);
+      if (VEC == 4) reinterpret_cast<float4*>(ow)[o] = reinterpret_cast<const float4*>(sw)[s];
+      else ow[o] = sw[s];
+    }
   }
 }
 
@@ -268,17 +301,42 @@ heads_split_transpose_kernel(const float* __restrict__ src, float* __restrict__ 
 }
 
 // z_l = x_l * w+ + x_u * w-,  z_u = x_l * w- + x_u * w+ with w a vector over the feature axis (Bounds.py:653-664);
-// n elements of rows of length Do.
+// rows of length Do.
+__device__ __forceinline__ void mul_feature(float wv, float a, float b, float& zl, float& zu) {
+  const float wp = wv > 0.f ? wv : 0.f;
+  const float wn = fsub(wv, wp);
+  zl = fadd(fmul(a, wp), fmul(b, wn));
+  zu = fadd(fmul(a, wn), fmul(b, wp));
+}
+template <int VEC>
 __global__ void __launch_bounds__(kThreads)
-mul_features_kernel(const float* xl, const float* xu, const float* __restrict__ w, float* zl, float* zu, int64_t n, int Do) {
+mul_features_kernel(Lines xw, OutLines zw, Lines xb, OutLines zb, const float* __restrict__ w, int64_t nv, int64_t nb, int Do) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const float wv = w[i % Do];
-    const float wp = wv > 0.f ? wv : 0.f;
-    const float wn = fsub(wv, wp);
-    const float a = xl[i], b = xu[i];   // both read before either is written: z may alias x
-    zl[i] = fadd(fmul(a, wp), fmul(b, wn));
-    zu[i] = fadd(fmul(a, wn), fmul(b, wp));
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv + nb; i += stride) {
+    // (every element is read before it is written: z may alias x)
+    if (i >= nv) {
+      const int64_t k = i - nv;
+      float zl, zu;
+      mul_feature(w[k % Do], xb.l[k], xb.u[k], zl, zu);
+      zb.l[k] = zl;
+      zb.u[k] = zu;
+    } else if (VEC == 4) {
+      const int j = nv <= 0x7fffffff ? (int)((uint32_t)i % (uint32_t)(Do / 4)) : (int)(i % (Do / 4));
+      const float4 a = reinterpret_cast<const float4*>(xw.l)[i], b = reinterpret_cast<const float4*>(xw.u)[i];
+      const float* wq = w + 4 * j;
+      float4 l, u;
+      mul_feature(__ldg(wq), a.x, b.x, l.x, u.x);
+      mul_feature(__ldg(wq + 1), a.y, b.y, l.y, u.y);
+      mul_feature(__ldg(wq + 2), a.z, b.z, l.z, u.z);
+      mul_feature(__ldg(wq + 3), a.w, b.w, l.w, u.w);
+      reinterpret_cast<float4*>(zw.l)[i] = l;
+      reinterpret_cast<float4*>(zw.u)[i] = u;
+    } else {
+      float zl, zu;
+      mul_feature(w[i % Do], xw.l[i], xw.u[i], zl, zu);
+      zw.l[i] = zl;
+      zw.u[i] = zu;
+    }
   }
 }
 
@@ -347,10 +405,11 @@ extern "C" int fb_add_f32(const float* x_lw, const float* x_uw, const float* x_l
   ProfileScope prof(PK_ELEMENTWISE, 2.0 * (nw + nb), 4.0 * 6 * (nw + nb), stream);
   const bool vw = nw % 4 == 0 && aligned16(x_lw) && aligned16(x_uw) && aligned16(y_lw) && aligned16(y_uw) &&
                   aligned16(z_lw) && aligned16(z_uw);
-  if (vw) add_kernel<4><<<stream_blocks(nw / 4), kThreads, 0, st>>>(x_lw, y_lw, z_lw, x_uw, y_uw, z_uw, nw);
-  else add_kernel<1><<<stream_blocks(nw), kThreads, 0, st>>>(x_lw, y_lw, z_lw, x_uw, y_uw, z_uw, nw);
-  add_kernel<1><<<stream_blocks(nb), kThreads, 0, st>>>(x_lb, y_lb, z_lb, x_ub, y_ub, z_ub, nb);
-  FB_LAUNCH_OK_N(2);
+  const Lines xw = {x_lw, x_uw}, yw = {y_lw, y_uw}, xb = {x_lb, x_ub}, yb = {y_lb, y_ub};
+  const OutLines zw = {z_lw, z_uw}, zb = {z_lb, z_ub};
+  if (vw) add_kernel<4><<<stream_blocks(nw / 4 + nb), kThreads, 0, st>>>(xw, yw, zw, xb, yb, zb, nw / 4, nb);
+  else add_kernel<1><<<stream_blocks(nw + nb), kThreads, 0, st>>>(xw, yw, zw, xb, yb, zb, nw, nb);
+  FB_LAUNCH_OK();
   return FB_OK;
 }
 
@@ -371,10 +430,11 @@ extern "C" int fb_scale_f32(const float* x_lw, const float* x_uw, const float* x
   const float* s_lb = c > 0.f ? x_lb : x_ub;
   const float* s_ub = c > 0.f ? x_ub : x_lb;
   const bool vw = nw % 4 == 0 && aligned16(x_lw) && aligned16(x_uw) && aligned16(z_lw) && aligned16(z_uw);
-  if (vw) scale_kernel<4><<<stream_blocks(nw / 4), kThreads, 0, st>>>(s_lw, z_lw, s_uw, z_uw, c, nw);
-  else scale_kernel<1><<<stream_blocks(nw), kThreads, 0, st>>>(s_lw, z_lw, s_uw, z_uw, c, nw);
-  scale_kernel<1><<<stream_blocks(nb), kThreads, 0, st>>>(s_lb, z_lb, s_ub, z_ub, c, nb);
-  FB_LAUNCH_OK_N(2);
+  const Lines xw = {s_lw, s_uw}, xb = {s_lb, s_ub};
+  const OutLines zw = {z_lw, z_uw}, zb = {z_lb, z_ub};
+  if (vw) scale_kernel<4><<<stream_blocks(nw / 4 + nb), kThreads, 0, st>>>(xw, zw, xb, zb, c, nw / 4, nb);
+  else scale_kernel<1><<<stream_blocks(nw + nb), kThreads, 0, st>>>(xw, zw, xb, zb, c, nw, nb);
+  FB_LAUNCH_OK();
   return FB_OK;
 }
 
@@ -435,6 +495,34 @@ extern "C" int fb_layernorm_novar_f32(const float* x_lw, const float* x_uw, cons
                                     Do, nullptr, stream);
 }
 
+namespace {
+// One line (z.u == nullptr) or both lines of a bound.
+template <bool SPLIT>
+int permute_heads(Lines xw, Lines xb, OutLines zw, OutLines zb, int B, int L, int Di, int H, int d, cudaStream_t st) {
+  const int lines = zw.u != nullptr ? 2 : 1;
+  const bool vec = d % 4 == 0 && aligned16(xw.l) && aligned16(zw.l) && (lines == 1 || (aligned16(xw.u) && aligned16(zw.u)));
+  const int64_t nw = (int64_t)B * L * Di * H * d / (vec ? 4 : 1), nb = (int64_t)B * L * H * d;
+  const dim3 grid(stream_blocks(nw + nb), (unsigned)lines);
+  const bool small = nw + nb + (int64_t)grid.x * kThreads < (1ll << 32);
+#define FB_PERMUTE(V, I) heads_permute_kernel<V, SPLIT, I><<<grid, kThreads, 0, st>>>(xw, zw, xb, zb, (I)nw, (I)nb, L, Di, H, d)
+  if (vec && small) FB_PERMUTE(4, uint32_t);
+  else if (vec) FB_PERMUTE(4, uint64_t);
+  else if (small) FB_PERMUTE(1, uint32_t);
+  else FB_PERMUTE(1, uint64_t);
+#undef FB_PERMUTE
+  FB_LAUNCH_OK();
+  return FB_OK;
+}
+int split_transpose(const float* x_w, const float* x_b, float* z_w, float* z_b, int B, int L, int Di, int H, int d, cudaStream_t st) {
+  const int64_t bw = (int64_t)B * H * Di, bb = (int64_t)B * H;
+  FB_REQUIRE(bw <= 0x7fffffff, FB_ERR_SHAPE);
+  heads_split_transpose_kernel<<<(unsigned)bw, kThreads, 0, st>>>(x_w, z_w, B, L, Di, H, d);
+  heads_split_transpose_kernel<<<(unsigned)bb, kThreads, 0, st>>>(x_b, z_b, B, L, 1, H, d);
+  FB_LAUNCH_OK_N(2);
+  return FB_OK;
+}
+}  // namespace
+
 extern "C" int fb_split_heads_f32(const float* x_w, const float* x_b, float* z_w, float* z_b,
                                   int B, int L, int Di, int H, int d, int transpose_ld, void* stream) {
   FB_REQUIRE(x_w && x_b && z_w && z_b, FB_ERR_ARG);
@@ -442,20 +530,8 @@ extern "C" int fb_split_heads_f32(const float* x_w, const float* x_b, float* z_w
   if (B == 0) return FB_OK;
   cudaStream_t st = (cudaStream_t)stream;
   ProfileScope prof(PK_ELEMENTWISE, 0.0, 4.0 * 2 * ((double)B * L * (Di + 1) * H * d), stream);
-  if (transpose_ld) {
-    const int64_t bw = (int64_t)B * H * Di, bb = (int64_t)B * H;
-    FB_REQUIRE(bw <= 0x7fffffff, FB_ERR_SHAPE);
-    heads_split_transpose_kernel<<<(unsigned)bw, kThreads, 0, st>>>(x_w, z_w, B, L, Di, H, d);
-    heads_split_transpose_kernel<<<(unsigned)bb, kThreads, 0, st>>>(x_b, z_b, B, L, 1, H, d);
-  } else {
-    const bool vec = d % 4 == 0 && aligned16(x_w) && aligned16(z_w);
-    const int64_t nw = (int64_t)B * L * Di * H * d, nb = (int64_t)B * L * H * d;
-    if (vec) heads_permute_kernel<4, true><<<stream_blocks(nw / 4), kThreads, 0, st>>>(x_w, z_w, B, L, Di, H, d);
-    else heads_permute_kernel<1, true><<<stream_blocks(nw), kThreads, 0, st>>>(x_w, z_w, B, L, Di, H, d);
-    heads_permute_kernel<1, true><<<stream_blocks(nb), kThreads, 0, st>>>(x_b, z_b, B, L, 1, H, d);
-  }
-  FB_LAUNCH_OK_N(2);
-  return FB_OK;
+  if (transpose_ld) return split_transpose(x_w, x_b, z_w, z_b, B, L, Di, H, d, st);
+  return permute_heads<true>({x_w, nullptr}, {x_b, nullptr}, {z_w, nullptr}, {z_b, nullptr}, B, L, Di, H, d, st);
 }
 
 extern "C" int fb_merge_heads_f32(const float* x_w, const float* x_b, float* z_w, float* z_b,
@@ -463,15 +539,32 @@ extern "C" int fb_merge_heads_f32(const float* x_w, const float* x_b, float* z_w
   FB_REQUIRE(x_w && x_b && z_w && z_b, FB_ERR_ARG);
   FB_REQUIRE(B >= 0 && L > 0 && Di > 0 && H > 0 && d > 0, FB_ERR_ARG);
   if (B == 0) return FB_OK;
-  cudaStream_t st = (cudaStream_t)stream;
   ProfileScope prof(PK_ELEMENTWISE, 0.0, 4.0 * 2 * ((double)B * L * (Di + 1) * H * d), stream);
-  const bool vec = d % 4 == 0 && aligned16(x_w) && aligned16(z_w);
-  const int64_t nw = (int64_t)B * L * Di * H * d, nb = (int64_t)B * L * H * d;
-  if (vec) heads_permute_kernel<4, false><<<stream_blocks(nw / 4), kThreads, 0, st>>>(x_w, z_w, B, L, Di, H, d);
-  else heads_permute_kernel<1, false><<<stream_blocks(nw), kThreads, 0, st>>>(x_w, z_w, B, L, Di, H, d);
-  heads_permute_kernel<1, false><<<stream_blocks(nb), kThreads, 0, st>>>(x_b, z_b, B, L, 1, H, d);
-  FB_LAUNCH_OK_N(2);
-  return FB_OK;
+  return permute_heads<false>({x_w, nullptr}, {x_b, nullptr}, {z_w, nullptr}, {z_b, nullptr}, B, L, Di, H, d, (cudaStream_t)stream);
+}
+
+extern "C" int fb_split_heads_bound_f32(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub, float* z_lw,
+                                        float* z_uw, float* z_lb, float* z_ub, int B, int L, int Di, int H, int d, int transpose_ld,
+                                        void* stream) {
+  FB_REQUIRE(x_lw && x_uw && x_lb && x_ub && z_lw && z_uw && z_lb && z_ub, FB_ERR_ARG);
+  FB_REQUIRE(B >= 0 && L > 0 && Di > 0 && H > 0 && d > 0, FB_ERR_ARG);
+  if (B == 0) return FB_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  ProfileScope prof(PK_ELEMENTWISE, 0.0, 4.0 * 4 * ((double)B * L * (Di + 1) * H * d), stream);
+  if (transpose_ld) {
+    const int rc = split_transpose(x_lw, x_lb, z_lw, z_lb, B, L, Di, H, d, st);
+    return rc != FB_OK ? rc : split_transpose(x_uw, x_ub, z_uw, z_ub, B, L, Di, H, d, st);
+  }
+  return permute_heads<true>({x_lw, x_uw}, {x_lb, x_ub}, {z_lw, z_uw}, {z_lb, z_ub}, B, L, Di, H, d, st);
+}
+
+extern "C" int fb_merge_heads_bound_f32(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub, float* z_lw,
+                                        float* z_uw, float* z_lb, float* z_ub, int B, int L, int Di, int H, int d, void* stream) {
+  FB_REQUIRE(x_lw && x_uw && x_lb && x_ub && z_lw && z_uw && z_lb && z_ub, FB_ERR_ARG);
+  FB_REQUIRE(B >= 0 && L > 0 && Di > 0 && H > 0 && d > 0, FB_ERR_ARG);
+  if (B == 0) return FB_OK;
+  ProfileScope prof(PK_ELEMENTWISE, 0.0, 4.0 * 4 * ((double)B * L * (Di + 1) * H * d), stream);
+  return permute_heads<false>({x_lw, x_uw}, {x_lb, x_ub}, {z_lw, z_uw}, {z_lb, z_ub}, B, L, Di, H, d, (cudaStream_t)stream);
 }
 
 extern "C" int fb_mul_features_f32(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub,
@@ -483,9 +576,12 @@ extern "C" int fb_mul_features_f32(const float* x_lw, const float* x_uw, const f
   if (nb == 0) return FB_OK;
   ProfileScope prof(PK_ELEMENTWISE, 4.0 * (nw + nb), 4.0 * 4 * (nw + nb), stream);
   cudaStream_t st = (cudaStream_t)stream;
-  mul_features_kernel<<<stream_blocks(nw), kThreads, 0, st>>>(x_lw, x_uw, w, z_lw, z_uw, nw, Do);
-  mul_features_kernel<<<stream_blocks(nb), kThreads, 0, st>>>(x_lb, x_ub, w, z_lb, z_ub, nb, Do);
-  FB_LAUNCH_OK_N(2);
+  const Lines xw = {x_lw, x_uw}, xb = {x_lb, x_ub};
+  const OutLines zw = {z_lw, z_uw}, zb = {z_lb, z_ub};
+  const bool vw = Do % 4 == 0 && aligned16(x_lw) && aligned16(x_uw) && aligned16(z_lw) && aligned16(z_uw);
+  if (vw) mul_features_kernel<4><<<stream_blocks(nw / 4 + nb), kThreads, 0, st>>>(xw, zw, xb, zb, w, nw / 4, nb, Do);
+  else mul_features_kernel<1><<<stream_blocks(nw + nb), kThreads, 0, st>>>(xw, zw, xb, zb, w, nw, nb, Do);
+  FB_LAUNCH_OK();
   return FB_OK;
 }
 

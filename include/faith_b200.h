@@ -357,6 +357,14 @@ int fb_layernorm_novar_f32(const float* x_lw, const float* x_uw, const float* x_
                            float* z_lw, float* z_uw, float* z_lb, float* z_ub,
                            int64_t rows, int Di, int Do, void* stream);
 
+/* Layer normalisation with the variance ("standard", Bounds.py:1111-1131) in one kernel: centre, square, mean + 1e-12, root,
+ * reciprocal, McCormick product, gain and shift.  `violation` as in fb_relax_f32(FB_SQRT / FB_RECIPROCAL).  z must not alias x.
+ * FB_ERR_SHAPE when Di or Do is too large for the per-row vectors in shared memory (thousands). */
+int fb_layernorm_standard_f32(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub,
+                              const float* gamma, const float* beta,
+                              float* z_lw, float* z_uw, float* z_lb, float* z_ub,
+                              int64_t rows, int Di, int Do, int words, int p, float eps, int* violation, void* stream);
+
 /* Head split [B, L, Di, H*d] -> [B*H, L, Di, d] (VerifierForward.py:208-229) and its inverse
  * (VerifierForward.py:253-265).  With transpose_ld != 0 the split additionally swaps the
  * position and feature axes, giving [B*H, d, Di, L]: the operand `value.t()` of the attention
@@ -365,6 +373,13 @@ int fb_split_heads_f32(const float* x_w, const float* x_b, float* z_w, float* z_
                        int B, int L, int Di, int H, int d, int transpose_ld, void* stream);
 int fb_merge_heads_f32(const float* x_w, const float* x_b, float* z_w, float* z_b,
                        int B, int L, int Di, int H, int d, void* stream);
+/* The same for both lines of a bound in one launch. */
+int fb_split_heads_bound_f32(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub,
+                             float* z_lw, float* z_uw, float* z_lb, float* z_ub,
+                             int B, int L, int Di, int H, int d, int transpose_ld, void* stream);
+int fb_merge_heads_bound_f32(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub,
+                             float* z_lw, float* z_uw, float* z_lb, float* z_ub,
+                             int B, int L, int Di, int H, int d, void* stream);
 
 /* Bound of a 2-D convolution with constant weights (split by sign like fb_matmul_f32); dim_in
  * is the batch axis of the convolution.  Replaces the commented-out

@@ -995,6 +995,22 @@ def test_layer_norm_applied_by_the_epilogue_of_the_product(with_slopes, Do):
                                rs, gamma[:64].contiguous(), beta[:64].contiguous(), *extra)
 
 
+@pytest.mark.parametrize("L,Di,Do,p,words", [(3, 8, 3, 2.0, 1), (2, 24, 33, float("inf"), 2), (2, 128, 128, 1.0, 1),
+                                             (1, 256, 128, 2.0, 2), (2, 10, 600, float("inf"), 1)])
+def test_standard_layer_norm_in_one_kernel(L, Di, Do, p, words):
+    """fb_layernorm_standard_f32 (tile in shared memory or re-read, few columns to more columns than threads) against the
+    operator chain of the oracle, fp64 as arbiter."""
+    import faith_b200
+    t = cases.rand_bounds(1201, 2, L, Di, Do, -0.5, 0.02, 0.02)
+    g = torch.Generator().manual_seed(1202)
+    norm = types.SimpleNamespace(weight=torch.rand(Do, generator=g) * 2 - 0.5, bias=torch.rand(Do, generator=g) - 0.5)
+    x = faith_b200.BoundsLite(p, 0.05, *[v.to(DEV) for v in t], perturbed_words=words)
+    dev = types.SimpleNamespace(weight=norm.weight.to(DEV), bias=norm.bias.to(DEV))
+    o = O.OBounds(p, 0.05, *t, words=words).layer_norm(norm.weight, norm.bias, "standard")
+    o64 = O.OBounds(p, 0.05, *[v.double() for v in t], words=words).layer_norm(norm.weight.double(), norm.bias.double(), "standard")
+    helpers.assert_bounds_arbitrated(x.layer_norm(dev, "standard"), o, o64, "standard layer norm %d x %d" % (Di, Do))
+
+
 @pytest.mark.parametrize("B,L,Do,Dy", [(1, 1, 128, 17), (1, 8, 516, 33), (1, 9, 1030, 128), (5, 51, 37, 96), (1, 255, 128, 512)])
 def test_product_of_few_rows(B, L, Do, Dy):
     """The kernel for a few output tiles (8 rows x 32 columns per block, K split over the warps): remainders of rows, columns
