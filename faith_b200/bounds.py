@@ -54,6 +54,20 @@ class Bounds:
     def _new(self, lw, uw, lb, ub):
         return Bounds(self.args, self.p, self.eps, lw=lw, lb=lb, uw=uw, ub=ub)
 
+    def _same(self, t):
+        """The bound with the tensors lw, uw, lb, ub of `t` and everything else as here (what _new gives for a result of an
+        operator in linear mode, without evaluating the arguments again: an operator of one sentence is bound by the host)."""
+        if self.ibp:
+            return self._new(t[0], t[1], t[2], t[3])
+        b = object.__new__(Bounds)
+        d = b.__dict__
+        d["args"], d["ibp"], d["p"], d["q"], d["eps"] = self.args, False, self.p, self.q, self.eps
+        d["perturbed_words"], d["device"], d["FLAG"] = self.perturbed_words, self.device, self.FLAG
+        lw = t[0]
+        d["lw"], d["uw"], d["lb"], d["ub"] = lw, t[1], t[2], t[3]
+        d["batch_size"], d["length"], d["dim_in"], d["dim_out"] = lw.shape
+        return b
+
     def _t4(self):
         return _c(self.lw), _c(self.uw), _c(self.lb), _c(self.ub)
 
@@ -71,15 +85,13 @@ class Bounds:
 
     def add(self, delta):
         if isinstance(delta, Bounds):
-            lw, uw, lb, ub = ops.add(self._t4(), delta._t4())
-            return self._new(lw, uw, lb, ub)
+            return self._same(ops.add(self._t4(), delta._t4()))
         # a constant only moves the bias terms; memory-only op
         return self._new(self.lw, self.uw, self.lb + delta, self.ub + delta)
 
     def multiply(self, W):
         if isinstance(W, float):
-            lw, uw, lb, ub = ops.scale(self._t4(), W)
-            return self._new(lw, uw, lb, ub)
+            return self._same(ops.scale(self._t4(), W))
         if isinstance(W, Bounds):
             assert self.lw.shape == W.lw.shape
             if self.ibp:
@@ -89,23 +101,19 @@ class Bounds:
                 lb, ub = ops.interval_mul(l_a, u_a, l_b, u_b)
                 zero = torch.zeros_like(self.lw)
                 return self._new(zero, zero.clone(), lb, ub)
-            lw, uw, lb, ub = ops.mul_bounds(self._t4(), W._t4(), self.p, self.eps, self.perturbed_words)
-            return self._new(lw, uw, lb, ub)
+            return self._same(ops.mul_bounds(self._t4(), W._t4(), self.p, self.eps, self.perturbed_words))
         # constant vector over the feature axis (the gain of a layer norm), split by sign (Bounds.py:653-664)
-        lw, uw, lb, ub = ops.mul_features(self._t4(), _c(W.detach().reshape(-1)))
-        return self._new(lw, uw, lb, ub)
+        return self._same(ops.mul_features(self._t4(), _c(W.detach().reshape(-1))))
 
     def matmul(self, W, *unused, **unused_kw):
         if isinstance(W, Bounds) or W.dim() != 2:
             raise NotImplementedError
         lw, uw, lb, ub = self._t4()
-        y = ops.matmul(lw, uw, lb, ub, _c(W.detach()), None)
-        return self._new(y[0], y[1], y[2], y[3])
+        return self._same(ops.matmul(lw, uw, lb, ub, _c(W), None))
 
     def dense(self, dense, *unused, **unused_kw):
         lw, uw, lb, ub = self._t4()
-        y = ops.matmul(lw, uw, lb, ub, _c(dense.weight.detach()), _c(dense.bias.detach()))
-        return self._new(y[0], y[1], y[2], y[3])
+        return self._same(ops.matmul(lw, uw, lb, ub, _c(dense.weight), _c(dense.bias)))
 
     def dot_product(self, other, debug=False, verbose=False, lower=True, upper=True):
         if self.dim_in == 1 or self.ibp:
@@ -114,22 +122,26 @@ class Bounds:
             lb, ub = ops.interval_dot(_c(self.lb), _c(self.ub), _c(other.lb), _c(other.ub))
             w = torch.zeros(lb.shape[0], lb.shape[1], self.dim_in, lb.shape[2], device=lb.device)
             return self._new(w, w.clone(), lb, ub)
-        z = ops.dot_product(self._t4(), other._t4(), self.p, self.eps, self.perturbed_words)
-        return self._new(z[0], z[1], z[2], z[3])
+        return self._same(ops.dot_product(self._t4(), other._t4(), self.p, self.eps, self.perturbed_words))
 
     def context(self, value):
+        if self.dim_in != 1 and not self.ibp:
+            # the product that reads the values as they are, where the shape is one of its: no transposed copies
+            z = ops.context_kmajor_or_none(self._t4(), value._t4(), self.p, self.eps, self.perturbed_words)
+            if z is not None:
+                return self._same(z)
         return self.dot_product(value.t())
 
     def _relax(self, op):
         lw, uw, lb, ub = self._t4()
-        violation = None
+        code = op + (FB_INTERVAL if self.ibp else 0)
         if op in (FB_RECIPROCAL, FB_SQRT):
-            violation = torch.zeros(1, dtype=torch.int32, device=lw.device)
-        o = ops.relax(op + (FB_INTERVAL if self.ibp else 0), lw, uw, lb, ub, self.p, self.eps, self.perturbed_words,
-                      violation=violation)
-        if violation is not None and int(violation.item()) != 0:
-            raise AssertionError("reciprocal or square root of a bound that is not strictly positive")
-        return self._new(o[0], o[1], o[2], o[3])
+            o = ops.relax_checked(code, lw, uw, lb, ub, self.p, self.eps, self.perturbed_words)
+            if o[4] != 0:
+                raise AssertionError("reciprocal or square root of a bound that is not strictly positive")
+        else:
+            o = ops.relax(code, lw, uw, lb, ub, self.p, self.eps, self.perturbed_words)
+        return self._same(o)
 
     def sqr(self):
         return self._relax(FB_SQR)
@@ -160,24 +172,28 @@ class Bounds:
         raise NotImplementedError
 
     def softmax(self, verbose=False):
-        violation = torch.zeros(1, dtype=torch.int32, device=self.lw.device)
-        fused = None if self.ibp else ops.softmax_fused(self._t4(), self.p, self.eps, self.perturbed_words, violation)
+        fused = None if self.ibp else ops.softmax_checked(self._t4(), self.p, self.eps, self.perturbed_words)
         if fused is not None:
-            if int(violation.item()) != 0:
+            if fused[4] != 0:
                 raise AssertionError("reciprocal of a bound that is not strictly positive")
-            return self._new(fused[0], fused[1], fused[2], fused[3])
+            return self._same(fused)
         e = self.exp()
-        s = ops.rowsum(e._t4())
-        return e.divide(self._new(s[0], s[1], s[2], s[3]))
+        return e.divide(self._same(ops.rowsum(e._t4())))
 
     def layer_norm(self, normalizer, layer_norm):
         if layer_norm == "no":
             return self
         if layer_norm == "no_var":
-            o = ops.layernorm_novar(self._t4(), _c(normalizer.weight.detach()), _c(normalizer.bias.detach()))
-            return self._new(o[0], o[1], o[2], o[3])
+            return self._same(ops.layernorm_novar(self._t4(), _c(normalizer.weight), _c(normalizer.bias)))
         if layer_norm != "standard":
             raise NotImplementedError("layer_norm mode %r" % (layer_norm,))
+        if not self.ibp:
+            o = ops.layernorm_standard_checked(self._t4(), _c(normalizer.weight), _c(normalizer.bias), self.p, self.eps,
+                                               self.perturbed_words)
+            if o is not None:
+                if o[4] != 0:
+                    raise AssertionError("reciprocal or square root of a bound that is not strictly positive")
+                return self._same(o)
         # Bounds.py:1111-1131: x - mean, variance = mean of the squares, division by its root, gain and shift; the mean
         # subtraction is the no_var kernel with unit gain, the rest is the reference's own chain of operators
         ones = torch.ones(self.dim_out, device=self.device)

@@ -1,4 +1,5 @@
-"""Builds faith_b200/libfaith_b200.so from csrc/ with nvcc for sm_100a (cross-compiles without a GPU).
+"""Builds faith_b200/libfaith_b200.so from csrc/ with nvcc for sm_100a (cross-compiles without a GPU), and the Python
+boundary faith_b200/_binding.so from csrc/binding/ with the host compiler.
 
     python -m faith_b200.build            # incremental
     python -m faith_b200.build --force    # rebuild everything
@@ -7,19 +8,22 @@ import concurrent.futures
 import os
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(CSRC, "build")
 INCLUDE = os.path.join(os.path.dirname(PKG), "include")
 LIB = os.path.join(PKG, "libfaith_b200.so")
+BINDING_SRC = os.path.join(CSRC, "binding", "binding.cpp")
+BINDING = os.path.join(PKG, "_binding.so")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-I" + INCLUDE, "-I" + CSRC]
 
 
 def _nvcc():
-    cand = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "bin", "nvcc")
+    cand = os.path.join(_cuda_home(), "bin", "nvcc")
     return cand if os.path.exists(cand) else "nvcc"
 
 
@@ -31,6 +35,32 @@ def _newest_header():
     hs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
     hs += [os.path.join(INCLUDE, f) for f in os.listdir(INCLUDE)]
     return max(os.path.getmtime(h) for h in hs)
+
+
+def _cuda_home():
+    return os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+def _build_binding(force, verbose):
+    """The extension module that faith_b200/ops.py calls: host code only, linked against the C-ABI library next to it."""
+    newest = max(os.path.getmtime(BINDING_SRC), max(os.path.getmtime(os.path.join(INCLUDE, f)) for f in os.listdir(INCLUDE)))
+    if not force and os.path.exists(BINDING) and os.path.getmtime(BINDING) >= newest:
+        return
+    import torch
+    troot = os.path.dirname(torch.__file__)
+    tlib = os.path.join(troot, "lib")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
+           "-I" + INCLUDE, "-I" + os.path.join(troot, "include"),
+           "-I" + os.path.join(troot, "include", "torch", "csrc", "api", "include"),
+           "-I" + os.path.join(_cuda_home(), "include"), "-I" + sysconfig.get_paths()["include"],
+           BINDING_SRC, "-o", BINDING, "-L" + PKG, "-lfaith_b200", "-L" + tlib, "-ltorch_python", "-ltorch_cpu", "-lc10",
+           "-lc10_cuda", "-ltorch_cuda", "-L" + os.path.join(_cuda_home(), "lib64"), "-lcudart", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+    if r.returncode != 0:
+        raise RuntimeError("building %s failed" % BINDING)
 
 
 def build(force=False, verbose=False):
@@ -62,6 +92,7 @@ def build(force=False, verbose=False):
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError("link failed:\n" + r.stdout + r.stderr)
+    _build_binding(force, verbose)
     return LIB
 
 

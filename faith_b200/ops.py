@@ -1,7 +1,9 @@
 """Thin tensor-level wrappers over the C ABI: argument checks, output allocation, stream.
 
 PyTorch is used only for device memory and the current stream; all arithmetic happens in
-libfaith_b200.so.  Every tensor must be a contiguous float32 CUDA tensor.
+libfaith_b200.so.  Every tensor must be a contiguous float32 CUDA tensor.  The operators of the `Bounds` class go through
+the native boundary (csrc/binding/binding.cpp): their small calls are bound by the host, and the same steps over ctypes cost 25
+to 40 us per operator; the remaining entry points, which the C++ driver calls itself, are bound here with ctypes.
 """
 import math
 
@@ -41,6 +43,9 @@ def _chk(*tensors):
     return dev
 
 
+_native = _lib.binding
+
+
 def _stream():
     return torch.cuda.current_stream().cuda_stream
 
@@ -50,50 +55,20 @@ def _p(t):
 
 
 def concretize(lw, uw, lb, ub, p, eps, words=1, layout=FB_NATIVE):
-    dev = _chk(lw, uw, lb, ub)
-    rows = lb.numel() // lb.shape[-1]
-    Do = lb.shape[-1]
-    Di = lw.shape[-2] if layout == FB_NATIVE else lw.shape[-1]
-    l, u = torch.empty_like(lb), torch.empty_like(ub)
-    with torch.cuda.device(dev):
-        check(load().fb_concretize_f32(_p(lw), _p(uw), _p(lb), _p(ub), _p(l), _p(u), rows, Di, Do, words,
-                                       norm_code(p), eps, layout, _stream()), "fb_concretize_f32")
-    return l, u
+    return _native().concretize(lw, uw, lb, ub, p, eps, words, layout)
 
 
 def relax(op, lw, uw, lb, ub, p, eps, words=1, layout=FB_NATIVE, out=None, violation=None):
-    dev = _chk(lw, uw, lb, ub)
-    rows = lb.numel() // lb.shape[-1]
-    Do = lb.shape[-1]
-    Di = lw.shape[-2] if layout == FB_NATIVE else lw.shape[-1]
-    if out is None:
-        out = (torch.empty_like(lw), torch.empty_like(uw), torch.empty_like(lb), torch.empty_like(ub))
-    o_lw, o_uw, o_lb, o_ub = out
-    _chk(o_lw, o_uw, o_lb, o_ub)
-    if violation is not None and (violation.dtype != torch.int32 or not violation.is_cuda):
-        raise _lib.FaithError("violation flag must be an int32 CUDA tensor")
-    with torch.cuda.device(dev):
-        check(load().fb_relax_f32(op, _p(lw), _p(uw), _p(lb), _p(ub), _p(o_lw), _p(o_uw), _p(o_lb), _p(o_ub),
-                                  rows, Di, Do, words, norm_code(p), eps, layout, _p(violation), _stream()),
-              "fb_relax_f32")
-    return o_lw, o_uw, o_lb, o_ub
+    return _native().relax(op, lw, uw, lb, ub, p, eps, words, layout, out, violation)
+
+
+def relax_checked(op, lw, uw, lb, ub, p, eps, words=1):
+    """relax() that also reads the status word of the call back (waits for the stream): (lw, uw, lb, ub, word)."""
+    return _native().relax_checked(op, lw, uw, lb, ub, p, eps, words)
 
 
 def matmul(lw, uw, lb, ub, W, bias=None):
-    dev = _chk(lw, uw, lb, ub, W, bias)
-    rows = lb.numel() // lb.shape[-1]
-    Di, Do = lw.shape[-2], lw.shape[-1]
-    Dy = W.shape[0]
-    if W.shape[1] != Do:
-        raise _lib.FaithError("weight shape %s does not match feature size %d" % (tuple(W.shape), Do))
-    y_lw = torch.empty(lw.shape[:-1] + (Dy,), device=dev, dtype=torch.float32)
-    y_uw = torch.empty_like(y_lw)
-    y_lb = torch.empty(lb.shape[:-1] + (Dy,), device=dev, dtype=torch.float32)
-    y_ub = torch.empty_like(y_lb)
-    with torch.cuda.device(dev):
-        check(load().fb_matmul_f32(_p(lw), _p(uw), _p(lb), _p(ub), _p(W), _p(bias), _p(y_lw), _p(y_uw), _p(y_lb),
-                                   _p(y_ub), rows, Di, Do, Dy, _stream()), "fb_matmul_f32")
-    return y_lw, y_uw, y_lb, y_ub
+    return _native().matmul(lw, uw, lb, ub, W, bias)
 
 
 def relax_coef(op, lw, uw, lb, ub, p, eps, words=1, violation=None):
@@ -203,99 +178,39 @@ def matmul_heads_ranges(lw, uw, lb, ub, W, bias, heads, p, eps, words=1):
 
 def dot_product(x, y, p, eps, words=1, out_scale=1.0, layout=FB_NATIVE, scratch=None, out=None):
     """x, y: (lw, uw, lb, ub).  Returns (z_lw, z_uw, z_lb, z_ub)."""
-    x_lw, x_uw, x_lb, x_ub = x
-    y_lw, y_uw, y_lb, y_ub = y
-    dev = _chk(*x, *y)
-    B, Lx, K = x_lb.shape
-    Ly = y_lb.shape[1]
-    Di = x_lw.shape[2] if layout == FB_NATIVE else x_lw.shape[3]
-    if out is None:
-        zshape = (B, Lx, Di, Ly) if layout == FB_NATIVE else (B, Lx, Ly, Di)
-        out = (torch.empty(zshape, device=dev), torch.empty(zshape, device=dev),
-               torch.empty((B, Lx, Ly), device=dev), torch.empty((B, Lx, Ly), device=dev))
-    if scratch is None:
-        scratch = (torch.empty_like(x_lb), torch.empty_like(x_lb), torch.empty_like(y_lb), torch.empty_like(y_lb))
-    x_l, x_u, y_l, y_u = scratch
-    z_lw, z_uw, z_lb, z_ub = out
-    _chk(*out, *scratch)
-    with torch.cuda.device(dev):
-        check(load().fb_dot_product_f32(_p(x_lw), _p(x_uw), _p(x_lb), _p(x_ub), _p(y_lw), _p(y_uw), _p(y_lb), _p(y_ub),
-                                        _p(z_lw), _p(z_uw), _p(z_lb), _p(z_ub), _p(x_l), _p(x_u), _p(y_l), _p(y_u),
-                                        B, Lx, Ly, Di, K, words, norm_code(p), eps, out_scale, layout, _stream()),
-              "fb_dot_product_f32")
-    return out
+    return _native().dot_product(*x, *y, p, eps, words, out_scale, layout, scratch, out)
 
 
 def context_kmajor(x, v, p, eps, words=1, out_scale=1.0, merge_heads=1):
     """Context product with the values in the projection's own layout: x (lw, uw [B, Lx, Di, K], lb, ub
     [B, Lx, K]), v (lw, uw [B, K, Di, Ly], lb, ub [B, K, Ly]).  Returns z as fb_dot_product_heads_f32 does.
     Raises FaithError (FB_ERR_SHAPE) outside the tensor-core shapes."""
-    x_lw, x_uw, x_lb, x_ub = x
-    v_lw, v_uw, v_lb, v_ub = v
-    dev = _chk(*x, *v)
-    B, Lx, K = x_lb.shape
-    Ly = v_lb.shape[2]
-    Di = x_lw.shape[2]
-    S = B // merge_heads
-    zw = (S, Lx, Di, merge_heads * Ly) if merge_heads > 1 else (B, Lx, Di, Ly)
-    zb = (S, Lx, merge_heads * Ly) if merge_heads > 1 else (B, Lx, Ly)
-    out = (torch.empty(zw, device=dev), torch.empty(zw, device=dev), torch.empty(zb, device=dev), torch.empty(zb, device=dev))
-    scratch = (torch.empty_like(x_lb), torch.empty_like(x_lb), torch.empty((B, Ly, K), device=dev), torch.empty((B, Ly, K), device=dev))
-    with torch.cuda.device(dev):
-        check(load().fb_context_heads_f32(_p(x_lw), _p(x_uw), _p(x_lb), _p(x_ub), _p(v_lw), _p(v_uw), _p(v_lb), _p(v_ub),
-                                          *[_p(t) for t in out], *[_p(t) for t in scratch], B, Lx, Ly, Di, K, words,
-                                          norm_code(p), eps, out_scale, merge_heads, _stream()), "fb_context_heads_f32")
-    return out
+    z = _native().context_kmajor(*x, *v, p, eps, words, out_scale, merge_heads)
+    if z is None:
+        check(2, "fb_context_heads_f32")
+    return z
+
+
+def context_kmajor_or_none(x, v, p, eps, words=1):
+    """context_kmajor(), or None where the shape is not one it takes."""
+    return _native().context_kmajor(*x, *v, p, eps, words, 1.0, 1)
 
 
 def mul_bounds(x, y, p, eps, words=1):
-    dev = _chk(*x, *y)
-    x_lw, x_uw, x_lb, x_ub = x
-    rows = x_lb.numel() // x_lb.shape[-1]
-    Di, Do = x_lw.shape[-2], x_lw.shape[-1]
-    out = (torch.empty_like(x_lw), torch.empty_like(x_lw), torch.empty_like(x_lb), torch.empty_like(x_lb))
-    with torch.cuda.device(dev):
-        check(load().fb_mul_bounds_f32(*[_p(t) for t in x], *[_p(t) for t in y], *[_p(t) for t in out],
-                                       rows, Di, Do, words, norm_code(p), eps, _stream()), "fb_mul_bounds_f32")
-    return out
+    return _native().mul_bounds(*x, *y, p, eps, words)
 
 
 def add(x, y):
-    dev = _chk(*x, *y)
-    x_lw, x_uw, x_lb, x_ub = x
-    rows = x_lb.numel() // x_lb.shape[-1]
-    Di, Do = x_lw.shape[-2], x_lw.shape[-1]
-    out = (torch.empty_like(x_lw), torch.empty_like(x_lw), torch.empty_like(x_lb), torch.empty_like(x_lb))
-    with torch.cuda.device(dev):
-        check(load().fb_add_f32(*[_p(t) for t in x], *[_p(t) for t in y], *[_p(t) for t in out], rows, Di, Do,
-                                _stream()), "fb_add_f32")
-    return out
+    return _native().add(*x, *y)
 
 
 def scale(x, c):
-    dev = _chk(*x)
-    x_lw, x_uw, x_lb, x_ub = x
-    rows = x_lb.numel() // x_lb.shape[-1]
-    Di, Do = x_lw.shape[-2], x_lw.shape[-1]
-    out = (torch.empty_like(x_lw), torch.empty_like(x_lw), torch.empty_like(x_lb), torch.empty_like(x_lb))
-    with torch.cuda.device(dev):
-        check(load().fb_scale_f32(*[_p(t) for t in x], *[_p(t) for t in out], rows, Di, Do, float(c), _stream()),
-              "fb_scale_f32")
-    return out
+    return _native().scale(*x, c)
 
 
 def mul_features(x, w):
     """x * w with w a vector over the feature axis, split by sign (Bounds.py:653-664)."""
-    dev = _chk(*x, w)
-    lw, uw, lb, ub = x
-    rows, Di, Do = lb.numel() // lb.shape[-1], lw.shape[-2], lw.shape[-1]
-    if w.numel() != Do:
-        raise _lib.FaithError("feature vector of %d elements against %d features" % (w.numel(), Do))
-    z = tuple(torch.empty_like(t) for t in x)
-    with torch.cuda.device(dev):
-        check(load().fb_mul_features_f32(_p(lw), _p(uw), _p(lb), _p(ub), _p(w), _p(z[0]), _p(z[1]), _p(z[2]), _p(z[3]),
-                                         rows, Di, Do, _stream()), "fb_mul_features_f32")
-    return z
+    return _native().mul_features(*x, w)
 
 
 def interval_mul(xl, xu, yl, yu):
@@ -324,78 +239,32 @@ def interval_dot(xl, xu, yl, yu):
 
 
 def rowsum(x):
-    dev = _chk(*x)
-    x_lw, x_uw, x_lb, x_ub = x
-    rows = x_lb.numel() // x_lb.shape[-1]
-    Di, Do = x_lw.shape[-2], x_lw.shape[-1]
-    out = (torch.empty_like(x_lw), torch.empty_like(x_lw), torch.empty_like(x_lb), torch.empty_like(x_lb))
-    with torch.cuda.device(dev):
-        check(load().fb_rowsum_f32(*[_p(t) for t in x], *[_p(t) for t in out], rows, Di, Do, _stream()),
-              "fb_rowsum_f32")
-    return out
+    return _native().rowsum(*x)
 
 
 def layernorm_novar(x, gamma, beta, residual=None):
-    dev = _chk(*x, gamma, beta, *(residual or ()))
-    x_lw, x_uw, x_lb, x_ub = x
-    rows = x_lb.numel() // x_lb.shape[-1]
-    Di, Do = x_lw.shape[-2], x_lw.shape[-1]
-    out = (torch.empty_like(x_lw), torch.empty_like(x_lw), torch.empty_like(x_lb), torch.empty_like(x_lb))
-    r = [_p(t) for t in residual] if residual is not None else [None] * 4
-    with torch.cuda.device(dev):
-        check(load().fb_layernorm_novar_f32(*[_p(t) for t in x], *r, _p(gamma), _p(beta), *[_p(t) for t in out],
-                                            rows, Di, Do, _stream()), "fb_layernorm_novar_f32")
-    return out
+    return _native().layernorm_novar(*x, gamma, beta, residual)
+
+
+def layernorm_standard_checked(x, gamma, beta, p, eps, words=1):
+    """Layer norm with the variance in one kernel (fb_layernorm_standard_f32); waits for the stream and returns
+    (lw, uw, lb, ub, status word), or None where the row is too wide for it."""
+    return _native().layernorm_standard_checked(*x, gamma, beta, p, eps, words)
 
 
 def split_heads(x, heads, transpose_ld=False):
     """(lw, uw, lb, ub) [B, L, Di, H*d] -> [B*H, L, Di, d], or [B*H, d, Di, L] with transpose_ld."""
-    dev = _chk(*x)
-    lw, uw, lb, ub = x
-    B, L, Di, D = lw.shape
-    d = D // heads
-    wshape = (B * heads, d, Di, L) if transpose_ld else (B * heads, L, Di, d)
-    bshape = (B * heads, d, L) if transpose_ld else (B * heads, L, d)
-    out = (torch.empty(wshape, device=dev), torch.empty(wshape, device=dev),
-           torch.empty(bshape, device=dev), torch.empty(bshape, device=dev))
-    with torch.cuda.device(dev):
-        for w, b, ow, ob in ((lw, lb, out[0], out[2]), (uw, ub, out[1], out[3])):
-            check(load().fb_split_heads_f32(_p(w), _p(b), _p(ow), _p(ob), B, L, Di, heads, d, int(transpose_ld),
-                                            _stream()), "fb_split_heads_f32")
-    return out
+    return _native().split_heads(*x, heads, int(transpose_ld))
 
 
 def merge_heads(x, heads):
     """(lw, uw, lb, ub) [B*H, L, Di, d] -> [B, L, Di, H*d]."""
-    dev = _chk(*x)
-    lw, uw, lb, ub = x
-    BH, L, Di, d = lw.shape
-    B = BH // heads
-    out = (torch.empty((B, L, Di, heads * d), device=dev), torch.empty((B, L, Di, heads * d), device=dev),
-           torch.empty((B, L, heads * d), device=dev), torch.empty((B, L, heads * d), device=dev))
-    with torch.cuda.device(dev):
-        for w, b, ow, ob in ((lw, lb, out[0], out[2]), (uw, ub, out[1], out[3])):
-            check(load().fb_merge_heads_f32(_p(w), _p(b), _p(ow), _p(ob), B, L, Di, heads, d, _stream()),
-                  "fb_merge_heads_f32")
-    return out
+    return _native().merge_heads(*x, heads)
 
 
 def conv2d(x, weight, bias, stride, padding):
     """x: (lw, uw, lb, ub) with lw, uw [B, Di, C, H, W] and lb, ub [B, C, H, W]."""
-    dev = _chk(*x, weight, bias)
-    lw, uw, lb, ub = x
-    B, Di, C, H, W = lw.shape
-    Co, Ci, Kh, Kw = weight.shape
-    if Ci != C:
-        raise _lib.FaithError("conv weight expects %d input channels, bounds have %d" % (Ci, C))
-    Ho = (H + 2 * padding - Kh) // stride + 1
-    Wo = (W + 2 * padding - Kw) // stride + 1
-    out = (torch.empty((B, Di, Co, Ho, Wo), device=dev), torch.empty((B, Di, Co, Ho, Wo), device=dev),
-           torch.empty((B, Co, Ho, Wo), device=dev), torch.empty((B, Co, Ho, Wo), device=dev))
-    with torch.cuda.device(dev):
-        check(load().fb_conv2d_f32(*[_p(t) for t in x], _p(weight), _p(bias), *[_p(t) for t in out],
-                                   B, Di, C, H, W, Co, Kh, Kw, stride, padding, _stream()), "fb_conv2d_f32")
-    return out
+    return _native().conv2d(*x, weight, bias, stride, padding)
 
 
 def norm_partials(lw, uw, p):
@@ -426,17 +295,10 @@ def relax_with_norms(op, lw, uw, lb, ub, norm_l, norm_u, p, eps, violation=None)
 def softmax_fused(x, p, eps, words=1, violation=None, ranges=False):
     """Fused softmax bound; returns None when the shape needs the unfused chain.  ranges=True appends the
     concretised range (l, u) of the result to the returned tuple."""
-    dev = _chk(*x)
-    lw, uw, lb, ub = x
-    Di, Do = lw.shape[-2], lw.shape[-1]
-    rows = lb.numel() // Do
-    out = (torch.empty_like(lw), torch.empty_like(uw), torch.empty_like(lb), torch.empty_like(ub))
-    if ranges:
-        out = out + (torch.empty_like(lb), torch.empty_like(ub))
-    with torch.cuda.device(dev):
-        rc = load().fb_softmax_ranges_f32(*[_p(t) for t in x], *[_p(t) for t in out], *([] if ranges else [None, None]),
-                                          rows, Di, Do, words, norm_code(p), eps, _p(violation), _stream())
-    if rc in (2, 3):   # FB_ERR_SHAPE / FB_ERR_ALIGN: not a fused shape
-        return None
-    check(rc, "fb_softmax_ranges_f32")
-    return out
+    return _native().softmax(*x, p, eps, words, violation, ranges)
+
+
+def softmax_checked(x, p, eps, words=1):
+    """softmax_fused() that also reads the status word of the call back (waits for the stream): None or
+    (lw, uw, lb, ub, word)."""
+    return _native().softmax_checked(*x, p, eps, words)
