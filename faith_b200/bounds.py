@@ -126,8 +126,8 @@ class Bounds:
 
     def context(self, value):
         if self.dim_in != 1 and not self.ibp:
-            # the product that reads the values as they are, where the shape is one of its: no transposed copies
-            z = ops.context_kmajor_or_none(self._t4(), value._t4(), self.p, self.eps, self.perturbed_words)
+            # the product that reads the values as they are: no transposed copies
+            z = ops.context(self._t4(), value._t4(), self.p, self.eps, self.perturbed_words)
             if z is not None:
                 return self._same(z)
         return self.dot_product(value.t())

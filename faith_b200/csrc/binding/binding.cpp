@@ -336,6 +336,31 @@ FB_FN(context_kmajor) {
   END_HANDLE_TH_ERRORS
 }
 
+// x (4) [B, Lx, Di, K], v (4) [B, K, Di, Ly], p, eps, words; None when the shape is not one of fb_context_f32's
+FB_FN(context) {
+  HANDLE_TH_ERRORS
+  Call c(args, nargs, 11, "context");
+  const Four x(c, 0), v(c, 4);
+  const int p = c.norm(8), words = c.integer(10);
+  const float eps = c.real(9);
+  if (x.lb->dim() != 3 || x.lw->dim() != 4 || v.lb->dim() != 3) fail("context: bounds of shape [B, L, Di, K] required");
+  const int64_t B = x.lb->size(0), Lx = x.lb->size(1), K = x.lb->size(2), Ly = v.lb->size(2), Di = x.lw->size(2);
+  std::array<at::Tensor, 4> z = {empty({B, Lx, Di, Ly}, c.device()), empty({B, Lx, Di, Ly}, c.device()), empty({B, Lx, Ly}, c.device()),
+                                 empty({B, Lx, Ly}, c.device())};
+  const std::array<at::Tensor, 4> r = {empty_like(*x.lb), empty_like(*x.lb), empty({B, Ly, K}, c.device()), empty({B, Ly, K}, c.device())};
+  int rc;
+  {
+    Launch l(c.device());
+    rc = fb_context_f32(ptr(x.lw), ptr(x.uw), ptr(x.lb), ptr(x.ub), ptr(v.lw), ptr(v.uw), ptr(v.lb), ptr(v.ub), ptr(z[0]), ptr(z[1]),
+                        ptr(z[2]), ptr(z[3]), ptr(r[0]), ptr(r[1]), ptr(r[2]), ptr(r[3]), (int)B, (int)Lx, (int)Ly, (int)Di, (int)K,
+                        words, p, eps, 1.0f, 1, l.stream());
+  }
+  if (rc == FB_ERR_SHAPE) Py_RETURN_NONE;
+  check_status(rc, "fb_context_f32");
+  return tuple(z);
+  END_HANDLE_TH_ERRORS
+}
+
 FB_FN(mul_bounds) {   // x (4), y (4), p, eps, words
   HANDLE_TH_ERRORS
   Call c(args, nargs, 11, "mul_bounds");
@@ -598,7 +623,7 @@ FB_FN(setup) {   // FaithError, _lib.check
 
 #define FB_DEF(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {FB_DEF(setup), FB_DEF(concretize), FB_DEF(relax), FB_DEF(relax_checked), FB_DEF(matmul), FB_DEF(dot_product),
-                          FB_DEF(context_kmajor), FB_DEF(mul_bounds), FB_DEF(add), FB_DEF(scale), FB_DEF(mul_features), FB_DEF(rowsum),
+                          FB_DEF(context_kmajor), FB_DEF(context), FB_DEF(mul_bounds), FB_DEF(add), FB_DEF(scale), FB_DEF(mul_features), FB_DEF(rowsum),
                           FB_DEF(layernorm_novar), FB_DEF(layernorm_standard_checked), FB_DEF(split_heads), FB_DEF(merge_heads), FB_DEF(conv2d), FB_DEF(softmax),
                           FB_DEF(softmax_checked), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_binding", "Native boundary of the tensor-level operators.", -1, kMethods,

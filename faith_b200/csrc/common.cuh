@@ -83,6 +83,25 @@ int layernorm_novar_rowsum(const float* x_lw, const float* x_uw, const float* x_
                            float* z_lw, float* z_uw, float* z_lb, float* z_ub, int64_t rows, int Di, int Do, float* rowsum,
                            void* stream);
 
+// softmax.cu: fb_softmax_ranges_f32 with rows `ld` floats apart.
+int softmax_ex(const float* lw, const float* uw, const float* lb, const float* ub, float* out_lw, float* out_uw, float* out_lb,
+               float* out_ub, float* out_l, float* out_u, int64_t rows, int Di, int Do, int ld, int words, int p, float eps,
+               int* violation, void* stream);
+
+bool softmax_fused_shape(int Di, int Do);   // whether the fused kernel takes the shape
+
+// dot_product.cu: whether the tensor-core kernel takes the shape (rows of any pitch; more than a few query rows).
+bool dot_pitched_supported(int B, int Lx, int Ly, int Di, int K);
+// The dot product and the context product with the options of the encoder driver (see the definitions).
+int dot_product_ex(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub, const float* y_lw, const float* y_uw,
+                   const float* y_lb, const float* y_ub, float* z_lw, float* z_uw, float* z_lb, float* z_ub, float* x_l, float* x_u,
+                   float* y_l, float* y_u, int B, int Lx, int Ly, int Di, int K, int words, int p, float eps, float out_scale,
+                   int layout, int merge_heads, int given, int ldz, void* stream);
+int context_ex(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub, const float* v_lw, const float* v_uw,
+               const float* v_lb, const float* v_ub, float* z_lw, float* z_uw, float* z_lb, float* z_ub, float* x_l, float* x_u,
+               float* y_l, float* y_u, int B, int Lx, int Ly, int Di, int K, int words, int p, float eps, float out_scale,
+               int merge_heads, int given, int ldx, bool transposed_ranges, void* stream);
+
 // Opts `kernel` in to `bytes` of dynamic shared memory on the current device (nothing to do up to 48 KB, or when it
 // already has that much): FB_OK or FB_ERR_CUDA.
 int ensure_dynamic_smem_impl(const void* func, size_t bytes);

@@ -77,51 +77,60 @@ dot_bias_kernel(const float* __restrict__ x_lb, const float* __restrict__ x_ub, 
   }
 }
 
-// Tiled version of the bias part: one block per (b, 32 i, 32 j) tile; the seven row tiles are staged
-// in shared memory (row stride 33 floats: conflict-free both for the row-wise fill and for the
-// column-wise reads), K in chunks of 32; thread (i, jq) owns the outputs (i, jq + 8 c), c = 0..3.
-// Same partial sums and the same final order of additions as dot_bias_kernel.
+// Tiled version of the bias part: one block per (b, RI i, 32 j) tile; the seven row tiles are staged in shared memory (row
+// stride 33 floats: conflict-free both for the row-wise fill and for the column-wise reads), K in chunks of 32; a thread owns
+// the outputs (warp + 8 c, lane), c = 0 .. RI / 8 - 1.  Same partial sums and the same final order of additions as
+// dot_bias_kernel.  RI = 8 where 32-row tiles would leave SMs idle: the kernel is bound by the latency of one chunk, and four
+// blocks of 32 rows (one sentence, four heads) took 7.5 us.
+// y_kmajor: y_lb / y_ub are stored [b, k, j] instead of [b, j, k]; ranges_kmajor: y_l / y_u likewise.
+template <int RI>
 __global__ void __launch_bounds__(kThreads)
 dot_bias_tiled(const float* __restrict__ x_lb, const float* __restrict__ x_ub, const float* __restrict__ y_lb,
                const float* __restrict__ y_ub, const float* __restrict__ x_l, const float* __restrict__ y_l,
                const float* __restrict__ y_u, float* __restrict__ z_lb, float* __restrict__ z_ub,
-               int Lx, int Ly, int K, int n_it, int n_jt, float out_scale, int heads, int y_kmajor) {
-  __shared__ float sm[7][32][33];   // x_lb, x_ub, x_l, y_lb, y_ub, y_l, y_u
+               int Lx, int Ly, int K, int n_it, int n_jt, float out_scale, int heads, int y_kmajor, int ranges_kmajor) {
+  constexpr int C = RI / 8;
+  __shared__ float sx[3][RI][33];   // x_lb, x_ub, x_l
+  __shared__ float sy[4][32][33];   // y_lb, y_ub, y_l, y_u
   int w = blockIdx.x;
   const int jt = w % n_jt; w /= n_jt;
   const int it = w % n_it;
   const int64_t b = w / n_it;
-  const int i0 = it * 32, j0 = jt * 32;
-  const int tid = threadIdx.x, ti = tid >> 3, tj = tid & 7;
-  float gl[4], gu[4], l1[4], l2[4], l3[4], l4[4], u1[4], u2[4], u3[4], u4[4];
+  const int i0 = it * RI, j0 = jt * 32;
+  const int tid = threadIdx.x, warp = tid >> 5, j = tid & 31;
+  float gl[C], gu[C], l1[C], l2[C], l3[C], l4[C], u1[C], u2[C], u3[C], u4[C];
 #pragma unroll
-  for (int c = 0; c < 4; ++c) gl[c] = gu[c] = l1[c] = l2[c] = l3[c] = l4[c] = u1[c] = u2[c] = u3[c] = u4[c] = 0.f;
+  for (int c = 0; c < C; ++c) gl[c] = gu[c] = l1[c] = l2[c] = l3[c] = l4[c] = u1[c] = u2[c] = u3[c] = u4[c] = 0.f;
   for (int k0 = 0; k0 < K; k0 += 32) {
-    const float* src[7] = {x_lb, x_ub, x_l, y_lb, y_ub, y_l, y_u};
+    const float* const xs[3] = {x_lb, x_ub, x_l};
+    const float* const ys[4] = {y_lb, y_ub, y_l, y_u};
 #pragma unroll
-    for (int a = 0; a < 7; ++a) {
-      const bool isx = a < 3;
-      const int L = isx ? Lx : Ly, r0 = isx ? i0 : j0;
-      for (int f = tid; f < 32 * 32; f += kThreads) {
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int f = tid; f < RI * 32; f += kThreads) {
         const int r = f >> 5, k = f & 31;
-        const bool ok = r0 + r < L && k0 + k < K;
-        // y_kmajor: y_lb / y_ub (a = 3, 4) are stored [b, k, j] instead of [b, j, k]
-        const bool km = y_kmajor && (a == 3 || a == 4);
-        const int64_t idx = km ? ((int64_t)b * K + k0 + k) * L + r0 + r : ((int64_t)b * L + r0 + r) * K + k0 + k;
-        sm[a][r][k] = ok ? src[a][idx] : 0.f;
+        sx[a][r][k] = (i0 + r < Lx && k0 + k < K) ? xs[a][((int64_t)b * Lx + i0 + r) * K + k0 + k] : 0.f;
+      }
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      const bool km = a < 2 ? y_kmajor != 0 : ranges_kmajor != 0;
+#pragma unroll
+      for (int f = tid; f < 32 * 32; f += kThreads) {
+        const int hi = f >> 5, lo = f & 31, r = km ? lo : hi, k = km ? hi : lo;   // the fast index is the contiguous one
+        const int64_t idx = km ? ((int64_t)b * K + k0 + k) * Ly + j0 + r : ((int64_t)b * Ly + j0 + r) * K + k0 + k;
+        sy[a][r][k] = (j0 + r < Ly && k0 + k < K) ? ys[a][idx] : 0.f;
       }
     }
     __syncthreads();
 #pragma unroll 4
     for (int k = 0; k < 32; ++k) {
-      const float xl = sm[0][ti][k], xu = sm[1][ti][k], lx = sm[2][ti][k];
-      const float lxp = lx > 0.f ? lx : 0.f, lxn = lx < 0.f ? lx : 0.f;
+      const float yl = sy[0][j][k], yu = sy[1][j][k], ly = sy[2][j][k], uy = sy[3][j][k];
+      const float lyp = ly > 0.f ? ly : 0.f, lyn = ly < 0.f ? ly : 0.f;
+      const float uyp = uy > 0.f ? uy : 0.f, uyn = uy < 0.f ? uy : 0.f;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int j = tj + 8 * c;
-        const float yl = sm[3][j][k], yu = sm[4][j][k], ly = sm[5][j][k], uy = sm[6][j][k];
-        const float lyp = ly > 0.f ? ly : 0.f, lyn = ly < 0.f ? ly : 0.f;
-        const float uyp = uy > 0.f ? uy : 0.f, uyn = uy < 0.f ? uy : 0.f;
+      for (int c = 0; c < C; ++c) {
+        const float xl = sx[0][warp + 8 * c][k], xu = sx[1][warp + 8 * c][k], lx = sx[2][warp + 8 * c][k];
+        const float lxp = lx > 0.f ? lx : 0.f, lxn = lx < 0.f ? lx : 0.f;
         gl[c] = fadd(gl[c], fmul(-ly, lx));
         gu[c] = fadd(gu[c], fmul(-uy, lx));
         l1[c] = fmaf(xl, lyp, l1[c]); l2[c] = fmaf(xu, lyn, l2[c]); l3[c] = fmaf(yl, lxp, l3[c]); l4[c] = fmaf(yu, lxn, l4[c]);
@@ -130,17 +139,15 @@ dot_bias_tiled(const float* __restrict__ x_lb, const float* __restrict__ x_ub, c
     }
     __syncthreads();
   }
-  const int i = i0 + ti;
-  if (i < Lx) {
+  if (j0 + j >= Ly) return;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int j = j0 + tj + 8 * c;
-      if (j < Ly) {
-        // heads > 1: head-merged output [S, Lx, heads * Ly]
-        const int64_t od = (((b / heads) * Lx + i) * heads + b % heads) * Ly + j;
-        z_lb[od] = fmul(fadd(fadd(fadd(fadd(gl[c], l1[c]), l2[c]), l3[c]), l4[c]), out_scale);
-        z_ub[od] = fmul(fadd(fadd(fadd(fadd(gu[c], u1[c]), u2[c]), u3[c]), u4[c]), out_scale);
-      }
+  for (int c = 0; c < C; ++c) {
+    const int i = i0 + warp + 8 * c;
+    if (i < Lx) {
+      // heads > 1: head-merged output [S, Lx, heads * Ly]
+      const int64_t od = (((b / heads) * Lx + i) * heads + b % heads) * Ly + j0 + j;
+      z_lb[od] = fmul(fadd(fadd(fadd(fadd(gl[c], l1[c]), l2[c]), l3[c]), l4[c]), out_scale);
+      z_ub[od] = fmul(fadd(fadd(fadd(fadd(gu[c], u1[c]), u2[c]), u3[c]), u4[c]), out_scale);
     }
   }
 }
@@ -340,6 +347,29 @@ int launch_dot_weight_rows(const float* x_lw, const float* x_uw, const float* y_
 }
 
 
+int launch_dot_bias(const float* x_lb, const float* x_ub, const float* y_lb, const float* y_ub, const float* x_l, const float* y_l,
+                    const float* y_u, float* z_lb, float* z_ub, int B, int Lx, int Ly, int K, float out_scale, int heads,
+                    int y_kmajor, int ranges_kmajor, cudaStream_t st) {
+  const int n_jt = (int)ceil_div(Ly, 32);
+  const int64_t b32 = (int64_t)B * ceil_div(Lx, 32) * n_jt, b8 = (int64_t)B * ceil_div(Lx, 8) * n_jt;
+  if (b32 < 2 * (int64_t)device_info().sms && b8 <= 0x7fffffff) {
+    dot_bias_tiled<8><<<(unsigned)b8, kThreads, 0, st>>>(x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u, z_lb, z_ub, Lx, Ly, K, (int)ceil_div(Lx, 8),
+                                                         n_jt, out_scale, heads, y_kmajor, ranges_kmajor);
+  } else if (b32 <= 0x7fffffff) {
+    dot_bias_tiled<32><<<(unsigned)b32, kThreads, 0, st>>>(x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u, z_lb, z_ub, Lx, Ly, K,
+                                                           (int)ceil_div(Lx, 32), n_jt, out_scale, heads, y_kmajor, ranges_kmajor);
+  } else {
+    if (y_kmajor || ranges_kmajor) return FB_ERR_SHAPE;
+    const int64_t total = (int64_t)B * Lx * Ly;
+    const int64_t want = ceil_div(total, kThreads / 32);
+    const int64_t cap = (int64_t)device_info().sms * 32;
+    dot_bias_kernel<<<(unsigned)(want < cap ? want : cap), kThreads, 0, st>>>(x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u, z_lb, z_ub, total,
+                                                                              Lx, Ly, K, out_scale, heads);
+  }
+  FB_LAUNCH_OK();
+  return FB_OK;
+}
+
 // --------------------------------------------- weight part, transposed layout
 // x [B, Lx, K, Di], y [B, Ly, K, Di] -> z [B, Lx, Ly, Di]   (Di contiguous).
 // One thread per symbolic coordinate m (coalesced along Di), 4 x 4 (i, j) outputs per thread;
@@ -433,6 +463,11 @@ bool dot_tc_supported(const float* x_lw, const float* x_uw, const float* y_lw, c
 int launch_dot_weight_tc(const float* x_lw, const float* x_uw, const float* y_lw, const float* y_uw, const float* x_l,
                          const float* y_l, const float* y_u, float* z_lw, float* z_uw, int B, int Lx, int Ly, int Di,
                          float out_scale, int heads, int y_kmajor, cudaStream_t st);
+// dot_product_tc_any.cu
+bool dot_tc_any_supported(int B, int Lx, int Ly, int Di, int K);
+int launch_dot_weight_tc_any(const float* x_lw, const float* x_uw, const float* y_lw, const float* y_uw, const float* x_l,
+                             const float* y_l, const float* y_u, float* z_lw, float* z_uw, int B, int Lx, int Ly, int Di, int K,
+                             float out_scale, int heads, int y_kmajor, int y_ranges_kmajor, int ldx, int ldz, cudaStream_t st);
 namespace {
 // FB_DOT_IMPL=ffma in the environment keeps the dot product on the CUDA-core kernels (exact fp32 products)
 bool dot_force_cuda_cores() {
@@ -447,14 +482,19 @@ bool dot_force_cuda_cores() {
 
 using namespace fb;
 
+bool fb::dot_pitched_supported(int B, int Lx, int Ly, int Di, int K) {
+  return !dot_force_cuda_cores() && Lx > kFewRows && Di > 1 && dot_tc_any_supported(B, Lx, Ly, Di, K);
+}
+
+// ldz: floats between consecutive m of z_lw / z_uw (0: contiguous; anything else takes the tensor-core kernel or nothing).
 // given: bit 0 = x_l / x_u already hold the concretised range of x, bit 1 = y_l / y_u that of y
 // (e.g. from fb_matmul_heads_ranges_f32); the corresponding concretisation pass is skipped.
-static int dot_heads_impl(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub,
+int fb::dot_product_ex(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub,
                           const float* y_lw, const float* y_uw, const float* y_lb, const float* y_ub,
                           float* z_lw, float* z_uw, float* z_lb, float* z_ub,
                           float* x_l, float* x_u, float* y_l, float* y_u,
                           int B, int Lx, int Ly, int Di, int K, int words, int p, float eps,
-                          float out_scale, int layout, int merge_heads, int given, void* stream) {
+                          float out_scale, int layout, int merge_heads, int given, int ldz, void* stream) {
   if (given < 0 || given > 3) return FB_ERR_ARG;
   if (merge_heads < 1 || (merge_heads > 1 && (layout != FB_NATIVE || B % merge_heads != 0 || K % 4 != 0))) return FB_ERR_ARG;
   if (!x_lw || !x_uw || !x_lb || !x_ub || !y_lw || !y_uw || !y_lb || !y_ub || !z_lw || !z_uw || !z_lb || !z_ub ||
@@ -477,26 +517,17 @@ static int dot_heads_impl(const float* x_lw, const float* x_uw, const float* x_l
   if (rc != FB_OK) return rc;
   if (!(given & 2)) rc = fb_concretize_f32(y_lw, y_uw, y_lb, y_ub, y_l, y_u, (int64_t)B * Ly, Di, K, words, p, eps, layout, stream);
   if (rc != FB_OK) return rc;
-  {
-    const int n_it = (int)ceil_div(Lx, 32), n_jt = (int)ceil_div(Ly, 32);
-    const int64_t blocks = (int64_t)B * n_it * n_jt;
-    if (blocks <= 0x7fffffff) {
-      dot_bias_tiled<<<(unsigned)blocks, kThreads, 0, st>>>(x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u, z_lb, z_ub, Lx, Ly, K,
-                                                           n_it, n_jt, out_scale, merge_heads, 0);
-    } else {
-      const int64_t total = (int64_t)B * Lx * Ly;
-      const int64_t want = ceil_div(total, kThreads / 32);
-      const int64_t cap = (int64_t)device_info().sms * 32;
-      dot_bias_kernel<<<(unsigned)(want < cap ? want : cap), kThreads, 0, st>>>(x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u,
-                                                                                 z_lb, z_ub, total, Lx, Ly, K, out_scale, merge_heads);
-    }
-    FB_LAUNCH_OK();
-  }
-  if (layout == FB_NATIVE && !dot_force_cuda_cores() &&
-      dot_tc_supported(x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, K, merge_heads)) {
-    // attention shapes: tensor-core kernel
+  rc = launch_dot_bias(x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u, z_lb, z_ub, B, Lx, Ly, K, out_scale, merge_heads, 0, 0, st);
+  if (rc != FB_OK) return rc;
+  // Tensor-core kernels: the one for the attention shapes with lengths that are multiples of 32 (5.6 TB/s on a large batch,
+  // where the other reaches 4.8), else the one for any shape of the native layout; a few query rows would be padded to 32 there.
+  if (layout == FB_NATIVE && !dot_force_cuda_cores() && ldz == 0 &&
+      dot_tc_supported(x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, K, merge_heads))
     return launch_dot_weight_tc(x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, out_scale, merge_heads, 0, st);
-  }
+  if (layout == FB_NATIVE && !dot_force_cuda_cores() && Lx > kFewRows && dot_tc_any_supported(B, Lx, Ly, Di, K))
+    return launch_dot_weight_tc_any(x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, K, out_scale, merge_heads, 0, 0,
+                                    0, ldz, st);
+  if (ldz != 0) return FB_ERR_SHAPE;
   if (layout == FB_NATIVE && Lx <= kFewRows)
     return launch_dot_weight_rows(x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, K, out_scale, merge_heads, 0, st);
   if (layout == FB_NATIVE) {
@@ -539,8 +570,8 @@ extern "C" int fb_dot_product_heads_f32(const float* x_lw, const float* x_uw, co
                                   float* x_l, float* x_u, float* y_l, float* y_u,
                                   int B, int Lx, int Ly, int Di, int K, int words, int p, float eps,
                                   float out_scale, int layout, int merge_heads, void* stream) {
-  return dot_heads_impl(x_lw, x_uw, x_lb, x_ub, y_lw, y_uw, y_lb, y_ub, z_lw, z_uw, z_lb, z_ub, x_l, x_u, y_l, y_u, B, Lx,
-                        Ly, Di, K, words, p, eps, out_scale, layout, merge_heads, 0, stream);
+  return fb::dot_product_ex(x_lw, x_uw, x_lb, x_ub, y_lw, y_uw, y_lb, y_ub, z_lw, z_uw, z_lb, z_ub, x_l, x_u, y_l, y_u, B, Lx,
+                        Ly, Di, K, words, p, eps, out_scale, layout, merge_heads, 0, 0, stream);
 }
 
 // fb_dot_product_heads_f32 for operands whose concretised ranges the caller already has (written by the
@@ -551,8 +582,8 @@ extern "C" int fb_dot_product_given_f32(const float* x_lw, const float* x_uw, co
                                   float* x_l, float* x_u, float* y_l, float* y_u,
                                   int B, int Lx, int Ly, int Di, int K, int words, int p, float eps,
                                   float out_scale, int layout, int merge_heads, int given, void* stream) {
-  return dot_heads_impl(x_lw, x_uw, x_lb, x_ub, y_lw, y_uw, y_lb, y_ub, z_lw, z_uw, z_lb, z_ub, x_l, x_u, y_l, y_u, B, Lx,
-                        Ly, Di, K, words, p, eps, out_scale, layout, merge_heads, given, stream);
+  return fb::dot_product_ex(x_lw, x_uw, x_lb, x_ub, y_lw, y_uw, y_lb, y_ub, z_lw, z_uw, z_lb, z_ub, x_l, x_u, y_l, y_u, B, Lx,
+                        Ly, Di, K, words, p, eps, out_scale, layout, merge_heads, given, 0, stream);
 }
 
 extern "C" int fb_dot_product_f32(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub,
@@ -605,11 +636,38 @@ extern "C" int fb_context_given_f32(const float* x_lw, const float* x_uw, const 
   if (!(out_scale > 0.f)) return FB_ERR_ARG;
   if (Di % words != 0 || Di == 1) return FB_ERR_SHAPE;
   if (B == 0) return FB_OK;
+  // (the shapes of the attention of the forward verifier; fb_context_f32 takes any)
   const bool tc = !dot_force_cuda_cores() &&
                   dot_tc_supported(x_lw, x_uw, v_lw, v_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, K, merge_heads);
   // (a few query rows go through the thread-per-output kernel, which reads the values in this layout as well)
   const bool rows_kernel = !tc && Lx <= kFewRows && (int64_t)K * Ly <= 4096;
   if (!tc && !rows_kernel) return FB_ERR_SHAPE;
+  return fb::context_ex(x_lw, x_uw, x_lb, x_ub, v_lw, v_uw, v_lb, v_ub, z_lw, z_uw, z_lb, z_ub, x_l, x_u, y_l, y_u, B, Lx, Ly,
+                                Di, K, words, p, eps, out_scale, merge_heads, given, 0, true, stream);
+}
+
+// The general form: any shape, x rows ldx floats apart (0: contiguous).  transposed_ranges: the value ranges end up as
+// [B, Ly, K] in y_l / y_u (small matrices only), as the entry points above document; otherwise they stay [B, K, Ly].
+int fb::context_ex(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub, const float* v_lw, const float* v_uw,
+                   const float* v_lb, const float* v_ub, float* z_lw, float* z_uw, float* z_lb, float* z_ub, float* x_l, float* x_u,
+                   float* y_l, float* y_u, int B, int Lx, int Ly, int Di, int K, int words, int p, float eps, float out_scale,
+                   int merge_heads, int given, int ldx, bool transposed_ranges, void* stream) {
+  if (given < 0 || given > 3) return FB_ERR_ARG;
+  if (!x_lw || !x_uw || !x_lb || !x_ub || !v_lw || !v_uw || !v_lb || !v_ub || !z_lw || !z_uw || !z_lb || !z_ub ||
+      !x_l || !x_u || !y_l || !y_u)
+    return FB_ERR_ARG;
+  if (B < 0 || Lx <= 0 || Ly <= 0 || Di <= 0 || K <= 0 || words <= 0 || !valid_norm(p) || merge_heads < 1 || B % merge_heads != 0)
+    return FB_ERR_ARG;
+  if (!(out_scale > 0.f)) return FB_ERR_ARG;
+  if (Di % words != 0 || Di == 1) return FB_ERR_SHAPE;
+  if (B == 0) return FB_OK;
+  const bool few = Lx <= kFewRows && ldx == 0;
+  const bool tc32 = !dot_force_cuda_cores() && ldx == 0 &&
+                    dot_tc_supported(x_lw, x_uw, v_lw, v_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, K, merge_heads);
+  const bool tc = tc32 || (!few && !dot_force_cuda_cores() && dot_tc_any_supported(B, Lx, Ly, Di, K));
+  if (!tc && (!few || (!transposed_ranges && (int64_t)K * Ly > 4096))) return FB_ERR_SHAPE;
+  if ((int64_t)B * ceil_div(Lx, 32) * ceil_div(Ly, 32) > 0x7fffffff) return FB_ERR_SHAPE;
+  if (ldx != 0 && !(given & 1)) return FB_ERR_ARG;   // (the concretisation pass reads contiguous rows)
   cudaStream_t st = (cudaStream_t)stream;
   const double d1 = (double)Di + 1;
   ProfileScope prof(PK_DOT, 16.0 * B * Lx * Ly * d1 * K,
@@ -617,20 +675,31 @@ extern "C" int fb_context_given_f32(const float* x_lw, const float* x_uw, const 
   int rc = FB_OK;
   if (!(given & 1)) rc = fb_concretize_f32(x_lw, x_uw, x_lb, x_ub, x_l, x_u, (int64_t)B * Lx, Di, K, words, p, eps, FB_NATIVE, stream);
   if (rc != FB_OK) return rc;
-  // ranges of the values in their own layout [B, K, Ly], then transposed in place to [B, Ly, K]
+  // ranges of the values in their own layout [B, K, Ly]
   if (!(given & 2)) rc = fb_concretize_f32(v_lw, v_uw, v_lb, v_ub, y_l, y_u, (int64_t)B * K, Di, Ly, words, p, eps, FB_NATIVE, stream);
   if (rc != FB_OK) return rc;
-  transpose_small_inplace<<<(unsigned)B, 256, 0, st>>>(y_l, y_u, K, Ly);
-  FB_LAUNCH_OK();
-  {
-    const int n_it = (int)ceil_div(Lx, 32), n_jt = (int)ceil_div(Ly, 32);
-    dot_bias_tiled<<<(unsigned)((int64_t)B * n_it * n_jt), kThreads, 0, st>>>(x_lb, x_ub, v_lb, v_ub, x_l, y_l, y_u, z_lb, z_ub,
-                                                                            Lx, Ly, K, n_it, n_jt, out_scale, merge_heads, 1);
+  const bool transpose = transposed_ranges || !tc || tc32;
+  if (transpose) {
+    transpose_small_inplace<<<(unsigned)B, 256, 0, st>>>(y_l, y_u, K, Ly);
     FB_LAUNCH_OK();
   }
-  if (rows_kernel)
+  rc = launch_dot_bias(x_lb, x_ub, v_lb, v_ub, x_l, y_l, y_u, z_lb, z_ub, B, Lx, Ly, K, out_scale, merge_heads, 1, transpose ? 0 : 1, st);
+  if (rc != FB_OK) return rc;
+  if (!tc)
     return launch_dot_weight_rows(x_lw, x_uw, v_lw, v_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, K, out_scale, merge_heads, 1, st);
-  return launch_dot_weight_tc(x_lw, x_uw, v_lw, v_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, out_scale, merge_heads, 1, st);
+  if (tc32) return launch_dot_weight_tc(x_lw, x_uw, v_lw, v_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, out_scale, merge_heads, 1, st);
+  return launch_dot_weight_tc_any(x_lw, x_uw, v_lw, v_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, K, out_scale, merge_heads, 1,
+                                  transpose ? 0 : 1, ldx, 0, st);
+}
+
+extern "C" int fb_context_f32(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub,
+                              const float* v_lw, const float* v_uw, const float* v_lb, const float* v_ub,
+                              float* z_lw, float* z_uw, float* z_lb, float* z_ub,
+                              float* x_l, float* x_u, float* y_l, float* y_u,
+                              int B, int Lx, int Ly, int Di, int K, int words, int p, float eps,
+                              float out_scale, int merge_heads, void* stream) {
+  return fb::context_ex(x_lw, x_uw, x_lb, x_ub, v_lw, v_uw, v_lb, v_ub, z_lw, z_uw, z_lb, z_ub, x_l, x_u, y_l, y_u, B, Lx, Ly, Di, K,
+                        words, p, eps, out_scale, merge_heads, 0, 0, false, stream);
 }
 
 extern "C" int fb_context_heads_f32(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub,

@@ -453,16 +453,22 @@ static int encoder_forward_impl(const fb_encoder* enc, const float* emb, int S, 
     } else {
       return qrc;
     }
-    // scores [S*H, L, Di, L], scaled by 1/sqrt(d) -> T1
-    FB_TRY(fb_dot_product_given_f32(Qh.lw, Qh.uw, T2.lb, T2.ub, Kh.lw, Kh.uw, T3.lb, T3.ub, T1.lw, T1.uw, T1.lb, T1.ub,
-                                    range[0], range[1], range[2], range[3], S * H, L, L, Di, d, words, p, eps, inv_sqrt_d,
-                                    FB_NATIVE, 1, given, stream));
+    // scores [S*H, L, Di, L], scaled by 1/sqrt(d) -> T1.  A length that is not a multiple of four leaves rows that TMA and
+    // 128-bit accesses cannot address: the rows of the scores and of the probabilities are then kept `ls` floats apart,
+    // where the slot has room for that and every consumer takes it.
+    const int lp = (L + 3) / 4 * 4;
+    const bool pitched = L != lp && (int64_t)S * H * L * Di * lp <= plan.cap_w && softmax_fused_shape(Di, L) &&
+                         dot_pitched_supported(S * H, L, L, Di, d) && dot_pitched_supported(S * H, L, d, Di, L);
+    const int ls = pitched ? lp : L;
+    FB_TRY(dot_product_ex(Qh.lw, Qh.uw, T2.lb, T2.ub, Kh.lw, Kh.uw, T3.lb, T3.ub, T1.lw, T1.uw, T1.lb, T1.ub,
+                          range[0], range[1], range[2], range[3], S * H, L, L, Di, d, words, p, eps, inv_sqrt_d,
+                          FB_NATIVE, 1, given, pitched ? ls : 0, stream));
     const int64_t hrows = (int64_t)S * H * L;
     // softmax: fused kernel when the score row fits one tile, else exp / row sum / reciprocal / product
     // (the fused kernel also returns the concretised range of the probabilities for the context product)
     int pgiven = 0;
-    int src = fb_softmax_ranges_f32(T1.lw, T1.uw, T1.lb, T1.ub, T2.lw, T2.uw, T2.lb, T2.ub, range[0], range[1], hrows, Di,
-                                    L, words, p, eps, violation, stream);
+    int src = softmax_ex(T1.lw, T1.uw, T1.lb, T1.ub, T2.lw, T2.uw, T2.lb, T2.ub, range[0], range[1], hrows, Di, L, ls, words, p, eps,
+                         violation, stream);
     if (src == FB_OK) {
       pgiven = 1;
       // probabilities are in T2; the stages below expect them in T1
@@ -479,7 +485,7 @@ static int encoder_forward_impl(const fb_encoder* enc, const float* emb, int S, 
     }
     // values, split into heads [S*H, L, Di, d]; the tensor-core context product reads them in this layout
     int crc = FB_ERR_SHAPE;
-    if (L % 4 == 0) {
+    if (pitched || dot_pitched_supported(S * H, L, d, Di, L)) {
       int vgiven = pgiven;
       BoundSet Vh = T3;
       if (li == 0) Vh.uw = Vh.lw;
@@ -495,9 +501,8 @@ static int encoder_forward_impl(const fb_encoder* enc, const float* emb, int S, 
         return vrc;
       }
       // context, written head-merged as [S, L, Di, D] -> T2
-      crc = fb_context_given_f32(T1.lw, T1.uw, T1.lb, T1.ub, Vh.lw, Vh.uw, T3.lb, T3.ub, T2.lw, T2.uw, T2.lb, T2.ub,
-                                 range[0], range[1], range[2], range[3], S * H, L, d, Di, L, words, p, eps, 1.0f, H, vgiven,
-                                 stream);
+      crc = context_ex(T1.lw, T1.uw, T1.lb, T1.ub, Vh.lw, Vh.uw, T3.lb, T3.ub, T2.lw, T2.uw, T2.lb, T2.ub, range[0], range[1],
+                       range[2], range[3], S * H, L, d, Di, L, words, p, eps, 1.0f, H, vgiven, pitched ? ls : 0, false, stream);
       if (crc != FB_OK && crc != FB_ERR_SHAPE) return crc;
     }
     if (crc == FB_ERR_SHAPE) {
@@ -509,7 +514,7 @@ static int encoder_forward_impl(const fb_encoder* enc, const float* emb, int S, 
                                       range[0], range[1], range[2], range[3], S * H, L, d, Di, L, words, p, eps, 1.0f,
                                       FB_NATIVE, (L % 4 == 0) ? H : 1, stream));
     }
-    if (L % 4 != 0) {  // unvectorised path: merge with the permute kernel
+    if (crc == FB_ERR_SHAPE && L % 4 != 0) {  // unvectorised path: merge with the permute kernel
       FB_TRY(fb_merge_heads_f32(T2.lw, T2.lb, T1.lw, T1.lb, S, L, Di, H, d, stream));
       FB_TRY(fb_merge_heads_f32(T2.uw, T2.ub, T1.uw, T1.ub, S, L, Di, H, d, stream));
       FB_CUDA_OK(cudaMemcpyAsync(T2.lw, T1.lw, (size_t)rows * Di * D * 4, cudaMemcpyDeviceToDevice, (cudaStream_t)stream));

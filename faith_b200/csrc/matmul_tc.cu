@@ -1032,7 +1032,10 @@ int launch_split_sign_tc(const float* a_lo, const float* a_up, const float* W, c
 
 // Reads (and clears) the device-side flag that the tensor-core kernels raise when one of their bounded
 // waits expires.  Synchronises the device.
-namespace fb { int dot_tc_error_flag(int* flag); }
+namespace fb {
+int dot_tc_error_flag(int* flag);
+int dot_tc_any_error_flag(int* flag);
+}  // namespace fb
 
 extern "C" int fb_tc_error_flag(int* flag) {
   if (!flag) return FB_ERR_ARG;
@@ -1044,9 +1047,12 @@ extern "C" int fb_tc_error_flag(int* flag) {
     FB_CUDA_OK(cudaMemcpyToSymbol(fb::g_tc_error, &zero, sizeof(int)));
   }
   int v2 = 0;
-  const int rc = fb::dot_tc_error_flag(&v2);   // the tensor-core dot product keeps a flag of its own
+  const int rc = fb::dot_tc_error_flag(&v2);   // the tensor-core dot product kernels keep flags of their own
   if (rc != FB_OK) return rc;
-  *flag = (v != 0 || v2 != 0) ? 1 : 0;
+  int v3 = 0;
+  const int rc3 = fb::dot_tc_any_error_flag(&v3);
+  if (rc3 != FB_OK) return rc3;
+  *flag = (v != 0 || v2 != 0 || v3 != 0) ? 1 : 0;
   return FB_OK;
 }
 

@@ -115,6 +115,16 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int x, int 
   asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];"
                ::"l"(map), "r"(x), "r"(y), "r"(z), "r"(src) : "memory");
 }
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, int w, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+      ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void tma_store_5d(const CUtensorMap* map, int x, int y, int z, int w, int v, uint32_t src) {
+  asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4, %5}], [%6];"
+               ::"l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(v), "r"(src) : "memory");
+}
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // waits until the bulk stores committed so far have finished READING shared memory
 __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
@@ -159,6 +169,18 @@ __device__ __forceinline__ void mma_tf32_ts_lean(uint32_t d_tmem, uint32_t a_tme
         ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(0u)
         : "memory");
   }
+}
+
+// The same with bf16 operands (kind::f16), K = 16 per instruction.
+template <bool kAccumulate>
+__device__ __forceinline__ void mma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 bd;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "mov.b64 bd, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %4, {%5, %5, %5, %5}, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(0u), "n"(kAccumulate ? 1 : 0)
+      : "memory");
 }
 
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
@@ -241,6 +263,18 @@ __device__ __forceinline__ void split_tf32_pair(uint64_t v, uint64_t& hi, uint64
   lo = sub2(v, hi);
 }
 
+// Exact split of two fp32 values into three bf16 parts each, packed two to a word: v = h + m + l with 8 significant bits per
+// part.  h and m are taken by truncation, so every part carries the sign of v (or is zero) and l is what is left of the 24
+// bits, which fits bf16 exactly.
+__device__ __forceinline__ void split_bf16_pair(uint64_t v, uint32_t& h, uint32_t& m, uint32_t& l) {
+  constexpr uint64_t kTop = 0xffff0000ffff0000ull;
+  h = __byte_perm((uint32_t)v, (uint32_t)(v >> 32), 0x7632);
+  const uint64_t r = sub2(v, v & kTop);
+  m = __byte_perm((uint32_t)r, (uint32_t)(r >> 32), 0x7632);
+  const uint64_t q = sub2(r, r & kTop);
+  l = __byte_perm((uint32_t)q, (uint32_t)(q >> 32), 0x7632);
+}
+
 // Byte offset of (row, 16-byte chunk) inside a 128-row x 128-byte tile with the 128-byte swizzle
 // (chunk index XOR row mod 8); tiles are 1024-byte aligned.
 __device__ __forceinline__ uint32_t swz(int row, int chunk) { return (uint32_t)(row * 128 + ((chunk ^ (row & 7)) << 4)); }
@@ -278,28 +312,28 @@ EncodeTiledFn encode_fn() {
 // arena addresses over and over, and an encode costs a driver call each.
 struct MapKey {
   const void* ptr;
-  uint64_t d0, d1, d2, s0, s1;
-  uint32_t b0, b1, b2, rank;
+  uint64_t dim[5], stride[4];   // extents innermost first; byte strides of dimensions 1 .. rank-1
+  uint32_t box[5], rank;
   bool operator==(const MapKey& o) const {
-    return ptr == o.ptr && d0 == o.d0 && d1 == o.d1 && d2 == o.d2 && s0 == o.s0 && s1 == o.s1 && b0 == o.b0 && b1 == o.b1 &&
-           b2 == o.b2 && rank == o.rank;
+    if (ptr != o.ptr || rank != o.rank) return false;
+    for (uint32_t i = 0; i < 5; ++i)
+      if (dim[i] != o.dim[i] || box[i] != o.box[i] || (i < 4 && stride[i] != o.stride[i])) return false;
+    return true;
   }
 };
 struct MapKeyHash {
   size_t operator()(const MapKey& k) const {
-    uint64_t h = reinterpret_cast<uintptr_t>(k.ptr) * 0x9E3779B97F4A7C15ull;
-    h ^= (k.d0 + 0x632BE59BD9B4E019ull) * 0xFF51AFD7ED558CCDull + (k.d1 << 17) + (k.d2 << 40) + k.s0 * 31 + k.s1 * 131 + k.b1 * 7 + k.b2 * 3 + k.rank;
+    uint64_t h = reinterpret_cast<uintptr_t>(k.ptr) * 0x9E3779B97F4A7C15ull + k.rank;
+    for (int i = 0; i < 5; ++i) h = (h ^ (k.dim[i] + ((uint64_t)k.box[i] << 40) + (i < 4 ? k.stride[i] << 17 : 0))) * 0xFF51AFD7ED558CCDull;
     return (size_t)(h ^ (h >> 29));
   }
 };
 std::mutex g_map_mu;
 std::unordered_map<MapKey, CUtensorMap, MapKeyHash> g_maps;
 
-// fp32 tensor of up to three dimensions (innermost first; s0, s1: byte strides of dimensions 1 and 2), box
-// {b0, b1, b2}, 128-byte swizzle, zero fill.
-bool get_map(CUtensorMap* out, const float* ptr, uint32_t rank, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s0, uint64_t s1,
-             uint32_t b0, uint32_t b1, uint32_t b2 = 1) {
-  const MapKey key = {ptr, d0, d1, d2, s0, s1, b0, b1, b2, rank};
+// fp32 tensor of `rank` dimensions, 128-byte swizzle, zero fill.  dim and box as in MapKey, 1 beyond the rank; stride 0
+// beyond it.
+bool get_map(CUtensorMap* out, const MapKey& key) {
   {
     std::lock_guard<std::mutex> lk(g_map_mu);
     auto it = g_maps.find(key);
@@ -307,11 +341,15 @@ bool get_map(CUtensorMap* out, const float* ptr, uint32_t rank, uint64_t d0, uin
   }
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
-  const cuuint64_t dims[3] = {d0, d1, d2};
-  const cuuint64_t strides[2] = {s0, s1};
-  const cuuint32_t box[3] = {b0, b1, b2};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  if (fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, rank, const_cast<float*>(ptr), dims, strides, box, estr,
+  cuuint64_t dims[5], strides[4];
+  cuuint32_t box[5];
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  for (int i = 0; i < 5; ++i) {
+    dims[i] = key.dim[i];
+    box[i] = key.box[i];
+    if (i < 4) strides[i] = key.stride[i];
+  }
+  if (fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, key.rank, const_cast<void*>(key.ptr), dims, strides, box, estr,
          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return false;
@@ -320,4 +358,8 @@ bool get_map(CUtensorMap* out, const float* ptr, uint32_t rank, uint64_t d0, uin
   g_maps.emplace(key, *out);
   return true;
 }
-
+// Up to three dimensions (innermost first; s0, s1: byte strides of dimensions 1 and 2), box {b0, b1, b2}.
+bool get_map(CUtensorMap* out, const float* ptr, uint32_t rank, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s0, uint64_t s1,
+             uint32_t b0, uint32_t b1, uint32_t b2 = 1) {
+  return get_map(out, MapKey{ptr, {d0, d1, d2, 1, 1}, {s0, s1, 0, 0}, {b0, b1, b2, 1, 1}, rank});
+}

@@ -191,9 +191,10 @@ def context_kmajor(x, v, p, eps, words=1, out_scale=1.0, merge_heads=1):
     return z
 
 
-def context_kmajor_or_none(x, v, p, eps, words=1):
-    """context_kmajor(), or None where the shape is not one it takes."""
-    return _native().context_kmajor(*x, *v, p, eps, words, 1.0, 1)
+def context(x, v, p, eps, words=1):
+    """Context product of any shape with the values in the projection's own layout (fb_context_f32), or None where the
+    shape is not one it takes (a few query rows against large values)."""
+    return _native().context(*x, *v, p, eps, words)
 
 
 def mul_bounds(x, y, p, eps, words=1):

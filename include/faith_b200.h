@@ -251,6 +251,15 @@ int fb_context_heads_f32(const float* x_lw, const float* x_uw, const float* x_lb
                          int B, int Lx, int Ly, int Di, int K, int words, int p, float eps,
                          float out_scale, int merge_heads, void* stream);
 
+/* The same operator for any shape (tensor-core kernel; up to four query rows go through a kernel of their own, which
+ * wants K * Ly <= 4096, else FB_ERR_SHAPE).  x_l, x_u, y_l, y_u are scratch. */
+int fb_context_f32(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub,
+                   const float* v_lw, const float* v_uw, const float* v_lb, const float* v_ub,
+                   float* z_lw, float* z_uw, float* z_lb, float* z_ub,
+                   float* x_l, float* x_u, float* y_l, float* y_u,
+                   int B, int Lx, int Ly, int Di, int K, int words, int p, float eps,
+                   float out_scale, int merge_heads, void* stream);
+
 /* fb_context_heads_f32 with `given` as in fb_dot_product_given_f32; given value ranges are expected as
  * [B, K, Ly] (the layout of v_lb / v_ub) and are transposed in place to [B, Ly, K] like computed ones. */
 int fb_context_given_f32(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub,
@@ -332,8 +341,8 @@ int fb_rowsum_f32(const float* x_lw, const float* x_uw, const float* x_lb, const
                   int64_t rows, int Di, int Do, void* stream);
 
 /* Fused softmax bound: exp, feature-axis sum, reciprocal and McCormick product in one kernel
- * (Bounds.softmax, Bounds.py:1005-1014).  Needs the feature axis in one tile: Do <= 32, Do % 4 == 0
- * and the two [Di, 32] tiles in shared memory; other shapes return FB_ERR_SHAPE (callers then run the
+ * (Bounds.softmax, Bounds.py:1005-1014).  Needs the feature axis in one tile: Do <= 64
+ * and the two [Di, 16 | 32 | 64] tiles in shared memory; other shapes return FB_ERR_SHAPE (callers then run the
  * chain fb_relax_f32(FB_EXP) / fb_rowsum_f32 / fb_relax_f32(FB_RECIPROCAL) / fb_mul_bounds_f32).
  * `violation` as in fb_relax_f32(FB_RECIPROCAL). */
 int fb_softmax_f32(const float* lw, const float* uw, const float* lb, const float* ub,

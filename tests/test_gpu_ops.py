@@ -1023,3 +1023,58 @@ def test_product_of_few_rows(B, L, Do, Dy):
     o = O.OBounds(2.0, 0.1, *t).dense(W, bias)
     o64 = O.OBounds(2.0, 0.1, *[v.double() for v in t]).dense(W.double(), bias.double())
     helpers.assert_bounds_arbitrated(got, o, o64, "product of few rows %d %d %d" % (B * L, Do, Dy))
+
+
+@pytest.mark.parametrize("B,Lx,Ly,Di,K,words", [(2, 5, 5, 6, 3, 1), (3, 21, 21, 64, 32, 2), (2, 33, 40, 32, 32, 1), (1, 64, 31, 10, 64, 1),
+                                                (2, 32, 23, 16, 21, 1)])
+def test_dot_and_context_of_ragged_lengths(B, Lx, Ly, Di, K, words):
+    """The tensor-core dot product for any length (tiles cut short in every direction, one and two chunks of the contraction,
+    operand and result rows that TMA cannot address): scores, and the context product that reads the values untransposed."""
+    import faith_b200
+    from faith_b200 import ops
+    p, eps = 2.0, 0.1
+    tx, ty = cases.rand_bounds(1401, B, Lx, Di, K, -0.5, 1.0), cases.rand_bounds(1402, B, Ly, Di, K, -0.5, 1.0)
+    ob = lambda t, d=torch.float32: O.OBounds(p, eps, *[v.to(d) for v in t], words=words)
+    gb = lambda t: faith_b200.BoundsLite(p, eps, *[v.to(DEV) for v in t], perturbed_words=words)
+    helpers.assert_bounds_arbitrated(gb(tx).dot_product(gb(ty)), ob(tx).dot_product(ob(ty)),
+                                     ob(tx, torch.float64).dot_product(ob(ty, torch.float64)), "ragged dot %d x %d, K %d" % (Lx, Ly, K))
+    tp, tv = cases.rand_bounds(1403, B, Lx, Di, Ly, 0.0, 0.2), cases.rand_bounds(1404, B, Ly, Di, K, -0.5, 1.0)
+    helpers.assert_bounds_arbitrated(gb(tp).context(gb(tv)), ob(tp).context(ob(tv)),
+                                     ob(tp, torch.float64).context(ob(tv, torch.float64)), "ragged context %d x %d, K %d" % (Lx, K, Ly))
+    ten = [gb(tx).dot_product(gb(ty)).lw for _ in range(10)]
+    assert all(torch.equal(ten[0], t) for t in ten)
+
+
+@pytest.mark.parametrize("Di,Do,words", [(64, 5, 1), (128, 16, 2), (256, 12, 2), (128, 31, 1), (64, 32, 1), (48, 33, 1), (128, 64, 1)])
+@pytest.mark.parametrize("p", [1.0, 2.0, float("inf")])
+def test_fused_softmax_of_any_length(Di, Do, words, p):
+    """Tiles of 16, 32 and 64 columns, rows of any length, in registers where the rows split evenly and in shared memory
+    otherwise; the returned range equals a concretisation of the result."""
+    import faith_b200
+    from faith_b200 import ops
+    t = cases.rand_bounds(1501, 2, 3, Di, Do, -0.5, 0.2)
+    g = faith_b200.BoundsLite(p, 0.02, *[v.to(DEV) for v in t], perturbed_words=words)
+    z = ops.softmax_fused(g._t4(), p, 0.02, words, ranges=True)
+    assert z is not None
+    o = O.OBounds(p, 0.02, *t, words=words).softmax()
+    for a, k in zip(z, ("lw", "uw", "lb", "ub")):
+        helpers.assert_close(a, getattr(o, k), "softmax %s of %d" % (k, Do), atol=2e-6)
+    l, u = ops.concretize(*z[:4], p, 0.02, words)
+    helpers.assert_close(z[4], l.cpu(), "range l")
+    helpers.assert_close(z[5], u.cpu(), "range u")
+
+
+@pytest.mark.parametrize("L,words", [(21, 2), (35, 1)])
+def test_encoder_of_a_length_that_is_not_a_multiple_of_four(L, words):
+    """The driver keeps scores and probabilities of such lengths with padded rows; same bounds as the CUDA-core route of the
+    oracle within the fp32 noise."""
+    import faith_b200
+    model = O.make_encoder(7, layers=2, d_model=128, heads=4, ffn=512)
+    emb = torch.randn(3, L, 128, generator=torch.Generator().manual_seed(8))
+    pos, p, eps = [1, 4][:words], float("inf"), 1e-3
+    l32, u32 = O.encoder_forward(model, emb, pos, p, eps)
+    l64, u64 = O.encoder_forward(O.model_to(model, torch.float64), emb.double(), pos, p, eps)
+    l, u, viol = faith_b200.EncoderVerifier(model, DEV).forward(emb.to(DEV), pos, p, eps)
+    assert int(viol.item()) == 0
+    helpers.assert_within_noise(l, l32, l64, "l")
+    helpers.assert_within_noise(u, u32, u64, "u")
