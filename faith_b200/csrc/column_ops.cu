@@ -9,6 +9,8 @@
 // Transposed layout [rows, Do, Di] (the reference's pybind layout): one warp per column.
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace fb {
@@ -17,7 +19,6 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kCW = 32;  // columns per block tile
 
-constexpr int OP_CONCRETIZE = -1;
 constexpr int OP_COEF_ONLY = 16;   // added to a relaxation op: write the column coefficients instead of rescaling
 
 // ---------------------------------------------------------------------------
@@ -202,13 +203,6 @@ col_relax_native(int op, const float* __restrict__ lw, const float* __restrict__
   }
   float l, u;
   tile_concretize<VEC, STAGED>(gl, gu, Di, Do, c0, words, p, eps, s_l, s_u, s_red, lbv, ubv, l, u);
-  if (op == OP_CONCRETIZE) {
-    if (mine) {
-      o_lb[(size_t)row * Do + c0 + tid] = l;
-      o_ub[(size_t)row * Do + c0 + tid] = u;
-    }
-    return;
-  }
   if (op >= OP_COEF_ONLY) {
     // coefficients only: o_lw / o_uw are [rows, Do] arrays that receive the own-side slopes; a column
     // with a cross term (possible only for an inverted range l > u) raises bit 1 of the flag
@@ -492,25 +486,17 @@ col_relax_apply_native(int op, const float* __restrict__ lw, const float* __rest
 }
 
 // ------------------------------------------------------------ transposed layout
-// [rows, Do, Di]: the Di values of a column are contiguous; one warp per column, two passes
-// (the second is served by L1/L2, a column is at most a few KB).
+// [rows, Do, Di]: the Di values of a column are contiguous; one warp per column.
+// Concretised range of a column; every lane returns it.
 template <int VEC>
-__global__ void __launch_bounds__(kThreads)
-col_relax_transposed(int op, const float* __restrict__ lw, const float* __restrict__ uw,
-                     const float* __restrict__ lb, const float* __restrict__ ub,
-                     float* __restrict__ o_lw, float* __restrict__ o_uw, float* __restrict__ o_lb,
-                     float* __restrict__ o_ub, int64_t ncols, int Di, int words, int p, float eps,
-                     int* __restrict__ violation) {
+__device__ __forceinline__ void transposed_concretize(const float* __restrict__ gl, const float* __restrict__ gu, int Di, int words,
+                                                      int p, float eps, float lbv, float ubv, float& l, float& u) {
   const int lane = threadIdx.x & 31;
-  const int64_t col = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
-  if (col >= ncols) return;
-  const float* gl = lw + (size_t)col * Di;
-  const float* gu = uw + (size_t)col * Di;
   const int blk = Di / words;
-  const float lbv = lb[col], ubv = ub[col];
-  float l = lbv, u = ubv;
+  l = lbv, u = ubv;
   for (int w = 0; w < words; ++w) {
     float al = 0.f, au = 0.f;
+#pragma unroll 2
     for (int r = w * blk + lane * VEC; r < (w + 1) * blk; r += 32 * VEC) {
       if (VEC == 4) {
         const float4 a = __ldg(reinterpret_cast<const float4*>(gl + r));
@@ -530,9 +516,52 @@ col_relax_transposed(int op, const float* __restrict__ lw, const float* __restri
     l = fadd(l, fmul(-eps, norm_finish(p, al)));
     u = fadd(u, fmul(eps, norm_finish(p, au)));
   }
-  if (op == OP_CONCRETIZE) {
-    if (lane == 0) { o_lb[col] = l; o_ub[col] = u; }
-    return;
+}
+
+// HELD > 0: one word and Di <= 128 * HELD, so that a lane keeps its HELD vectors of either line in registers from the norm to
+// the rescale (all its loads in flight at once, no second read); otherwise two passes, the second served by L1 / L2.
+// [128, 256, 512]: 51 us in two passes, 41.7 us held (6.4 TB/s).
+template <int VEC, int HELD>
+__global__ void __launch_bounds__(kThreads)
+col_relax_transposed(int op, const float* __restrict__ lw, const float* __restrict__ uw,
+                     const float* __restrict__ lb, const float* __restrict__ ub,
+                     float* __restrict__ o_lw, float* __restrict__ o_uw, float* __restrict__ o_lb,
+                     float* __restrict__ o_ub, int64_t ncols, int Di, int words, int p, float eps,
+                     int* __restrict__ violation) {
+  const int lane = threadIdx.x & 31;
+  const int64_t col = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+  if (col >= ncols) return;
+  const float* gl = lw + (size_t)col * Di;
+  const float* gu = uw + (size_t)col * Di;
+  const float lbv = lb[col], ubv = ub[col];
+  constexpr int N = HELD > 0 ? HELD : 1;
+  float4 va[N], vb[N];
+  float l, u;
+  if (HELD > 0) {
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+      const int r = (t * 32 + lane) * 4;
+      va[t] = vb[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r < Di) {
+        va[t] = __ldg(reinterpret_cast<const float4*>(gl + r));
+        vb[t] = __ldg(reinterpret_cast<const float4*>(gu + r));
+      }
+    }
+    float al = 0.f, au = 0.f;   // (a zero leaves every norm as it is)
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+      al = norm_accum(p, norm_accum(p, norm_accum(p, norm_accum(p, al, va[t].x), va[t].y), va[t].z), va[t].w);
+      au = norm_accum(p, norm_accum(p, norm_accum(p, norm_accum(p, au, vb[t].x), vb[t].y), vb[t].z), vb[t].w);
+    }
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+      al = norm_combine(p, al, __shfl_xor_sync(0xffffffffu, al, s));
+      au = norm_combine(p, au, __shfl_xor_sync(0xffffffffu, au, s));
+    }
+    l = fadd(lbv, fmul(-eps, norm_finish(p, al)));
+    u = fadd(ubv, fmul(eps, norm_finish(p, au)));
+  } else {
+    transposed_concretize<VEC>(gl, gu, Di, words, p, eps, lbv, ubv, l, u);
   }
   bool bad = false;
   const ColCoef c = relax_column(op, l, u, lbv, ubv, bad);  // every lane computes the same scalars
@@ -543,23 +572,101 @@ col_relax_transposed(int op, const float* __restrict__ lw, const float* __restri
   }
   float* ol = o_lw + (size_t)col * Di;
   float* ou = o_uw + (size_t)col * Di;
+  auto rescale4 = [&](const float4 a, const float4 b, int r) {
+    float4 x, y;
+    x.x = fmaf(c.c_ll, a.x, fmul(c.c_lu, b.x)); y.x = fmaf(c.c_uu, b.x, fmul(c.c_ul, a.x));
+    x.y = fmaf(c.c_ll, a.y, fmul(c.c_lu, b.y)); y.y = fmaf(c.c_uu, b.y, fmul(c.c_ul, a.y));
+    x.z = fmaf(c.c_ll, a.z, fmul(c.c_lu, b.z)); y.z = fmaf(c.c_uu, b.z, fmul(c.c_ul, a.z));
+    x.w = fmaf(c.c_ll, a.w, fmul(c.c_lu, b.w)); y.w = fmaf(c.c_uu, b.w, fmul(c.c_ul, a.w));
+    *reinterpret_cast<float4*>(ol + r) = x;
+    *reinterpret_cast<float4*>(ou + r) = y;
+  };
+  if (HELD > 0) {
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+      const int r = (t * 32 + lane) * 4;
+      if (r < Di) rescale4(va[t], vb[t], r);
+    }
+    return;
+  }
   for (int r = lane * VEC; r < Di; r += 32 * VEC) {
     if (VEC == 4) {
-      const float4 a = __ldg(reinterpret_cast<const float4*>(gl + r));
-      const float4 b = __ldg(reinterpret_cast<const float4*>(gu + r));
-      float4 x, y;
-      x.x = fmaf(c.c_ll, a.x, fmul(c.c_lu, b.x)); y.x = fmaf(c.c_uu, b.x, fmul(c.c_ul, a.x));
-      x.y = fmaf(c.c_ll, a.y, fmul(c.c_lu, b.y)); y.y = fmaf(c.c_uu, b.y, fmul(c.c_ul, a.y));
-      x.z = fmaf(c.c_ll, a.z, fmul(c.c_lu, b.z)); y.z = fmaf(c.c_uu, b.z, fmul(c.c_ul, a.z));
-      x.w = fmaf(c.c_ll, a.w, fmul(c.c_lu, b.w)); y.w = fmaf(c.c_uu, b.w, fmul(c.c_ul, a.w));
-      *reinterpret_cast<float4*>(ol + r) = x;
-      *reinterpret_cast<float4*>(ou + r) = y;
+      rescale4(__ldg(reinterpret_cast<const float4*>(gl + r)), __ldg(reinterpret_cast<const float4*>(gu + r)), r);
     } else {
       const float a = __ldg(gl + r), b = __ldg(gu + r);
       ol[r] = fmaf(c.c_ll, a, fmul(c.c_lu, b));
       ou[r] = fmaf(c.c_uu, b, fmul(c.c_ul, a));
     }
   }
+}
+
+// Concretisation alone, of one bound or of two (the operands of a product) in one launch: blocks below `n_first` take the
+// first, the others the second.
+struct ConcretizeOne {
+  const float *lw, *uw, *lb, *ub;
+  float *l, *u;
+  int64_t rows;
+  int Do, ntiles;
+};
+
+template <int VEC>
+__global__ void __launch_bounds__(kThreads)
+concretize_native(const ConcretizeOne first, const ConcretizeOne second, int64_t n_first, int Di, int words, int p, float eps) {
+  __shared__ float s_red[2 * 8 * kCW];
+  const bool is_first = blockIdx.x < n_first;
+  const ConcretizeOne& q = is_first ? first : second;
+  const int64_t blk = is_first ? blockIdx.x : blockIdx.x - n_first;
+  const int64_t row = blk / q.ntiles;
+  const int c0 = (int)(blk % q.ntiles) * kCW;
+  const int tid = threadIdx.x;
+  const bool mine = tid < kCW && c0 + tid < q.Do;
+  const size_t o = (size_t)row * q.Do + c0 + tid;
+  float lbv = 0.f, ubv = 0.f, l, u;
+  if (mine) {
+    lbv = q.lb[o];
+    ubv = q.ub[o];
+  }
+  const size_t w = (size_t)row * Di * q.Do;
+  tile_concretize<VEC, false>(q.lw + w, q.uw + w, Di, q.Do, c0, words, p, eps, nullptr, nullptr, s_red, lbv, ubv, l, u);
+  if (mine) {
+    q.l[o] = l;
+    q.u[o] = u;
+  }
+}
+
+template <int VEC>
+__global__ void __launch_bounds__(kThreads)
+concretize_transposed(const ConcretizeOne first, const ConcretizeOne second, int64_t n_first, int Di, int words, int p, float eps) {
+  const bool is_first = blockIdx.x < n_first;
+  const ConcretizeOne& q = is_first ? first : second;
+  const int64_t col = (is_first ? blockIdx.x : blockIdx.x - n_first) * (kThreads / 32) + (threadIdx.x >> 5);
+  if (col >= q.rows * q.Do) return;
+  float l, u;
+  transposed_concretize<VEC>(q.lw + (size_t)col * Di, q.uw + (size_t)col * Di, Di, words, p, eps, q.lb[col], q.ub[col], l, u);
+  if ((threadIdx.x & 31) == 0) {
+    q.l[col] = l;
+    q.u[col] = u;
+  }
+}
+
+int launch_concretize(ConcretizeOne first, ConcretizeOne second, int Di, int words, int p, float eps, int layout, cudaStream_t st) {
+  bool vec = aligned16(first.lw) && aligned16(first.uw) && (second.rows == 0 || (aligned16(second.lw) && aligned16(second.uw)));
+  if (layout == FB_TRANSPOSED) {
+    vec = vec && (Di / words) % 4 == 0;
+    const int64_t n1 = ceil_div(first.rows * first.Do, kThreads / 32), blocks = n1 + ceil_div(second.rows * second.Do, kThreads / 32);
+    if (blocks > 0x7fffffff) return FB_ERR_SHAPE;
+    (vec ? concretize_transposed<4> : concretize_transposed<1>)<<<(unsigned)blocks, kThreads, 0, st>>>(first, second, n1, Di, words, p,
+                                                                                                     eps);
+  } else {
+    vec = vec && first.Do % 4 == 0 && (second.rows == 0 || second.Do % 4 == 0);
+    first.ntiles = (int)ceil_div(first.Do, kCW);
+    second.ntiles = std::max(1, (int)ceil_div(second.Do, kCW));
+    const int64_t n1 = first.rows * first.ntiles, blocks = n1 + second.rows * second.ntiles;
+    if (blocks > 0x7fffffff) return FB_ERR_SHAPE;
+    (vec ? concretize_native<4> : concretize_native<1>)<<<(unsigned)blocks, kThreads, 0, st>>>(first, second, n1, Di, words, p, eps);
+  }
+  FB_LAUNCH_OK();
+  return FB_OK;
 }
 
 size_t relax_smem_bytes(int Di, bool staged, int tiles) {
@@ -579,14 +686,12 @@ int launch_relax(int op, const float* lw, const float* uw, const float* lb, cons
     const int64_t ncols = rows * Do;
     const int64_t blocks = ceil_div(ncols, kThreads / 32);
     if (blocks > 0x7fffffff) return FB_ERR_SHAPE;
-    const bool vec = (Di / words) % 4 == 0 && aligned16(lw) && aligned16(uw) &&
-                     (op == OP_CONCRETIZE || (aligned16(o_lw) && aligned16(o_uw)));
-    if (vec)
-      col_relax_transposed<4><<<(unsigned)blocks, kThreads, 0, st>>>(op, lw, uw, lb, ub, o_lw, o_uw, o_lb, o_ub,
-                                                                      ncols, Di, words, p, eps, violation);
-    else
-      col_relax_transposed<1><<<(unsigned)blocks, kThreads, 0, st>>>(op, lw, uw, lb, ub, o_lw, o_uw, o_lb, o_ub,
-                                                                      ncols, Di, words, p, eps, violation);
+    const bool vec = (Di / words) % 4 == 0 && aligned16(lw) && aligned16(uw) && aligned16(o_lw) && aligned16(o_uw);
+    // 4 vectors of either line per lane are 32 registers; a longer column is read twice
+    const bool held = vec && words == 1 && Di <= 512;
+    auto kern = !vec ? col_relax_transposed<1, 0> : !held ? col_relax_transposed<4, 0> : Di <= 128 ? col_relax_transposed<4, 1>
+                : Di <= 256 ? col_relax_transposed<4, 2> : col_relax_transposed<4, 4>;
+    kern<<<(unsigned)blocks, kThreads, 0, st>>>(op, lw, uw, lb, ub, o_lw, o_uw, o_lb, o_ub, ncols, Di, words, p, eps, violation);
     FB_LAUNCH_OK();
     return FB_OK;
   }
@@ -594,13 +699,13 @@ int launch_relax(int op, const float* lw, const float* uw, const float* lb, cons
   const int64_t blocks = rows * ntiles;
   if (blocks > 0x7fffffff) return FB_ERR_SHAPE;
   const bool vec = Do % 4 == 0 && aligned16(lw) && aligned16(uw) &&
-                   (op == OP_CONCRETIZE || op >= OP_COEF_ONLY || (aligned16(o_lw) && aligned16(o_uw)));
-  // Keep the tile in shared memory when a few blocks per SM still fit; concretise alone and the
-  // coefficient-only mode have no second pass and never stage.
+                   (op >= OP_COEF_ONLY || (aligned16(o_lw) && aligned16(o_uw)));
+  // Keep the tile in shared memory when a few blocks per SM still fit; the coefficient-only mode has no second pass and never
+  // stages.
   const size_t staged_bytes = relax_smem_bytes(Di, true, 2);
   // (40 KB: dim_in up to 128 + the scratch.  A 64 KB tile, dim_in 256, leaves three blocks per SM and was slower staged than
   // re-read through L2: tanh on [8, 64, 256, 256] 0.172 ms staged, 0.137 ms not, 0.48 -> 0.60 of the HBM roof.)
-  const bool staged = op != OP_CONCRETIZE && op < OP_COEF_ONLY && staged_bytes <= 40 * 1024;
+  const bool staged = op < OP_COEF_ONLY && staged_bytes <= 40 * 1024;
   const size_t smem = staged ? staged_bytes : relax_smem_bytes(Di, false, 2);
 #define FB_RELAX_LAUNCH(V, S)                                                                              \
   do {                                                                                                     \
@@ -652,8 +757,17 @@ extern "C" int fb_concretize_f32(const float* lw, const float* uw, const float* 
   if (Di % words != 0) return FB_ERR_SHAPE;
   const double mw = (double)rows * Di * Do, mb = (double)rows * Do;
   ProfileScope prof(PK_RELAX, 4.0 * mw, 4.0 * (2 * mw + 4 * mb), stream);
-  return launch_relax(OP_CONCRETIZE, lw, uw, lb, ub, nullptr, nullptr, l, u, rows, Di, Do, words, p, eps, layout,
-                      nullptr, (cudaStream_t)stream);
+  return launch_concretize({lw, uw, lb, ub, l, u, rows, Do, 0}, {}, Di, words, p, eps, layout, (cudaStream_t)stream);
+}
+
+// (the callers have checked the arguments; both bounds have rows)
+int fb::concretize_pair(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub, float* x_l, float* x_u,
+                        int64_t x_rows, int x_do, const float* y_lw, const float* y_uw, const float* y_lb, const float* y_ub, float* y_l,
+                        float* y_u, int64_t y_rows, int y_do, int Di, int words, int p, float eps, int layout, cudaStream_t st) {
+  const double mw = ((double)x_rows * x_do + (double)y_rows * y_do) * Di, mb = (double)x_rows * x_do + (double)y_rows * y_do;
+  ProfileScope prof(PK_RELAX, 4.0 * mw, 4.0 * (2 * mw + 4 * mb), (void*)st);
+  return launch_concretize({x_lw, x_uw, x_lb, x_ub, x_l, x_u, x_rows, x_do, 0}, {y_lw, y_uw, y_lb, y_ub, y_l, y_u, y_rows, y_do, 0}, Di,
+                           words, p, eps, layout, st);
 }
 
 extern "C" int fb_relax_f32(int op, const float* lw, const float* uw, const float* lb, const float* ub,

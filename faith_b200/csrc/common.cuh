@@ -83,6 +83,11 @@ int layernorm_novar_rowsum(const float* x_lw, const float* x_uw, const float* x_
                            float* z_lw, float* z_uw, float* z_lb, float* z_ub, int64_t rows, int Di, int Do, float* rowsum,
                            void* stream);
 
+// column_ops.cu: the concretised ranges of two bounds over the same dim_in in one launch.
+int concretize_pair(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub, float* x_l, float* x_u, int64_t x_rows,
+                    int x_do, const float* y_lw, const float* y_uw, const float* y_lb, const float* y_ub, float* y_l, float* y_u,
+                    int64_t y_rows, int y_do, int Di, int words, int p, float eps, int layout, cudaStream_t st);
+
 // softmax.cu: fb_softmax_ranges_f32 with rows `ld` floats apart.
 int softmax_ex(const float* lw, const float* uw, const float* lb, const float* ub, float* out_lw, float* out_uw, float* out_lb,
                float* out_ub, float* out_l, float* out_u, int64_t rows, int Di, int Do, int ld, int words, int p, float eps,
@@ -134,6 +139,23 @@ __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b)
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdiv_rn(a, b); }
+
+// Two FP32 multiply-adds per instruction (fma.rn.f32x2), lanes in a 64-bit register pair.
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 d;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(v));
+  return d;
+}
 
 constexpr float kGuard = 1e-12f;  // additive guard of every chord slope (Bounds.py:27)
 

@@ -11,8 +11,8 @@
 // against the ranges of y, the last two a GEMM of y against the ranges of x whose result lands
 // transposed; both are fused here so that x and y are read once per tile and z is written once.
 //
-// Three launches: concretise x, concretise y (column kernels), then one kernel for the bias
-// part and one for the weight part.
+// Launches: one that concretises both operands, then one kernel for the bias part and one for the weight part (a single one
+// for both in the transposed layout).
 #include <mutex>
 
 #include <cstdlib>
@@ -78,50 +78,72 @@ dot_bias_kernel(const float* __restrict__ x_lb, const float* __restrict__ x_ub, 
 }
 
 // Tiled version of the bias part: one block per (b, RI i, 32 j) tile; the seven row tiles are staged in shared memory (row
-// stride 33 floats: conflict-free both for the row-wise fill and for the column-wise reads), K in chunks of 32; a thread owns
-// the outputs (warp + 8 c, lane), c = 0 .. RI / 8 - 1.  Same partial sums and the same final order of additions as
-// dot_bias_kernel.  RI = 8 where 32-row tiles would leave SMs idle: the kernel is bound by the latency of one chunk, and four
-// blocks of 32 rows (one sentence, four heads) took 7.5 us.
+// stride 33 floats: conflict-free both for the row-wise fill and for the column-wise reads), K in chunks of 32 whose global
+// loads are issued before the arithmetic of the chunk before; a thread owns the outputs (warp + 8 c, lane),
+// c = 0 .. RI / 8 - 1.  Same partial sums and the same final order of additions as dot_bias_kernel.  RI = 8 where 32-row
+// tiles would leave SMs idle: the kernel is bound by the latency of one chunk, and four blocks of 32 rows (one sentence, four
+// heads) took 7.5 us.
 // y_kmajor: y_lb / y_ub are stored [b, k, j] instead of [b, j, k]; ranges_kmajor: y_l / y_u likewise.
+struct DotBias {
+  const float *x_lb, *x_ub, *y_lb, *y_ub, *x_l, *y_l, *y_u;
+  float *z_lb, *z_ub;
+  int Lx, Ly, K, n_it, n_jt, heads, y_kmajor, ranges_kmajor;
+  float out_scale;
+};
+__host__ __device__ constexpr int dot_bias_smem_floats(int ri) { return (3 * ri + 4 * 32) * 33; }
+
 template <int RI>
-__global__ void __launch_bounds__(kThreads)
-dot_bias_tiled(const float* __restrict__ x_lb, const float* __restrict__ x_ub, const float* __restrict__ y_lb,
-               const float* __restrict__ y_ub, const float* __restrict__ x_l, const float* __restrict__ y_l,
-               const float* __restrict__ y_u, float* __restrict__ z_lb, float* __restrict__ z_ub,
-               int Lx, int Ly, int K, int n_it, int n_jt, float out_scale, int heads, int y_kmajor, int ranges_kmajor) {
+__device__ __forceinline__ void dot_bias_tile(const DotBias& q, int w, float* smem) {
   constexpr int C = RI / 8;
-  __shared__ float sx[3][RI][33];   // x_lb, x_ub, x_l
-  __shared__ float sy[4][32][33];   // y_lb, y_ub, y_l, y_u
-  int w = blockIdx.x;
-  const int jt = w % n_jt; w /= n_jt;
-  const int it = w % n_it;
-  const int64_t b = w / n_it;
+  float (*sx)[RI][33] = reinterpret_cast<float (*)[RI][33]>(smem);                  // x_lb, x_ub, x_l
+  float (*sy)[32][33] = reinterpret_cast<float (*)[32][33]>(smem + 3 * RI * 33);    // y_lb, y_ub, y_l, y_u
+  const int jt = w % q.n_jt; w /= q.n_jt;
+  const int it = w % q.n_it;
+  const int64_t b = w / q.n_it;
   const int i0 = it * RI, j0 = jt * 32;
   const int tid = threadIdx.x, warp = tid >> 5, j = tid & 31;
   float gl[C], gu[C], l1[C], l2[C], l3[C], l4[C], u1[C], u2[C], u3[C], u4[C];
 #pragma unroll
   for (int c = 0; c < C; ++c) gl[c] = gu[c] = l1[c] = l2[c] = l3[c] = l4[c] = u1[c] = u2[c] = u3[c] = u4[c] = 0.f;
-  for (int k0 = 0; k0 < K; k0 += 32) {
-    const float* const xs[3] = {x_lb, x_ub, x_l};
-    const float* const ys[4] = {y_lb, y_ub, y_l, y_u};
+  float vx[3][C], vy[4][4];
+  auto load = [&](int k0) {
+    const float* const xs[3] = {q.x_lb, q.x_ub, q.x_l};
+    const float* const ys[4] = {q.y_lb, q.y_ub, q.y_l, q.y_u};
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
-      for (int f = tid; f < RI * 32; f += kThreads) {
-        const int r = f >> 5, k = f & 31;
-        sx[a][r][k] = (i0 + r < Lx && k0 + k < K) ? xs[a][((int64_t)b * Lx + i0 + r) * K + k0 + k] : 0.f;
+      for (int c = 0; c < C; ++c) {
+        const int r = warp + 8 * c;
+        vx[a][c] = (i0 + r < q.Lx && k0 + j < q.K) ? xs[a][((int64_t)b * q.Lx + i0 + r) * q.K + k0 + j] : 0.f;
       }
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
-      const bool km = a < 2 ? y_kmajor != 0 : ranges_kmajor != 0;
+      const bool km = a < 2 ? q.y_kmajor != 0 : q.ranges_kmajor != 0;
 #pragma unroll
-      for (int f = tid; f < 32 * 32; f += kThreads) {
-        const int hi = f >> 5, lo = f & 31, r = km ? lo : hi, k = km ? hi : lo;   // the fast index is the contiguous one
-        const int64_t idx = km ? ((int64_t)b * K + k0 + k) * Ly + j0 + r : ((int64_t)b * Ly + j0 + r) * K + k0 + k;
-        sy[a][r][k] = (j0 + r < Ly && k0 + k < K) ? ys[a][idx] : 0.f;
+      for (int c = 0; c < 4; ++c) {
+        const int hi = warp + 8 * c, r = km ? j : hi, k = km ? hi : j;   // the fast index is the contiguous one
+        const int64_t idx = km ? ((int64_t)b * q.K + k0 + k) * q.Ly + j0 + r : ((int64_t)b * q.Ly + j0 + r) * q.K + k0 + k;
+        vy[a][c] = (j0 + r < q.Ly && k0 + k < q.K) ? ys[a][idx] : 0.f;
+      }
+    }
+  };
+  load(0);
+  for (int k0 = 0; k0 < q.K; k0 += 32) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int c = 0; c < C; ++c) sx[a][warp + 8 * c][j] = vx[a][c];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      const bool km = a < 2 ? q.y_kmajor != 0 : q.ranges_kmajor != 0;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int hi = warp + 8 * c;
+        sy[a][km ? j : hi][km ? hi : j] = vy[a][c];
       }
     }
     __syncthreads();
+    if (k0 + 32 < q.K) load(k0 + 32);
 #pragma unroll 4
     for (int k = 0; k < 32; ++k) {
       const float yl = sy[0][j][k], yu = sy[1][j][k], ly = sy[2][j][k], uy = sy[3][j][k];
@@ -139,17 +161,23 @@ dot_bias_tiled(const float* __restrict__ x_lb, const float* __restrict__ x_ub, c
     }
     __syncthreads();
   }
-  if (j0 + j >= Ly) return;
+  if (j0 + j >= q.Ly) return;
 #pragma unroll
   for (int c = 0; c < C; ++c) {
     const int i = i0 + warp + 8 * c;
-    if (i < Lx) {
+    if (i < q.Lx) {
       // heads > 1: head-merged output [S, Lx, heads * Ly]
-      const int64_t od = (((b / heads) * Lx + i) * heads + b % heads) * Ly + j0 + j;
-      z_lb[od] = fmul(fadd(fadd(fadd(fadd(gl[c], l1[c]), l2[c]), l3[c]), l4[c]), out_scale);
-      z_ub[od] = fmul(fadd(fadd(fadd(fadd(gu[c], u1[c]), u2[c]), u3[c]), u4[c]), out_scale);
+      const int64_t od = (((b / q.heads) * q.Lx + i) * q.heads + b % q.heads) * q.Ly + j0 + j;
+      q.z_lb[od] = fmul(fadd(fadd(fadd(fadd(gl[c], l1[c]), l2[c]), l3[c]), l4[c]), q.out_scale);
+      q.z_ub[od] = fmul(fadd(fadd(fadd(fadd(gu[c], u1[c]), u2[c]), u3[c]), u4[c]), q.out_scale);
     }
   }
+}
+
+template <int RI>
+__global__ void __launch_bounds__(kThreads) dot_bias_tiled(const DotBias q) {
+  __shared__ float smem[dot_bias_smem_floats(RI)];
+  dot_bias_tile<RI>(q, blockIdx.x, smem);
 }
 
 // ------------------------------------------------- weight part, native layout
@@ -352,12 +380,13 @@ int launch_dot_bias(const float* x_lb, const float* x_ub, const float* y_lb, con
                     int y_kmajor, int ranges_kmajor, cudaStream_t st) {
   const int n_jt = (int)ceil_div(Ly, 32);
   const int64_t b32 = (int64_t)B * ceil_div(Lx, 32) * n_jt, b8 = (int64_t)B * ceil_div(Lx, 8) * n_jt;
+  DotBias q = {x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u, z_lb, z_ub, Lx, Ly, K, 0, n_jt, heads, y_kmajor, ranges_kmajor, out_scale};
   if (b32 < 2 * (int64_t)device_info().sms && b8 <= 0x7fffffff) {
-    dot_bias_tiled<8><<<(unsigned)b8, kThreads, 0, st>>>(x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u, z_lb, z_ub, Lx, Ly, K, (int)ceil_div(Lx, 8),
-                                                         n_jt, out_scale, heads, y_kmajor, ranges_kmajor);
+    q.n_it = (int)ceil_div(Lx, 8);
+    dot_bias_tiled<8><<<(unsigned)b8, kThreads, 0, st>>>(q);
   } else if (b32 <= 0x7fffffff) {
-    dot_bias_tiled<32><<<(unsigned)b32, kThreads, 0, st>>>(x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u, z_lb, z_ub, Lx, Ly, K,
-                                                           (int)ceil_div(Lx, 32), n_jt, out_scale, heads, y_kmajor, ranges_kmajor);
+    q.n_it = (int)ceil_div(Lx, 32);
+    dot_bias_tiled<32><<<(unsigned)b32, kThreads, 0, st>>>(q);
   } else {
     if (y_kmajor || ranges_kmajor) return FB_ERR_SHAPE;
     const int64_t total = (int64_t)B * Lx * Ly;
@@ -370,87 +399,7 @@ int launch_dot_bias(const float* x_lb, const float* x_ub, const float* y_lb, con
   return FB_OK;
 }
 
-// --------------------------------------------- weight part, transposed layout
-// x [B, Lx, K, Di], y [B, Ly, K, Di] -> z [B, Lx, Ly, Di]   (Di contiguous).
-// One thread per symbolic coordinate m (coalesced along Di), 4 x 4 (i, j) outputs per thread;
-// the operand ranges of the tile live in shared memory and are broadcast.
-constexpr int TTI = 4, TTJ = 4, TTK = 128, TThreads = 128;
-
-__global__ void __launch_bounds__(TThreads)
-dot_weight_transposed(const float* __restrict__ x_lw, const float* __restrict__ x_uw, const float* __restrict__ y_lw,
-                      const float* __restrict__ y_uw, const float* __restrict__ x_l, const float* __restrict__ y_l,
-                      const float* __restrict__ y_u, float* __restrict__ z_lw, float* __restrict__ z_uw,
-                      int Lx, int Ly, int Di, int K, int n_it, int n_jt, float out_scale) {
-  __shared__ float s_lx[TTI][TTK], s_ly[TTJ][TTK], s_uy[TTJ][TTK];
-  int64_t bid = blockIdx.x;
-  const int jt = (int)(bid % n_jt); bid /= n_jt;
-  const int it = (int)(bid % n_it); bid /= n_it;
-  const int64_t b = bid;
-  const int i0 = it * TTI, j0 = jt * TTJ;
-  const int m = blockIdx.y * TThreads + threadIdx.x;
-  const bool m_ok = m < Di;
-  float acc_l[TTI][TTJ], acc_u[TTI][TTJ];
-#pragma unroll
-  for (int a = 0; a < TTI; ++a)
-#pragma unroll
-    for (int c = 0; c < TTJ; ++c) { acc_l[a][c] = 0.f; acc_u[a][c] = 0.f; }
-  for (int k0 = 0; k0 < K; k0 += TTK) {
-    const int nk = min(TTK, K - k0);
-    for (int f = threadIdx.x; f < TTI * TTK; f += TThreads) {
-      const int r = f / TTK, k = f % TTK;
-      const bool kin = k < nk;
-      s_lx[r][k] = (kin && i0 + r < Lx) ? x_l[(b * Lx + i0 + r) * (int64_t)K + k0 + k] : 0.f;
-      s_ly[r][k] = (kin && j0 + r < Ly) ? y_l[(b * Ly + j0 + r) * (int64_t)K + k0 + k] : 0.f;
-      s_uy[r][k] = (kin && j0 + r < Ly) ? y_u[(b * Ly + j0 + r) * (int64_t)K + k0 + k] : 0.f;
-    }
-    __syncthreads();
-    if (m_ok) {
-      for (int k = 0; k < nk; ++k) {
-        float xl[TTI], xu[TTI], yl[TTJ], yu[TTJ];
-#pragma unroll
-        for (int a = 0; a < TTI; ++a) {
-          const bool ok = i0 + a < Lx;
-          const int64_t o = ((b * Lx + i0 + a) * (int64_t)K + k0 + k) * Di + m;
-          xl[a] = ok ? __ldg(x_lw + o) : 0.f;
-          xu[a] = ok ? __ldg(x_uw + o) : 0.f;
-        }
-#pragma unroll
-        for (int c = 0; c < TTJ; ++c) {
-          const bool ok = j0 + c < Ly;
-          const int64_t o = ((b * Ly + j0 + c) * (int64_t)K + k0 + k) * Di + m;
-          yl[c] = ok ? __ldg(y_lw + o) : 0.f;
-          yu[c] = ok ? __ldg(y_uw + o) : 0.f;
-        }
-#pragma unroll
-        for (int a = 0; a < TTI; ++a) {
-          const float lx = s_lx[a][k];
-          const float lxp = fmaxf(lx, 0.f), lxn = fminf(lx, 0.f);
-#pragma unroll
-          for (int c = 0; c < TTJ; ++c) {
-            const float ly = s_ly[c][k], uy = s_uy[c][k];
-            float l = acc_l[a][c], u = acc_u[a][c];
-            l = fmaf(xl[a], fmaxf(ly, 0.f), l); l = fmaf(xu[a], fminf(ly, 0.f), l);
-            l = fmaf(yl[c], lxp, l);            l = fmaf(yu[c], lxn, l);
-            u = fmaf(xu[a], fmaxf(uy, 0.f), u); u = fmaf(xl[a], fminf(uy, 0.f), u);
-            u = fmaf(yu[c], lxp, u);            u = fmaf(yl[c], lxn, u);
-            acc_l[a][c] = l; acc_u[a][c] = u;
-          }
-        }
-      }
-    }
-    __syncthreads();
-  }
-  if (!m_ok) return;
-#pragma unroll
-  for (int a = 0; a < TTI; ++a)
-#pragma unroll
-    for (int c = 0; c < TTJ; ++c)
-      if (i0 + a < Lx && j0 + c < Ly) {
-        const int64_t o = ((b * Lx + i0 + a) * (int64_t)Ly + j0 + c) * Di + m;
-        z_lw[o] = fmul(acc_l[a][c], out_scale);
-        z_uw[o] = fmul(acc_u[a][c], out_scale);
-      }
-}
+#include "dot_product_transposed.cuh"
 
 }  // namespace
 }  // namespace fb
@@ -513,10 +462,19 @@ int fb::dot_product_ex(const float* x_lw, const float* x_uw, const float* x_lb, 
   ProfileScope prof(PK_DOT, 16.0 * B * Lx * Ly * d1 * K,
                     4.0 * (2.0 * B * Lx * d1 * K + 2.0 * B * Ly * d1 * K + 2.0 * B * Lx * Ly * d1), stream);
   int rc = FB_OK;
-  if (!(given & 1)) rc = fb_concretize_f32(x_lw, x_uw, x_lb, x_ub, x_l, x_u, (int64_t)B * Lx, Di, K, words, p, eps, layout, stream);
+  if (given == 0)
+    rc = concretize_pair(x_lw, x_uw, x_lb, x_ub, x_l, x_u, (int64_t)B * Lx, K, y_lw, y_uw, y_lb, y_ub, y_l, y_u, (int64_t)B * Ly, K, Di,
+                         words, p, eps, layout, st);
+  else if (given == 2)
+    rc = fb_concretize_f32(x_lw, x_uw, x_lb, x_ub, x_l, x_u, (int64_t)B * Lx, Di, K, words, p, eps, layout, stream);
+  else if (given == 1)
+    rc = fb_concretize_f32(y_lw, y_uw, y_lb, y_ub, y_l, y_u, (int64_t)B * Ly, Di, K, words, p, eps, layout, stream);
   if (rc != FB_OK) return rc;
-  if (!(given & 2)) rc = fb_concretize_f32(y_lw, y_uw, y_lb, y_ub, y_l, y_u, (int64_t)B * Ly, Di, K, words, p, eps, layout, stream);
-  if (rc != FB_OK) return rc;
+  if (layout == FB_TRANSPOSED && ldz == 0) {
+    const DotBias q = {x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u, z_lb, z_ub, Lx, Ly, K, (int)ceil_div(Lx, 8), (int)ceil_div(Ly, 32), 1, 0, 0,
+                       out_scale};
+    return launch_dot_transposed(x_lw, x_uw, y_lw, y_uw, z_lw, z_uw, q, B, Di, st);
+  }
   rc = launch_dot_bias(x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u, z_lb, z_ub, B, Lx, Ly, K, out_scale, merge_heads, 0, 0, st);
   if (rc != FB_OK) return rc;
   // Tensor-core kernels: the one for the attention shapes with lengths that are multiples of 32 (5.6 TB/s on a large batch,
@@ -530,7 +488,8 @@ int fb::dot_product_ex(const float* x_lw, const float* x_uw, const float* x_lb, 
   if (ldz != 0) return FB_ERR_SHAPE;
   if (layout == FB_NATIVE && Lx <= kFewRows)
     return launch_dot_weight_rows(x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, K, out_scale, merge_heads, 0, st);
-  if (layout == FB_NATIVE) {
+  if (layout != FB_NATIVE) return FB_ERR_SHAPE;
+  {
     const int n_it = (int)ceil_div(Lx, TI), n_jt = (int)ceil_div(Ly, TJ), n_mt = (int)ceil_div(Di, TM);
     const int64_t blocks = (int64_t)B * n_it * n_jt * n_mt;
     if (blocks > 0x7fffffff) return FB_ERR_SHAPE;
@@ -552,13 +511,6 @@ int fb::dot_product_ex(const float* x_lw, const float* x_uw, const float* x_lb, 
       dot_weight_native<false><<<(unsigned)blocks, kThreads, smem, st>>>(x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw,
                                                                          z_uw, Lx, Ly, Di, K, n_it, n_jt, n_mt, out_scale);
     }
-  } else {
-    const int n_it = (int)ceil_div(Lx, TTI), n_jt = (int)ceil_div(Ly, TTJ);
-    const int64_t blocks = (int64_t)B * n_it * n_jt;
-    const int64_t my = ceil_div(Di, TThreads);
-    if (blocks > 0x7fffffff || my > 65535) return FB_ERR_SHAPE;
-    dot_weight_transposed<<<dim3((unsigned)blocks, (unsigned)my), TThreads, 0, st>>>(
-        x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, Lx, Ly, Di, K, n_it, n_jt, out_scale);
   }
   FB_LAUNCH_OK();
   return FB_OK;
@@ -673,10 +625,14 @@ int fb::context_ex(const float* x_lw, const float* x_uw, const float* x_lb, cons
   ProfileScope prof(PK_DOT, 16.0 * B * Lx * Ly * d1 * K,
                     4.0 * (2.0 * B * Lx * d1 * K + 2.0 * B * Ly * d1 * K + 2.0 * B * Lx * Ly * d1), stream);
   int rc = FB_OK;
-  if (!(given & 1)) rc = fb_concretize_f32(x_lw, x_uw, x_lb, x_ub, x_l, x_u, (int64_t)B * Lx, Di, K, words, p, eps, FB_NATIVE, stream);
-  if (rc != FB_OK) return rc;
   // ranges of the values in their own layout [B, K, Ly]
-  if (!(given & 2)) rc = fb_concretize_f32(v_lw, v_uw, v_lb, v_ub, y_l, y_u, (int64_t)B * K, Di, Ly, words, p, eps, FB_NATIVE, stream);
+  if (given == 0)
+    rc = concretize_pair(x_lw, x_uw, x_lb, x_ub, x_l, x_u, (int64_t)B * Lx, K, v_lw, v_uw, v_lb, v_ub, y_l, y_u, (int64_t)B * K, Ly, Di,
+                         words, p, eps, FB_NATIVE, st);
+  else if (given == 2)
+    rc = fb_concretize_f32(x_lw, x_uw, x_lb, x_ub, x_l, x_u, (int64_t)B * Lx, Di, K, words, p, eps, FB_NATIVE, stream);
+  else if (given == 1)
+    rc = fb_concretize_f32(v_lw, v_uw, v_lb, v_ub, y_l, y_u, (int64_t)B * K, Di, Ly, words, p, eps, FB_NATIVE, stream);
   if (rc != FB_OK) return rc;
   const bool transpose = transposed_ranges || !tc || tc32;
   if (transpose) {

@@ -1078,3 +1078,34 @@ def test_encoder_of_a_length_that_is_not_a_multiple_of_four(L, words):
     assert int(viol.item()) == 0
     helpers.assert_within_noise(l, l32, l64, "l")
     helpers.assert_within_noise(u, u32, u64, "u")
+
+
+# (one coordinate past a 64-wide tile, odd dim_in, K past the 128 values staged at a time, a tile of one row, both block
+# shapes)
+@pytest.mark.parametrize("B,Lx,Ly,Di,K", [(1, 1, 3, 2, 1), (1, 5, 9, 65, 130), (2, 9, 4, 66, 7), (4, 33, 31, 128, 33), (2, 40, 48, 250, 150)])
+def test_dot_product_transposed_edges(B, Lx, Ly, Di, K):
+    from faith_b200 import ops
+    from faith_b200._lib import FB_TRANSPOSED
+    tx, ty = cases.rand_bounds(420, B, Lx, Di, K, -0.5, 1.0), cases.rand_bounds(421, B, Ly, Di, K, -0.5, 1.0)
+    o64 = O.OBounds(1.0, 0.1, *[v.double() for v in tx]).dot_product(O.OBounds(1.0, 0.1, *[v.double() for v in ty]))
+    o = O.OBounds(1.0, 0.1, *tx).dot_product(O.OBounds(1.0, 0.1, *ty))
+
+    def dev(t):
+        return t[0].transpose(2, 3).contiguous().to(DEV), t[2].transpose(2, 3).contiguous().to(DEV), t[1].to(DEV), t[3].to(DEV)
+    z = ops.dot_product(dev(tx), dev(ty), 1.0, 0.1, 1, 1.0, FB_TRANSPOSED)
+    for got, name in ((z[0].transpose(2, 3), "lw"), (z[1].transpose(2, 3), "uw"), (z[2], "lb"), (z[3], "ub")):
+        helpers.assert_arbitrated(got, getattr(o, name), getattr(o64, name), "transposed dot %s %s" % (name, (B, Lx, Ly, Di, K)))
+
+
+@pytest.mark.parametrize("Di", [1, 4, 126, 128, 132, 256, 260, 512, 516])
+@pytest.mark.parametrize("p", [1.0, 2.0, float("inf")])
+def test_relax_transposed_columns_held_in_registers(Di, p):
+    from faith_b200 import ops
+    from faith_b200._lib import FB_RELU, FB_TRANSPOSED
+    t = cases.rand_bounds(422, 1, 3, Di, 9, -0.7, 0.2)
+    o = O.OBounds(p, 0.02, *t).relu()
+    lw, lb, uw, ub = t
+    z = ops.relax(FB_RELU, lw.transpose(2, 3).contiguous().to(DEV), uw.transpose(2, 3).contiguous().to(DEV), lb.to(DEV), ub.to(DEV), p,
+                  0.02, 1, FB_TRANSPOSED)
+    helpers.assert_close(z[0].transpose(2, 3), o.lw, "lw"); helpers.assert_close(z[1].transpose(2, 3), o.uw, "uw")
+    helpers.assert_close(z[2], o.lb, "lb"); helpers.assert_close(z[3], o.ub, "ub")
