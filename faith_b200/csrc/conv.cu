@@ -3,10 +3,7 @@
 // evaluated in centre/radius form like the FFMA GEMM:
 //   c = (x_lw + x_uw)/2, r = (x_uw - x_lw)/2, y_c = conv(c, W), y_r = conv(r, |W|),
 //   y_lw = y_c - y_r, y_uw = y_c + y_r.
-// Direct convolution on CUDA cores: a block owns one image, a TH x TW tile of output pixels
-// (8 x 32, or 16 x 16 for narrow outputs such as the 16 x 16 map of a stride-2 layer) and CO
-// output channels (16 or 32); input channels are staged through shared memory four at a time
-// (centre and radius planes with halo), the weights of the chunk are broadcast from shared memory.
+// Direct convolution on CUDA cores, bound by the FP32 rate (one multiply-add per tap for the centre and one for the radius).
 #include <algorithm>
 #include <cstdint>
 #include "common.cuh"
@@ -15,225 +12,245 @@
 namespace fb {
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int CC = 4;            // input channels per shared-memory stage
-constexpr int kStageBatch = 6;   // input elements per thread whose global loads are in flight together
+// One block: the output channels [chunk * G * CPT, + G * CPT) of a tile of NI images x TH x TW output pixels.  A thread owns
+// PX pixels x CPT channels, a warp of each channel group PX * 32 pixels.  The centre and the radius of a value make one packed
+// multiply-add (fma.rn.f32x2: half the instructions) with a (w, |w|) pair; a tap costs a thread PX 64-bit reads of (centre,
+// radius) pairs and CPT / 2 broadcast 128-bit reads of (w, |w|) pairs, two cycles each, for PX * CPT packed multiply-adds of
+// two cycles on one of four pipes: with 4 x 8 the shared-memory pipe and the arithmetic are level.  CC input channels are
+// staged at a time, by a table of source and destination offsets made once per block; the columns of a stride-2 layer are
+// stored even ones first, so that consecutive pixels read consecutive words.  The tile is cut from the output map at run time
+// (whole rows of narrow maps, several images of small ones): a fixed 16 x 16 or 8 x 32 tile spent up to two thirds of its
+// threads on padding.  Every output accumulates over (input channel, tap row, tap column) in that order, whatever the tile.
+// 384 images, 16 -> 32 channels, 32 x 32, 3 x 3, stride 2: 100 us with one pixel x 32 channels per thread and scalar
+// multiply-adds (and 21 us more for the bias image in a launch of its own), 83 us now; 25 us are arithmetic, the staging alone
+// takes 35 us and overlaps with it only across the four blocks of an SM, and the last of 1.3 rounds of blocks is thin.
+struct ConvArgs {
+  const float *x_lo, *x_up, *b_lo, *b_up;   // n_img images without the bias, then n_bias with it
+  float *y_lo, *y_up, *yb_lo, *yb_up;
+  const float *Wt, *bias;
+  int64_t n_img, n_bias, blocks_bias;
+  int Cin, H, W, Cout, Kh, Kw, stride, pad, Ho, Wo;
+  int TH, TW, NI, tiles_h, tiles_w, chunks, G, CC;
+  int in_h, in_w, pw, row, chan;   // staged tile: rows, columns, columns per phase, pairs per row and per channel
+};
 
-// KS: filter size when it is the same in both directions and known at compile time (3), 0 = taken from the
-// arguments; with KS the tap loops are unrolled and their index arithmetic disappears.
-template <int TH, int TW, int CO, int KS>
-__global__ void __launch_bounds__(kThreads, 2)
-conv_bounds_kernel(const float* __restrict__ x_lo, const float* __restrict__ x_up, const float* __restrict__ Wt,
-                   const float* __restrict__ bias, float* __restrict__ y_lo, float* __restrict__ y_up,
-                   int Cin, int H, int W, int Cout, int Kh_arg, int Kw_arg, int stride, int pad, int Ho, int Wo,
-                   int tiles_h, int tiles_w, int co_chunks) {
-  const int Kh = KS ? KS : Kh_arg, Kw = KS ? KS : Kw_arg;
+constexpr int kConvThreads = 256;   // at most: 8 channel groups
+constexpr int kConvPos = 3, kConvLoads = 4;   // positions x input channels whose loads a thread has in flight together
+
+__device__ __forceinline__ uint64_t lds64(uint32_t a) {
+  uint64_t v;
+  asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void lds128(uint32_t a, uint64_t& v, uint64_t& w) {
+  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(v), "=l"(w) : "r"(a) : "memory");
+}
+
+// KS: filter size when it is the same in both directions and known at compile time (3, 5), 0 = taken from the arguments; with
+// KS the tap loops are unrolled.  ST: 2 = even columns first, 1 = stride 1, 0 = any stride, columns as they are.
+template <int CPT, int PX, int KS, int ST>
+__global__ void __launch_bounds__(kConvThreads)
+conv_bounds_kernel(const ConvArgs q) {
+  static_assert(CPT % 2 == 0 && 32 % CPT == 0, "two channels per read; every thread stages the weights of one channel");
   extern __shared__ __align__(16) float smem[];
-  const int in_h = (TH - 1) * stride + Kh, in_w = (TW - 1) * stride + Kw;
-  const int plane = in_h * in_w;
-  float* s_c = smem;                        // [CC][in_h][in_w]
-  float* s_r = s_c + CC * plane;            // [CC][in_h][in_w]
-  float* s_w = s_r + CC * plane;            // [CC][Kh][Kw][CO]
+  const int Kh = KS ? KS : q.Kh, Kw = KS ? KS : q.Kw, taps = Kh * Kw, co_n = q.G * CPT;
+  float2* s_w = reinterpret_cast<float2*>(smem);            // [CC][Kh][Kw][co_n] (w, |w|)
+  float2* s_x = s_w + q.CC * taps * co_n;                   // [CC][NI][in_h][row] (centre, radius)
+  int2* s_pos = reinterpret_cast<int2*>(s_x + q.CC * q.chan);   // [NI][in_h][in_w] offset in a channel of x (-1: outside), in s_x
+  const int tid = threadIdx.x, nthr = blockDim.x;
 
   int64_t bid = blockIdx.x;
-  const int tw_i = (int)(bid % tiles_w); bid /= tiles_w;
-  const int th_i = (int)(bid % tiles_h); bid /= tiles_h;
-  const int cq = (int)(bid % co_chunks); bid /= co_chunks;
-  const int64_t n = bid;  // image index
-  const int tid = threadIdx.x;
-  const int tw = tid % TW, th = tid / TW;
-  const int oh = th_i * TH + th, ow = tw_i * TW + tw;
-  const int ih0 = th_i * TH * stride - pad, iw0 = tw_i * TW * stride - pad;
-  const int co0 = cq * CO;
+  const bool is_bias = bid < q.blocks_bias;
+  if (!is_bias) bid -= q.blocks_bias;
+  const int tw_i = (int)(bid % q.tiles_w); bid /= q.tiles_w;
+  const int th_i = (int)(bid % q.tiles_h); bid /= q.tiles_h;
+  const int cq = (int)(bid % q.chunks);
+  const int64_t n0 = (bid / q.chunks) * q.NI, n_all = is_bias ? q.n_bias : q.n_img;
+  const int ni = (int)min((int64_t)q.NI, n_all - n0);   // images of this block
+  const int ih0 = th_i * q.TH * q.stride - q.pad, iw0 = tw_i * q.TW * q.stride - q.pad;
+  const int co0 = cq * co_n, g = tid / 32;
+  const int64_t hw = (int64_t)q.H * q.W;
+  const float* x_lo = (is_bias ? q.b_lo : q.x_lo) + n0 * q.Cin * hw;
+  const float* x_up = (is_bias ? q.b_up : q.x_up) + n0 * q.Cin * hw;
 
-  float acc_c[CO], acc_r[CO];
+  const int n_pos = ni * q.in_h * q.in_w;
+  for (int f = tid; f < n_pos; f += nthr) {
+    const int rw = f % q.in_w, rh = (f / q.in_w) % q.in_h, im = f / (q.in_w * q.in_h);
+    const int ih = ih0 + rh, iw = iw0 + rw;
+    const bool in = ih >= 0 && ih < q.H && iw >= 0 && iw < q.W;
+    s_pos[f] = make_int2(in ? (im * q.Cin * q.H + ih) * q.W + iw : -1,
+                         (im * q.in_h + rh) * q.row + (ST == 2 ? (rw & 1) * q.pw + (rw >> 1) : rw));
+  }
+  // this thread's pixels: offset of the window in a staged channel, or the first window for a pixel it does not have
+  int s0[PX];
 #pragma unroll
-  for (int o = 0; o < CO; ++o) { acc_c[o] = 0.f; acc_r[o] = 0.f; }
+  for (int e = 0; e < PX; ++e) {
+    const int t = tid % 32 + e * 32, im = t / (q.TH * q.TW), th = (t / q.TW) % q.TH, tw = t % q.TW;
+    s0[e] = im < ni ? (im * q.in_h + th * q.stride) * q.row + tw * (ST ? 1 : q.stride) : 0;
+  }
+  uint64_t acc[PX][CPT];
+#pragma unroll
+  for (int e = 0; e < PX; ++e)
+#pragma unroll
+    for (int o = 0; o < CPT; ++o) acc[e][o] = 0;
 
-  const float* img_lo = x_lo + n * (int64_t)Cin * H * W;
-  const float* img_up = x_up + n * (int64_t)Cin * H * W;
-  for (int c0 = 0; c0 < Cin; c0 += CC) {
-    // staged in batches of kStageBatch elements per thread: all global loads of a batch are issued before
-    // the first of them is used, so their latencies overlap instead of adding up
-    for (int f0 = tid; f0 < CC * plane; f0 += kThreads * kStageBatch) {
-      float lo[kStageBatch], up[kStageBatch];
-#pragma unroll
-      for (int b = 0; b < kStageBatch; ++b) {
-        const int f = f0 + b * kThreads;
-        const int c = f / plane, rem = f - c * plane;
-        const int rh = rem / in_w;
-        const int ih = ih0 + rh, iw = iw0 + rem - rh * in_w;
-        lo[b] = 0.f;
-        up[b] = 0.f;
-        if (f < CC * plane && c0 + c < Cin && ih >= 0 && ih < H && iw >= 0 && iw < W) {
-          const int64_t o = ((int64_t)(c0 + c) * H + ih) * W + iw;
-          lo[b] = __ldg(img_lo + o);
-          up[b] = __ldg(img_up + o);
-        }
-      }
-#pragma unroll
-      for (int b = 0; b < kStageBatch; ++b) {
-        const int f = f0 + b * kThreads;
-        if (f < CC * plane) {
-          s_c[f] = fmul(fadd(lo[b], up[b]), 0.5f);
-          s_r[f] = fmul(fsub(up[b], lo[b]), 0.5f);
-        }
-      }
+  // weights: 32 / CPT taps at a time, a thread always the same channel
+  const int wo = tid % co_n, wt0 = tid / co_n;
+  const bool w_in = co0 + wo < q.Cout;
+  const float* w_src = q.Wt + (int64_t)(w_in ? co0 + wo : 0) * q.Cin * taps;
+  for (int c0 = 0; c0 < q.Cin; c0 += q.CC) {
+    const int cc = min(q.CC, q.Cin - c0);
+    __syncthreads();
+    const float* xl = x_lo + c0 * hw;
+    const float* xu = x_up + c0 * hw;
+    for (int t = wt0; t < cc * taps; t += 32 / CPT) {   // t = c * taps + tap
+      const float w = w_in ? __ldg(w_src + (int64_t)c0 * taps + t) : 0.f;
+      s_w[t * co_n + wo] = make_float2(w, fabsf(w));
     }
-    for (int f = tid; f < CC * Kh * Kw * CO; f += kThreads) {
-      const int o = f % CO, t = f / CO;
-      const int kw = t % Kw, kh = (t / Kw) % Kh, c = t / (Kw * Kh);
-      float w = 0.f;
-      if (c0 + c < Cin && co0 + o < Cout) w = __ldg(Wt + (((int64_t)(co0 + o) * Cin + c0 + c) * Kh + kh) * Kw + kw);
-      s_w[f] = w;
+    for (int f0 = tid; f0 < n_pos; f0 += kConvPos * nthr) {
+      int2 pos[kConvPos];
+#pragma unroll
+      for (int u = 0; u < kConvPos; ++u) pos[u] = f0 + u * nthr < n_pos ? s_pos[f0 + u * nthr] : make_int2(-1, -1);
+      for (int c = 0; c < cc; c += kConvLoads) {
+        float lo[kConvPos][kConvLoads], up[kConvPos][kConvLoads];
+#pragma unroll
+        for (int u = 0; u < kConvPos; ++u)
+#pragma unroll
+          for (int d = 0; d < kConvLoads; ++d) {
+            const bool ok = pos[u].x >= 0 && c + d < cc;
+            lo[u][d] = ok ? __ldg(xl + pos[u].x + (c + d) * hw) : 0.f;
+            up[u][d] = ok ? __ldg(xu + pos[u].x + (c + d) * hw) : 0.f;
+          }
+#pragma unroll
+        for (int u = 0; u < kConvPos; ++u)
+#pragma unroll
+          for (int d = 0; d < kConvLoads; ++d)
+            if (c + d < cc && pos[u].y >= 0)
+              s_x[pos[u].y + (c + d) * q.chan] = make_float2(fmul(fadd(lo[u][d], up[u][d]), 0.5f), fmul(fsub(up[u][d], lo[u][d]), 0.5f));
+      }
     }
     __syncthreads();
-    const int s0 = th * stride * in_w + tw * stride;   // this thread's window in a staged plane
-#pragma unroll(KS ? CC : 1)
-    for (int c = 0; c < CC; ++c) {
+    // addresses in shared memory by hand: one addition per row, phase and pixel, one per tap for the weights
+    const uint32_t row_b = q.row * 8, chan_b = q.chan * 8, pw_b = ST == 2 ? q.pw * 8 : 0, tap_b = co_n * 8;
+    uint32_t wa = (uint32_t)__cvta_generic_to_shared(s_w + g * CPT);
+    uint32_t xa[PX];
+#pragma unroll
+    for (int e = 0; e < PX; ++e) xa[e] = (uint32_t)__cvta_generic_to_shared(s_x + s0[e]);
+    for (int c = 0; c < cc; ++c) {
 #pragma unroll
       for (int kh = 0; kh < (KS ? KS : Kh); ++kh) {
+        uint32_t x0[PX], x1[PX];
+#pragma unroll
+        for (int e = 0; e < PX; ++e) {
+          x0[e] = xa[e] + kh * row_b;
+          x1[e] = x0[e] + pw_b;
+        }
 #pragma unroll
         for (int kw = 0; kw < (KS ? KS : Kw); ++kw) {
-          const int si = s0 + c * plane + kh * in_w + kw;
-          const float vc = s_c[si], vr = s_r[si];
-          const float* wp = s_w + ((c * Kh + kh) * Kw + kw) * CO;
+          uint64_t w[CPT];
 #pragma unroll
-          for (int o4 = 0; o4 < CO; o4 += 4) {
-            const float4 w = *reinterpret_cast<const float4*>(wp + o4);
-            acc_c[o4 + 0] = fmaf(vc, w.x, acc_c[o4 + 0]); acc_r[o4 + 0] = fmaf(vr, fabsf(w.x), acc_r[o4 + 0]);
-            acc_c[o4 + 1] = fmaf(vc, w.y, acc_c[o4 + 1]); acc_r[o4 + 1] = fmaf(vr, fabsf(w.y), acc_r[o4 + 1]);
-            acc_c[o4 + 2] = fmaf(vc, w.z, acc_c[o4 + 2]); acc_r[o4 + 2] = fmaf(vr, fabsf(w.z), acc_r[o4 + 2]);
-            acc_c[o4 + 3] = fmaf(vc, w.w, acc_c[o4 + 3]); acc_r[o4 + 3] = fmaf(vr, fabsf(w.w), acc_r[o4 + 3]);
+          for (int o = 0; o < CPT; o += 2) lds128(wa + o * 8, w[o], w[o + 1]);
+          wa += tap_b;
+#pragma unroll
+          for (int e = 0; e < PX; ++e) {
+            const uint64_t v = lds64(ST == 2 ? (kw & 1 ? x1[e] : x0[e]) + (kw >> 1) * 8 : x0[e] + kw * 8);
+#pragma unroll
+            for (int o = 0; o < CPT; ++o) acc[e][o] = fma2(v, w[o], acc[e][o]);
           }
         }
       }
-    }
-    __syncthreads();
-  }
-  if (oh >= Ho || ow >= Wo) return;
 #pragma unroll
-  for (int o = 0; o < CO; ++o) {
-    if (co0 + o < Cout) {
-      float lo = fsub(acc_c[o], acc_r[o]), up = fadd(acc_c[o], acc_r[o]);
-      if (bias != nullptr) { lo = fadd(lo, bias[co0 + o]); up = fadd(up, bias[co0 + o]); }
-      const int64_t off = ((n * Cout + co0 + o) * (int64_t)Ho + oh) * Wo + ow;
-      y_lo[off] = lo;
-      y_up[off] = up;
+      for (int e = 0; e < PX; ++e) xa[e] += chan_b;
+    }
+  }
+  float* y_lo = is_bias ? q.yb_lo : q.y_lo;
+  float* y_up = is_bias ? q.yb_up : q.y_up;
+#pragma unroll
+  for (int e = 0; e < PX; ++e) {
+    const int t = tid % 32 + e * 32, im = t / (q.TH * q.TW), oh = th_i * q.TH + (t / q.TW) % q.TH, ow = tw_i * q.TW + t % q.TW;
+    if (im >= ni || oh >= q.Ho || ow >= q.Wo) continue;
+    const int64_t off = (n0 + im) * q.Cout * (int64_t)q.Ho * q.Wo + (int64_t)oh * q.Wo + ow;
+#pragma unroll
+    for (int o = 0; o < CPT; ++o) {
+      const int co = co0 + g * CPT + o;
+      if (co >= q.Cout) break;
+      const float2 v = unpack2(acc[e][o]);
+      float lo = fsub(v.x, v.y), up = fadd(v.x, v.y);
+      if (is_bias && q.bias != nullptr) { lo = fadd(lo, q.bias[co]); up = fadd(up, q.bias[co]); }
+      y_lo[off + (int64_t)co * q.Ho * q.Wo] = lo;
+      y_up[off + (int64_t)co * q.Ho * q.Wo] = up;
     }
   }
 }
 
-// A few images only (the bias part of a bound: one image per batch element): the tiled kernel above would occupy a
-// handful of SMs and run at the latency of its staging loop (51 us for one 16 -> 32 channel image of 32 x 32).  Here a
-// thread owns one output element and accumulates in the same order (input channel, tap row, tap column; taps outside
-// the image are the exact zeros the tiled kernel multiplies), so the value is the tiled kernel's bit for bit.
-// KS: filter size when it is the same in both directions and known at compile time (3), 0 = from the arguments.  With KS
-// every tap is visited (those outside the image with a zero input: fmaf(0, w, acc) leaves the sum as it is), so the tap
-// loops unroll and the loads of a channel are in flight together.
-template <int KS>
-__global__ void __launch_bounds__(128)
-conv_bounds_small_kernel(const float* __restrict__ x_lo, const float* __restrict__ x_up, const float* __restrict__ Wt,
-                         const float* __restrict__ bias, float* __restrict__ y_lo, float* __restrict__ y_up, int64_t total,
-                         int Cin, int H, int W, int Cout, int Kh_arg, int Kw_arg, int stride, int pad, int Ho, int Wo) {
-  const int Kh = KS ? KS : Kh_arg, Kw = KS ? KS : Kw_arg;
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= total) return;
-  const int ow = (int)(t % Wo), oh = (int)((t / Wo) % Ho), co = (int)((t / ((int64_t)Wo * Ho)) % Cout);
-  const int64_t n = t / ((int64_t)Wo * Ho * Cout);
-  const int ih0 = oh * stride - pad, iw0 = ow * stride - pad;
-  const float* il = x_lo + n * (int64_t)Cin * H * W;
-  const float* iu = x_up + n * (int64_t)Cin * H * W;
-  float ac = 0.f, ar = 0.f;
-  if (KS) {
-    for (int c = 0; c < Cin; ++c) {
-      const float* wp = Wt + ((int64_t)co * Cin + c) * KS * KS;
-      float lo[KS ? KS * KS : 1], up[KS ? KS * KS : 1], w[KS ? KS * KS : 1];
-#pragma unroll
-      for (int kh = 0; kh < KS; ++kh)
-#pragma unroll
-        for (int kw = 0; kw < KS; ++kw) {
-          const int ih = ih0 + kh, iw = iw0 + kw;
-          const bool in = ih >= 0 && ih < H && iw >= 0 && iw < W;
-          const int64_t o = ((int64_t)c * H + ih) * W + iw;
-          lo[kh * KS + kw] = in ? __ldg(il + o) : 0.f;
-          up[kh * KS + kw] = in ? __ldg(iu + o) : 0.f;
-          w[kh * KS + kw] = __ldg(wp + kh * KS + kw);
-        }
-#pragma unroll
-      for (int k = 0; k < KS * KS; ++k) {
-        ac = fmaf(fmul(fadd(lo[k], up[k]), 0.5f), w[k], ac);
-        ar = fmaf(fmul(fsub(up[k], lo[k]), 0.5f), fabsf(w[k]), ar);
-      }
-    }
-  } else {
-    const int kh0 = max(0, -ih0), kh1 = min(Kh, H - ih0), kw0 = max(0, -iw0), kw1 = min(Kw, W - iw0);
-    for (int c = 0; c < Cin; ++c) {
-      const float* wp = Wt + ((int64_t)co * Cin + c) * Kh * Kw;
-      const int64_t ib = ((int64_t)c * H + ih0) * W + iw0;
-      for (int kh = kh0; kh < kh1; ++kh)
-        for (int kw = kw0; kw < kw1; ++kw) {
-          const float lo = __ldg(il + ib + (int64_t)kh * W + kw), up = __ldg(iu + ib + (int64_t)kh * W + kw);
-          const float w = __ldg(wp + kh * Kw + kw);
-          ac = fmaf(fmul(fadd(lo, up), 0.5f), w, ac);
-          ar = fmaf(fmul(fsub(up, lo), 0.5f), fabsf(w), ar);
-        }
-    }
+// Cuts the tile (`pixels` at most, up to g_max channel groups of CPT) and returns the number of blocks; 0: no tile fits.
+int64_t plan_conv(ConvArgs& q, int cpt, int pixels, int g_max, int cc_max, size_t& smem) {
+  const int groups = (int)ceil_div(q.Cout, cpt);
+  q.chunks = (int)ceil_div(groups, g_max);
+  q.G = (int)ceil_div(groups, q.chunks);
+  q.TW = (int)ceil_div(q.Wo, ceil_div(q.Wo, std::min(pixels, 64)));   // even parts of at most 64 columns
+  q.TH = std::max(1, std::min(q.Ho, pixels / q.TW));
+  q.TH = (int)ceil_div(q.Ho, ceil_div(q.Ho, q.TH));
+  q.NI = q.TW == q.Wo && q.TH == q.Ho ? std::max(1, pixels / (q.TW * q.TH)) : 1;
+  q.NI = (int)std::max<int64_t>(1, std::min<int64_t>(q.NI, 0x7fffffff / ((int64_t)q.Cin * q.H * q.W)));   // 32-bit offsets
+  q.CC = std::min(q.Cin, cc_max);
+  for (;;) {
+    const bool phases = q.stride == 2;
+    q.in_h = (q.TH - 1) * q.stride + q.Kh;
+    q.in_w = (q.TW - 1) * q.stride + q.Kw;
+    q.pw = (q.in_w + 1) / 2;
+    q.row = phases ? 2 * q.pw : q.in_w;
+    q.chan = q.NI * q.in_h * q.row;
+    smem = 8 * (q.CC * ((size_t)q.Kh * q.Kw * q.G * cpt + (size_t)q.chan) + (size_t)q.NI * q.in_h * q.in_w);
+    // below 45 KB five blocks fit an SM; fewer channels a stage get there first, then (only if nothing fits) smaller tiles
+    if (smem <= 45 * 1024 || (q.CC == 1 && smem <= (size_t)device_info().smem_optin)) break;
+    if (q.CC > 1) q.CC = (q.CC + 1) / 2;
+    else if (q.NI > 1) q.NI /= 2;
+    else if (q.TH > 1) q.TH = (q.TH + 1) / 2;
+    else if (q.TW > 1) q.TW = (q.TW + 1) / 2;
+    else if (q.G > 1) { q.G = (q.G + 1) / 2; q.chunks = (int)ceil_div(groups, q.G); }
+    else return 0;
   }
-  float lo = fsub(ac, ar), up = fadd(ac, ar);
-  if (bias != nullptr) { lo = fadd(lo, bias[co]); up = fadd(up, bias[co]); }
-  y_lo[t] = lo;
-  y_up[t] = up;
+  q.tiles_h = (int)ceil_div(q.Ho, q.TH);
+  q.tiles_w = (int)ceil_div(q.Wo, q.TW);
+  const int64_t per_set = (int64_t)q.chunks * q.tiles_h * q.tiles_w;
+  q.blocks_bias = ceil_div(q.n_bias, q.NI) * per_set;
+  return q.blocks_bias + ceil_div(q.n_img, q.NI) * per_set;
 }
 
-template <int TH, int TW, int CO, int KS>
-int launch_conv_t(const float* x_lo, const float* x_up, const float* Wt, const float* bias, float* y_lo, float* y_up,
-                  int64_t N, int Cin, int H, int W, int Cout, int Kh, int Kw, int stride, int pad, int Ho, int Wo,
-                  cudaStream_t st) {
-  static_assert(TH * TW == kThreads, "one thread per output pixel of the tile");
-  const int in_h = (TH - 1) * stride + Kh, in_w = (TW - 1) * stride + Kw;
-  const size_t smem = sizeof(float) * ((size_t)2 * CC * in_h * in_w + (size_t)CC * Kh * Kw * CO);
-  if (smem > (size_t)device_info().smem_optin) return FB_ERR_SHAPE;
-  const int tiles_h = (int)ceil_div(Ho, TH), tiles_w = (int)ceil_div(Wo, TW), co_chunks = (int)ceil_div(Cout, CO);
-  const int64_t blocks = N * co_chunks * tiles_h * tiles_w;
-  if (blocks > 0x7fffffff) return FB_ERR_SHAPE;
-  if (int rc = ensure_dynamic_smem(conv_bounds_kernel<TH, TW, CO, KS>, smem)) return rc;
-  conv_bounds_kernel<TH, TW, CO, KS><<<(unsigned)blocks, kThreads, smem, st>>>(x_lo, x_up, Wt, bias, y_lo, y_up, Cin, H, W, Cout,
-                                                                         Kh, Kw, stride, pad, Ho, Wo, tiles_h, tiles_w,
-                                                                         co_chunks);
+template <int CPT, int PX>
+int launch_conv_t(const ConvArgs& q, int64_t blocks, size_t smem, cudaStream_t st) {
+  if (blocks <= 0 || blocks > 0x7fffffff) return FB_ERR_SHAPE;
+  const int ks = q.Kh == q.Kw && (q.Kh == 3 || q.Kh == 5) ? q.Kh : 0;
+#define FB_CONV_ST(K) (q.stride == 2 ? conv_bounds_kernel<CPT, PX, K, 2> : q.stride == 1 ? conv_bounds_kernel<CPT, PX, K, 1> \
+                                     : conv_bounds_kernel<CPT, PX, K, 0>)
+  auto kern = ks == 3 ? FB_CONV_ST(3) : ks == 5 ? FB_CONV_ST(5) : FB_CONV_ST(0);
+#undef FB_CONV_ST
+  if (int rc = ensure_dynamic_smem(kern, smem)) return rc;
+  kern<<<(unsigned)blocks, q.G * 32, smem, st>>>(q);
   FB_LAUNCH_OK();
   return FB_OK;
 }
 
-int launch_conv(const float* x_lo, const float* x_up, const float* Wt, const float* bias, float* y_lo, float* y_up,
-                int64_t N, int Cin, int H, int W, int Cout, int Kh, int Kw, int stride, int pad, int Ho, int Wo,
-                cudaStream_t st) {
-  if (N == 0) return FB_OK;
-  {
-    // blocks the tiled kernel would launch (its smallest tile: 256 pixels x 16 or 32 channels); fewer than one per
-    // SM and it is latency-bound
-    const int64_t tiled = N * ceil_div(Cout, Cout > 16 ? 32 : 16) * ceil_div((int64_t)Ho * Wo, 256);
-    const int64_t total = N * (int64_t)Cout * Ho * Wo;
-    if (tiled < device_info().sms && ceil_div(total, 128) <= 0x7fffffff) {
-      if (Kh == 3 && Kw == 3)
-        conv_bounds_small_kernel<3><<<(unsigned)ceil_div(total, 128), 128, 0, st>>>(x_lo, x_up, Wt, bias, y_lo, y_up, total, Cin, H,
-                                                                                    W, Cout, Kh, Kw, stride, pad, Ho, Wo);
-      else
-        conv_bounds_small_kernel<0><<<(unsigned)ceil_div(total, 128), 128, 0, st>>>(x_lo, x_up, Wt, bias, y_lo, y_up, total, Cin, H,
-                                                                                    W, Cout, Kh, Kw, stride, pad, Ho, Wo);
-      FB_LAUNCH_OK();
-      return FB_OK;
-    }
-  }
-  const bool narrow = Wo <= 16, wide_co = Cout > 16;
-#define FB_CONV_ARGS x_lo, x_up, Wt, bias, y_lo, y_up, N, Cin, H, W, Cout, Kh, Kw, stride, pad, Ho, Wo, st
-  if (Kh == 3 && Kw == 3) {
-    if (narrow) return wide_co ? launch_conv_t<16, 16, 32, 3>(FB_CONV_ARGS) : launch_conv_t<16, 16, 16, 3>(FB_CONV_ARGS);
-    return wide_co ? launch_conv_t<8, 32, 32, 3>(FB_CONV_ARGS) : launch_conv_t<8, 32, 16, 3>(FB_CONV_ARGS);
-  }
-  if (narrow) return wide_co ? launch_conv_t<16, 16, 32, 0>(FB_CONV_ARGS) : launch_conv_t<16, 16, 16, 0>(FB_CONV_ARGS);
-  return wide_co ? launch_conv_t<8, 32, 32, 0>(FB_CONV_ARGS) : launch_conv_t<8, 32, 16, 0>(FB_CONV_ARGS);
-#undef FB_CONV_ARGS
+// n_img images without bias (the weight part) and n_bias with it (the bias part) in one launch.
+int launch_conv(const float* x_lo, const float* x_up, float* y_lo, float* y_up, int64_t n_img, const float* b_lo, const float* b_up,
+                float* yb_lo, float* yb_up, int64_t n_bias, const float* Wt, const float* bias, int Cin, int H, int W, int Cout,
+                int Kh, int Kw, int stride, int pad, int Ho, int Wo, cudaStream_t st) {
+  if (n_img + n_bias == 0) return FB_OK;
+  if ((int64_t)H * W > 0x7fffffff) return FB_ERR_SHAPE;   // (offsets inside a plane are 32-bit)
+  ConvArgs q = {};
+  q.x_lo = x_lo, q.x_up = x_up, q.b_lo = b_lo, q.b_up = b_up;
+  q.y_lo = y_lo, q.y_up = y_up, q.yb_lo = yb_lo, q.yb_up = yb_up;
+  q.Wt = Wt, q.bias = bias, q.n_img = n_img, q.n_bias = n_bias;
+  q.Cin = Cin, q.H = H, q.W = W, q.Cout = Cout, q.Kh = Kh, q.Kw = Kw, q.stride = stride, q.pad = pad, q.Ho = Ho, q.Wo = Wo;
+  size_t smem;
+  // up to 5 channel groups a block share its staged input (48 channels are 2 x 3 groups, 40 are 5)
+  int64_t blocks = plan_conv(q, 8, 128, 5, 4, smem);
+  if (blocks >= device_info().sms) return launch_conv_t<8, 4>(q, blocks, smem, st);
+  // a few images only (the bias part alone: one image per batch element): less than a block per SM and bound by the latency
+  // of the stages, so one pixel x 2 channels per thread, 32 pixels x up to 8 channels per block, all channels in one stage
+  blocks = plan_conv(q, 2, 32, 4, Cin, smem);
+  return launch_conv_t<2, 1>(q, blocks, smem, st);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -459,7 +476,8 @@ extern "C" int fb_conv2d_identity_relax_f32(int op, const float* x_lb, const flo
   const int64_t ncol = (int64_t)Cout * Ho * Wo;
   fb::ProfileScope prof(fb::PK_CONV, 8.0 * (rows + 1) * ncol * Cin * Kh * Kw, 4.0 * (2.0 * (rows + 1) * ncol), stream);
   // bias part: an ordinary convolution of one image
-  int rc = fb::launch_conv(x_lb, x_ub, Wt, bias, y_lb, y_ub, 1, Cin, H, W, Cout, Kh, Kw, stride, pad, Ho, Wo, st);
+  int rc = fb::launch_conv(nullptr, nullptr, nullptr, nullptr, 0, x_lb, x_ub, y_lb, y_ub, 1, Wt, bias, Cin, H, W, Cout, Kh, Kw, stride, pad,
+                           Ho, Wo, st);
   if (rc != FB_OK) return rc;
   float* k_l = col_ws;
   float* k_u = col_ws + ncol;
@@ -547,8 +565,6 @@ extern "C" int fb_conv2d_f32(const float* x_lw, const float* x_uw, const float* 
   const double n1 = (double)B * (Di + 1);
   fb::ProfileScope prof(fb::PK_CONV, 8.0 * n1 * Cout * Ho * Wo * Cin * Kh * Kw,
                         4.0 * (2 * n1 * Cin * H * W + 2 * n1 * Cout * Ho * Wo + (double)Cout * Cin * Kh * Kw), stream);
-  int rc = fb::launch_conv(x_lw, x_uw, Wt, nullptr, y_lw, y_uw, (int64_t)B * Di, Cin, H, W, Cout, Kh, Kw, stride, pad,
-                           Ho, Wo, st);
-  if (rc != FB_OK) return rc;
-  return fb::launch_conv(x_lb, x_ub, Wt, bias, y_lb, y_ub, B, Cin, H, W, Cout, Kh, Kw, stride, pad, Ho, Wo, st);
+  return fb::launch_conv(x_lw, x_uw, y_lw, y_uw, (int64_t)B * Di, x_lb, x_ub, y_lb, y_ub, B, Wt, bias, Cin, H, W, Cout, Kh, Kw, stride, pad,
+                         Ho, Wo, st);
 }

@@ -1109,3 +1109,23 @@ def test_relax_transposed_columns_held_in_registers(Di, p):
                   0.02, 1, FB_TRANSPOSED)
     helpers.assert_close(z[0].transpose(2, 3), o.lw, "lw"); helpers.assert_close(z[1].transpose(2, 3), o.uw, "uw")
     helpers.assert_close(z[2], o.lb, "lb"); helpers.assert_close(z[3], o.ub, "ub")
+
+
+# many images: maps smaller than a tile (several images per block), one column past 64, 8 / 16 channels a thread, stride 3, a
+# filter that is neither 3 x 3 nor 5 x 5, more channels than a block's groups
+@pytest.mark.parametrize("N,C,H,W,Co,kh,kw,s,p", [(700, 3, 5, 6, 16, 3, 3, 1, 1), (160, 5, 9, 65, 8, 3, 3, 1, 1), (75, 2, 66, 13, 40, 5, 5, 2, 1),
+                                                  (150, 9, 13, 13, 50, 3, 3, 2, 0), (300, 4, 14, 11, 24, 2, 4, 3, 2)])
+def test_conv_of_many_images_tiles(N, C, H, W, Co, kh, kw, s, p):
+    from faith_b200 import ops
+    g = torch.Generator().manual_seed(504)
+    lw = torch.rand(1, N, C, H, W, generator=g) - 0.5
+    uw = lw + torch.rand(1, N, C, H, W, generator=g)
+    lb = torch.rand(1, C, H, W, generator=g)
+    ub = lb + torch.rand(1, C, H, W, generator=g)
+    wt = torch.randn(Co, C, kh, kw, generator=g) * math.sqrt(2.0 / (C * kh * kw))
+    bias = torch.randn(Co, generator=g) * 0.1
+    o = O.conv_bounds(O.OBounds(1.0, 0.01, lw, lb, uw, ub), wt, bias, s, p)
+    o64 = O.conv_bounds(O.OBounds(1.0, 0.01, lw.double(), lb.double(), uw.double(), ub.double()), wt.double(), bias.double(), s, p)
+    r = ops.conv2d((lw.to(DEV), uw.to(DEV), lb.to(DEV), ub.to(DEV)), wt.to(DEV), bias.to(DEV), s, p)
+    for got, k in zip(r, ("lw", "uw", "lb", "ub")):
+        helpers.assert_arbitrated(got, getattr(o, k), getattr(o64, k), "conv %s %s" % ((N, C, H, W, Co, kh, kw, s, p), k))
