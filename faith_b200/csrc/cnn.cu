@@ -11,12 +11,13 @@
 #include <cstdint>
 
 #include "common.cuh"
+#include "conv_window.cuh"
 
 namespace fb {
 namespace {
 
 struct Geometry {
-  int64_t wt;      // elements of the weight of the linear layer that ends the spatial part (transposed copy), or 0
+  int64_t part;    // partial norms of the linear layer that ends the spatial part, or 0
   int64_t f_max;   // widest layer output (features of one row)
   int n_out;       // features of the last layer
   bool ok;
@@ -40,7 +41,7 @@ Geometry walk(const fb_cnn* net) {
       feat = (int64_t)c * h * w;
     } else if (ly.kind == FB_CNN_LINEAR) {
       if (!ly.weight || ly.n_out <= 0) return g;
-      if (spatial) g.wt = feat * ly.n_out;
+      if (spatial) g.part = 2 * ly.n_out * cw_linear_tiles(net->h, net->w);
       spatial = false;
       feat = ly.n_out;
     } else if (ly.kind != FB_CNN_RELU) {
@@ -67,9 +68,9 @@ extern "C" int64_t fb_cnn_workspace_bytes(const fb_cnn* net, int64_t rows) {
   const Geometry g = walk(net);
   if (!g.ok || rows < 0) return -1;
   // two bound sets (lw, uw [rows, f_max]; lb, ub [f_max]), the column scratch of the first convolution and the norm
-  // partials (2 * f_max each), the relaxation coefficients of the compact route (4 * f_max)
+  // partials (2 * f_max each), the relaxation coefficients of the compact route (4 * f_max), the linear layer's partial norms
   const int64_t per_set = 2 * round_up(rows * g.f_max) + 2 * round_up(g.f_max);
-  return 4 * (2 * per_set + 8 * round_up(g.f_max) + round_up(g.wt));
+  return 4 * (2 * per_set + 8 * round_up(g.f_max) + round_up(g.part));
 }
 
 extern "C" int fb_cnn_forward_f32(const fb_cnn* net, const float* image, int p, float eps, int64_t row_start, int64_t rows,
@@ -95,22 +96,35 @@ extern "C" int fb_cnn_forward_f32(const fb_cnn* net, const float* image, int p, 
   float* col_ws = base; base += 2 * bsz;
   float* part_ws = base; base += 2 * bsz;
   float* coef_ws = base; base += 4 * bsz;
-  float* wt_ws = base;
+  float* lin_ws = base;
 
+  cudaStream_t st = (cudaStream_t)stream;
   int c = net->cin, h = net->h, w = net->w;
   int64_t feat = di;
   int chain[4 * 8];
   int n_chain = 0;
-  int cur = 0;
   int i = 0;
-  bool cw = compact != 0;   // rows still kept as their windows (compact route, until the first linear layer)
+  Set x = set[0], y = set[1];   // input and output of the layer at hand
+  // compact route, until the first linear layer: rows kept as their windows only, and not written where the next layer can take
+  // them as they come: first (the rows behind the first convolution follow from its filter and the slopes in col_ws), rescaled
+  // (the rows still have to go through the coefficients in coef_ws).
+  bool cw = compact != 0, first = false, rescaled = false;
   {
     // the first convolution (and the relaxation behind it, if any) from the filter alone
     const fb_cnn_layer& ly = net->layer[0];
     const bool fuse = net->n_layers > 1 && net->layer[1].kind == FB_CNN_RELU;
-    int rc = (cw ? fb_cw_identity_relax_f32 : fb_conv2d_identity_relax_f32)(
-        fuse ? FB_RELU : -1, image, image, ly.weight, ly.bias, 1.0f, set[0].lw, set[0].uw, set[0].lb, set[0].ub, col_ws, rows,
-        row_start, c, h, w, ly.cout, ly.kh, ly.kw, ly.stride, ly.pad, p, eps, violation, stream);
+    const int next = fuse ? 2 : 1, op = fuse ? FB_RELU : -1;
+    first = cw && next < net->n_layers && net->layer[next].kind == FB_CNN_CONV;
+    int rc;
+    if (first) {
+      const int ho = (h + 2 * ly.pad - ly.kh) / ly.stride + 1, wo = (w + 2 * ly.pad - ly.kw) / ly.stride + 1;
+      rc = launch_identity_columns(op, image, image, ly.weight, ly.bias, x.lb, x.ub, col_ws, col_ws + (int64_t)ly.cout * ho * wo, 1.0f, c, h, w,
+                                   ly.cout, ly.kh, ly.kw, ly.stride, ly.pad, ho, wo, p, eps, violation, st);
+    } else {
+      rc = (cw ? fb_cw_identity_relax_f32 : fb_conv2d_identity_relax_f32)(op, image, image, ly.weight, ly.bias, 1.0f, x.lw, x.uw, x.lb, x.ub,
+                                                                          col_ws, rows, row_start, c, h, w, ly.cout, ly.kh, ly.kw,
+                                                                          ly.stride, ly.pad, p, eps, violation, stream);
+    }
     if (rc != FB_OK) return rc;
     chain[0] = ly.kh, chain[1] = ly.kw, chain[2] = ly.stride, chain[3] = ly.pad;
     n_chain = 1;
@@ -118,37 +132,39 @@ extern "C" int fb_cnn_forward_f32(const fb_cnn* net, const float* image, int p, 
     w = (w + 2 * ly.pad - ly.kw) / ly.stride + 1;
     c = ly.cout;
     feat = (int64_t)c * h * w;
-    i = fuse ? 2 : 1;
+    i = next;
   }
   // leaves the compact route: dense rows from here on (a layer the compact operators do not cover)
   auto expand = [&]() -> int {
-    const Set& x = set[cur];
-    const Set& y = set[cur ^ 1];
+    if (rescaled) {
+      int rc = cw_rescale_rows(x.lw, x.uw, coef_ws, y.lw, y.uw, rows, row_start, net->h, net->w, chain, n_chain, c, h, w, st);
+      if (rc != FB_OK) return rc;
+      std::swap(x.lw, y.lw);
+      std::swap(x.uw, y.uw);
+      rescaled = false;
+    }
     int rc = fb_cw_expand_f32(x.lw, x.uw, y.lw, y.uw, rows, row_start, net->h, net->w, chain, n_chain, c, h, w, stream);
     if (rc != FB_OK) return rc;
-    FB_CUDA_OK(cudaMemcpyAsync(y.lb, x.lb, sizeof(float) * feat, cudaMemcpyDeviceToDevice, (cudaStream_t)stream));
-    FB_CUDA_OK(cudaMemcpyAsync(y.ub, x.ub, sizeof(float) * feat, cudaMemcpyDeviceToDevice, (cudaStream_t)stream));
-    cur ^= 1;
+    std::swap(x.lw, y.lw);
+    std::swap(x.uw, y.uw);
     cw = false;
     return FB_OK;
   };
   for (; i < net->n_layers; ++i) {
     const fb_cnn_layer& ly = net->layer[i];
+    const bool last = i + 1 == net->n_layers;
     int rc = FB_OK;
     if (cw && ly.kind == FB_CNN_CONV && n_chain + 1 > 8) {
       rc = expand();
       if (rc != FB_OK) return rc;
     }
-    const Set& x = set[cur];
-    const Set& y = set[cur ^ 1];
     if (ly.kind == FB_CNN_CONV) {
       const int ho = (h + 2 * ly.pad - ly.kh) / ly.stride + 1, wo = (w + 2 * ly.pad - ly.kw) / ly.stride + 1;
       if (cw) {
-        rc = fb_cw_conv2d_f32(x.lw, x.uw, ly.weight, y.lw, y.uw, rows, row_start, net->h, net->w, chain, n_chain, c, h, w, ly.cout,
-                              ly.kh, ly.kw, ly.stride, ly.pad, stream);
-        if (rc == FB_OK)
-          rc = fb_conv2d_f32(x.lb, x.ub, x.lb, x.ub, ly.weight, ly.bias, y.lb, y.ub, y.lb, y.ub, 1, 0, c, h, w, ly.cout, ly.kh,
-                             ly.kw, ly.stride, ly.pad, stream);
+        rc = cw_conv_ex(first ? nullptr : x.lw, first ? nullptr : x.uw, first ? net->layer[0].weight : nullptr, col_ws, col_ws + feat, 1.0f,
+                        net->cin, ly.weight, y.lw, y.uw, x.lb, x.ub, ly.bias, y.lb, y.ub, rows, row_start, net->h, net->w, chain, n_chain, c,
+                        h, w, ly.cout, ly.kh, ly.kw, ly.stride, ly.pad, st);
+        first = false;
       } else {
         rc = n_chain < 8 ? fb_conv2d_windowed_f32(x.lw, x.uw, ly.weight, y.lw, y.uw, rows, row_start, net->h, net->w, chain,
                                                   n_chain, c, h, w, ly.cout, ly.kh, ly.kw, ly.stride, ly.pad, stream)
@@ -169,39 +185,54 @@ extern "C" int fb_cnn_forward_f32(const fb_cnn* net, const float* image, int p, 
       feat = (int64_t)c * h * w;
     } else if (ly.kind == FB_CNN_RELU) {
       if (cw) {
-        float* part_l = part_ws;
-        float* part_u = part_ws + feat;
-        rc = fb_cw_norm_partials_f32(x.lw, x.uw, part_l, part_u, rows, row_start, net->cin, net->h, net->w, chain, n_chain, c, h, w,
-                                     p, stream);
-        if (rc == FB_OK && comm != nullptr) rc = fb_allreduce_f32(comm, part_ws, 2 * feat, p == FB_P1 ? 1 : 0, algo, stream);
-        if (rc == FB_OK)   // relaxation coefficients in their own scratch
-          rc = fb_cw_relax_apply_f32(FB_RELU, x.lw, x.uw, x.lb, x.ub, part_l, part_u, y.lw, y.uw, y.lb, y.ub, coef_ws, rows,
-                                     row_start, net->h, net->w, chain, n_chain, c, h, w, p, eps, violation, stream);
+        if (comm == nullptr) {
+          rc = cw_norm_ex(FB_RELU, x.lw, x.uw, nullptr, nullptr, x.lb, x.ub, y.lb, y.ub, coef_ws, rows, row_start, net->cin, net->h, net->w,
+                          chain, n_chain, c, h, w, p, eps, violation, st);
+        } else {
+          rc = cw_norm_ex(-1, x.lw, x.uw, part_ws, part_ws + feat, nullptr, nullptr, nullptr, nullptr, nullptr, rows, row_start, net->cin,
+                          net->h, net->w, chain, n_chain, c, h, w, p, eps, violation, st);
+          if (rc == FB_OK) rc = fb_allreduce_f32(comm, part_ws, 2 * feat, p == FB_P1 ? 1 : 0, algo, stream);
+          if (rc == FB_OK)
+            rc = cw_relax_columns(FB_RELU, x.lb, x.ub, part_ws, part_ws + feat, y.lb, y.ub, coef_ws, c, (int64_t)h * w, p, eps, violation, st);
+        }
+        if (rc != FB_OK) return rc;
+        std::swap(x.lb, y.lb);
+        std::swap(x.ub, y.ub);
+        rescaled = !last && net->layer[i + 1].kind == FB_CNN_LINEAR;
+        if (rescaled) continue;
+        rc = cw_rescale_rows(x.lw, x.uw, coef_ws, y.lw, y.uw, rows, row_start, net->h, net->w, chain, n_chain, c, h, w, st);
+        if (rc != FB_OK) return rc;
+        std::swap(x.lw, y.lw);
+        std::swap(x.uw, y.uw);
+        continue;
       } else {
         rc = fb_relax_sharded_f32(comm, algo, FB_RELU, x.lw, x.uw, x.lb, x.ub, y.lw, y.uw, y.lb, y.ub, part_ws, 1, (int)rows,
                                   (int)feat, 1, p, eps, violation, stream);
       }
     } else {
+      bool dense = !cw;
       if (cw) {
-        rc = fb_cw_linear_f32(x.lw, x.uw, ly.weight, y.lw, y.uw, wt_ws, rows, row_start, net->h, net->w, chain, n_chain, c, h, w, ly.n_out,
-                              stream);
-        if (rc == FB_OK)
-          rc = fb_matmul_f32(x.lb, x.ub, x.lb, x.ub, ly.weight, ly.bias, y.lb, y.ub, y.lb, y.ub, 1, 0, (int)feat, ly.n_out, stream);
+        // the last layer's rows are needed for their norms only (several ranks: exchanged below)
+        const bool norms = last && comm == nullptr;
+        rc = cw_linear_ex(x.lw, x.uw, rescaled ? coef_ws : nullptr, ly.weight, norms ? nullptr : y.lw, norms ? nullptr : y.uw,
+                          norms ? lin_ws : nullptr, x.lb, x.ub, ly.bias, y.lb, y.ub, rows, row_start, net->h, net->w, chain, n_chain, c, h, w,
+                          ly.n_out, p, st);
+        if (rc == FB_OK && norms) return cw_linear_range(lin_ws, y.lb, y.ub, out_l, out_u, net->h, net->w, ly.n_out, p, eps, st);
+        dense = rc == FB_ERR_SHAPE;   // a row of positions does not fit into shared memory
+        if (dense) rc = expand();
+        if (rc != FB_OK) return rc;
         cw = false;
-      } else {
-        rc = fb_matmul_f32(x.lw, x.uw, x.lb, x.ub, ly.weight, ly.bias, y.lw, y.uw, y.lb, y.ub, 1, (int)rows, (int)feat, ly.n_out,
-                           stream);
       }
+      if (dense)
+        rc = fb_matmul_f32(x.lw, x.uw, x.lb, x.ub, ly.weight, ly.bias, y.lw, y.uw, y.lb, y.ub, 1, (int)rows, (int)feat, ly.n_out, stream);
       feat = ly.n_out;
     }
     if (rc != FB_OK) return rc;
-    cur ^= 1;
+    std::swap(x, y);
   }
   if (cw) {   // the network ended on a feature map
     int rc = expand();
     if (rc != FB_OK) return rc;
   }
-  const Set& z = set[cur];
-  return fb_concretize_sharded_f32(comm, algo, z.lw, z.uw, z.lb, z.ub, out_l, out_u, part_ws, 1, (int)rows, (int)feat, 1, p,
-                                   eps, stream);
+  return fb_concretize_sharded_f32(comm, algo, x.lw, x.uw, x.lb, x.ub, out_l, out_u, part_ws, 1, (int)rows, (int)feat, 1, p, eps, stream);
 }

@@ -88,6 +88,25 @@ int concretize_pair(const float* x_lw, const float* x_uw, const float* x_lb, con
                     int x_do, const float* y_lw, const float* y_uw, const float* y_lb, const float* y_ub, float* y_l, float* y_u,
                     int64_t y_rows, int y_do, int Di, int words, int p, float eps, int layout, cudaStream_t st);
 
+// conv_compact.cu: the operators on compact rows with the options of the CNN driver (see the definitions).
+int cw_conv_ex(const float* z_lo, const float* z_up, const float* W1, const float* k_l, const float* k_u, float scale, int Cin0,
+               const float* Wt, float* y_lo, float* y_up, const float* b_lo, const float* b_up, const float* bias, float* yb_lo,
+               float* yb_up, int64_t rows, int64_t row_start, int H0, int W0, const int* chain, int n_chain, int Cin, int H, int W,
+               int Cout, int Kh, int Kw, int stride, int pad, cudaStream_t st);
+int cw_norm_ex(int op, const float* z_lw, const float* z_uw, float* part_l, float* part_u, const float* lb, const float* ub, float* out_lb,
+               float* out_ub, float* coef, int64_t rows, int64_t row_start, int Cin0, int H0, int W0, const int* chain, int n_chain, int C,
+               int H, int W, int p, float eps, int* violation, cudaStream_t st);
+int cw_relax_columns(int op, const float* lb, const float* ub, const float* norm_l, const float* norm_u, float* out_lb, float* out_ub,
+                     float* coef, int C, int64_t hw, int p, float eps, int* violation, cudaStream_t st);
+int cw_rescale_rows(const float* z_lw, const float* z_uw, const float* coef, float* out_lw, float* out_uw, int64_t rows, int64_t row_start,
+                    int H0, int W0, const int* chain, int n_chain, int C, int H, int W, cudaStream_t st);
+int64_t cw_linear_tiles(int H0, int W0);
+int cw_linear_ex(const float* z_lw, const float* z_uw, const float* coef, const float* Wl, float* y_lw, float* y_uw, float* part,
+                 const float* lb, const float* ub, const float* bias, float* y_lb, float* y_ub, int64_t rows, int64_t row_start, int H0,
+                 int W0, const int* chain, int n_chain, int C, int H, int W, int N, int p, cudaStream_t st);
+int cw_linear_range(const float* part, const float* lb, const float* ub, float* l, float* u, int H0, int W0, int N, int p, float eps,
+                    cudaStream_t st);
+
 // softmax.cu: fb_softmax_ranges_f32 with rows `ld` floats apart.
 int softmax_ex(const float* lw, const float* uw, const float* lb, const float* ub, float* out_lw, float* out_uw, float* out_lb,
                float* out_ub, float* out_l, float* out_u, int64_t rows, int Di, int Do, int ld, int words, int p, float eps,

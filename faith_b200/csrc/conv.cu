@@ -264,35 +264,50 @@ int launch_conv(const float* x_lo, const float* x_up, float* y_lo, float* y_up, 
 //  * further layers keep the rows local: row r is zero outside a small window around its pixel, so a later
 //    convolution only has to compute the outputs whose taps reach into that window and store zeros elsewhere.
 
-// Per output column (co, y, x): slopes and bias terms of the relaxation `op` of conv(identity input) (op < 0: no
-// relaxation).  col_ws: k_l, k_u, then the bias terms are written to y_lb, y_ub in place (they hold the conv of
-// the bias part on entry).
-__global__ void __launch_bounds__(256)
-identity_conv_columns_kernel(int op, const float* __restrict__ Wt, float* __restrict__ y_lb, float* __restrict__ y_ub,
-                             float* __restrict__ k_l, float* __restrict__ k_u, float scale, int Cin, int H, int W,
-                             int Cout, int Kh, int Kw, int stride, int pad, int Ho, int Wo, int p, float eps,
+// Per output column (co, y, x): the bias part (an ordinary convolution of the image, accumulated in the order of
+// conv_bounds_kernel), the norm of the taps inside the image, and from both the slopes k_l, k_u and the relaxed bias terms of
+// the relaxation `op` (op < 0: no relaxation, slopes 1).  Bound by latency (a thread per column): with KS, as above, the loads
+// of an input channel's taps are in flight together, and one pass serves both sums (the image's convolution and the columns
+// took 4 + 5 us as two launches for 3 -> 16 channels of 32 x 32).
+template <int KS>
+__global__ void __launch_bounds__(128)
+identity_conv_columns_kernel(int op, const float* __restrict__ x_lb, const float* __restrict__ x_ub, const float* __restrict__ Wt,
+                             const float* __restrict__ bias, float* __restrict__ y_lb, float* __restrict__ y_ub,
+                             float* __restrict__ k_l, float* __restrict__ k_u, float scale, int Cin, int H, int W, int Cout,
+                             int Kh_arg, int Kw_arg, int stride, int pad, int Ho, int Wo, int p, float eps,
                              int* __restrict__ violation) {
+  const int Kh = KS ? KS : Kh_arg, Kw = KS ? KS : Kw_arg;
   const int64_t n = (int64_t)Cout * Ho * Wo;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
     const int x = (int)(t % Wo), y = (int)((t / Wo) % Ho), co = (int)(t / ((int64_t)Wo * Ho));
-    float acc = 0.f;
-    for (int ci = 0; ci < Cin; ++ci)
-      for (int ky = 0; ky < Kh; ++ky) {
-        const int iy = y * stride - pad + ky;
-        if (iy < 0 || iy >= H) continue;
-        for (int kx = 0; kx < Kw; ++kx) {
-          const int ix = x * stride - pad + kx;
-          if (ix < 0 || ix >= W) continue;
-          acc = norm_accum(p, acc, fmul(scale, Wt[(((int64_t)co * Cin + ci) * Kh + ky) * Kw + kx]));
+    const int iy0 = y * stride - pad, ix0 = x * stride - pad;
+    float ac = 0.f, ar = 0.f, acc = 0.f;
+    for (int ci = 0; ci < Cin; ++ci) {
+      const float* wp = Wt + ((int64_t)co * Cin + ci) * Kh * Kw;
+      const int64_t plane = (int64_t)ci * H * W;
+#pragma unroll
+      for (int ky = 0; ky < (KS ? KS : Kh); ++ky)
+#pragma unroll
+        for (int kx = 0; kx < (KS ? KS : Kw); ++kx) {
+          const int iy = iy0 + ky, ix = ix0 + kx;
+          const bool in = iy >= 0 && iy < H && ix >= 0 && ix < W;
+          const int64_t o = plane + (int64_t)iy * W + ix;
+          const float w = __ldg(wp + ky * Kw + kx), lo = in ? __ldg(x_lb + o) : 0.f, up = in ? __ldg(x_ub + o) : 0.f;
+          ac = fmaf(fmul(fadd(lo, up), 0.5f), w, ac);
+          ar = fmaf(fmul(fsub(up, lo), 0.5f), fabsf(w), ar);
+          acc = norm_accum(p, acc, in ? fmul(scale, w) : 0.f);
         }
-      }
-    const float nrm = norm_finish(p, acc);
-    const float lbv = y_lb[t], ubv = y_ub[t];
+    }
+    float lbv = fsub(ac, ar), ubv = fadd(ac, ar);
+    if (bias != nullptr) { lbv = fadd(lbv, bias[co]); ubv = fadd(ubv, bias[co]); }
     if (op < 0) {
       k_l[t] = 1.f;
       k_u[t] = 1.f;
+      y_lb[t] = lbv;
+      y_ub[t] = ubv;
       continue;
     }
+    const float nrm = norm_finish(p, acc);
     const float l = fadd(lbv, fmul(-eps, nrm)), u = fadd(ubv, fmul(eps, nrm));
     bool bad = false;
     const ColCoef c = relax_column(op, l, u, lbv, ubv, bad);
@@ -447,13 +462,14 @@ conv_window_kernel(const float* __restrict__ x_lo, const float* __restrict__ x_u
 
 }  // namespace
 
-int launch_identity_columns(int op, const float* Wt, float* y_lb, float* y_ub, float* k_l, float* k_u, float scale, int Cin,
-                            int H, int W, int Cout, int Kh, int Kw, int stride, int pad, int Ho, int Wo, int p, float eps,
-                            int* violation, cudaStream_t st) {
+int launch_identity_columns(int op, const float* x_lb, const float* x_ub, const float* Wt, const float* bias, float* y_lb, float* y_ub,
+                            float* k_l, float* k_u, float scale, int Cin, int H, int W, int Cout, int Kh, int Kw, int stride, int pad,
+                            int Ho, int Wo, int p, float eps, int* violation, cudaStream_t st) {
   const int64_t ncol = (int64_t)Cout * Ho * Wo;
-  const int64_t want = ceil_div(ncol, 256), cap = (int64_t)device_info().sms * 8;
-  identity_conv_columns_kernel<<<(unsigned)(want < cap ? want : cap), 256, 0, st>>>(
-      op, Wt, y_lb, y_ub, k_l, k_u, scale, Cin, H, W, Cout, Kh, Kw, stride, pad, Ho, Wo, p, eps, violation);
+  const int64_t want = ceil_div(ncol, 128), cap = (int64_t)device_info().sms * 16;
+  auto kern = Kh == 3 && Kw == 3 ? identity_conv_columns_kernel<3> : identity_conv_columns_kernel<0>;
+  kern<<<(unsigned)(want < cap ? want : cap), 128, 0, st>>>(op, x_lb, x_ub, Wt, bias, y_lb, y_ub, k_l, k_u, scale, Cin, H, W, Cout, Kh, Kw,
+                                                            stride, pad, Ho, Wo, p, eps, violation);
   FB_LAUNCH_OK();
   return FB_OK;
 }
@@ -475,14 +491,10 @@ extern "C" int fb_conv2d_identity_relax_f32(int op, const float* x_lb, const flo
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t ncol = (int64_t)Cout * Ho * Wo;
   fb::ProfileScope prof(fb::PK_CONV, 8.0 * (rows + 1) * ncol * Cin * Kh * Kw, 4.0 * (2.0 * (rows + 1) * ncol), stream);
-  // bias part: an ordinary convolution of one image
-  int rc = fb::launch_conv(nullptr, nullptr, nullptr, nullptr, 0, x_lb, x_ub, y_lb, y_ub, 1, Wt, bias, Cin, H, W, Cout, Kh, Kw, stride, pad,
-                           Ho, Wo, st);
-  if (rc != FB_OK) return rc;
   float* k_l = col_ws;
   float* k_u = col_ws + ncol;
-  rc = fb::launch_identity_columns(op, Wt, y_lb, y_ub, k_l, k_u, scale, Cin, H, W, Cout, Kh, Kw, stride, pad, Ho, Wo, p, eps,
-                                   violation, st);
+  int rc = fb::launch_identity_columns(op, x_lb, x_ub, Wt, bias, y_lb, y_ub, k_l, k_u, scale, Cin, H, W, Cout, Kh, Kw, stride, pad, Ho, Wo,
+                                       p, eps, violation, st);
   if (rc != FB_OK) return rc;
   if (rows == 0) return FB_OK;
   if (rows > 0x7fffffff) return FB_ERR_SHAPE;

@@ -5,8 +5,9 @@
 // The dense-row kernels of conv.cu still write and read those zeros: [rows, C, H, W] per tensor, 98 % zeros for the
 // benchmark CNN.  Here a row is kept as its window only:
 //
-//     z[r, c, dy, dx] = row r at (c, wy.lo(r) + dy, wx.lo(r) + dx),   dy < wh, dx < ww,
+//     z[r, dy, dx, c] = row r at (c, wy.lo(r) + dy, wx.lo(r) + dx),   dy < wh, dx < ww,
 //
+// (channels innermost: the kernels have their lanes on the channels, and their loads and stores of rows are whole sectors)
 // with (wh, ww) the largest window over all pixels (fb_cw_extent) and zeros where a pixel's own window is smaller.
 // The origin (wy.lo, wx.lo) is recomputed from the pixel and the chain wherever it is needed.  Every operator of the
 // CNN pass has a compact form: first convolution + relaxation, later convolutions, the column norms over dim_in
@@ -46,7 +47,7 @@ cw_identity_rows_kernel(const float* __restrict__ Wt, const float* __restrict__ 
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < rows * per_row; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t lr = t / per_row;
     const int e = (int)(t - lr * per_row);
-    const int dx = e % ww, dy = (e / ww) % wh, co = e / (ww * wh);
+    const int co = e % Cout, dx = (e / Cout) % ww, dy = e / (Cout * ww);
     const int64_t r = row_start + lr;
     const int xi = (int)(r % W), yi = (int)((r / W) % H), ci = (int)(r / ((int64_t)W * H));
     Span sy = {yi, yi}, sx = {xi, xi};
@@ -68,187 +69,334 @@ cw_identity_rows_kernel(const float* __restrict__ Wt, const float* __restrict__ 
   }
 }
 
-// A later convolution, compact -> compact.  A block takes kCwRows consecutive rows: the filter is staged in shared
-// memory once per block with the output channel innermost ([Cin, Kh, Kw, Cout]: the lanes of a warp, which differ in the
-// output channel, read consecutive words), the compact inputs of the rows as (centre, radius) pairs.  A work item is one
-// output element; items are ordered (row, y, x, channel), so with Cout a multiple of 32 a warp shares its row and its
-// output pixel, its tap loops are uniform and its input reads are broadcasts.  Every output accumulates over (input
-// channel, tap row, tap column) in that order, as the dense kernel does.
-// Shared memory: Cin*Kh*Kw*(Cout+1) + 2 * kCwRows * Cin*iwh*iww floats (the filter rows are padded by one word, so that
-// both the staging stores, whose lanes differ in the tap, and the reads, whose lanes differ in the channel, are free of
-// bank conflicts).
-constexpr int kCwRows = 8;
-// CPT: output channels per work item (4 when Cout is a multiple of 4: the four weights of a tap are one 128-bit read and
-// the input pair is read once for four channels, which halves the instructions per multiply-add; else 1).
-template <int CPT>
-__global__ void __launch_bounds__(256)
-cw_conv_kernel(const float* __restrict__ x_lo, const float* __restrict__ x_up, const float* __restrict__ Wt,
-               float* __restrict__ y_lo, float* __restrict__ y_up, int64_t rows, int64_t row_start, int H0, int W0,
-               const ConvChain ch, int Cin, int Cout, int Kh, int Kw, int stride, int pad, int Ho, int Wo, int iwh, int iww,
-               int owh, int oww) {
+// A later convolution, compact -> compact.  Rows whose pixels agree modulo S, the product of all strides up to and including
+// this convolution's, have the same geometry up to a shift: the same windows, the same taps for the same output.  A block takes
+// G * 8 rows of one such class, so that nothing in its loops depends on the row: a thread owns one output position and channel of
+// eight rows, reads a weight once for all of them, and its tap bounds are the same for the whole block.  The windows are taken
+// without the borders of the maps (rows at the border are filled up with zeros, whose products leave every sum as it is), and
+// what falls outside is not stored.  Every output accumulates over (input channel, tap row, tap column) in that order, as the
+// dense kernel does.  Centre and radius share a packed multiply-add with a (w, |w|) pair.
+// The input comes from compact rows, or (W1 != nullptr) is the first convolution and its relaxation, evaluated from the filter
+// while it is staged: those rows are never written.  The first blocks compute the bias image.
+// Bound by latency and shared-memory reads: 3072 rows, 16 -> 32 channels, 3 x 3 stride 2 took 35 us with a thread per output of
+// one row, whose tap bounds differ from lane to lane, and 8 us before it to write its input.
+constexpr int kCwR = 8;             // rows per thread
+constexpr int kCwConvThreads = 512;
+constexpr int kCwMaxRows = 32;      // rows per block at most: one per lane
+constexpr size_t kCwStatic = 4096;  // static shared memory of the kernels below, at most
+
+struct CwConvArgs {
+  const float *z_lo, *z_up;                    // compact rows, or
+  const float *W1, *k_l, *k_u;                 // the first convolution (ch.kh[0] ...): filter [Cin, Cin0, kh, kw], slopes per column
+  float scale;
+  int Cin0;
+  const float* Wt;
+  float *y_lo, *y_up;
+  const float *b_lo, *b_up, *bias;             // bias image (blocks_bias > 0)
+  float *yb_lo, *yb_up;
+  int blocks_bias;
+  int64_t rows, row_start;
+  int ci0, n_ci;                               // input channels of the image that the rows span
+  int H0, W0, Cin, H, W, Cout, Kh, Kw, stride, pad, Ho, Wo, iwh, iww, owh, oww;
+  int S, cls_x, per_class, G, CC;
+  int uih, uiw;                                // largest window of the input without borders
+  ConvChain ch;
+};
+
+struct CwRow {
+  int lr, yi, xi, ci;      // local row (-1: none), pixel
+  int uy, ux;              // input window without borders: first row and column
+  int iy, ix, ih, iw;      // input window: first row and column, size
+  int oy, ox, oh, ow;      // output window
+  int voy, vox;            // output window without borders: first row and column
+};
+
+// KS: filter size when it is the same in both directions and known at compile time (3), 0 = from the arguments.
+template <int KS>
+__global__ void __launch_bounds__(kCwConvThreads)
+cw_conv_kernel(const CwConvArgs q) {
   extern __shared__ __align__(16) float cw_smem[];
-  const int ldw = Cout + (CPT == 4 ? 4 : 1), ctaps = Cin * Kh * Kw;   // padded: staging stores and reads spread over the banks
-  const int n_in = Cin * iwh * iww, n_out = Cout * owh * oww, n_w = ctaps * ldw;
-  float* s_w = cw_smem;                                        // [Cin][Kh][Kw][ldw]
-  float2* s_x = reinterpret_cast<float2*>(cw_smem + n_w + (n_w & 1));   // [kCwRows][Cin][iwh][iww] (centre, radius)
-  __shared__ int s_geo[kCwRows][8];   // wy.lo, wx.lo, ah, aw, oy.lo, ox.lo, bh, bw (bh = 0: nothing to compute)
-  const int64_t lr0 = (int64_t)blockIdx.x * kCwRows;
-  const int nr = (int)min((int64_t)kCwRows, rows - lr0);
-  for (int f = threadIdx.x; f < ctaps * Cout; f += blockDim.x) {   // coalesced read of [Cout][Cin*Kh*Kw]
-    const int t = f % ctaps, co = f / ctaps;        // t = (c * Kh + ky) * Kw + kx
-    s_w[t * ldw + co] = __ldg(Wt + f);
-  }
-  for (int f = threadIdx.x; f < nr * n_in; f += blockDim.x) {
-    const float lo = __ldg(x_lo + lr0 * n_in + f), up = __ldg(x_up + lr0 * n_in + f);
-    s_x[f] = make_float2(fmul(fadd(lo, up), 0.5f), fmul(fsub(up, lo), 0.5f));
-  }
-  if (threadIdx.x < nr) {
-    int yi, xi;
-    pixel_of_row(row_start + lr0 + threadIdx.x, H0, W0, yi, xi);
-    Span wy, wx;
-    chain_window(ch, H0, W0, yi, xi, wy, wx);
-    const Span oy = span_after_conv(wy, Kh, stride, pad, Ho), ox = span_after_conv(wx, Kw, stride, pad, Wo);
-    const bool empty = wy.lo > wy.hi || wx.lo > wx.hi || oy.lo > oy.hi || ox.lo > ox.hi;
-    int* gq = s_geo[threadIdx.x];
-    gq[0] = wy.lo, gq[1] = wx.lo, gq[2] = wy.hi - wy.lo + 1, gq[3] = wx.hi - wx.lo + 1;
-    gq[4] = oy.lo, gq[5] = ox.lo, gq[6] = empty ? 0 : oy.hi - oy.lo + 1, gq[7] = empty ? 0 : ox.hi - ox.lo + 1;
-  }
-  __syncthreads();
-  const int taps = Kh * Kw, cgroups = Cout / CPT;
-  for (int i = threadIdx.x; i < nr * owh * oww * cgroups; i += blockDim.x) {
-    const int co = (i % cgroups) * CPT, q = i / cgroups;
-    const int x = q % oww, y = (q / oww) % owh, lr = q / (oww * owh);
-    const int* gq = s_geo[lr];
-    float ac[CPT], ar[CPT];
+  __shared__ CwRow s_row[kCwMaxRows];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, Kh = KS ? KS : q.Kh, Kw = KS ? KS : q.Kw, taps = Kh * Kw;
+  if ((int)blockIdx.x < q.blocks_bias) {   // an ordinary convolution of one image, a thread per output
+    const int64_t total = (int64_t)q.Cout * q.Ho * q.Wo;
+    for (int64_t t = (int64_t)blockIdx.x * kCwConvThreads + tid; t < total; t += (int64_t)q.blocks_bias * kCwConvThreads) {
+      const int ow = (int)(t % q.Wo), oh = (int)((t / q.Wo) % q.Ho), co = (int)(t / ((int64_t)q.Wo * q.Ho));
+      const int ih0 = oh * q.stride - q.pad, iw0 = ow * q.stride - q.pad;
+      float ac = 0.f, ar = 0.f;
+#pragma unroll 2
+      for (int c = 0; c < q.Cin; ++c) {
+        const float* wp = q.Wt + ((int64_t)co * q.Cin + c) * taps;
+        const int64_t plane = (int64_t)c * q.H * q.W;
 #pragma unroll
-    for (int e = 0; e < CPT; ++e) { ac[e] = 0.f; ar[e] = 0.f; }
-    const bool live = y < gq[6] && x < gq[7];
-    if (live) {
-      const int iy0 = (gq[4] + y) * stride - pad - gq[0], ix0 = (gq[5] + x) * stride - pad - gq[1];   // window coordinates
-      const int ky0 = max(0, -iy0), ky1 = min(Kh, gq[2] - iy0), kx0 = max(0, -ix0), kx1 = min(Kw, gq[3] - ix0);
-      const float2* xp = s_x + (lr * Cin * iwh + iy0) * iww + ix0;
-      const float* wp = s_w + co;
-      for (int c = 0; c < Cin; ++c, xp += iwh * iww, wp += taps * ldw)
-        for (int ky = ky0; ky < ky1; ++ky)
-          for (int kx = kx0; kx < kx1; ++kx) {
-            const float2 v = xp[ky * iww + kx];
-            if (CPT == 4) {
-              const float4 w = *reinterpret_cast<const float4*>(wp + (ky * Kw + kx) * ldw);
-              ac[0] = fmaf(v.x, w.x, ac[0]); ar[0] = fmaf(v.y, fabsf(w.x), ar[0]);
-              ac[1 % CPT] = fmaf(v.x, w.y, ac[1 % CPT]); ar[1 % CPT] = fmaf(v.y, fabsf(w.y), ar[1 % CPT]);
-              ac[2 % CPT] = fmaf(v.x, w.z, ac[2 % CPT]); ar[2 % CPT] = fmaf(v.y, fabsf(w.z), ar[2 % CPT]);
-              ac[3 % CPT] = fmaf(v.x, w.w, ac[3 % CPT]); ar[3 % CPT] = fmaf(v.y, fabsf(w.w), ar[3 % CPT]);
-            } else {
-              const float w = wp[(ky * Kw + kx) * ldw];
-              ac[0] = fmaf(v.x, w, ac[0]);
-              ar[0] = fmaf(v.y, fabsf(w), ar[0]);
+        for (int kh = 0; kh < (KS ? KS : Kh); ++kh)
+#pragma unroll
+          for (int kw = 0; kw < (KS ? KS : Kw); ++kw) {
+            const int ih = ih0 + kh, iw = iw0 + kw;
+            const bool in = ih >= 0 && ih < q.H && iw >= 0 && iw < q.W;
+            const int64_t o = plane + (int64_t)ih * q.W + iw;
+            const float w = __ldg(wp + kh * Kw + kw), lo = in ? __ldg(q.b_lo + o) : 0.f, up = in ? __ldg(q.b_up + o) : 0.f;
+            ac = fmaf(fmul(fadd(lo, up), 0.5f), w, ac);
+            ar = fmaf(fmul(fsub(up, lo), 0.5f), fabsf(w), ar);
+          }
+      }
+      float lo = fsub(ac, ar), up = fadd(ac, ar);
+      if (q.bias != nullptr) { lo = fadd(lo, q.bias[co]); up = fadd(up, q.bias[co]); }
+      q.yb_lo[t] = lo;
+      q.yb_up[t] = up;
+    }
+    return;
+  }
+  const int bid = blockIdx.x - q.blocks_bias, cls = bid / q.per_class, chunk = bid - cls * q.per_class;
+  const int ry = cls / q.cls_x, rx = cls % q.cls_x, n_rows = q.G * kCwR;
+  {
+    const int ny = (q.H0 - ry + q.S - 1) / q.S, nx = (q.W0 - rx + q.S - 1) / q.S, n_cls = q.n_ci * ny * nx;
+    if (chunk * n_rows >= n_cls) return;
+    bool live = false;
+    if (tid < n_rows) {
+      const int k = chunk * n_rows + tid;
+      CwRow r;
+      r.lr = -1;
+      const int kx = k % nx, ky = (k / nx) % ny;
+      r.xi = rx + q.S * kx;
+      r.yi = ry + q.S * ky;
+      r.ci = q.ci0 + k / (nx * ny);
+      if (k < n_cls) {
+        const int64_t lr = ((int64_t)r.ci * q.H0 + r.yi) * q.W0 + r.xi - q.row_start;
+        if (lr >= 0 && lr < q.rows) r.lr = (int)lr;
+      }
+      live = r.lr >= 0;
+      Span wy, wx, vy, vx;
+      chain_window(q.ch, q.H0, q.W0, r.yi, r.xi, wy, wx);
+      chain_window_free(q.ch, r.yi, r.xi, vy, vx);
+      r.uy = vy.lo, r.ux = vx.lo;
+      r.iy = wy.lo, r.ix = wx.lo, r.ih = wy.hi - wy.lo + 1, r.iw = wx.hi - wx.lo + 1;
+      const Span oy = span_after_conv(wy, q.Kh, q.stride, q.pad, q.Ho), ox = span_after_conv(wx, q.Kw, q.stride, q.pad, q.Wo);
+      const bool empty = wy.lo > wy.hi || wx.lo > wx.hi || oy.lo > oy.hi || ox.lo > ox.hi;
+      r.oy = oy.lo, r.ox = ox.lo, r.oh = empty ? 0 : oy.hi - oy.lo + 1, r.ow = empty ? 0 : ox.hi - ox.lo + 1;
+      r.voy = span_after_conv_free(vy, q.Kh, q.stride, q.pad).lo;
+      r.vox = span_after_conv_free(vx, q.Kw, q.stride, q.pad).lo;
+      s_row[tid] = r;
+    }
+    if (!__syncthreads_or(live)) return;
+  }
+  // geometry of the class, from its first pixel
+  Span vy, vx;
+  chain_window_free(q.ch, ry, rx, vy, vx);
+  const Span wy = span_after_conv_free(vy, q.Kh, q.stride, q.pad), wx = span_after_conv_free(vx, q.Kw, q.stride, q.pad);
+  const int ih = max(0, vy.hi - vy.lo + 1), iw = max(0, vx.hi - vx.lo + 1);
+  const int oh = ih > 0 ? max(0, wy.hi - wy.lo + 1) : 0, ow = iw > 0 ? max(0, wx.hi - wx.lo + 1) : 0;
+  const int ty0 = wy.lo * q.stride - q.pad - vy.lo, tx0 = wx.lo * q.stride - q.pad - vx.lo;   // first tap of the first output
+  const int npos = oh * ow, ldw = q.Cout + 1, n_w = q.CC * taps * ldw;
+  float2* s_w = reinterpret_cast<float2*>(cw_smem);            // [CC][Kh][Kw][ldw] (w, |w|)
+  float2* s_x = s_w + n_w + (n_w & 1);                         // [CC][uih][uiw][G * 8] (centre, radius)
+  const bool once = q.CC >= q.Cin;
+  const int items = q.G * npos * q.Cout;
+  for (int i0 = 0; i0 < items; i0 += kCwConvThreads) {
+    const int item = i0 + tid, co = item % q.Cout, pos = (item / q.Cout) % max(npos, 1), g = item / (q.Cout * max(npos, 1));
+    const int py = pos / max(ow, 1), px = pos - py * ow;
+    const int by = ty0 + py * q.stride, bx = tx0 + px * q.stride;
+    const int ky0 = max(0, -by), ky1 = min(Kh, ih - by), kx0 = max(0, -bx), kx1 = min(Kw, iw - bx);
+    uint64_t acc[kCwR];
+#pragma unroll
+    for (int j = 0; j < kCwR; ++j) acc[j] = 0;
+    for (int c0 = 0; c0 < q.Cin; c0 += q.CC) {
+      const int cc = min(q.CC, q.Cin - c0);
+      if (!once || i0 == 0) {
+        if (i0 > 0 || c0 > 0) __syncthreads();
+        const int wn = cc * taps;
+        for (int o = warp; o < q.Cout; o += kCwConvThreads / 32) {   // lanes along (channel, tap)
+          const float* src = q.Wt + ((int64_t)o * q.Cin + c0) * taps;
+#pragma unroll 4
+          for (int t = lane; t < wn; t += 32) {
+            const float w = __ldg(src + t);
+            s_w[t * ldw + o] = make_float2(w, fabsf(w));
+          }
+        }
+        if (q.W1 != nullptr) {
+          // lanes along the rows (n_rows <= 32): neighbouring columns of the slopes
+          const CwRow r = s_row[min(lane, n_rows - 1)];
+#pragma unroll 3
+          for (int u = warp; u < cc * ih * iw; u += kCwConvThreads / 32) {
+            const int ux = u % iw, uy = (u / iw) % ih, c = u / (iw * ih), y = r.uy + uy, x = r.ux + ux;
+            const int ky = r.yi - (y * q.ch.stride[0] - q.ch.pad[0]), kx = r.xi - (x * q.ch.stride[0] - q.ch.pad[0]);
+            const bool in = r.lr >= 0 && y >= 0 && y < q.H && x >= 0 && x < q.W && ky >= 0 && ky < q.ch.kh[0] && kx >= 0 && kx < q.ch.kw[0];
+            const int64_t col = in ? ((int64_t)(c0 + c) * q.H + y) * q.W + x : 0;
+            const float w = in ? __ldg(q.W1 + (((int64_t)(c0 + c) * q.Cin0 + r.ci) * q.ch.kh[0] + ky) * q.ch.kw[0] + kx) : 0.f;
+            const float kl = __ldg(q.k_l + col), ku = __ldg(q.k_u + col);
+            const float tap = fmul(q.scale, w), lo = fmul(tap, kl), up = fmul(tap, ku);
+            if (lane < n_rows)
+              s_x[((c * q.uih + uy) * q.uiw + ux) * n_rows + lane] =
+                  in ? make_float2(fmul(fadd(lo, up), 0.5f), fmul(fsub(up, lo), 0.5f)) : make_float2(0.f, 0.f);
+          }
+        } else {
+          // lanes along the channel: neighbouring words of a row
+          for (int u = warp; u < ih * iw * n_rows; u += kCwConvThreads / 32) {
+            const int t = u % n_rows, v = u / n_rows, ux = v % iw, uy = v / iw;
+            const CwRow& r = s_row[t];
+            const int dy = r.uy + uy - r.iy, dx = r.ux + ux - r.ix;
+            const bool in = r.lr >= 0 && dy >= 0 && dy < r.ih && dx >= 0 && dx < r.iw;
+            const int64_t o = (((int64_t)r.lr * q.iwh + dy) * q.iww + dx) * q.Cin + c0;
+#pragma unroll 2
+            for (int c = lane; c < cc; c += 32) {
+              const float lo = in ? __ldg(q.z_lo + o + c) : 0.f, up = in ? __ldg(q.z_up + o + c) : 0.f;
+              s_x[((c * q.uih + uy) * q.uiw + ux) * n_rows + t] = make_float2(fmul(fadd(lo, up), 0.5f), fmul(fsub(up, lo), 0.5f));
             }
           }
-    }
+        }
+        __syncthreads();
+      }
+      if (item < items) {
+        const float2* xc = s_x + ((int64_t)by * q.uiw + bx) * n_rows + g * kCwR;
+        const float2* wc = s_w + co;
+        for (int c = 0; c < cc; ++c, xc += q.uih * q.uiw * n_rows, wc += taps * ldw)
+          for (int ky = ky0; ky < ky1; ++ky) {
+            const float2* xp = xc + (ky * q.uiw + kx0) * n_rows;
+            const float2* wp = wc + (ky * Kw + kx0) * ldw;
+#pragma unroll 3
+            for (int kx = kx0; kx < kx1; ++kx, xp += n_rows, wp += ldw) {
+              const uint64_t w = *reinterpret_cast<const uint64_t*>(wp);
 #pragma unroll
-    for (int e = 0; e < CPT; ++e) {
-      const int64_t o = (lr0 + lr) * n_out + ((int64_t)(co + e) * owh + y) * oww + x;
-      y_lo[o] = live ? fsub(ac[e], ar[e]) : 0.f;
-      y_up[o] = live ? fadd(ac[e], ar[e]) : 0.f;
-    }
-  }
-}
-
-// Unfinished dual-norm accumulation of every column (c, y, x) over the rows [row_start, row_start + rows): a gather over
-// the pixels whose window holds (y, x).  The spans of all pixel coordinates are tabulated in shared memory first
-// (H0 + W0 entries); a warp takes a column, its lanes interleave over the candidate pixels (the pixel rows and columns
-// between the first and the last whose span holds y resp. x), and the lane sums are combined by a butterfly: the order
-// of the additions is fixed by the geometry alone, so the result does not depend on scheduling.
-__global__ void __launch_bounds__(256)
-cw_norm_partials_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw, float* __restrict__ part_l,
-                        float* __restrict__ part_u, int64_t rows, int64_t row_start, int Cin0, const CwShape g, int p) {
-  extern __shared__ int cw_spans[];   // ylo[H0], yhi[H0], xlo[W0], xhi[W0], then ya[H], yb[H], xa[W], xb[W]
-  int* ylo = cw_spans;
-  int* yhi = ylo + g.H0;
-  int* xlo = yhi + g.H0;
-  int* xhi = xlo + g.W0;
-  int* t_ya = xhi + g.W0;
-  int* t_yb = t_ya + g.H;
-  int* t_xa = t_yb + g.H;
-  int* t_xb = t_xa + g.W;
-  for (int i = threadIdx.x; i < g.H0 + g.W0; i += blockDim.x) {
-    Span wy, wx;
-    if (i < g.H0) {
-      chain_window(g.ch, g.H0, g.W0, i, 0, wy, wx);
-      ylo[i] = wy.lo, yhi[i] = wy.hi;
-    } else {
-      chain_window(g.ch, g.H0, g.W0, 0, i - g.H0, wy, wx);
-      xlo[i - g.H0] = wx.lo, xhi[i - g.H0] = wx.hi;
-    }
-  }
-  __syncthreads();
-  // per dense coordinate: first and last pixel row / column whose span holds it
-  for (int i = threadIdx.x; i < g.H + g.W; i += blockDim.x) {
-    const bool is_y = i < g.H;
-    const int v = is_y ? i : i - g.H, n0 = is_y ? g.H0 : g.W0;
-    const int* lo = is_y ? ylo : xlo;
-    const int* hi = is_y ? yhi : xhi;
-    int a = n0, b = -1;
-    for (int k = 0; k < n0; ++k)
-      if (v >= lo[k] && v <= hi[k]) { a = min(a, k); b = k; }
-    (is_y ? t_ya : t_xa)[v] = a;
-    (is_y ? t_yb : t_xb)[v] = b;
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int64_t ncol = (int64_t)g.C * g.H * g.W, per_row = (int64_t)g.C * g.wh * g.ww;
-  const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ncol; t += warps) {
-    const int x = (int)(t % g.W), y = (int)((t / g.W) % g.H), c = (int)(t / ((int64_t)g.W * g.H));
-    const int ya = t_ya[y], yb = t_yb[y], xa = t_xa[x], xb = t_xb[x];
-    float al = 0.f, au = 0.f;
-    if (yb >= ya && xb >= xa) {
-      const int ny = yb - ya + 1, nx = xb - xa + 1, cand = Cin0 * ny * nx;
-      for (int k = lane; k < cand; k += 32) {
-        const int xi = xa + k % nx, yi = ya + (k / nx) % ny, ci = k / (nx * ny);
-        if (y < ylo[yi] || y > yhi[yi] || x < xlo[xi] || x > xhi[xi]) continue;
-        const int64_t lr = ((int64_t)ci * g.H0 + yi) * g.W0 + xi - row_start;
-        if (lr < 0 || lr >= rows) continue;
-        const int64_t o = lr * per_row + ((int64_t)c * g.wh + (y - ylo[yi])) * g.ww + (x - xlo[xi]);
-        al = norm_accum(p, al, __ldg(z_lw + o));
-        au = norm_accum(p, au, __ldg(z_uw + o));
+              for (int j = 0; j < kCwR; j += 2) {
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(xp + j);
+                acc[j] = fma2(v.x, w, acc[j]);
+                acc[j + 1] = fma2(v.y, w, acc[j + 1]);
+              }
+            }
+          }
       }
     }
+    if (item < items) {
 #pragma unroll
-    for (int sft = 16; sft > 0; sft >>= 1) {
-      al = norm_combine(p, al, __shfl_xor_sync(0xffffffffu, al, sft));
-      au = norm_combine(p, au, __shfl_xor_sync(0xffffffffu, au, sft));
+      for (int j = 0; j < kCwR; ++j) {
+        const CwRow& r = s_row[g * kCwR + j];
+        const int dy = r.voy + py - r.oy, dx = r.vox + px - r.ox;
+        if (r.lr >= 0 && dy >= 0 && dy < r.oh && dx >= 0 && dx < r.ow) {
+          const float2 v = unpack2(acc[j]);
+          const int64_t o = (((int64_t)r.lr * q.owh + dy) * q.oww + dx) * q.Cout + co;
+          q.y_lo[o] = fsub(v.x, v.y);
+          q.y_up[o] = fadd(v.x, v.y);
+        }
+      }
     }
-    if (lane == 0) {
-      part_l[t] = al;
-      part_u[t] = au;
+  }
+  // zeros where a row's window is smaller than the largest one
+  for (int t = 0; t < n_rows; ++t) {
+    const CwRow& r = s_row[t];
+    if (r.lr < 0 || (r.oh == q.owh && r.ow == q.oww)) continue;
+    for (int f = tid; f < q.owh * q.oww * q.Cout; f += kCwConvThreads) {
+      const int u = f / q.Cout, dx = u % q.oww, dy = u / q.oww;
+      if (dy < r.oh && dx < r.ow) continue;
+      const int64_t o = (int64_t)r.lr * q.owh * q.oww * q.Cout + f;
+      q.y_lo[o] = 0.f;
+      q.y_up[o] = 0.f;
     }
   }
 }
 
-// Relaxation coefficients per column from the (reduced) norms; the relaxed bias terms are written to out_lb / out_ub.
+// Dual-norm accumulation of every column (c, y, x) over the rows [row_start, row_start + rows): a gather over the pixels whose
+// window holds (y, x).  A block takes one position and 32 channels; its warps interleave over the candidate pixels (the hull of
+// the position's receptive field, whose spans are tabulated in shared memory) and read 32 consecutive words of a row; their sums
+// are combined in the order of the warps, so the result depends on the geometry alone.
+// op < 0: the unfinished accumulations go to part_l / part_u.  Otherwise the relaxation's coefficients follow at once (no
+// exchange between ranks in between): out_lb / out_ub receive the relaxed bias terms, coef as cw_relax_columns_kernel writes it.
+// 3072 rows of 3 x 3 x 32 windows, 8192 columns: 13 us with a warp per column of channel-major rows, whose 32 lanes touch 32
+// sectors per load.
+constexpr int kCwNormWarps = 16, kCwNormLoads = 4;
+
+__device__ __forceinline__ void cw_relax_column(int op, float lbv, float ubv, float nl, float nu, int p, float eps, int64_t dense,
+                                                int64_t at, int64_t ncol, float* out_lb, float* out_ub, float* coef, int* violation) {
+  const float l = fadd(lbv, fmul(-eps, norm_finish(p, nl)));
+  const float u = fadd(ubv, fmul(eps, norm_finish(p, nu)));
+  bool bad = false;
+  const ColCoef c = relax_column(op, l, u, lbv, ubv, bad);
+  if (bad && violation != nullptr) *violation = 1;
+  out_lb[dense] = c.nlb;
+  out_ub[dense] = c.nub;
+  coef[at] = c.c_ll;
+  coef[ncol + at] = c.c_lu;
+  coef[2 * ncol + at] = c.c_ul;
+  coef[3 * ncol + at] = c.c_uu;
+}
+
+__global__ void __launch_bounds__(32 * kCwNormWarps)
+cw_norm_kernel(int op, const float* __restrict__ z_lw, const float* __restrict__ z_uw, float* __restrict__ part_l,
+               float* __restrict__ part_u, const float* __restrict__ lb, const float* __restrict__ ub, float* __restrict__ out_lb,
+               float* __restrict__ out_ub, float* __restrict__ coef, int64_t rows, int64_t row_start, int Cin0, const CwShape g, int p,
+               float eps, int* __restrict__ violation) {
+  extern __shared__ int2 cw_spans[];   // windows of the candidate pixel rows, then columns
+  __shared__ float s_part[2][kCwNormWarps][32];
+  const int y = blockIdx.x / g.W, x = blockIdx.x - y * g.W, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = blockIdx.y * 32 + lane;
+  const Span py = chain_pixels(g.ch, g.ch.kh, {y, y}, g.H0), px = chain_pixels(g.ch, g.ch.kw, {x, x}, g.W0);
+  const int ny = max(0, py.hi - py.lo + 1), nx = max(0, px.hi - px.lo + 1);
+  for (int i = threadIdx.x; i < ny + nx; i += blockDim.x) {
+    Span wy, wx;
+    chain_window(g.ch, g.H0, g.W0, i < ny ? py.lo + i : 0, i < ny ? 0 : px.lo + i - ny, wy, wx);
+    cw_spans[i] = i < ny ? make_int2(wy.lo, wy.hi) : make_int2(wx.lo, wx.hi);
+  }
+  __syncthreads();
+  float al = 0.f, au = 0.f;
+  for (int k = warp; k < Cin0 * ny; k += kCwNormWarps) {
+    const int ky = k % ny, ci = k / ny;
+    const int2 wy = cw_spans[ky];
+    if (y < wy.x || y > wy.y) continue;
+    const int64_t lr0 = ((int64_t)ci * g.H0 + py.lo + ky) * g.W0 + px.lo - row_start;
+    for (int kx = 0; kx < nx; kx += kCwNormLoads) {
+      float vl[kCwNormLoads], vu[kCwNormLoads];   // zeros leave every norm as it is
+#pragma unroll
+      for (int e = 0; e < kCwNormLoads; ++e) {
+        const int2 wx = cw_spans[ny + min(kx + e, nx - 1)];
+        const int64_t lr = lr0 + kx + e;
+        const bool in = kx + e < nx && x >= wx.x && x <= wx.y && lr >= 0 && lr < rows && c < g.C;
+        const int64_t o = in ? ((lr * g.wh + (y - wy.x)) * g.ww + (x - wx.x)) * g.C + c : 0;
+        vl[e] = in ? __ldg(z_lw + o) : 0.f;
+        vu[e] = in ? __ldg(z_uw + o) : 0.f;
+      }
+#pragma unroll
+      for (int e = 0; e < kCwNormLoads; ++e) {
+        al = norm_accum(p, al, vl[e]);
+        au = norm_accum(p, au, vu[e]);
+      }
+    }
+  }
+  s_part[0][warp][lane] = al;
+  s_part[1][warp][lane] = au;
+  __syncthreads();
+  if (warp != 0 || c >= g.C) return;
+#pragma unroll
+  for (int w = 1; w < kCwNormWarps; ++w) {
+    al = norm_combine(p, al, s_part[0][w][lane]);
+    au = norm_combine(p, au, s_part[1][w][lane]);
+  }
+  const int64_t dense = ((int64_t)c * g.H + y) * g.W + x;
+  if (op < 0) {
+    part_l[dense] = al;
+    part_u[dense] = au;
+  } else {
+    cw_relax_column(op, lb[dense], ub[dense], al, au, p, eps, dense, (int64_t)blockIdx.x * g.C + c, (int64_t)g.C * g.H * g.W, out_lb, out_ub,
+                    coef, violation);
+  }
+}
+
+// Relaxation coefficients per column from the (reduced) norms, coef [4][H * W][C]; the relaxed bias terms go to out_lb / out_ub.
 __global__ void __launch_bounds__(256)
 cw_relax_columns_kernel(int op, const float* __restrict__ lb, const float* __restrict__ ub, const float* __restrict__ norm_l,
                         const float* __restrict__ norm_u, float* __restrict__ out_lb, float* __restrict__ out_ub,
-                        float* __restrict__ coef /* [4][ncol] */, int64_t ncol, int p, float eps, int* __restrict__ violation) {
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < ncol; t += (int64_t)gridDim.x * blockDim.x) {
-    const float lbv = lb[t], ubv = ub[t];
-    const float l = fadd(lbv, fmul(-eps, norm_finish(p, norm_l[t])));
-    const float u = fadd(ubv, fmul(eps, norm_finish(p, norm_u[t])));
-    bool bad = false;
-    const ColCoef c = relax_column(op, l, u, lbv, ubv, bad);
-    if (bad && violation != nullptr) *violation = 1;
-    out_lb[t] = c.nlb;
-    out_ub[t] = c.nub;
-    coef[t] = c.c_ll;
-    coef[ncol + t] = c.c_lu;
-    coef[2 * ncol + t] = c.c_ul;
-    coef[3 * ncol + t] = c.c_uu;
-  }
+                        float* __restrict__ coef, int C, int64_t hw, int p, float eps, int* __restrict__ violation) {
+  const int64_t ncol = C * hw;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < ncol; t += (int64_t)gridDim.x * blockDim.x)
+    cw_relax_column(op, lb[t], ub[t], norm_l[t], norm_u[t], p, eps, t, (t % hw) * C + t / hw, ncol, out_lb, out_ub, coef, violation);
 }
 
 // Rescale of a relaxation on compact rows: out_lw = c_ll lw + c_lu uw, out_uw = c_uu uw + c_ul lw (the expressions of
 // the dense kernel).  A warp per row: the window is worked out once, the lanes interleave over its elements.
+__device__ __forceinline__ void cw_rescale(const float* __restrict__ coef, int64_t ncol, int64_t col, float a, float b, float& lo,
+                                           float& up) {
+  lo = fmaf(__ldg(coef + col), a, fmul(__ldg(coef + ncol + col), b));
+  up = fmaf(__ldg(coef + 3 * ncol + col), b, fmul(__ldg(coef + 2 * ncol + col), a));
+}
+
 __global__ void __launch_bounds__(256)
 cw_rescale_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw, const float* __restrict__ coef,
                   float* __restrict__ o_lw, float* __restrict__ o_uw, int64_t rows, int64_t row_start, const CwShape g) {
@@ -264,90 +412,199 @@ cw_rescale_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw
   const bool empty = wy.lo > wy.hi || wx.lo > wx.hi;
   const int ah = wy.hi - wy.lo + 1, aw = wx.hi - wx.lo + 1;
   for (int e = lane; e < per_row; e += 32) {
-    const int dx = e % g.ww, dy = (e / g.ww) % g.wh, c = e / (g.ww * g.wh);
+    const int c = e % g.C, dx = (e / g.C) % g.ww, dy = e / (g.C * g.ww);
     float lo = 0.f, up = 0.f;
     if (!empty && dy < ah && dx < aw) {
-      const int64_t col = ((int64_t)c * g.H + wy.lo + dy) * g.W + wx.lo + dx;
-      const float a = z_lw[lr * per_row + e], b = z_uw[lr * per_row + e];
-      lo = fmaf(coef[col], a, fmul(coef[ncol + col], b));
-      up = fmaf(coef[3 * ncol + col], b, fmul(coef[2 * ncol + col], a));
+      const int64_t col = ((int64_t)(wy.lo + dy) * g.W + wx.lo + dx) * g.C + c;
+      cw_rescale(coef, ncol, col, z_lw[lr * per_row + e], z_uw[lr * per_row + e], lo, up);
     }
     o_lw[lr * per_row + e] = lo;
     o_uw[lr * per_row + e] = up;
   }
 }
 
-// Linear layer on compact rows (weight part): y[r, n] = sum_e c_e W[n, col(e)] -/+ r_e |W[n, col(e)]|.  One warp per
-// (row, group of kCwNB outputs): the lanes interleave over the elements, partial sums are combined by shuffles.
-// The weight is read as WT [F, N] (the transpose of the nn.Linear layout, made once per call by cw_transpose_kernel): the
-// kCwNB weights of an element are then consecutive words, while in the [N, F] layout every one of them is a sector of
-// its own (measured on the 8192 -> 10 head: 37 us against 9 us).
-constexpr int kCwNB = 16;
-__global__ void __launch_bounds__(256)
-cw_linear_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw, const float* __restrict__ WT,
-                 float* __restrict__ y_lw, float* __restrict__ y_uw, int64_t rows, int64_t row_start, const CwShape g, int N) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int groups = (N + kCwNB - 1) / kCwNB;
-  const int64_t lr = warp / groups;
-  if (lr >= rows) return;
-  const int n0 = (int)(warp % groups) * kCwNB;
-  const int per_row = g.C * g.wh * g.ww;
-  int yi, xi;
-  pixel_of_row(row_start + lr, g.H0, g.W0, yi, xi);
+// Linear layer on compact rows: y[r, n] = sum_e c_e W[n, col(e)] -/+ r_e |W[n, col(e)]|, where (coef != nullptr) the rows go
+// through the rescale of a relaxation on the way.  A block takes the pixels of one image row, kCwPx of its columns and every
+// channel of the image: their windows overlap, so the weights they need (the union of the windows) are staged in shared memory
+// once, [position][32 channels][NB outputs], 32 channels and as many rows of positions at a time as fit.  A warp owns a row
+// of the result, its lanes the channels; the sums over the lanes go through a transposing butterfly (31 shuffles for 32 values).
+// Where this is the last layer (part != nullptr), the rows are not written: what is left of them is their dual norm, one partial
+// accumulation per block, tile and output.  The first bias_blocks blocks compute the bias part, an output each.
+// Bound by L2 reads: with W^T in global memory every row read its own copy of the weights (20 us and 2 us for the transpose at
+// 3072 rows, 288 elements, 10 outputs, and 9 us to write the rescaled rows first).
+constexpr int kCwPx = 8, kCwLinWarps = 24, kCwLinThreads = 32 * kCwLinWarps;   // 24: the rows of 8 pixels of 3 channels
+
+struct CwLinearArgs {
+  const float *z_lw, *z_uw, *coef, *W;
+  float *y_lw, *y_uw, *part;
+  const float *lb, *ub, *bias;
+  float *y_lb, *y_ub;
+  int bias_blocks;
+  int64_t rows, row_start;
+  int ci0, n_ci, N, nb, ny_max, nx_max, p;
+  CwShape g;
+};
+
+template <int NB>
+__global__ void __launch_bounds__(kCwLinThreads)
+cw_linear_kernel(const CwLinearArgs q) {
+  constexpr int LDN = NB + 2, LDP = 32 * LDN + 2;   // the lanes' 64-bit reads, along the channels, and the stores, along the
+                                                    // positions, fall on different banks
+  extern __shared__ __align__(16) float cw_smem[];
+  __shared__ float s_red[2][kCwLinWarps][16];
+  __shared__ int2 s_win[kCwPx];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const CwShape& g = q.g;
+  const int64_t ncol = (int64_t)g.C * g.H * g.W;
+  if ((int)blockIdx.x < q.bias_blocks) {
+    if (blockIdx.y > 0) return;
+    const float* w = q.W + (int64_t)blockIdx.x * ncol;
+    float c = 0.f, r = 0.f;
+#pragma unroll 4
+    for (int64_t f = tid; f < ncol; f += kCwLinThreads) {
+      const float lo = __ldg(q.lb + f), up = __ldg(q.ub + f), v = __ldg(w + f);
+      c = fmaf(fmul(fadd(lo, up), 0.5f), v, c);
+      r = fmaf(fmul(fsub(up, lo), 0.5f), fabsf(v), r);
+    }
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+      c += __shfl_xor_sync(0xffffffffu, c, s);
+      r += __shfl_xor_sync(0xffffffffu, r, s);
+    }
+    if (lane == 0) s_red[0][warp][0] = c, s_red[1][warp][0] = r;
+    __syncthreads();
+    if (tid == 0) {
+      for (int i = 1; i < kCwLinWarps; ++i) c += s_red[0][i][0], r += s_red[1][i][0];
+      const float b = q.bias != nullptr ? q.bias[blockIdx.x] : 0.f;
+      q.y_lb[blockIdx.x] = fadd(fsub(c, r), b);
+      q.y_ub[blockIdx.x] = fadd(fadd(c, r), b);
+    }
+    return;
+  }
+  const int tiles_x = (g.W0 + kCwPx - 1) / kCwPx, tile = blockIdx.x - q.bias_blocks;
+  const int yi = tile / tiles_x, x0 = (tile - yi * tiles_x) * kCwPx, npx = min(kCwPx, g.W0 - x0);
+  const int n0 = blockIdx.y * q.nb, nb = min(q.nb, q.N - n0);
+  if (tid < kCwPx) {
+    Span ty, tx;
+    chain_window(g.ch, g.H0, g.W0, yi, min(x0 + tid, g.W0 - 1), ty, tx);
+    s_win[tid] = make_int2(tx.lo, tx.hi);
+  }
+  __syncthreads();
   Span wy, wx;
-  chain_window(g.ch, g.H0, g.W0, yi, xi, wy, wx);
-  const int ah = wy.hi - wy.lo + 1, aw = wx.hi - wx.lo + 1;
-  float sc[kCwNB], sr[kCwNB];
+  chain_window(g.ch, g.H0, g.W0, yi, x0, wy, wx);
+  int xl = g.W, xh = -1;
 #pragma unroll
-  for (int j = 0; j < kCwNB; ++j) { sc[j] = 0.f; sr[j] = 0.f; }
-  if (wy.lo <= wy.hi && wx.lo <= wx.hi) {
-    const float* zl = z_lw + lr * per_row;
-    const float* zu = z_uw + lr * per_row;
+  for (int i = 0; i < kCwPx; ++i)
+    if (s_win[i].x <= s_win[i].y) { xl = min(xl, s_win[i].x); xh = max(xh, s_win[i].y); }
+  const int nxr = max(0, xh - xl + 1), rows_here = npx * q.n_ci;
+  const int64_t per_pos = g.C, per_row = (int64_t)g.wh * g.ww * g.C;
+  float pl = 0.f, pu = 0.f;   // accumulated norms of this lane's output
+  for (int r0 = 0; r0 < rows_here; r0 += kCwLinWarps) {
+    float sc[NB], sr[NB];
+#pragma unroll
+    for (int n = 0; n < NB; ++n) sc[n] = sr[n] = 0.f;
+    const int t = r0 + warp, px = t % npx, ci = q.ci0 + t / npx;
+    int64_t lr = -1;
+    int2 win = make_int2(1, 0);
+    if (t < rows_here) {
+      const int64_t l = ((int64_t)ci * g.H0 + yi) * g.W0 + x0 + px - q.row_start;
+      if (l >= 0 && l < q.rows) { lr = l; win = s_win[px]; }
+    }
+    const int aw = win.y - win.x + 1;
+    for (int c0 = 0; c0 < g.C; c0 += 32) {
+      const int c = c0 + lane;
+      for (int ya = wy.lo; ya <= wy.hi; ya += q.ny_max) {
+        const int yb = min(wy.hi, ya + q.ny_max - 1), npos = (yb - ya + 1) * nxr;
+        __syncthreads();
+        for (int pos = lane; pos < npos; pos += 32) {   // a warp per (output, channel), lanes along the positions
+          const int yy = pos / nxr;
+          const float* src = q.W + (int64_t)n0 * ncol + ((int64_t)c0 * g.H + ya + yy) * g.W + xl + pos - yy * nxr;
+#pragma unroll 8
+          for (int u = warp; u < 32 * NB; u += kCwLinWarps) {
+            const int cl = u % 32, n = u / 32;
+            const float w = n < nb && c0 + cl < g.C ? __ldg(src + n * ncol + (int64_t)cl * g.H * g.W) : 0.f;
+            cw_smem[pos * LDP + cl * LDN + n] = w;
+          }
+        }
+        __syncthreads();
+        if (lr >= 0 && c < g.C) {
+          const int n_el = (yb - ya + 1) * aw;
+          const int64_t zb = lr * per_row + (int64_t)(ya - wy.lo) * g.ww * per_pos + c;
 #pragma unroll 3
-    for (int e = lane; e < per_row; e += 32) {
-      const int dx = e % g.ww, dy = (e / g.ww) % g.wh, c = e / (g.ww * g.wh);
-      if (dy >= ah || dx >= aw) continue;
-      const float lo = zl[e], up = zu[e];
-      const float vc = fmul(fadd(lo, up), 0.5f), vr = fmul(fsub(up, lo), 0.5f);
-      const int64_t col = ((int64_t)c * g.H + wy.lo + dy) * g.W + wx.lo + dx;
-      const float* wp = WT + col * N + n0;
+          for (int k = 0; k < n_el; ++k) {
+            const int dy = k / aw, dx = k - dy * aw;
+            const int64_t o = zb + (dy * g.ww + dx) * per_pos;
+            float lo = __ldg(q.z_lw + o), up = __ldg(q.z_uw + o);
+            if (q.coef != nullptr) {
+              const float a = lo, b = up;
+              cw_rescale(q.coef, ncol, ((int64_t)(ya + dy) * g.W + win.x + dx) * g.C + c, a, b, lo, up);
+            }
+            const float vc = fmul(fadd(lo, up), 0.5f), vr = fmul(fsub(up, lo), 0.5f);
+            const float2* w = reinterpret_cast<const float2*>(cw_smem + (dy * nxr + win.x - xl + dx) * LDP + lane * LDN);
 #pragma unroll
-      for (int j = 0; j < kCwNB; ++j) {
-        if (n0 + j < N) {
-          const float w = __ldg(wp + j);
-          sc[j] = fmaf(vc, w, sc[j]);
-          sr[j] = fmaf(vr, fabsf(w), sr[j]);
+            for (int n = 0; n < NB; n += 2) {
+              const float2 v = w[n / 2];
+              sc[n] = fmaf(vc, v.x, sc[n]);
+              sr[n] = fmaf(vr, fabsf(v.x), sr[n]);
+              sc[n + 1] = fmaf(vc, v.y, sc[n + 1]);
+              sr[n + 1] = fmaf(vr, fabsf(v.y), sr[n + 1]);
+            }
+          }
         }
       }
     }
+    // lane i ends with the sum of value i of (sc[0 .. 15], sr[0 .. 15])
+    float v[32];
+#pragma unroll
+    for (int n = 0; n < 16; ++n) {
+      v[n] = n < NB ? sc[n < NB ? n : 0] : 0.f;
+      v[16 + n] = n < NB ? sr[n < NB ? n : 0] : 0.f;
+    }
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1)
+#pragma unroll
+      for (int i = 0; i < s; ++i) {
+        const bool upper = (lane & s) != 0;
+        const float keep = upper ? v[i + s] : v[i], give = upper ? v[i] : v[i + s];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, give, s);
+      }
+    const float other = __shfl_xor_sync(0xffffffffu, v[0], 16);
+    if (lr >= 0 && lane < nb) {   // (the lanes below 16 hold the centres)
+      const float lo = fsub(v[0], other), up = fadd(v[0], other);
+      if (q.part != nullptr) {
+        pl = norm_accum(q.p, pl, lo);
+        pu = norm_accum(q.p, pu, up);
+      } else {
+        q.y_lw[lr * q.N + n0 + lane] = lo;
+        q.y_uw[lr * q.N + n0 + lane] = up;
+      }
+    }
   }
-#pragma unroll
-  for (int j = 0; j < kCwNB; ++j) {
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) {
-      sc[j] += __shfl_xor_sync(0xffffffffu, sc[j], s);
-      sr[j] += __shfl_xor_sync(0xffffffffu, sr[j], s);
-    }
-    if (lane == 0 && n0 + j < N) {
-      y_lw[lr * N + n0 + j] = fsub(sc[j], sr[j]);
-      y_uw[lr * N + n0 + j] = fadd(sc[j], sr[j]);
-    }
+  if (q.part == nullptr) return;
+  if (lane < 16) s_red[0][warp][lane] = pl, s_red[1][warp][lane] = pu;
+  __syncthreads();
+  if (tid < nb) {
+    pl = s_red[0][0][tid], pu = s_red[1][0][tid];
+    for (int i = 1; i < kCwLinWarps; ++i) pl = norm_combine(q.p, pl, s_red[0][i][tid]), pu = norm_combine(q.p, pu, s_red[1][i][tid]);
+    q.part[((int64_t)tile * 2 + 0) * q.N + n0 + tid] = pl;
+    q.part[((int64_t)tile * 2 + 1) * q.N + n0 + tid] = pu;
   }
 }
 
-// [N, F] -> [F, N] through a 32 x 32 shared-memory tile.
-__global__ void __launch_bounds__(256)
-cw_transpose_kernel(const float* __restrict__ W, float* __restrict__ WT, int N, int64_t F) {
-  __shared__ float tile[32][33];
-  const int64_t f0 = (int64_t)blockIdx.x * 32;
-  const int n0 = blockIdx.y * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  for (int j = ty; j < 32; j += 8)
-    if (n0 + j < N && f0 + tx < F) tile[j][tx] = W[(int64_t)(n0 + j) * F + f0 + tx];
-  __syncthreads();
-  for (int j = ty; j < 32; j += 8)
-    if (f0 + j < F && n0 + tx < N) WT[(f0 + j) * N + n0 + tx] = tile[tx][j];
+// Concretised range of output blockIdx.x from the partial norms of cw_linear_kernel: warp 0 the lower, warp 1 the upper side.
+__global__ void __launch_bounds__(64)
+cw_linear_range_kernel(const float* __restrict__ part, const float* __restrict__ lb, const float* __restrict__ ub, float* __restrict__ l,
+                       float* __restrict__ u, int tiles, int N, int p, float eps) {
+  const int lane = threadIdx.x & 31, side = threadIdx.x >> 5, n = blockIdx.x;
+  float a = 0.f;
+#pragma unroll 4
+  for (int t = lane; t < tiles; t += 32) a = norm_combine(p, a, __ldg(part + ((int64_t)t * 2 + side) * N + n));
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) a = norm_combine(p, a, __shfl_xor_sync(0xffffffffu, a, s));
+  if (lane == 0) {
+    if (side == 0) l[n] = fadd(lb[n], fmul(-eps, norm_finish(p, a)));
+    else u[n] = fadd(ub[n], fmul(eps, norm_finish(p, a)));
+  }
 }
 
 // Dense rows from compact ones: one block per row, zeros outside the window.
@@ -370,7 +627,7 @@ cw_expand_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw,
     const unsigned q = t / uW, x = t - q * uW, c = q / uH, y = q - c * uH;
     float lo = 0.f, up = 0.f;
     if (!empty && (int)y >= wy.lo && (int)y <= wy.hi && (int)x >= wx.lo && (int)x <= wx.hi) {
-      const int e = ((int)c * g.wh + ((int)y - wy.lo)) * g.ww + ((int)x - wx.lo);
+      const int e = (((int)y - wy.lo) * g.ww + ((int)x - wx.lo)) * g.C + (int)c;
       lo = zl[e];
       up = zu[e];
     }
@@ -395,7 +652,184 @@ inline unsigned grid_for(int64_t items, int per_block) {
   return (unsigned)std::max<int64_t>(1, std::min(want, cap));
 }
 
+// Channels of the image that the rows [row_start, row_start + rows) span.
+inline void row_channels(int64_t row_start, int64_t rows, int H0, int W0, int& ci0, int& n_ci) {
+  const int64_t hw = (int64_t)H0 * W0;
+  ci0 = (int)(row_start / hw);
+  n_ci = (int)((row_start + rows - 1) / hw) - ci0 + 1;
+}
+
 }  // namespace
+
+// z_lo == nullptr: the rows of the first convolution, from its filter W1 and the slopes k_l, k_u (chain has one entry).
+// b_lo != nullptr: the bias image goes along (b_lo, b_up [Cin, H, W] -> yb_lo, yb_up).
+int cw_conv_ex(const float* z_lo, const float* z_up, const float* W1, const float* k_l, const float* k_u, float scale, int Cin0,
+               const float* Wt, float* y_lo, float* y_up, const float* b_lo, const float* b_up, const float* bias, float* yb_lo,
+               float* yb_up, int64_t rows, int64_t row_start, int H0, int W0, const int* chain, int n_chain, int Cin, int H, int W,
+               int Cout, int Kh, int Kw, int stride, int pad, cudaStream_t st) {
+  if (rows < 0 || row_start < 0 || Cin <= 0 || Cout <= 0 || Kh <= 0 || Kw <= 0 || stride <= 0 || pad < 0 || n_chain < 1)
+    return FB_ERR_ARG;
+  if (n_chain >= kMaxChain) return FB_ERR_SHAPE;
+  CwShape gi, go;
+  int rc = make_shape(chain, n_chain, H0, W0, Cin, H, W, gi);
+  if (rc != FB_OK) return rc;
+  const int Ho = (H + 2 * pad - Kh) / stride + 1, Wo = (W + 2 * pad - Kw) / stride + 1;
+  if (Ho <= 0 || Wo <= 0) return FB_ERR_SHAPE;
+  int out_chain[4 * kMaxChain];
+  std::copy(chain, chain + 4 * n_chain, out_chain);
+  out_chain[4 * n_chain] = Kh, out_chain[4 * n_chain + 1] = Kw, out_chain[4 * n_chain + 2] = stride, out_chain[4 * n_chain + 3] = pad;
+  rc = make_shape(out_chain, n_chain + 1, H0, W0, Cout, Ho, Wo, go);
+  if (rc != FB_OK) return rc;
+  if (rows == 0) return FB_OK;
+  if (rows > 0x7fffffff) return FB_ERR_SHAPE;
+
+  CwConvArgs q = {};
+  q.z_lo = z_lo, q.z_up = z_up, q.W1 = W1, q.k_l = k_l, q.k_u = k_u, q.scale = scale, q.Cin0 = Cin0;
+  q.Wt = Wt, q.y_lo = y_lo, q.y_up = y_up;
+  q.b_lo = b_lo, q.b_up = b_up, q.bias = bias, q.yb_lo = yb_lo, q.yb_up = yb_up;
+  q.rows = rows, q.row_start = row_start;
+  row_channels(row_start, rows, H0, W0, q.ci0, q.n_ci);
+  q.H0 = H0, q.W0 = W0, q.Cin = Cin, q.H = H, q.W = W, q.Cout = Cout, q.Kh = Kh, q.Kw = Kw, q.stride = stride, q.pad = pad;
+  q.Ho = Ho, q.Wo = Wo, q.iwh = gi.wh, q.iww = gi.ww, q.owh = go.wh, q.oww = go.ww;
+  q.ch = gi.ch;
+  const int64_t longest = std::max(H0, W0);
+  int64_t S = stride;
+  for (int i = 0; i < gi.ch.n; ++i) S = std::min(S * gi.ch.stride[i], longest);   // (beyond the image every pixel is its own class)
+  q.S = (int)S;
+  const int cls_y = std::min(q.S, H0);
+  q.cls_x = std::min(q.S, W0);
+  q.uih = q.uiw = 1;
+  for (int yi = 0; yi < cls_y; ++yi) {
+    Span wy, wx;
+    chain_window_free(gi.ch, yi, 0, wy, wx);
+    q.uih = std::max(q.uih, wy.hi - wy.lo + 1);
+  }
+  for (int xi = 0; xi < q.cls_x; ++xi) {
+    Span wy, wx;
+    chain_window_free(gi.ch, 0, xi, wy, wx);
+    q.uiw = std::max(q.uiw, wx.hi - wx.lo + 1);
+  }
+  const int64_t n_cls = (int64_t)q.n_ci * ceil_div(H0, q.S) * ceil_div(W0, q.S);   // rows of the largest class
+  if (n_cls > 0x7fffffff / 64) return FB_ERR_SHAPE;
+  // about a block per SM, the weights being staged once per block
+  q.G = (int)std::max<int64_t>(1, std::min<int64_t>(kCwMaxRows / kCwR, ceil_div((int64_t)cls_y * q.cls_x * n_cls, (int64_t)kCwR * device_info().sms)));
+  static_assert(sizeof(CwRow) * kCwMaxRows <= kCwStatic, "static shared memory");
+  const size_t limit = device_info().smem_optin - 2 * kCwStatic;
+  auto bytes = [&] {
+    const size_t n_w = (size_t)q.CC * Kh * Kw * (Cout + 1);
+    return 8 * (n_w + (n_w & 1) + (size_t)q.CC * q.uih * q.uiw * q.G * kCwR);
+  };
+  q.CC = Cin;
+  while (bytes() > limit && (q.CC > 1 || q.G > 1)) {
+    if (q.CC > 1) q.CC = (q.CC + 1) / 2;
+    else q.G = (q.G + 1) / 2;
+  }
+  if (bytes() > limit) return FB_ERR_SHAPE;
+  q.per_class = (int)ceil_div(n_cls, (int64_t)q.G * kCwR);
+  const int64_t out = (int64_t)Cout * Ho * Wo;
+  q.blocks_bias = b_lo != nullptr ? (int)std::min<int64_t>(ceil_div(out, kCwConvThreads), device_info().sms) : 0;
+  const int64_t blocks = q.blocks_bias + (int64_t)cls_y * q.cls_x * q.per_class;
+  if (blocks > 0x7fffffff) return FB_ERR_SHAPE;
+  auto kern = Kh == 3 && Kw == 3 ? cw_conv_kernel<3> : cw_conv_kernel<0>;
+  if (int rc = ensure_dynamic_smem(kern, bytes() + kCwStatic)) return rc;   // (48 KB without the attribute hold the static part too)
+  ProfileScope prof(PK_CONV, 8.0 * rows * Cout * go.wh * go.ww * Cin * Kh * Kw,
+                    4.0 * 2.0 * rows * ((double)Cin * gi.wh * gi.ww + (double)Cout * go.wh * go.ww), (void*)st);
+  kern<<<(unsigned)blocks, kCwConvThreads, bytes(), st>>>(q);
+  FB_LAUNCH_OK();
+  return FB_OK;
+}
+
+int64_t cw_linear_tiles(int H0, int W0) { return (int64_t)H0 * ceil_div(W0, kCwPx); }
+
+// coef != nullptr: the rows go through that rescale first.  part != nullptr: no rows are written, but the partial norms
+// [cw_linear_tiles][2][N].  lb != nullptr: the bias part goes along.
+int cw_linear_ex(const float* z_lw, const float* z_uw, const float* coef, const float* Wl, float* y_lw, float* y_uw, float* part,
+                 const float* lb, const float* ub, const float* bias, float* y_lb, float* y_ub, int64_t rows, int64_t row_start, int H0,
+                 int W0, const int* chain, int n_chain, int C, int H, int W, int N, int p, cudaStream_t st) {
+  if (rows < 0 || row_start < 0 || N <= 0) return FB_ERR_ARG;
+  CwLinearArgs q = {};
+  int rc = make_shape(chain, n_chain, H0, W0, C, H, W, q.g);
+  if (rc != FB_OK) return rc;
+  if (rows == 0) return FB_OK;
+  q.z_lw = z_lw, q.z_uw = z_uw, q.coef = coef, q.W = Wl, q.y_lw = y_lw, q.y_uw = y_uw, q.part = part;
+  q.lb = lb, q.ub = ub, q.bias = bias, q.y_lb = y_lb, q.y_ub = y_ub;
+  q.bias_blocks = lb != nullptr ? N : 0;
+  q.rows = rows, q.row_start = row_start, q.N = N, q.p = p;
+  row_channels(row_start, rows, H0, W0, q.ci0, q.n_ci);
+  // widest union of the windows of a tile
+  q.nx_max = 1;
+  for (int x0 = 0; x0 < W0; x0 += kCwPx) {
+    int lo = W, hi = -1;
+    for (int xi = x0; xi < std::min(W0, x0 + kCwPx); ++xi) {
+      Span wy, wx;
+      chain_window(q.g.ch, H0, W0, 0, xi, wy, wx);
+      if (wx.lo <= wx.hi) lo = std::min(lo, wx.lo), hi = std::max(hi, wx.hi);
+    }
+    q.nx_max = std::max(q.nx_max, hi - lo + 1);
+  }
+  // outputs a block: at most 16, fewer where a row of positions would not fit otherwise
+  const size_t limit = device_info().smem_optin - 2 * kCwStatic;
+  int NB = 16;
+  auto row_bytes = [&] { return sizeof(float) * (32 * (NB + 2) + 2) * (size_t)q.nx_max; };
+  while (NB > 4 && row_bytes() > limit) NB -= 4;
+  if (row_bytes() > limit) return FB_ERR_SHAPE;
+  const int groups = (int)ceil_div(N, NB);
+  q.nb = (int)ceil_div(N, groups);
+  NB = (int)ceil_div(q.nb, 4) * 4;
+  q.ny_max = (int)std::max<int64_t>(1, std::min<int64_t>(q.g.wh, (int64_t)(limit / 2 / row_bytes())));   // two blocks per SM where that is possible
+  const int64_t blocks = q.bias_blocks + cw_linear_tiles(H0, W0);
+  if (blocks > 0x7fffffff || groups > 65535) return FB_ERR_SHAPE;
+  const size_t smem = row_bytes() * q.ny_max;
+  auto kern = NB == 4 ? cw_linear_kernel<4> : NB == 8 ? cw_linear_kernel<8> : NB == 12 ? cw_linear_kernel<12> : cw_linear_kernel<16>;
+  if (int rc = ensure_dynamic_smem(kern, smem + kCwStatic)) return rc;
+  ProfileScope prof(PK_MATMUL, 8.0 * rows * C * q.g.wh * q.g.ww * N,
+                    4.0 * (2.0 * rows * C * q.g.wh * q.g.ww + 2.0 * rows * N + (double)C * H * W * N), (void*)st);
+  kern<<<dim3((unsigned)blocks, (unsigned)groups), kCwLinThreads, smem, st>>>(q);
+  FB_LAUNCH_OK();
+  return FB_OK;
+}
+
+int cw_linear_range(const float* part, const float* lb, const float* ub, float* l, float* u, int H0, int W0, int N, int p, float eps,
+                    cudaStream_t st) {
+  cw_linear_range_kernel<<<(unsigned)N, 64, 0, st>>>(part, lb, ub, l, u, (int)cw_linear_tiles(H0, W0), N, p, eps);
+  FB_LAUNCH_OK();
+  return FB_OK;
+}
+
+// op < 0: partial accumulations to part_l / part_u; else the coefficients of the relaxation and the relaxed bias terms.
+int cw_norm_ex(int op, const float* z_lw, const float* z_uw, float* part_l, float* part_u, const float* lb, const float* ub, float* out_lb,
+               float* out_ub, float* coef, int64_t rows, int64_t row_start, int Cin0, int H0, int W0, const int* chain, int n_chain, int C,
+               int H, int W, int p, float eps, int* violation, cudaStream_t st) {
+  if (rows < 0 || row_start < 0 || Cin0 <= 0 || !valid_norm(p) || row_start + rows > (int64_t)Cin0 * H0 * W0) return FB_ERR_ARG;
+  CwShape g;
+  int rc = make_shape(chain, n_chain, H0, W0, C, H, W, g);
+  if (rc != FB_OK) return rc;
+  const size_t smem = sizeof(int2) * ((size_t)H0 + W0);
+  if (smem > 40 * 1024 || ceil_div(C, 32) > 65535 || (int64_t)Cin0 * H0 * W0 > 0x7fffffff) return FB_ERR_SHAPE;
+  ProfileScope prof(PK_RELAX, 4.0 * rows * C * g.wh * g.ww, 4.0 * (2.0 * rows * C * g.wh * g.ww + 2.0 * C * H * W), (void*)st);
+  cw_norm_kernel<<<dim3((unsigned)(H * W), (unsigned)ceil_div(C, 32)), 32 * kCwNormWarps, smem, st>>>(
+      op, z_lw, z_uw, part_l, part_u, lb, ub, out_lb, out_ub, coef, rows, row_start, Cin0, g, p, eps, violation);
+  FB_LAUNCH_OK();
+  return FB_OK;
+}
+
+int cw_relax_columns(int op, const float* lb, const float* ub, const float* norm_l, const float* norm_u, float* out_lb, float* out_ub,
+                     float* coef, int C, int64_t hw, int p, float eps, int* violation, cudaStream_t st) {
+  cw_relax_columns_kernel<<<grid_for(C * hw, 256), 256, 0, st>>>(op, lb, ub, norm_l, norm_u, out_lb, out_ub, coef, C, hw, p, eps, violation);
+  FB_LAUNCH_OK();
+  return FB_OK;
+}
+
+int cw_rescale_rows(const float* z_lw, const float* z_uw, const float* coef, float* out_lw, float* out_uw, int64_t rows, int64_t row_start,
+                    int H0, int W0, const int* chain, int n_chain, int C, int H, int W, cudaStream_t st) {
+  CwShape g;
+  int rc = make_shape(chain, n_chain, H0, W0, C, H, W, g);
+  if (rc != FB_OK || rows == 0) return rc;
+  cw_rescale_kernel<<<(unsigned)ceil_div(rows, 8), 256, 0, st>>>(z_lw, z_uw, coef, out_lw, out_uw, rows, row_start, g);
+  FB_LAUNCH_OK();
+  return FB_OK;
+}
+
 }  // namespace fb
 
 using namespace fb;
@@ -428,13 +862,10 @@ extern "C" int fb_cw_identity_relax_f32(int op, const float* x_lb, const float* 
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t ncol = (int64_t)Cout * Ho * Wo;
   ProfileScope prof(PK_CONV, 2.0 * rows * Cout * g.wh * g.ww, 4.0 * 2.0 * rows * Cout * g.wh * g.ww, stream);
-  // bias part: an ordinary convolution of one image (x_lb doubles as the unused weight operand: Di = 0)
-  rc = fb_conv2d_f32(x_lb, x_ub, x_lb, x_ub, Wt, bias, y_lb, y_ub, y_lb, y_ub, 1, 0, Cin, H, W, Cout, Kh, Kw, stride, pad, stream);
-  if (rc != FB_OK) return rc;
   float* k_l = col_ws;
   float* k_u = col_ws + ncol;
-  rc = launch_identity_columns(op, Wt, y_lb, y_ub, k_l, k_u, scale, Cin, H, W, Cout, Kh, Kw, stride, pad, Ho, Wo, p, eps, violation,
-                               st);
+  rc = launch_identity_columns(op, x_lb, x_ub, Wt, bias, y_lb, y_ub, k_l, k_u, scale, Cin, H, W, Cout, Kh, Kw, stride, pad, Ho, Wo, p, eps,
+                               violation, st);
   if (rc != FB_OK || rows == 0) return rc;
   cw_identity_rows_kernel<<<grid_for(rows * Cout * g.wh * g.ww, 256), 256, 0, st>>>(Wt, k_l, k_u, z_lw, z_uw, scale, rows, row_start,
                                                                                    Cin, H, W, Cout, Kh, Kw, stride, pad, Ho, Wo,
@@ -447,51 +878,16 @@ extern "C" int fb_cw_conv2d_f32(const float* x_lw, const float* x_uw, const floa
                                 int64_t row_start, int H0, int W0, const int* chain, int n_chain, int Cin, int H, int W,
                                 int Cout, int Kh, int Kw, int stride, int pad, void* stream) {
   if (!x_lw || !x_uw || !Wt || !y_lw || !y_uw) return FB_ERR_ARG;
-  if (rows < 0 || row_start < 0 || Cin <= 0 || Cout <= 0 || Kh <= 0 || Kw <= 0 || stride <= 0 || pad < 0 || n_chain < 1)
-    return FB_ERR_ARG;
-  if (n_chain >= kMaxChain) return FB_ERR_SHAPE;
-  CwShape gi, go;
-  int rc = make_shape(chain, n_chain, H0, W0, Cin, H, W, gi);
-  if (rc != FB_OK) return rc;
-  const int Ho = (H + 2 * pad - Kh) / stride + 1, Wo = (W + 2 * pad - Kw) / stride + 1;
-  if (Ho <= 0 || Wo <= 0) return FB_ERR_SHAPE;
-  int out_chain[4 * kMaxChain];
-  std::copy(chain, chain + 4 * n_chain, out_chain);
-  out_chain[4 * n_chain] = Kh, out_chain[4 * n_chain + 1] = Kw, out_chain[4 * n_chain + 2] = stride, out_chain[4 * n_chain + 3] = pad;
-  rc = make_shape(out_chain, n_chain + 1, H0, W0, Cout, Ho, Wo, go);
-  if (rc != FB_OK) return rc;
-  if (rows == 0) return FB_OK;
-  if (rows > 0x7fffffff) return FB_ERR_SHAPE;
-  const bool by4 = Cout % 4 == 0;
-  const size_t n_w = (size_t)Cin * Kh * Kw * (Cout + (by4 ? 4 : 1));
-  const size_t smem = sizeof(float) * (n_w + (n_w & 1) + 2 * (size_t)kCwRows * Cin * gi.wh * gi.ww);
-  if (smem > (size_t)device_info().smem_optin) return FB_ERR_SHAPE;
-  auto kern = by4 ? cw_conv_kernel<4> : cw_conv_kernel<1>;
-  if (int rc = ensure_dynamic_smem(kern, smem)) return rc;
-  ProfileScope prof(PK_CONV, 8.0 * rows * Cout * go.wh * go.ww * Cin * Kh * Kw,
-                    4.0 * 2.0 * rows * ((double)Cin * gi.wh * gi.ww + (double)Cout * go.wh * go.ww), stream);
-  kern<<<(unsigned)ceil_div(rows, kCwRows), 256, smem, (cudaStream_t)stream>>>(
-      x_lw, x_uw, Wt, y_lw, y_uw, rows, row_start, H0, W0, gi.ch, Cin, Cout, Kh, Kw, stride, pad, Ho, Wo, gi.wh, gi.ww, go.wh, go.ww);
-  FB_LAUNCH_OK();
-  return FB_OK;
+  return cw_conv_ex(x_lw, x_uw, nullptr, nullptr, nullptr, 1.f, 0, Wt, y_lw, y_uw, nullptr, nullptr, nullptr, nullptr, nullptr, rows,
+                    row_start, H0, W0, chain, n_chain, Cin, H, W, Cout, Kh, Kw, stride, pad, (cudaStream_t)stream);
 }
 
 extern "C" int fb_cw_norm_partials_f32(const float* z_lw, const float* z_uw, float* part_l, float* part_u, int64_t rows,
                                        int64_t row_start, int Cin0, int H0, int W0, const int* chain, int n_chain, int C, int H,
                                        int W, int p, void* stream) {
   if (!z_lw || !z_uw || !part_l || !part_u) return FB_ERR_ARG;
-  if (rows < 0 || row_start < 0 || Cin0 <= 0 || !valid_norm(p) || row_start + rows > (int64_t)Cin0 * H0 * W0) return FB_ERR_ARG;
-  CwShape g;
-  int rc = make_shape(chain, n_chain, H0, W0, C, H, W, g);
-  if (rc != FB_OK) return rc;
-  const int64_t ncol = (int64_t)C * H * W;
-  const size_t smem = sizeof(int) * 2 * ((size_t)H0 + W0 + H + W);
-  if (smem > 48 * 1024) return FB_ERR_SHAPE;
-  ProfileScope prof(PK_RELAX, 4.0 * rows * C * g.wh * g.ww, 4.0 * (2.0 * rows * C * g.wh * g.ww + 2.0 * ncol), stream);
-  cw_norm_partials_kernel<<<grid_for(ncol, 8), 256, smem, (cudaStream_t)stream>>>(z_lw, z_uw, part_l, part_u, rows, row_start, Cin0,
-                                                                                    g, p);
-  FB_LAUNCH_OK();
-  return FB_OK;
+  return cw_norm_ex(-1, z_lw, z_uw, part_l, part_u, nullptr, nullptr, nullptr, nullptr, nullptr, rows, row_start, Cin0, H0, W0, chain,
+                    n_chain, C, H, W, p, 0.f, nullptr, (cudaStream_t)stream);
 }
 
 extern "C" int fb_cw_relax_apply_f32(int op, const float* z_lw, const float* z_uw, const float* lb, const float* ub,
@@ -506,36 +902,18 @@ extern "C" int fb_cw_relax_apply_f32(int op, const float* z_lw, const float* z_u
   int rc = make_shape(chain, n_chain, H0, W0, C, H, W, g);
   if (rc != FB_OK) return rc;
   const int64_t ncol = (int64_t)C * H * W, per_row = (int64_t)C * g.wh * g.ww;
-  cudaStream_t st = (cudaStream_t)stream;
   ProfileScope prof(PK_RELAX, 4.0 * rows * per_row, 4.0 * (4.0 * rows * per_row + 10.0 * ncol), stream);
-  cw_relax_columns_kernel<<<grid_for(ncol, 256), 256, 0, st>>>(op, lb, ub, norm_l, norm_u, out_lb, out_ub, coef_ws, ncol, p, eps,
-                                                               violation);
-  FB_LAUNCH_OK();
-  if (rows == 0) return FB_OK;
-  cw_rescale_kernel<<<(unsigned)ceil_div(rows, 8), 256, 0, st>>>(z_lw, z_uw, coef_ws, out_lw, out_uw, rows, row_start, g);
-  FB_LAUNCH_OK();
-  return FB_OK;
+  rc = cw_relax_columns(op, lb, ub, norm_l, norm_u, out_lb, out_ub, coef_ws, C, (int64_t)H * W, p, eps, violation, (cudaStream_t)stream);
+  if (rc != FB_OK) return rc;
+  return cw_rescale_rows(z_lw, z_uw, coef_ws, out_lw, out_uw, rows, row_start, H0, W0, chain, n_chain, C, H, W, (cudaStream_t)stream);
 }
 
 extern "C" int fb_cw_linear_f32(const float* z_lw, const float* z_uw, const float* Wl, float* y_lw, float* y_uw, float* wt_ws,
                                 int64_t rows, int64_t row_start, int H0, int W0, const int* chain, int n_chain, int C, int H,
                                 int W, int N, void* stream) {
   if (!z_lw || !z_uw || !Wl || !y_lw || !y_uw || !wt_ws) return FB_ERR_ARG;
-  if (rows < 0 || row_start < 0 || N <= 0) return FB_ERR_ARG;
-  CwShape g;
-  int rc = make_shape(chain, n_chain, H0, W0, C, H, W, g);
-  if (rc != FB_OK) return rc;
-  if (rows == 0) return FB_OK;
-  const int64_t warps = rows * ceil_div(N, kCwNB), F = (int64_t)C * H * W;
-  if (ceil_div(warps, 8) > 0x7fffffff || ceil_div(N, 32) > 65535) return FB_ERR_SHAPE;
-  cudaStream_t st = (cudaStream_t)stream;
-  ProfileScope prof(PK_MATMUL, 8.0 * rows * C * g.wh * g.ww * N, 4.0 * (2.0 * rows * C * g.wh * g.ww + 2.0 * rows * N + 2.0 * F * N),
-                    stream);
-  cw_transpose_kernel<<<dim3((unsigned)ceil_div(F, 32), (unsigned)ceil_div(N, 32)), 256, 0, st>>>(Wl, wt_ws, N, F);
-  FB_LAUNCH_OK();
-  cw_linear_kernel<<<(unsigned)ceil_div(warps, 8), 256, 0, st>>>(z_lw, z_uw, wt_ws, y_lw, y_uw, rows, row_start, g, N);
-  FB_LAUNCH_OK();
-  return FB_OK;
+  return cw_linear_ex(z_lw, z_uw, nullptr, Wl, y_lw, y_uw, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, rows, row_start, H0, W0,
+                      chain, n_chain, C, H, W, N, FB_PINF, (cudaStream_t)stream);
 }
 
 extern "C" int fb_cw_expand_f32(const float* z_lw, const float* z_uw, float* y_lw, float* y_uw, int64_t rows, int64_t row_start,

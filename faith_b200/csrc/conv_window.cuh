@@ -42,6 +42,34 @@ __host__ __device__ inline void chain_window(const ConvChain& ch, int H0, int W0
   }
 }
 
+// The same without the borders of the maps: a shift of the input by the product of the strides shifts the window by one.
+__host__ __device__ inline Span span_after_conv_free(Span s, int k, int stride, int pad) {
+  if (s.lo > s.hi) return s;
+  const int a = s.lo + pad - (k - 1), b = s.hi + pad;
+  Span o;
+  o.lo = a >= 0 ? (a + stride - 1) / stride : -(-a / stride);
+  o.hi = b >= 0 ? b / stride : -((-b + stride - 1) / stride);
+  return o;
+}
+__host__ __device__ inline void chain_window_free(const ConvChain& ch, int yi, int xi, Span& wy, Span& wx) {
+  wy.lo = wy.hi = yi;
+  wx.lo = wx.hi = xi;
+  for (int i = 0; i < ch.n; ++i) {
+    wy = span_after_conv_free(wy, ch.kh[i], ch.stride[i], ch.pad[i]);
+    wx = span_after_conv_free(wx, ch.kw[i], ch.stride[i], ch.pad[i]);
+  }
+}
+
+// Pixels (along one axis of n0) that can reach the outputs [s.lo, s.hi] of the chain: the hull of their receptive field.
+__host__ __device__ inline Span chain_pixels(const ConvChain& ch, const int* k, Span s, int n0) {
+  for (int i = ch.n - 1; i >= 0; --i) {
+    s.lo = s.lo * ch.stride[i] - ch.pad[i];
+    s.hi = s.hi * ch.stride[i] - ch.pad[i] + k[i] - 1;
+  }
+  if (s.lo < 0) s.lo = 0;
+  if (s.hi > n0 - 1) s.hi = n0 - 1;
+  return s;
+}
 
 // Host side: the chain as the C ABI passes it (n x 4 ints: kernel height, kernel width, stride, padding).  Fills `ch`
 // and the size (h, w) of the chain's last output; FB_ERR_ARG / FB_ERR_SHAPE on malformed input.
@@ -75,9 +103,9 @@ inline void chain_extent(const ConvChain& ch, int H0, int W0, int& win_h, int& w
   }
 }
 
-// Slopes and bias terms of the relaxation behind the first convolution, per output column (defined in conv.cu).
-int launch_identity_columns(int op, const float* Wt, float* y_lb, float* y_ub, float* k_l, float* k_u, float scale, int Cin,
-                            int H, int W, int Cout, int Kh, int Kw, int stride, int pad, int Ho, int Wo, int p, float eps,
-                            int* violation, cudaStream_t st);
+// Bias part, slopes and relaxed bias terms of the first convolution and the relaxation behind it, per output column (conv.cu).
+int launch_identity_columns(int op, const float* x_lb, const float* x_ub, const float* Wt, const float* bias, float* y_lb, float* y_ub,
+                            float* k_l, float* k_u, float scale, int Cin, int H, int W, int Cout, int Kh, int Kw, int stride, int pad,
+                            int Ho, int Wo, int p, float eps, int* violation, cudaStream_t st);
 
 }  // namespace fb

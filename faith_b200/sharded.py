@@ -134,7 +134,7 @@ def _chain_arr(chain):
 
 
 def cw_extent(H0, W0, chain):
-    """Largest window (wh, ww) any pixel of an H0 x W0 image reaches through `chain`: the trailing dimensions of a compact
+    """Largest window (wh, ww) any pixel of an H0 x W0 image reaches through `chain`: the middle dimensions of a compact
     tensor (fb_cw_extent)."""
     wh, ww = ctypes.c_int(0), ctypes.c_int(0)
     check(load().fb_cw_extent(H0, W0, _chain_arr(chain), len(chain), ctypes.byref(wh), ctypes.byref(ww)), "fb_cw_extent")
@@ -142,13 +142,13 @@ def cw_extent(H0, W0, chain):
 
 
 def cw_identity_relax(op, image_lb, image_ub, weight, bias, rows, row_start, stride, pad, p, eps, scale=1.0):
-    """conv_identity_relax with compact rows: z_lw, z_uw [rows, Cout, wh, ww] (fb_cw_identity_relax_f32)."""
+    """conv_identity_relax with compact rows: z_lw, z_uw [rows, wh, ww, Cout] (fb_cw_identity_relax_f32)."""
     dev = ops._chk(image_lb, image_ub, weight, bias)
     C, H, W = image_lb.shape[-3:]
     Co, _, Kh, Kw = weight.shape
     Ho, Wo = (H + 2 * pad - Kh) // stride + 1, (W + 2 * pad - Kw) // stride + 1
     wh, ww = cw_extent(H, W, [(Kh, Kw, stride, pad)])
-    z_lw = torch.empty(rows, Co, wh, ww, device=dev)
+    z_lw = torch.empty(rows, wh, ww, Co, device=dev)
     z_uw = torch.empty_like(z_lw)
     y_lb = torch.empty(1, Co, Ho, Wo, device=dev)
     y_ub = torch.empty_like(y_lb)
@@ -165,10 +165,10 @@ def cw_identity_relax(op, image_lb, image_ub, weight, bias, rows, row_start, str
 def cw_conv(z_lw, z_uw, weight, stride, pad, row_start, H0, W0, chain, H, W):
     """Weight part of a later convolution on compact rows (fb_cw_conv2d_f32); `chain` leads to the input [Cin, H, W]."""
     dev = ops._chk(z_lw, z_uw, weight)
-    rows, C = z_lw.shape[:2]
+    rows, C = z_lw.shape[0], z_lw.shape[3]
     Co, _, Kh, Kw = weight.shape
     wh, ww = cw_extent(H0, W0, list(chain) + [(Kh, Kw, stride, pad)])
-    y_lw = torch.empty(rows, Co, wh, ww, device=dev)
+    y_lw = torch.empty(rows, wh, ww, Co, device=dev)
     y_uw = torch.empty_like(y_lw)
     with torch.cuda.device(dev):
         check(load().fb_cw_conv2d_f32(z_lw.data_ptr(), z_uw.data_ptr(), weight.data_ptr(), y_lw.data_ptr(), y_uw.data_ptr(), rows,
@@ -180,7 +180,7 @@ def cw_conv(z_lw, z_uw, weight, stride, pad, row_start, H0, W0, chain, H, W):
 def cw_norm_partials(z_lw, z_uw, row_start, Cin0, H0, W0, chain, H, W, p):
     """Unfinished dual-norm accumulation of every dense column over the rows of a compact tensor (fb_cw_norm_partials_f32)."""
     dev = ops._chk(z_lw, z_uw)
-    rows, C = z_lw.shape[:2]
+    rows, C = z_lw.shape[0], z_lw.shape[3]
     part_l = torch.empty(C * H * W, device=dev)
     part_u = torch.empty_like(part_l)
     with torch.cuda.device(dev):
@@ -193,7 +193,7 @@ def cw_norm_partials(z_lw, z_uw, row_start, Cin0, H0, W0, chain, H, W, p):
 def cw_relax_apply(op, z_lw, z_uw, lb, ub, norm_l, norm_u, row_start, H0, W0, chain, H, W, p, eps):
     """Relaxation of compact rows from given (reduced) norm accumulations (fb_cw_relax_apply_f32)."""
     dev = ops._chk(z_lw, z_uw, lb, ub, norm_l, norm_u)
-    rows, C = z_lw.shape[:2]
+    rows, C = z_lw.shape[0], z_lw.shape[3]
     o_lw, o_uw, o_lb, o_ub = torch.empty_like(z_lw), torch.empty_like(z_uw), torch.empty_like(lb), torch.empty_like(ub)
     coef = torch.empty(4 * C * H * W, device=dev)
     with torch.cuda.device(dev):
@@ -207,7 +207,7 @@ def cw_relax_apply(op, z_lw, z_uw, lb, ub, norm_l, norm_u, row_start, H0, W0, ch
 def cw_linear(z_lw, z_uw, weight, row_start, H0, W0, chain, H, W):
     """Weight rows of the linear layer that ends the spatial part, from compact rows: [rows, N] (fb_cw_linear_f32)."""
     dev = ops._chk(z_lw, z_uw, weight)
-    rows, C = z_lw.shape[:2]
+    rows, C = z_lw.shape[0], z_lw.shape[3]
     N = weight.shape[0]
     y_lw = torch.empty(rows, N, device=dev)
     y_uw = torch.empty_like(y_lw)
@@ -223,7 +223,7 @@ def cw_linear(z_lw, z_uw, weight, row_start, H0, W0, chain, H, W):
 def cw_expand(z_lw, z_uw, row_start, H0, W0, chain, H, W):
     """Dense rows [rows, C, H, W] of a compact tensor (fb_cw_expand_f32)."""
     dev = ops._chk(z_lw, z_uw)
-    rows, C = z_lw.shape[:2]
+    rows, C = z_lw.shape[0], z_lw.shape[3]
     y_lw = torch.empty(rows, C, H, W, device=dev)
     y_uw = torch.empty_like(y_lw)
     with torch.cuda.device(dev):
@@ -287,21 +287,18 @@ class CnnVerifier:
         if self._arena is None or self._arena.numel() < need:
             self._graphs.clear()     # captured passes point into the arena that is about to be replaced
             self._arena = torch.empty(need, dtype=torch.uint8, device=self.device)
-        n_out = self._out_features(C, H, W)
-        l = torch.empty(n_out, device=self.device)
-        u = torch.empty(n_out, device=self.device)
-        violation = torch.zeros(1, dtype=torch.int32, device=self.device)
+        out = torch.empty(2, self._out_features(C, H, W), device=self.device)
         comm = self.comm._h if (self.comm is not None and world > 1) else None
         with torch.cuda.device(self.device):
             check(lib.fb_cnn_forward_f32(ctypes.byref(net), img.data_ptr(), ops.norm_code(p), float(eps), start, size, comm,
-                                         self.algo, 1 if self.compact else 0, l.data_ptr(), u.data_ptr(), violation.data_ptr(),
+                                         self.algo, 1 if self.compact else 0, out[0].data_ptr(), out[1].data_ptr(), None,
                                          self._arena.data_ptr(), self._arena.numel(), ops._stream()), "fb_cnn_forward_f32")
-        return l, u
+        return out
 
     def _forward_driver(self, image, p, eps, start, size, world):
         if not self.graph or world > 1:
             img = image.to(self.device, torch.float32, non_blocking=True).contiguous()
-            return self._run_driver(img, p, eps, start, size, world)
+            return self._run_driver(img, p, eps, start, size, world).unbind(0)
         # Single GPU: the pass is a dozen launches of a few microseconds each, which cost more to launch than to run;
         # they are captured once per (shape, norm, radius) into a CUDA graph that reads the image from a fixed device
         # buffer and writes the range to fixed outputs.  (Not with a communicator: the one-shot exchange takes its
@@ -316,12 +313,12 @@ class CnnVerifier:
                 torch.cuda.synchronize(self.device)
                 g = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(g, capture_error_mode="thread_local"):   # other threads (a collective's watchdog) stay free to call CUDA
-                    l, u = self._run_driver(static_img, p, eps, start, size, world)
-            ent = self._graphs[key] = (g, static_img, l, u)
-        g, static_img, l, u = ent
+                    out = self._run_driver(static_img, p, eps, start, size, world)
+            ent = self._graphs[key] = (g, static_img, out)
+        g, static_img, out = ent
         static_img.copy_(image, non_blocking=True)
         g.replay()
-        return l.clone(), u.clone()
+        return out.clone().unbind(0)
 
     def _out_features(self, C, H, W):
         c, h, w = C, H, W

@@ -534,7 +534,7 @@ int fb_concretize_sharded_f32(fb_comm* c, int algo,
 
 /* ---- compact rows for the convolutions behind an identity input ---------------------------
  * Row r of such a CNN is zero outside the window its pixel reaches (fb_conv2d_windowed_f32 above); here a row is stored
- * as that window only, z [rows, C, wh, ww] with z[r, c, dy, dx] = row r at (c, y_lo(r) + dy, x_lo(r) + dx) and zeros
+ * as that window only, z [rows, wh, ww, C] with z[r, dy, dx, c] = row r at (c, y_lo(r) + dy, x_lo(r) + dx) and zeros
  * where the pixel's own window is smaller than (wh, ww), the largest window over all pixels (fb_cw_extent).  `chain`
  * (host, n_chain x 4 ints: kernel height, kernel width, stride, padding) always lists the convolutions that lead from
  * the H0 x W0 image to the tensor in question, whose dense shape is [C, H, W].  For the benchmark CNN a row shrinks
@@ -551,8 +551,8 @@ int fb_concretize_sharded_f32(fb_comm* c, int algo,
  * fb_cw_relax_apply_f32     relaxation from (all-reduced) norms, the counterpart of fb_relax_with_norms_f32: rescaled
  *                           compact rows, relaxed bias terms out_lb / out_ub [C*H*W]; coef_ws: 4*C*H*W floats of scratch.
  * fb_cw_linear_f32          the linear layer that ends the spatial part, weight rows only: Wl [N, C*H*W] (nn.Linear
- *                           layout) -> y_lw, y_uw [rows, N] dense (bias rows: fb_matmul_f32 with Di = 0); wt_ws: N*C*H*W
- *                           floats of scratch (the call transposes the weight once so that its reads coalesce).
+ *                           layout) -> y_lw, y_uw [rows, N] dense (bias rows: fb_matmul_f32 with Di = 0); wt_ws:
+ *                           scratch, not used (N*C*H*W floats in earlier versions; must not be null).
  * fb_cw_expand_f32          dense rows [rows, C, H, W] from compact ones. */
 int fb_cw_extent(int H0, int W0, const int* chain, int n_chain, int* wh, int* ww);
 int fb_cw_identity_relax_f32(int op, const float* x_lb, const float* x_ub, const float* Wt, const float* bias,
