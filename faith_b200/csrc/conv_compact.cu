@@ -8,7 +8,7 @@
 //     z[r, dy, dx, c] = row r at (c, wy.lo(r) + dy, wx.lo(r) + dx),   dy < wh, dx < ww,
 //
 // (channels innermost: the kernels have their lanes on the channels, and their loads and stores of rows are whole sectors)
-// with (wh, ww) the largest window over all pixels (fb_cw_extent) and zeros where a pixel's own window is smaller.
+// with (wh, ww) the largest window over all pixels (fb_cw_extent); where a pixel's own window is smaller nothing is written.
 // The origin (wy.lo, wx.lo) is recomputed from the pixel and the chain wherever it is needed.  Every operator of the
 // CNN pass has a compact form: first convolution + relaxation, later convolutions, the column norms over dim_in
 // (a gather over the rows whose window holds the column, in row order: deterministic), the rescale of a relaxation,
@@ -27,15 +27,23 @@
 namespace fb {
 namespace {
 
-// Geometry of a compact tensor: the chain that leads to it and its dense shape.
+// Geometry of a compact tensor: its windows and its dense shape.
 struct CwShape {
-  ConvChain ch;
+  CwAxis y, x;
   int H0, W0, C, H, W, wh, ww;
 };
 
 __device__ __forceinline__ void pixel_of_row(int64_t r, int H0, int W0, int& yi, int& xi) {
   xi = (int)(r % W0);
   yi = (int)((r / W0) % H0);
+}
+
+// The arguments of a launch arrive in a constant bank that no cache has seen: every 64 bytes of them cost the first reader a miss.
+// The warps of a block touch one line each, so that the misses overlap.
+template <typename Args>
+__device__ __forceinline__ void touch_params(const Args& q) {
+  const unsigned at = (threadIdx.x >> 5) * 16;
+  if (at < sizeof(Args) / 4) asm volatile("" ::"r"(reinterpret_cast<const int*>(&q)[at]));
 }
 
 // First convolution (+ relaxation) of the identity input, compact: one thread per element of z.
@@ -81,15 +89,15 @@ cw_identity_rows_kernel(const float* __restrict__ Wt, const float* __restrict__ 
 // Bound by latency and shared-memory reads: 3072 rows, 16 -> 32 channels, 3 x 3 stride 2 took 35 us with a thread per output of
 // one row, whose tap bounds differ from lane to lane, and 8 us before it to write its input.
 constexpr int kCwR = 8;             // rows per thread
-constexpr int kCwConvThreads = 512;
+constexpr int kCwConvThreads = 512;   // at most; the items of a block in one round where that is possible
 constexpr int kCwMaxRows = 32;      // rows per block at most: one per lane
 constexpr size_t kCwStatic = 4096;  // static shared memory of the kernels below, at most
 
 struct CwConvArgs {
   const float *z_lo, *z_up;                    // compact rows, or
-  const float *W1, *k_l, *k_u;                 // the first convolution (ch.kh[0] ...): filter [Cin, Cin0, kh, kw], slopes per column
+  const float *W1, *k_l, *k_u;                 // the first convolution: filter [Cin, Cin0, kh1, kw1], slopes per column
   float scale;
-  int Cin0;
+  int Cin0, kh1, kw1, stride1, pad1;
   const float* Wt;
   float *y_lo, *y_up;
   const float *b_lo, *b_up, *bias;             // bias image (blocks_bias > 0)
@@ -97,30 +105,35 @@ struct CwConvArgs {
   int blocks_bias;
   int64_t rows, row_start;
   int ci0, n_ci;                               // input channels of the image that the rows span
-  int H0, W0, Cin, H, W, Cout, Kh, Kw, stride, pad, Ho, Wo, iwh, iww, owh, oww;
-  int S, cls_x, per_class, G, CC;
+  int H0, W0, Cin, H, W, Cout, stride, pad, Kh, Kw, Ho, Wo, iwh, iww, owh, oww;
+  int cls_x, per_class, G, CC;
   int uih, uiw;                                // largest window of the input without borders
-  ConvChain ch;
+  CwAxis iy, ix, oy, ox;                       // input and output windows
 };
 
-struct CwRow {
+struct __align__(16) CwRow {
   int lr, yi, xi, ci;      // local row (-1: none), pixel
   int uy, ux;              // input window without borders: first row and column
   int iy, ix, ih, iw;      // input window: first row and column, size
-  int oy, ox, oh, ow;      // output window
-  int voy, vox;            // output window without borders: first row and column
+  int oh, ow;              // output window: size (0 x 0: no row)
+  int py, px;              // its first row and column among the positions of the class
+  int64_t base;            // element (0, 0, 0) of the output row, shifted by (py, px)
 };
 
 // KS: filter size when it is the same in both directions and known at compile time (3), 0 = from the arguments.
-template <int KS>
+// CPT: output channels per thread (2 where Cout is even: the pairs of a tap are one 128-bit read, and the inputs, which every lane
+// reads, serve twice the multiply-adds).
+template <int KS, int CPT>
 __global__ void __launch_bounds__(kCwConvThreads)
-cw_conv_kernel(const CwConvArgs q) {
+cw_conv_kernel(const __grid_constant__ CwConvArgs q) {
   extern __shared__ __align__(16) float cw_smem[];
   __shared__ CwRow s_row[kCwMaxRows];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, Kh = KS ? KS : q.Kh, Kw = KS ? KS : q.Kw, taps = Kh * Kw;
+  touch_params(q);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x, nwarps = nthr >> 5;
+  const int Kh = KS ? KS : q.Kh, Kw = KS ? KS : q.Kw, taps = Kh * Kw;
   if ((int)blockIdx.x < q.blocks_bias) {   // an ordinary convolution of one image, a thread per output
     const int64_t total = (int64_t)q.Cout * q.Ho * q.Wo;
-    for (int64_t t = (int64_t)blockIdx.x * kCwConvThreads + tid; t < total; t += (int64_t)q.blocks_bias * kCwConvThreads) {
+    for (int64_t t = (int64_t)blockIdx.x * nthr + tid; t < total; t += (int64_t)q.blocks_bias * nthr) {
       const int ow = (int)(t % q.Wo), oh = (int)((t / q.Wo) % q.Ho), co = (int)(t / ((int64_t)q.Wo * q.Ho));
       const int ih0 = oh * q.stride - q.pad, iw0 = ow * q.stride - q.pad;
       float ac = 0.f, ar = 0.f;
@@ -148,156 +161,194 @@ cw_conv_kernel(const CwConvArgs q) {
     return;
   }
   const int bid = blockIdx.x - q.blocks_bias, cls = bid / q.per_class, chunk = bid - cls * q.per_class;
-  const int ry = cls / q.cls_x, rx = cls % q.cls_x, n_rows = q.G * kCwR;
+  const int ry = cls / q.cls_x, rx = cls - ry * q.cls_x, n_rows = q.G * kCwR;
+  // geometry of the class, from its first pixel
+  const int vy = q.iy.free_lo(ry), vx = q.ix.free_lo(rx), wy = q.oy.free_lo(ry), wx = q.ox.free_lo(rx);
+  const int ih = max(0, q.iy.free_hi(ry) - vy + 1), iw = max(0, q.ix.free_hi(rx) - vx + 1);
+  const int oh = max(0, q.oy.free_hi(ry) - wy + 1), ow = max(0, q.ox.free_hi(rx) - wx + 1);
+  const int ty0 = wy * q.stride - q.pad - vy, tx0 = wx * q.stride - q.pad - vx;   // first tap of the first output
   {
-    const int ny = (q.H0 - ry + q.S - 1) / q.S, nx = (q.W0 - rx + q.S - 1) / q.S, n_cls = q.n_ci * ny * nx;
-    if (chunk * n_rows >= n_cls) return;
+    const int S = q.oy.S, ny = (q.H0 - ry + S - 1) / S, nx = (q.W0 - rx + S - 1) / S, n_cls = q.n_ci * ny * nx;
     bool live = false;
     if (tid < n_rows) {
-      const int k = chunk * n_rows + tid;
+      const int k = chunk * n_rows + tid, kl = k / nx, kx = k - kl * nx, ci = kl / ny, ky = kl - ci * ny;
       CwRow r;
       r.lr = -1;
-      const int kx = k % nx, ky = (k / nx) % ny;
-      r.xi = rx + q.S * kx;
-      r.yi = ry + q.S * ky;
-      r.ci = q.ci0 + k / (nx * ny);
+      r.xi = rx + S * kx;
+      r.yi = ry + S * ky;
+      r.ci = q.ci0 + ci;
       if (k < n_cls) {
         const int64_t lr = ((int64_t)r.ci * q.H0 + r.yi) * q.W0 + r.xi - q.row_start;
         if (lr >= 0 && lr < q.rows) r.lr = (int)lr;
       }
       live = r.lr >= 0;
-      Span wy, wx, vy, vx;
-      chain_window(q.ch, q.H0, q.W0, r.yi, r.xi, wy, wx);
-      chain_window_free(q.ch, r.yi, r.xi, vy, vx);
-      r.uy = vy.lo, r.ux = vx.lo;
-      r.iy = wy.lo, r.ix = wx.lo, r.ih = wy.hi - wy.lo + 1, r.iw = wx.hi - wx.lo + 1;
-      const Span oy = span_after_conv(wy, q.Kh, q.stride, q.pad, q.Ho), ox = span_after_conv(wx, q.Kw, q.stride, q.pad, q.Wo);
-      const bool empty = wy.lo > wy.hi || wx.lo > wx.hi || oy.lo > oy.hi || ox.lo > ox.hi;
-      r.oy = oy.lo, r.ox = ox.lo, r.oh = empty ? 0 : oy.hi - oy.lo + 1, r.ow = empty ? 0 : ox.hi - ox.lo + 1;
-      r.voy = span_after_conv_free(vy, q.Kh, q.stride, q.pad).lo;
-      r.vox = span_after_conv_free(vx, q.Kw, q.stride, q.pad).lo;
+      r.uy = vy + q.stride * ky, r.ux = vx + q.stride * kx;
+      r.iy = max(0, r.uy), r.ix = max(0, r.ux);
+      r.ih = min(q.H, r.uy + ih) - r.iy, r.iw = min(q.W, r.ux + iw) - r.ix;
+      const int oy = max(0, wy + ky), ox = max(0, wx + kx);
+      r.oh = live ? max(0, min(q.Ho, wy + ky + oh) - oy) : 0, r.ow = live ? max(0, min(q.Wo, wx + kx + ow) - ox) : 0;
+      r.py = oy - wy - ky, r.px = ox - wx - kx;
+      r.base = (((int64_t)r.lr * q.owh - r.py) * q.oww - r.px) * q.Cout;
       s_row[tid] = r;
     }
     if (!__syncthreads_or(live)) return;
   }
-  // geometry of the class, from its first pixel
-  Span vy, vx;
-  chain_window_free(q.ch, ry, rx, vy, vx);
-  const Span wy = span_after_conv_free(vy, q.Kh, q.stride, q.pad), wx = span_after_conv_free(vx, q.Kw, q.stride, q.pad);
-  const int ih = max(0, vy.hi - vy.lo + 1), iw = max(0, vx.hi - vx.lo + 1);
-  const int oh = ih > 0 ? max(0, wy.hi - wy.lo + 1) : 0, ow = iw > 0 ? max(0, wx.hi - wx.lo + 1) : 0;
-  const int ty0 = wy.lo * q.stride - q.pad - vy.lo, tx0 = wx.lo * q.stride - q.pad - vx.lo;   // first tap of the first output
-  const int npos = oh * ow, ldw = q.Cout + 1, n_w = q.CC * taps * ldw;
-  float2* s_w = reinterpret_cast<float2*>(cw_smem);            // [CC][Kh][Kw][ldw] (w, |w|)
-  float2* s_x = s_w + n_w + (n_w & 1);                         // [CC][uih][uiw][G * 8] (centre, radius)
+  const int npos = oh * ow, ldw = q.Cout + CPT;                // (pairs of weights stay 8-byte aligned)
+  float2* s_x = reinterpret_cast<float2*>(cw_smem);            // [CC][uih][uiw][G * 8] (centre, radius)
+  float* s_w = cw_smem + 2 * (size_t)q.CC * q.uih * q.uiw * n_rows;   // [CC][Kh][Kw][ldw]
   const bool once = q.CC >= q.Cin;
-  const int items = q.G * npos * q.Cout;
-  for (int i0 = 0; i0 < items; i0 += kCwConvThreads) {
-    const int item = i0 + tid, co = item % q.Cout, pos = (item / q.Cout) % max(npos, 1), g = item / (q.Cout * max(npos, 1));
-    const int py = pos / max(ow, 1), px = pos - py * ow;
+  const int cgroups = q.Cout / CPT, items = npos * q.G * cgroups;
+  for (int i0 = 0; i0 < items; i0 += nthr) {
+    // channels fastest, then the groups of rows: the lanes of a warp that leave the channels' range keep their position
+    const int item = i0 + tid, u = item / cgroups, co = (item - u * cgroups) * CPT, pos = u / q.G, g = u - pos * q.G;
+    const int py = pos / ow, px = pos - py * ow;
     const int by = ty0 + py * q.stride, bx = tx0 + px * q.stride;
     const int ky0 = max(0, -by), ky1 = min(Kh, ih - by), kx0 = max(0, -bx), kx1 = min(Kw, iw - bx);
-    uint64_t acc[kCwR];
+    uint64_t acc[kCwR][CPT];
 #pragma unroll
-    for (int j = 0; j < kCwR; ++j) acc[j] = 0;
+    for (int j = 0; j < kCwR; ++j)
+#pragma unroll
+      for (int e = 0; e < CPT; ++e) acc[j][e] = 0;
     for (int c0 = 0; c0 < q.Cin; c0 += q.CC) {
       const int cc = min(q.CC, q.Cin - c0);
       if (!once || i0 == 0) {
         if (i0 > 0 || c0 > 0) __syncthreads();
         const int wn = cc * taps;
-        for (int o = warp; o < q.Cout; o += kCwConvThreads / 32) {   // lanes along (channel, tap)
+        for (int o = warp; o < q.Cout; o += nwarps) {   // asynchronous, lanes along (channel, tap)
           const float* src = q.Wt + ((int64_t)o * q.Cin + c0) * taps;
-#pragma unroll 4
-          for (int t = lane; t < wn; t += 32) {
-            const float w = __ldg(src + t);
-            s_w[t * ldw + o] = make_float2(w, fabsf(w));
-          }
+          uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_w + lane * ldw + o);
+          for (int t = lane; t < wn; t += 32, dst += 128 * ldw)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src + t) : "memory");
         }
         if (q.W1 != nullptr) {
-          // lanes along the rows (n_rows <= 32): neighbouring columns of the slopes
+          // lanes along the rows (n_rows <= 32): neighbouring columns of the slopes; two (channel, window row) pairs at a time, so
+          // that eighteen loads are in flight
           const CwRow r = s_row[min(lane, n_rows - 1)];
-#pragma unroll 3
-          for (int u = warp; u < cc * ih * iw; u += kCwConvThreads / 32) {
-            const int ux = u % iw, uy = (u / iw) % ih, c = u / (iw * ih), y = r.uy + uy, x = r.ux + ux;
-            const int ky = r.yi - (y * q.ch.stride[0] - q.ch.pad[0]), kx = r.xi - (x * q.ch.stride[0] - q.ch.pad[0]);
-            const bool in = r.lr >= 0 && y >= 0 && y < q.H && x >= 0 && x < q.W && ky >= 0 && ky < q.ch.kh[0] && kx >= 0 && kx < q.ch.kw[0];
-            const int64_t col = in ? ((int64_t)(c0 + c) * q.H + y) * q.W + x : 0;
-            const float w = in ? __ldg(q.W1 + (((int64_t)(c0 + c) * q.Cin0 + r.ci) * q.ch.kh[0] + ky) * q.ch.kw[0] + kx) : 0.f;
-            const float kl = __ldg(q.k_l + col), ku = __ldg(q.k_u + col);
-            const float tap = fmul(q.scale, w), lo = fmul(tap, kl), up = fmul(tap, ku);
-            if (lane < n_rows)
-              s_x[((c * q.uih + uy) * q.uiw + ux) * n_rows + lane] =
-                  in ? make_float2(fmul(fadd(lo, up), 0.5f), fmul(fsub(up, lo), 0.5f)) : make_float2(0.f, 0.f);
-          }
+          const int n_v = cc * ih;
+          for (int v0 = warp; v0 < n_v; v0 += 2 * nwarps)
+            for (int ux0 = 0; ux0 < iw; ux0 += 3) {
+              float w[2][3], kl[2][3], ku[2][3];
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const int v = min(v0 + h * nwarps, n_v - 1), c = v / ih, y = r.uy + v - c * ih, ky = r.yi - (y * q.stride1 - q.pad1);
+                const bool in_y = r.lr >= 0 && y >= 0 && y < q.H && ky >= 0 && ky < q.kh1;
+                const float* wp = q.W1 + (((int64_t)(c0 + c) * q.Cin0 + r.ci) * q.kh1 + ky) * q.kw1;
+                const int64_t col = ((int64_t)(c0 + c) * q.H + y) * q.W;
+#pragma unroll
+                for (int e = 0; e < 3; ++e) {
+                  const int x = r.ux + ux0 + e, kx = r.xi - (x * q.stride1 - q.pad1);
+                  const bool in = in_y && x >= 0 && x < q.W && kx >= 0 && kx < q.kw1;
+                  w[h][e] = in ? __ldg(wp + kx) : 0.f;
+                  kl[h][e] = in ? __ldg(q.k_l + col + x) : 0.f;
+                  ku[h][e] = in ? __ldg(q.k_u + col + x) : 0.f;
+                }
+              }
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const int v = min(v0 + h * nwarps, n_v - 1), c = v / ih, uy = v - c * ih;   // (a repeated pair writes the same)
+                float2* dst = s_x + ((c * q.uih + uy) * q.uiw + ux0) * n_rows + lane;
+#pragma unroll
+                for (int e = 0; e < 3; ++e) {
+                  const float tap = fmul(q.scale, w[h][e]), lo = fmul(tap, kl[h][e]), up = fmul(tap, ku[h][e]);
+                  if (ux0 + e < iw && lane < n_rows) dst[e * n_rows] = make_float2(fmul(fadd(lo, up), 0.5f), fmul(fsub(up, lo), 0.5f));
+                }
+              }
+            }
         } else {
           // lanes along the channel: neighbouring words of a row
-          for (int u = warp; u < ih * iw * n_rows; u += kCwConvThreads / 32) {
-            const int t = u % n_rows, v = u / n_rows, ux = v % iw, uy = v / iw;
+          for (int v = warp; v < ih * n_rows; v += nwarps) {
+            const int uy = v / n_rows, t = v - uy * n_rows;
             const CwRow& r = s_row[t];
-            const int dy = r.uy + uy - r.iy, dx = r.ux + ux - r.ix;
-            const bool in = r.lr >= 0 && dy >= 0 && dy < r.ih && dx >= 0 && dx < r.iw;
-            const int64_t o = (((int64_t)r.lr * q.iwh + dy) * q.iww + dx) * q.Cin + c0;
-#pragma unroll 2
+            const int dy = r.uy + uy - r.iy, dx0 = r.ux - r.ix;
+            const bool in_y = r.lr >= 0 && dy >= 0 && dy < r.ih;
+            const int64_t o = (((int64_t)r.lr * q.iwh + dy) * q.iww + dx0) * q.Cin + c0;
             for (int c = lane; c < cc; c += 32) {
-              const float lo = in ? __ldg(q.z_lo + o + c) : 0.f, up = in ? __ldg(q.z_up + o + c) : 0.f;
-              s_x[((c * q.uih + uy) * q.uiw + ux) * n_rows + t] = make_float2(fmul(fadd(lo, up), 0.5f), fmul(fsub(up, lo), 0.5f));
-            }
-          }
-        }
-        __syncthreads();
-      }
-      if (item < items) {
-        const float2* xc = s_x + ((int64_t)by * q.uiw + bx) * n_rows + g * kCwR;
-        const float2* wc = s_w + co;
-        for (int c = 0; c < cc; ++c, xc += q.uih * q.uiw * n_rows, wc += taps * ldw)
-          for (int ky = ky0; ky < ky1; ++ky) {
-            const float2* xp = xc + (ky * q.uiw + kx0) * n_rows;
-            const float2* wp = wc + (ky * Kw + kx0) * ldw;
+              float2* dst = s_x + (c * q.uih + uy) * q.uiw * n_rows + t;
 #pragma unroll 3
-            for (int kx = kx0; kx < kx1; ++kx, xp += n_rows, wp += ldw) {
-              const uint64_t w = *reinterpret_cast<const uint64_t*>(wp);
-#pragma unroll
-              for (int j = 0; j < kCwR; j += 2) {
-                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(xp + j);
-                acc[j] = fma2(v.x, w, acc[j]);
-                acc[j + 1] = fma2(v.y, w, acc[j + 1]);
+              for (int ux = 0; ux < iw; ++ux) {
+                const bool in = in_y && dx0 + ux >= 0 && dx0 + ux < r.iw;
+                const float lo = in ? __ldg(q.z_lo + o + ux * q.Cin + c) : 0.f, up = in ? __ldg(q.z_up + o + ux * q.Cin + c) : 0.f;
+                dst[ux * n_rows] = make_float2(fmul(fadd(lo, up), 0.5f), fmul(fsub(up, lo), 0.5f));
               }
             }
           }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+      }
+      if (item < items) {
+        // all taps of all channels in one loop (the loops over a position's one to three taps would each wait for their loads),
+        // the operands of the next tap loaded before the arithmetic of this one
+        const int nx = kx1 - kx0, ny = ky1 - ky0, n_tap = cc * max(0, ny) * max(0, nx);
+        const float2* xp = s_x + ((int64_t)(by + ky0) * q.uiw + bx + kx0) * n_rows + g * kCwR;
+        const float* wp = s_w + (ky0 * Kw + kx0) * ldw + co;
+        const int x_row = (q.uiw - nx) * n_rows, w_row = (Kw - nx) * ldw;
+        const int x_ch = (q.uih - ny) * q.uiw * n_rows, w_ch = (taps - ny * Kw) * ldw;
+        int kx = 0, ky = 0;
+        auto load = [&](ulonglong2 (&x)[kCwR / 2], float (&w)[CPT]) {
+#pragma unroll
+          for (int j = 0; j < kCwR / 2; ++j) x[j] = reinterpret_cast<const ulonglong2*>(xp)[j];
+          if (CPT == 2) {
+            const float2 v = *reinterpret_cast<const float2*>(wp);
+            w[0] = v.x, w[CPT - 1] = v.y;
+          } else {
+            w[0] = *wp;
+          }
+          xp += n_rows, wp += ldw;
+          if (++kx == nx) {
+            kx = 0, xp += x_row, wp += w_row;
+            if (++ky == ny) ky = 0, xp += x_ch, wp += w_ch;
+          }
+        };
+        auto mac = [&](const ulonglong2 (&x)[kCwR / 2], const float (&w)[CPT]) {
+#pragma unroll
+          for (int e = 0; e < CPT; ++e) {
+            const uint64_t p = pack2(w[e], fabsf(w[e]));
+#pragma unroll
+            for (int j = 0; j < kCwR / 2; ++j) {
+              acc[2 * j][e] = fma2(x[j].x, p, acc[2 * j][e]);
+              acc[2 * j + 1][e] = fma2(x[j].y, p, acc[2 * j + 1][e]);
+            }
+          }
+        };
+        if (n_tap > 0) {
+          ulonglong2 xa[kCwR / 2], xb[kCwR / 2];
+          float wa[CPT], wb[CPT];
+          load(xa, wa);
+          int t = 1;
+          for (; t + 1 < n_tap; t += 2) {
+            load(xb, wb);
+            mac(xa, wa);
+            load(xa, wa);
+            mac(xb, wb);
+          }
+          if (t < n_tap) load(xb, wb);
+          mac(xa, wa);
+          if (t < n_tap) mac(xb, wb);
+        }
       }
     }
     if (item < items) {
 #pragma unroll
       for (int j = 0; j < kCwR; ++j) {
         const CwRow& r = s_row[g * kCwR + j];
-        const int dy = r.voy + py - r.oy, dx = r.vox + px - r.ox;
-        if (r.lr >= 0 && dy >= 0 && dy < r.oh && dx >= 0 && dx < r.ow) {
-          const float2 v = unpack2(acc[j]);
-          const int64_t o = (((int64_t)r.lr * q.owh + dy) * q.oww + dx) * q.Cout + co;
-          q.y_lo[o] = fsub(v.x, v.y);
-          q.y_up[o] = fadd(v.x, v.y);
+        if ((unsigned)(py - r.py) < (unsigned)r.oh && (unsigned)(px - r.px) < (unsigned)r.ow) {
+          const int64_t o = r.base + (int64_t)(py * q.oww + px) * q.Cout + co;
+#pragma unroll
+          for (int e = 0; e < CPT; ++e) {
+            const float2 v = unpack2(acc[j][e]);
+            q.y_lo[o + e] = fsub(v.x, v.y);
+            q.y_up[o + e] = fadd(v.x, v.y);
+          }
         }
       }
-    }
-  }
-  // zeros where a row's window is smaller than the largest one
-  for (int t = 0; t < n_rows; ++t) {
-    const CwRow& r = s_row[t];
-    if (r.lr < 0 || (r.oh == q.owh && r.ow == q.oww)) continue;
-    for (int f = tid; f < q.owh * q.oww * q.Cout; f += kCwConvThreads) {
-      const int u = f / q.Cout, dx = u % q.oww, dy = u / q.oww;
-      if (dy < r.oh && dx < r.ow) continue;
-      const int64_t o = (int64_t)r.lr * q.owh * q.oww * q.Cout + f;
-      q.y_lo[o] = 0.f;
-      q.y_up[o] = 0.f;
     }
   }
 }
 
 // Dual-norm accumulation of every column (c, y, x) over the rows [row_start, row_start + rows): a gather over the pixels whose
-// window holds (y, x).  A block takes one position and 32 channels; its warps interleave over the candidate pixels (the hull of
-// the position's receptive field, whose spans are tabulated in shared memory) and read 32 consecutive words of a row; their sums
-// are combined in the order of the warps, so the result depends on the geometry alone.
+// window holds (y, x).  A block takes one position and 32 channels; its warps interleave over the rows of those pixels and read 32
+// consecutive words of a row of z; their sums are combined in the order of the warps, so the result depends on the geometry alone.
 // op < 0: the unfinished accumulations go to part_l / part_u.  Otherwise the relaxation's coefficients follow at once (no
 // exchange between ranks in between): out_lb / out_ub receive the relaxed bias terms, coef as cw_relax_columns_kernel writes it.
 // 3072 rows of 3 x 3 x 32 windows, 8192 columns: 13 us with a warp per column of channel-major rows, whose 32 lanes touch 32
@@ -322,41 +373,35 @@ __device__ __forceinline__ void cw_relax_column(int op, float lbv, float ubv, fl
 __global__ void __launch_bounds__(32 * kCwNormWarps)
 cw_norm_kernel(int op, const float* __restrict__ z_lw, const float* __restrict__ z_uw, float* __restrict__ part_l,
                float* __restrict__ part_u, const float* __restrict__ lb, const float* __restrict__ ub, float* __restrict__ out_lb,
-               float* __restrict__ out_ub, float* __restrict__ coef, int64_t rows, int64_t row_start, int Cin0, const CwShape g, int p,
+               float* __restrict__ out_ub, float* __restrict__ coef, int64_t rows, int64_t row_start, int Cin0, const __grid_constant__ CwShape g, int p,
                float eps, int* __restrict__ violation) {
-  extern __shared__ int2 cw_spans[];   // windows of the candidate pixel rows, then columns
   __shared__ float s_part[2][kCwNormWarps][32];
   const int y = blockIdx.x / g.W, x = blockIdx.x - y * g.W, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.y * 32 + lane;
-  const Span py = chain_pixels(g.ch, g.ch.kh, {y, y}, g.H0), px = chain_pixels(g.ch, g.ch.kw, {x, x}, g.W0);
-  const int ny = max(0, py.hi - py.lo + 1), nx = max(0, px.hi - px.lo + 1);
-  for (int i = threadIdx.x; i < ny + nx; i += blockDim.x) {
-    Span wy, wx;
-    chain_window(g.ch, g.H0, g.W0, i < ny ? py.lo + i : 0, i < ny ? 0 : px.lo + i - ny, wy, wx);
-    cw_spans[i] = i < ny ? make_int2(wy.lo, wy.hi) : make_int2(wx.lo, wx.hi);
-  }
-  __syncthreads();
+  // pixels whose window holds (y, x)
+  const int y0 = max(0, y * g.y.S - g.y.B), ny = min(g.H0 - 1, y * g.y.S - g.y.A) - y0 + 1;
+  const int x0 = max(0, x * g.x.S - g.x.B), nx = min(g.W0 - 1, x * g.x.S - g.x.A) - x0 + 1;
   float al = 0.f, au = 0.f;
-  for (int k = warp; k < Cin0 * ny; k += kCwNormWarps) {
-    const int ky = k % ny, ci = k / ny;
-    const int2 wy = cw_spans[ky];
-    if (y < wy.x || y > wy.y) continue;
-    const int64_t lr0 = ((int64_t)ci * g.H0 + py.lo + ky) * g.W0 + px.lo - row_start;
-    for (int kx = 0; kx < nx; kx += kCwNormLoads) {
-      float vl[kCwNormLoads], vu[kCwNormLoads];   // zeros leave every norm as it is
+  if (ny > 0) {
+    for (int k = warp; k < Cin0 * ny; k += kCwNormWarps) {
+      const int ci = k / ny, yi = y0 + k - ci * ny;
+      const int64_t lr0 = ((int64_t)ci * g.H0 + yi) * g.W0 + x0 - row_start;
+      const int dy = y - g.y.lo(yi);
+      for (int kx = 0; kx < nx; kx += kCwNormLoads) {
+        float vl[kCwNormLoads], vu[kCwNormLoads];   // zeros leave every norm as it is
 #pragma unroll
-      for (int e = 0; e < kCwNormLoads; ++e) {
-        const int2 wx = cw_spans[ny + min(kx + e, nx - 1)];
-        const int64_t lr = lr0 + kx + e;
-        const bool in = kx + e < nx && x >= wx.x && x <= wx.y && lr >= 0 && lr < rows && c < g.C;
-        const int64_t o = in ? ((lr * g.wh + (y - wy.x)) * g.ww + (x - wx.x)) * g.C + c : 0;
-        vl[e] = in ? __ldg(z_lw + o) : 0.f;
-        vu[e] = in ? __ldg(z_uw + o) : 0.f;
-      }
+        for (int e = 0; e < kCwNormLoads; ++e) {
+          const int64_t lr = lr0 + kx + e;
+          const bool in = kx + e < nx && lr >= 0 && lr < rows && c < g.C;
+          const int64_t o = in ? ((lr * g.wh + dy) * g.ww + (x - g.x.lo(x0 + kx + e))) * g.C + c : 0;
+          vl[e] = in ? __ldg(z_lw + o) : 0.f;
+          vu[e] = in ? __ldg(z_uw + o) : 0.f;
+        }
 #pragma unroll
-      for (int e = 0; e < kCwNormLoads; ++e) {
-        al = norm_accum(p, al, vl[e]);
-        au = norm_accum(p, au, vu[e]);
+        for (int e = 0; e < kCwNormLoads; ++e) {
+          al = norm_accum(p, al, vl[e]);
+          au = norm_accum(p, au, vu[e]);
+        }
       }
     }
   }
@@ -391,12 +436,6 @@ cw_relax_columns_kernel(int op, const float* __restrict__ lb, const float* __res
 
 // Rescale of a relaxation on compact rows: out_lw = c_ll lw + c_lu uw, out_uw = c_uu uw + c_ul lw (the expressions of
 // the dense kernel).  A warp per row: the window is worked out once, the lanes interleave over its elements.
-__device__ __forceinline__ void cw_rescale(const float* __restrict__ coef, int64_t ncol, int64_t col, float a, float b, float& lo,
-                                           float& up) {
-  lo = fmaf(__ldg(coef + col), a, fmul(__ldg(coef + ncol + col), b));
-  up = fmaf(__ldg(coef + 3 * ncol + col), b, fmul(__ldg(coef + 2 * ncol + col), a));
-}
-
 __global__ void __launch_bounds__(256)
 cw_rescale_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw, const float* __restrict__ coef,
                   float* __restrict__ o_lw, float* __restrict__ o_uw, int64_t rows, int64_t row_start, const CwShape g) {
@@ -407,16 +446,15 @@ cw_rescale_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw
   const int64_t ncol = (int64_t)g.C * g.H * g.W;
   int yi, xi;
   pixel_of_row(row_start + lr, g.H0, g.W0, yi, xi);
-  Span wy, wx;
-  chain_window(g.ch, g.H0, g.W0, yi, xi, wy, wx);
-  const bool empty = wy.lo > wy.hi || wx.lo > wx.hi;
-  const int ah = wy.hi - wy.lo + 1, aw = wx.hi - wx.lo + 1;
+  const int ylo = g.y.lo(yi), xlo = g.x.lo(xi), ah = g.y.hi(yi) - ylo + 1, aw = g.x.hi(xi) - xlo + 1;
   for (int e = lane; e < per_row; e += 32) {
     const int c = e % g.C, dx = (e / g.C) % g.ww, dy = e / (g.C * g.ww);
     float lo = 0.f, up = 0.f;
-    if (!empty && dy < ah && dx < aw) {
-      const int64_t col = ((int64_t)(wy.lo + dy) * g.W + wx.lo + dx) * g.C + c;
-      cw_rescale(coef, ncol, col, z_lw[lr * per_row + e], z_uw[lr * per_row + e], lo, up);
+    if (dy < ah && dx < aw) {
+      const int64_t col = ((int64_t)(ylo + dy) * g.W + xlo + dx) * g.C + c;
+      const float a = z_lw[lr * per_row + e], b = z_uw[lr * per_row + e];
+      lo = fmaf(coef[col], a, fmul(coef[ncol + col], b));
+      up = fmaf(coef[3 * ncol + col], b, fmul(coef[2 * ncol + col], a));
     }
     o_lw[lr * per_row + e] = lo;
     o_uw[lr * per_row + e] = up;
@@ -447,12 +485,12 @@ struct CwLinearArgs {
 
 template <int NB>
 __global__ void __launch_bounds__(kCwLinThreads)
-cw_linear_kernel(const CwLinearArgs q) {
+cw_linear_kernel(const __grid_constant__ CwLinearArgs q) {
+  touch_params(q);
   constexpr int LDN = NB + 2, LDP = 32 * LDN + 2;   // the lanes' 64-bit reads, along the channels, and the stores, along the
                                                     // positions, fall on different banks
   extern __shared__ __align__(16) float cw_smem[];
   __shared__ float s_red[2][kCwLinWarps][16];
-  __shared__ int2 s_win[kCwPx];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const CwShape& g = q.g;
   const int64_t ncol = (int64_t)g.C * g.H * g.W;
@@ -484,19 +522,8 @@ cw_linear_kernel(const CwLinearArgs q) {
   const int tiles_x = (g.W0 + kCwPx - 1) / kCwPx, tile = blockIdx.x - q.bias_blocks;
   const int yi = tile / tiles_x, x0 = (tile - yi * tiles_x) * kCwPx, npx = min(kCwPx, g.W0 - x0);
   const int n0 = blockIdx.y * q.nb, nb = min(q.nb, q.N - n0);
-  if (tid < kCwPx) {
-    Span ty, tx;
-    chain_window(g.ch, g.H0, g.W0, yi, min(x0 + tid, g.W0 - 1), ty, tx);
-    s_win[tid] = make_int2(tx.lo, tx.hi);
-  }
-  __syncthreads();
-  Span wy, wx;
-  chain_window(g.ch, g.H0, g.W0, yi, x0, wy, wx);
-  int xl = g.W, xh = -1;
-#pragma unroll
-  for (int i = 0; i < kCwPx; ++i)
-    if (s_win[i].x <= s_win[i].y) { xl = min(xl, s_win[i].x); xh = max(xh, s_win[i].y); }
-  const int nxr = max(0, xh - xl + 1), rows_here = npx * q.n_ci;
+  // the union of the windows (their ends do not decrease along the pixels)
+  const int ylo = g.y.lo(yi), yhi = g.y.hi(yi), xl = g.x.lo(x0), nxr = max(0, g.x.hi(x0 + npx - 1) - xl + 1), rows_here = npx * q.n_ci;
   const int64_t per_pos = g.C, per_row = (int64_t)g.wh * g.ww * g.C;
   float pl = 0.f, pu = 0.f;   // accumulated norms of this lane's output
   for (int r0 = 0; r0 < rows_here; r0 += kCwLinWarps) {
@@ -505,49 +532,69 @@ cw_linear_kernel(const CwLinearArgs q) {
     for (int n = 0; n < NB; ++n) sc[n] = sr[n] = 0.f;
     const int t = r0 + warp, px = t % npx, ci = q.ci0 + t / npx;
     int64_t lr = -1;
-    int2 win = make_int2(1, 0);
+    const int wlo = g.x.lo(x0 + px), aw = g.x.hi(x0 + px) - wlo + 1;
     if (t < rows_here) {
       const int64_t l = ((int64_t)ci * g.H0 + yi) * g.W0 + x0 + px - q.row_start;
-      if (l >= 0 && l < q.rows) { lr = l; win = s_win[px]; }
+      if (l >= 0 && l < q.rows) lr = l;
     }
-    const int aw = win.y - win.x + 1;
     for (int c0 = 0; c0 < g.C; c0 += 32) {
       const int c = c0 + lane;
-      for (int ya = wy.lo; ya <= wy.hi; ya += q.ny_max) {
-        const int yb = min(wy.hi, ya + q.ny_max - 1), npos = (yb - ya + 1) * nxr;
+      for (int ya = ylo; ya <= yhi; ya += q.ny_max) {
+        const int yb = min(yhi, ya + q.ny_max - 1), npos = (yb - ya + 1) * nxr;
         __syncthreads();
-        for (int pos = lane; pos < npos; pos += 32) {   // a warp per (output, channel), lanes along the positions
+        for (int pos = lane; pos < npos; pos += 32) {   // asynchronous; a warp per (output, channel), lanes along the positions
           const int yy = pos / nxr;
           const float* src = q.W + (int64_t)n0 * ncol + ((int64_t)c0 * g.H + ya + yy) * g.W + xl + pos - yy * nxr;
-#pragma unroll 8
+          const uint32_t dst = (uint32_t)__cvta_generic_to_shared(cw_smem + pos * LDP);
           for (int u = warp; u < 32 * NB; u += kCwLinWarps) {
             const int cl = u % 32, n = u / 32;
-            const float w = n < nb && c0 + cl < g.C ? __ldg(src + n * ncol + (int64_t)cl * g.H * g.W) : 0.f;
-            cw_smem[pos * LDP + cl * LDN + n] = w;
+            const bool in = n < nb && c0 + cl < g.C;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 4 * (cl * LDN + n)),
+                         "l"(src + (in ? n * ncol + (int64_t)cl * g.H * g.W : 0)), "r"(in ? 4 : 0) : "memory");
           }
         }
+        // the row's elements, three at a time: those of the next step are loaded before the arithmetic of this one
+        const bool mine = lr >= 0 && c < g.C && aw > 0;
+        const int steps_x = (aw + 2) / 3, steps = mine ? (yb - ya + 1) * steps_x : 0;
+        float zl[3], zu[3], kf[4][3];
+        int sy = ya, sx = 0;   // the next step: row, first column of the window
+        auto load = [&] {
+          const int64_t zb = lr * per_row + ((int64_t)(sy - ylo) * g.ww + sx) * per_pos + c, cb = ((int64_t)sy * g.W + wlo + sx) * g.C + c;
+#pragma unroll
+          for (int e = 0; e < 3; ++e) {
+            const bool in = sx + e < aw;
+            zl[e] = in ? __ldg(q.z_lw + zb + e * per_pos) : 0.f;
+            zu[e] = in ? __ldg(q.z_uw + zb + e * per_pos) : 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) kf[i][e] = in && q.coef != nullptr ? __ldg(q.coef + i * ncol + cb + e * g.C) : 0.f;
+          }
+        };
+        if (steps > 0) load();
+        asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
-        if (lr >= 0 && c < g.C) {
-          const int n_el = (yb - ya + 1) * aw;
-          const int64_t zb = lr * per_row + (int64_t)(ya - wy.lo) * g.ww * per_pos + c;
-#pragma unroll 3
-          for (int k = 0; k < n_el; ++k) {
-            const int dy = k / aw, dx = k - dy * aw;
-            const int64_t o = zb + (dy * g.ww + dx) * per_pos;
-            float lo = __ldg(q.z_lw + o), up = __ldg(q.z_uw + o);
-            if (q.coef != nullptr) {
-              const float a = lo, b = up;
-              cw_rescale(q.coef, ncol, ((int64_t)(ya + dy) * g.W + win.x + dx) * g.C + c, a, b, lo, up);
-            }
-            const float vc = fmul(fadd(lo, up), 0.5f), vr = fmul(fsub(up, lo), 0.5f);
-            const float2* w = reinterpret_cast<const float2*>(cw_smem + (dy * nxr + win.x - xl + dx) * LDP + lane * LDN);
+        for (int st = 0; st < steps; ++st) {
+          const float* wb = cw_smem + ((sy - ya) * nxr + wlo + sx - xl) * LDP + lane * LDN;
+          const int left = aw - sx;
+          float vc[3], vr[3];
+#pragma unroll
+          for (int e = 0; e < 3; ++e) {
+            const float lo = q.coef != nullptr ? fmaf(kf[0][e], zl[e], fmul(kf[1][e], zu[e])) : zl[e];
+            const float up = q.coef != nullptr ? fmaf(kf[3][e], zu[e], fmul(kf[2][e], zl[e])) : zu[e];
+            vc[e] = fmul(fadd(lo, up), 0.5f), vr[e] = fmul(fsub(up, lo), 0.5f);
+          }
+          sx += 3;
+          if (sx >= aw) sx = 0, ++sy;
+          if (st + 1 < steps) load();
+#pragma unroll
+          for (int e = 0; e < 3; ++e) {
+            const float2* w = reinterpret_cast<const float2*>(wb + (e < left ? e : 0) * LDP);
 #pragma unroll
             for (int n = 0; n < NB; n += 2) {
               const float2 v = w[n / 2];
-              sc[n] = fmaf(vc, v.x, sc[n]);
-              sr[n] = fmaf(vr, fabsf(v.x), sr[n]);
-              sc[n + 1] = fmaf(vc, v.y, sc[n + 1]);
-              sr[n + 1] = fmaf(vr, fabsf(v.y), sr[n + 1]);
+              sc[n] = fmaf(vc[e], v.x, sc[n]);
+              sr[n] = fmaf(vr[e], fabsf(v.x), sr[n]);
+              sc[n + 1] = fmaf(vc[e], v.y, sc[n + 1]);
+              sr[n + 1] = fmaf(vr[e], fabsf(v.y), sr[n + 1]);
             }
           }
         }
@@ -614,9 +661,7 @@ cw_expand_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw,
   const int64_t r = row_start + blockIdx.x;
   int yi, xi;
   pixel_of_row(r, g.H0, g.W0, yi, xi);
-  Span wy, wx;
-  chain_window(g.ch, g.H0, g.W0, yi, xi, wy, wx);
-  const bool empty = wy.lo > wy.hi || wx.lo > wx.hi;
+  const int ylo = g.y.lo(yi), yhi = g.y.hi(yi), xlo = g.x.lo(xi), xhi = g.x.hi(xi);
   const int per_row = g.C * g.wh * g.ww;
   const unsigned n = (unsigned)g.C * g.H * g.W, uW = g.W, uH = g.H;
   const float* zl = z_lw + (int64_t)blockIdx.x * per_row;
@@ -626,8 +671,8 @@ cw_expand_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw,
   for (unsigned t = threadIdx.x; t < n; t += blockDim.x) {
     const unsigned q = t / uW, x = t - q * uW, c = q / uH, y = q - c * uH;
     float lo = 0.f, up = 0.f;
-    if (!empty && (int)y >= wy.lo && (int)y <= wy.hi && (int)x >= wx.lo && (int)x <= wx.hi) {
-      const int e = (((int)y - wy.lo) * g.ww + ((int)x - wx.lo)) * g.C + (int)c;
+    if ((int)y >= ylo && (int)y <= yhi && (int)x >= xlo && (int)x <= xhi) {
+      const int e = (((int)y - ylo) * g.ww + ((int)x - xlo)) * g.C + (int)c;
       lo = zl[e];
       up = zu[e];
     }
@@ -638,11 +683,15 @@ cw_expand_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw,
 
 int make_shape(const int* chain, int n_chain, int H0, int W0, int C, int H, int W, CwShape& g) {
   int h, w;
-  int rc = chain_from_host(chain, n_chain, H0, W0, g.ch, h, w);
+  ConvChain ch;
+  int rc = chain_from_host(chain, n_chain, H0, W0, ch, h, w);
   if (rc != FB_OK) return rc;
   if (n_chain == 0 || C <= 0 || h != H || w != W) return FB_ERR_SHAPE;
   g.H0 = H0, g.W0 = W0, g.C = C, g.H = H, g.W = W;
-  chain_extent(g.ch, H0, W0, g.wh, g.ww);
+  rc = axis_from_chain(ch, ch.kh, H, g.y);
+  if (rc == FB_OK) rc = axis_from_chain(ch, ch.kw, W, g.x);
+  if (rc != FB_OK) return rc;
+  g.wh = axis_extent(g.y, H0), g.ww = axis_extent(g.x, W0);
   if ((int64_t)C * H * W > 0x7fffffff || (int64_t)C * g.wh * g.ww > 0x7fffffff) return FB_ERR_SHAPE;
   return FB_OK;
 }
@@ -691,33 +740,22 @@ int cw_conv_ex(const float* z_lo, const float* z_up, const float* W1, const floa
   row_channels(row_start, rows, H0, W0, q.ci0, q.n_ci);
   q.H0 = H0, q.W0 = W0, q.Cin = Cin, q.H = H, q.W = W, q.Cout = Cout, q.Kh = Kh, q.Kw = Kw, q.stride = stride, q.pad = pad;
   q.Ho = Ho, q.Wo = Wo, q.iwh = gi.wh, q.iww = gi.ww, q.owh = go.wh, q.oww = go.ww;
-  q.ch = gi.ch;
-  const int64_t longest = std::max(H0, W0);
-  int64_t S = stride;
-  for (int i = 0; i < gi.ch.n; ++i) S = std::min(S * gi.ch.stride[i], longest);   // (beyond the image every pixel is its own class)
-  q.S = (int)S;
-  const int cls_y = std::min(q.S, H0);
-  q.cls_x = std::min(q.S, W0);
+  q.iy = gi.y, q.ix = gi.x, q.oy = go.y, q.ox = go.x;
+  q.kh1 = chain[0], q.kw1 = chain[1], q.stride1 = chain[2], q.pad1 = chain[3];
+  const int S = go.y.S, cls_y = std::min(S, H0);
+  q.cls_x = std::min(S, W0);
   q.uih = q.uiw = 1;
-  for (int yi = 0; yi < cls_y; ++yi) {
-    Span wy, wx;
-    chain_window_free(gi.ch, yi, 0, wy, wx);
-    q.uih = std::max(q.uih, wy.hi - wy.lo + 1);
-  }
-  for (int xi = 0; xi < q.cls_x; ++xi) {
-    Span wy, wx;
-    chain_window_free(gi.ch, 0, xi, wy, wx);
-    q.uiw = std::max(q.uiw, wx.hi - wx.lo + 1);
-  }
-  const int64_t n_cls = (int64_t)q.n_ci * ceil_div(H0, q.S) * ceil_div(W0, q.S);   // rows of the largest class
+  for (int yi = 0; yi < cls_y; ++yi) q.uih = std::max(q.uih, gi.y.free_hi(yi) - gi.y.free_lo(yi) + 1);
+  for (int xi = 0; xi < q.cls_x; ++xi) q.uiw = std::max(q.uiw, gi.x.free_hi(xi) - gi.x.free_lo(xi) + 1);
+  const int64_t n_cls = (int64_t)q.n_ci * ceil_div(H0, S) * ceil_div(W0, S);   // rows of the largest class
   if (n_cls > 0x7fffffff / 64) return FB_ERR_SHAPE;
   // about a block per SM, the weights being staged once per block
   q.G = (int)std::max<int64_t>(1, std::min<int64_t>(kCwMaxRows / kCwR, ceil_div((int64_t)cls_y * q.cls_x * n_cls, (int64_t)kCwR * device_info().sms)));
+  const int cpt = Cout % 2 == 0 ? 2 : 1;
   static_assert(sizeof(CwRow) * kCwMaxRows <= kCwStatic, "static shared memory");
   const size_t limit = device_info().smem_optin - 2 * kCwStatic;
   auto bytes = [&] {
-    const size_t n_w = (size_t)q.CC * Kh * Kw * (Cout + 1);
-    return 8 * (n_w + (n_w & 1) + (size_t)q.CC * q.uih * q.uiw * q.G * kCwR);
+    return sizeof(float) * q.CC * ((size_t)Kh * Kw * (Cout + cpt) + 2 * (size_t)q.uih * q.uiw * q.G * kCwR);
   };
   q.CC = Cin;
   while (bytes() > limit && (q.CC > 1 || q.G > 1)) {
@@ -726,15 +764,18 @@ int cw_conv_ex(const float* z_lo, const float* z_up, const float* W1, const floa
   }
   if (bytes() > limit) return FB_ERR_SHAPE;
   q.per_class = (int)ceil_div(n_cls, (int64_t)q.G * kCwR);
+  const int64_t items = (int64_t)q.G * go.wh * go.ww * (Cout / cpt);
+  const int threads = (int)(ceil_div(ceil_div(items, ceil_div(items, kCwConvThreads)), 32) * 32);
   const int64_t out = (int64_t)Cout * Ho * Wo;
-  q.blocks_bias = b_lo != nullptr ? (int)std::min<int64_t>(ceil_div(out, kCwConvThreads), device_info().sms) : 0;
+  q.blocks_bias = b_lo != nullptr ? (int)std::min<int64_t>(ceil_div(out, threads), device_info().sms) : 0;
   const int64_t blocks = q.blocks_bias + (int64_t)cls_y * q.cls_x * q.per_class;
   if (blocks > 0x7fffffff) return FB_ERR_SHAPE;
-  auto kern = Kh == 3 && Kw == 3 ? cw_conv_kernel<3> : cw_conv_kernel<0>;
+  auto kern = Kh == 3 && Kw == 3 ? (cpt == 2 ? cw_conv_kernel<3, 2> : cw_conv_kernel<3, 1>)
+                                 : (cpt == 2 ? cw_conv_kernel<0, 2> : cw_conv_kernel<0, 1>);
   if (int rc = ensure_dynamic_smem(kern, bytes() + kCwStatic)) return rc;   // (48 KB without the attribute hold the static part too)
   ProfileScope prof(PK_CONV, 8.0 * rows * Cout * go.wh * go.ww * Cin * Kh * Kw,
                     4.0 * 2.0 * rows * ((double)Cin * gi.wh * gi.ww + (double)Cout * go.wh * go.ww), (void*)st);
-  kern<<<(unsigned)blocks, kCwConvThreads, bytes(), st>>>(q);
+  kern<<<(unsigned)blocks, threads, bytes(), st>>>(q);
   FB_LAUNCH_OK();
   return FB_OK;
 }
@@ -758,15 +799,7 @@ int cw_linear_ex(const float* z_lw, const float* z_uw, const float* coef, const 
   row_channels(row_start, rows, H0, W0, q.ci0, q.n_ci);
   // widest union of the windows of a tile
   q.nx_max = 1;
-  for (int x0 = 0; x0 < W0; x0 += kCwPx) {
-    int lo = W, hi = -1;
-    for (int xi = x0; xi < std::min(W0, x0 + kCwPx); ++xi) {
-      Span wy, wx;
-      chain_window(q.g.ch, H0, W0, 0, xi, wy, wx);
-      if (wx.lo <= wx.hi) lo = std::min(lo, wx.lo), hi = std::max(hi, wx.hi);
-    }
-    q.nx_max = std::max(q.nx_max, hi - lo + 1);
-  }
+  for (int x0 = 0; x0 < W0; x0 += kCwPx) q.nx_max = std::max(q.nx_max, q.g.x.hi(std::min(W0, x0 + kCwPx) - 1) - q.g.x.lo(x0) + 1);
   // outputs a block: at most 16, fewer where a row of positions would not fit otherwise
   const size_t limit = device_info().smem_optin - 2 * kCwStatic;
   int NB = 16;
@@ -804,10 +837,9 @@ int cw_norm_ex(int op, const float* z_lw, const float* z_uw, float* part_l, floa
   CwShape g;
   int rc = make_shape(chain, n_chain, H0, W0, C, H, W, g);
   if (rc != FB_OK) return rc;
-  const size_t smem = sizeof(int2) * ((size_t)H0 + W0);
-  if (smem > 40 * 1024 || ceil_div(C, 32) > 65535 || (int64_t)Cin0 * H0 * W0 > 0x7fffffff) return FB_ERR_SHAPE;
+  if (ceil_div(C, 32) > 65535 || (int64_t)Cin0 * H0 * W0 > 0x7fffffff) return FB_ERR_SHAPE;
   ProfileScope prof(PK_RELAX, 4.0 * rows * C * g.wh * g.ww, 4.0 * (2.0 * rows * C * g.wh * g.ww + 2.0 * C * H * W), (void*)st);
-  cw_norm_kernel<<<dim3((unsigned)(H * W), (unsigned)ceil_div(C, 32)), 32 * kCwNormWarps, smem, st>>>(
+  cw_norm_kernel<<<dim3((unsigned)(H * W), (unsigned)ceil_div(C, 32)), 32 * kCwNormWarps, 0, st>>>(
       op, z_lw, z_uw, part_l, part_u, lb, ub, out_lb, out_ub, coef, rows, row_start, Cin0, g, p, eps, violation);
   FB_LAUNCH_OK();
   return FB_OK;
@@ -840,7 +872,11 @@ extern "C" int fb_cw_extent(int H0, int W0, const int* chain, int n_chain, int* 
   int h, w;
   int rc = chain_from_host(chain, n_chain, H0, W0, ch, h, w);
   if (rc != FB_OK) return rc;
-  chain_extent(ch, H0, W0, *wh, *ww);
+  CwAxis y, x;
+  rc = axis_from_chain(ch, ch.kh, h, y);
+  if (rc == FB_OK) rc = axis_from_chain(ch, ch.kw, w, x);
+  if (rc != FB_OK) return rc;
+  *wh = axis_extent(y, H0), *ww = axis_extent(x, W0);
   return FB_OK;
 }
 

@@ -42,35 +42,6 @@ __host__ __device__ inline void chain_window(const ConvChain& ch, int H0, int W0
   }
 }
 
-// The same without the borders of the maps: a shift of the input by the product of the strides shifts the window by one.
-__host__ __device__ inline Span span_after_conv_free(Span s, int k, int stride, int pad) {
-  if (s.lo > s.hi) return s;
-  const int a = s.lo + pad - (k - 1), b = s.hi + pad;
-  Span o;
-  o.lo = a >= 0 ? (a + stride - 1) / stride : -(-a / stride);
-  o.hi = b >= 0 ? b / stride : -((-b + stride - 1) / stride);
-  return o;
-}
-__host__ __device__ inline void chain_window_free(const ConvChain& ch, int yi, int xi, Span& wy, Span& wx) {
-  wy.lo = wy.hi = yi;
-  wx.lo = wx.hi = xi;
-  for (int i = 0; i < ch.n; ++i) {
-    wy = span_after_conv_free(wy, ch.kh[i], ch.stride[i], ch.pad[i]);
-    wx = span_after_conv_free(wx, ch.kw[i], ch.stride[i], ch.pad[i]);
-  }
-}
-
-// Pixels (along one axis of n0) that can reach the outputs [s.lo, s.hi] of the chain: the hull of their receptive field.
-__host__ __device__ inline Span chain_pixels(const ConvChain& ch, const int* k, Span s, int n0) {
-  for (int i = ch.n - 1; i >= 0; --i) {
-    s.lo = s.lo * ch.stride[i] - ch.pad[i];
-    s.hi = s.hi * ch.stride[i] - ch.pad[i] + k[i] - 1;
-  }
-  if (s.lo < 0) s.lo = 0;
-  if (s.hi > n0 - 1) s.hi = n0 - 1;
-  return s;
-}
-
 // Host side: the chain as the C ABI passes it (n x 4 ints: kernel height, kernel width, stride, padding).  Fills `ch`
 // and the size (h, w) of the chain's last output; FB_ERR_ARG / FB_ERR_SHAPE on malformed input.
 inline int chain_from_host(const int* chain, int n_chain, int H0, int W0, ConvChain& ch, int& h, int& w) {
@@ -88,19 +59,40 @@ inline int chain_from_host(const int* chain, int n_chain, int H0, int W0, ConvCh
   return FB_OK;
 }
 
-// Largest window any pixel reaches through the chain (at least 1 x 1).
-inline void chain_extent(const ConvChain& ch, int H0, int W0, int& win_h, int& win_w) {
-  win_h = 1, win_w = 1;
-  for (int yi = 0; yi < H0; ++yi) {
-    Span wy, wx;
-    chain_window(ch, H0, W0, yi, 0, wy, wx);
-    win_h = std::max(win_h, wy.hi - wy.lo + 1);
+// The same for the compact rows (conv_compact.cu), along one axis.  Without the borders of the maps the nested divisions of a
+// chain collapse into one: pixel i reaches [ceil((i + A) / S), floor((i + B) / S)], S the product of the strides, so that a shift
+// of the pixel by S shifts the window by one; the compact window is that interval cut to the map.  (It holds the window above,
+// and is larger only where a padding exceeds its filter or a stride its filter; what is more is zero.)  Turned round, output y is
+// reached by the pixels [y S - B, y S - A].
+struct CwAxis {
+  int S, sh, A, B, n;   // sh: log2(S), or -1; n: outputs of the chain
+  __host__ __device__ int floor_s(int a) const { return sh >= 0 ? a >> sh : a >= 0 ? a / S : -((-a + S - 1) / S); }
+  __host__ __device__ int free_lo(int i) const { return floor_s(i + A + S - 1); }
+  __host__ __device__ int free_hi(int i) const { return floor_s(i + B); }
+  __host__ __device__ int lo(int i) const { const int v = free_lo(i); return v > 0 ? v : 0; }
+  __host__ __device__ int hi(int i) const { const int v = free_hi(i); return v < n - 1 ? v : n - 1; }
+};
+
+inline int axis_from_chain(const ConvChain& ch, const int* k, int n, CwAxis& ax) {
+  int64_t S = 1, A = 0, B = 0;
+  for (int i = 0; i < ch.n; ++i) {
+    A += (ch.pad[i] - (k[i] - 1)) * S;
+    B += ch.pad[i] * S;
+    S *= ch.stride[i];
+    if (S > (1 << 24) || A < -(1 << 28) || B > (1 << 28)) return FB_ERR_SHAPE;
   }
-  for (int xi = 0; xi < W0; ++xi) {
-    Span wy, wx;
-    chain_window(ch, H0, W0, 0, xi, wy, wx);
-    win_w = std::max(win_w, wx.hi - wx.lo + 1);
-  }
+  ax.S = (int)S, ax.A = (int)A, ax.B = (int)B, ax.n = n;
+  ax.sh = -1;
+  for (int i = 0; i < 25; ++i)
+    if (S == (int64_t)1 << i) ax.sh = i;
+  return FB_OK;
+}
+
+// Largest window any pixel of n0 reaches (at least 1).
+inline int axis_extent(const CwAxis& ax, int n0) {
+  int win = 1;
+  for (int i = 0; i < n0; ++i) win = std::max(win, ax.hi(i) - ax.lo(i) + 1);
+  return win;
 }
 
 // Bias part, slopes and relaxed bias terms of the first convolution and the relaxation behind it, per output column (conv.cu).

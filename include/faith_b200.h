@@ -534,8 +534,8 @@ int fb_concretize_sharded_f32(fb_comm* c, int algo,
 
 /* ---- compact rows for the convolutions behind an identity input ---------------------------
  * Row r of such a CNN is zero outside the window its pixel reaches (fb_conv2d_windowed_f32 above); here a row is stored
- * as that window only, z [rows, wh, ww, C] with z[r, dy, dx, c] = row r at (c, y_lo(r) + dy, x_lo(r) + dx) and zeros
- * where the pixel's own window is smaller than (wh, ww), the largest window over all pixels (fb_cw_extent).  `chain`
+ * as that window only, z [rows, wh, ww, C] with z[r, dy, dx, c] = row r at (c, y_lo(r) + dy, x_lo(r) + dx),
+ * (wh, ww) the largest window over all pixels (fb_cw_extent); what lies beyond a pixel's own window is not defined.  `chain`
  * (host, n_chain x 4 ints: kernel height, kernel width, stride, padding) always lists the convolutions that lead from
  * the H0 x W0 image to the tensor in question, whose dense shape is [C, H, W].  For the benchmark CNN a row shrinks
  * from 16 384 resp. 8 192 values to 144 resp. 288.  No counterpart in the reference.

@@ -258,3 +258,53 @@ def test_cnn_driver_other_layer_sequences():
             got = CnnVerifier(layers, DEV, compact=compact).forward(img, float("inf"), 0.01)
             helpers.assert_close(got[0], ref[0], "net %d l compact=%s" % (i, compact), atol=2e-6)
             helpers.assert_close(got[1], ref[1], "net %d u compact=%s" % (i, compact), atol=2e-6)
+
+
+# odd and single channels, a 5 x 5 filter with a stride of 3, padding beyond the filter, an image narrower than a tile of pixels,
+# rows starting in the middle of a channel, more outputs than a block takes
+@pytest.mark.parametrize("C,H,W,c1,c2,k2,s2,p2,n,start,drop", [(1, 7, 5, 3, 5, 3, 1, 1, 3, 0, 0), (3, 11, 13, 8, 33, 5, 3, 2, 17, 100, 57),
+                                                              (2, 9, 30, 2, 64, 2, 2, 3, 40, 5, 300), (4, 6, 9, 16, 1, 3, 2, 1, 1, 0, 1)])
+def test_compact_rows_of_odd_shapes(C, H, W, c1, c2, k2, s2, p2, n, start, drop):
+    from faith_b200 import ops, sharded
+    from faith_b200._lib import FB_RELU
+    g = torch.Generator().manual_seed(45)
+    rows, eps = C * H * W - start - drop, 0.05
+    img = torch.rand(1, C, H, W, generator=g).to(DEV)
+    w1 = (torch.randn(c1, C, 3, 3, generator=g) * 0.3).to(DEV)
+    w2 = (torch.randn(c2, c1, k2, k2, generator=g) * 0.3).to(DEV)
+    b1 = (torch.randn(c1, generator=g) * 0.1).to(DEV)
+    dense = sharded.conv_identity_relax(FB_RELU, img, img.clone(), w1, b1, rows, start, 1, 1, float("inf"), eps)
+    z = sharded.cw_identity_relax(FB_RELU, img, img.clone(), w1, b1, rows, start, 1, 1, float("inf"), eps)
+    d2 = ops.conv2d(dense, w2, None, s2, p2)
+    z2 = sharded.cw_conv(z[0], z[1], w2, s2, p2, start, H, W, [(3, 3, 1, 1)], H, W)
+    chain = [(3, 3, 1, 1), (k2, k2, s2, p2)]
+    h, w = d2[0].shape[-2:]
+    e = sharded.cw_expand(z2[0], z2[1], start, H, W, chain, h, w)
+    assert torch.equal(e[0], d2[0][0]) and torch.equal(e[1], d2[1][0])
+    feat = c2 * h * w
+    for p in (1.0, 2.0, float("inf")):
+        pl, pu = ops.norm_partials(d2[0].reshape(1, rows, feat), d2[1].reshape(1, rows, feat), p)
+        cl, cu = sharded.cw_norm_partials(z2[0], z2[1], start, C, H, W, chain, h, w, p)
+        helpers.assert_close(cl, pl.reshape(-1), "l p=%s" % p, rtol=1e-6, atol=1e-7)
+        helpers.assert_close(cu, pu.reshape(-1), "u p=%s" % p, rtol=1e-6, atol=1e-7)
+    wl = (torch.randn(n, feat, generator=g) / feat ** 0.5).to(DEV)
+    dl = ops.matmul(d2[0].reshape(1, 1, rows, feat), d2[1].reshape(1, 1, rows, feat), d2[2].reshape(1, 1, feat),
+                    d2[3].reshape(1, 1, feat), wl, None)
+    yl, yu = sharded.cw_linear(z2[0], z2[1], wl, start, H, W, chain, h, w)
+    helpers.assert_close(yl, dl[0].reshape(rows, n), "linear lw", atol=2e-6)
+    helpers.assert_close(yu, dl[1].reshape(rows, n), "linear uw", atol=2e-6)
+
+
+@pytest.mark.parametrize("C,HW,c1,c2,n,p", [(1, 16, 8, 16, 2, 1.0), (3, 23, 24, 48, 16, 2.0), (1, 21, 5, 7, 33, float("inf"))])
+def test_cnn_driver_with_the_head_reduced_to_its_norms(C, HW, c1, c2, n, p):
+    from faith_b200.sharded import CnnVerifier
+    g = torch.Generator().manual_seed(46)
+    h2 = (HW + 1) // 2
+    layers = [("conv", torch.randn(c1, C, 3, 3, generator=g) * 0.2, torch.randn(c1, generator=g) * 0.1, 1, 1), ("relu",),
+              ("conv", torch.randn(c2, c1, 3, 3, generator=g) * 0.1, torch.randn(c2, generator=g) * 0.1, 2, 1), ("relu",),
+              ("linear", torch.randn(n, c2 * h2 * h2, generator=g) * 0.02, torch.randn(n, generator=g) * 0.1)]
+    img = torch.rand(C, HW, HW, generator=g)
+    ref = CnnVerifier(layers, DEV).forward(img, p, 0.01, dense=True)
+    got = CnnVerifier(layers, DEV).forward(img, p, 0.01)
+    helpers.assert_close(got[0], ref[0], "l", atol=5e-6)
+    helpers.assert_close(got[1], ref[1], "u", atol=5e-6)
