@@ -185,6 +185,7 @@ col_relax_native(int op, const float* __restrict__ lw, const float* __restrict__
                  float* __restrict__ o_lw, float* __restrict__ o_uw, float* __restrict__ o_lb,
                  float* __restrict__ o_ub, int Di, int Do, int ntiles, int words, int p, float eps,
                  int* __restrict__ violation) {
+  pdl_sync();
   extern __shared__ __align__(16) float smem[];
   float* s_red = smem;                    // [2][8][kCW]
   float* s_coef = s_red + 2 * 8 * kCW;    // [4][kCW]
@@ -247,6 +248,7 @@ col_mul_bounds_native(const float* __restrict__ x_lw, const float* __restrict__ 
                       const float* __restrict__ y_lb, const float* __restrict__ y_ub,
                       float* __restrict__ z_lw, float* __restrict__ z_uw, float* __restrict__ z_lb,
                       float* __restrict__ z_ub, int Di, int Do, int ntiles, int words, int p, float eps) {
+  pdl_sync();
   extern __shared__ __align__(16) float smem[];
   float* s_red = smem;
   float* s_coef = s_red + 2 * 8 * kCW;  // [8][kCW]: lower (x own, x other, y own, y other), upper (same)
@@ -340,6 +342,7 @@ template <int VEC>
 __global__ void __launch_bounds__(kThreads)
 col_norm_partials_native(const float* __restrict__ lw, const float* __restrict__ uw, float* __restrict__ part_l,
                          float* __restrict__ part_u, int Di, int Do, int ntiles, int p) {
+  pdl_sync();
   extern __shared__ __align__(16) float smem[];
   const int64_t row = blockIdx.x / ntiles;
   const int c0 = (int)(blockIdx.x % ntiles) * kCW;
@@ -362,6 +365,7 @@ template <int VEC>
 __global__ void __launch_bounds__(kThreads)
 col_norm_partials_split(const float* __restrict__ lw, const float* __restrict__ uw, float* __restrict__ part_l,
                         float* __restrict__ part_u, int Di, int Do, int ntiles, int p) {
+  pdl_sync();
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ __align__(16) float s_red[2 * 8 * kCW];
@@ -403,6 +407,7 @@ col_norm_partials_split(const float* __restrict__ lw, const float* __restrict__ 
 __global__ void __launch_bounds__(kThreads)
 col_norm_partials_narrow(const float* __restrict__ lw, const float* __restrict__ uw, float* __restrict__ part_l,
                          float* __restrict__ part_u, int Di, int Do, int p) {
+  pdl_sync();
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ float s_l[kThreads], s_u[kThreads];
@@ -458,6 +463,7 @@ col_relax_apply_native(int op, const float* __restrict__ lw, const float* __rest
                        float* __restrict__ o_lw, float* __restrict__ o_uw, float* __restrict__ o_lb,
                        float* __restrict__ o_ub, int Di, int Do, int ntiles, int p, float eps,
                        int* __restrict__ violation) {
+  pdl_sync();
   __shared__ float s_coef[4 * kCW];
   const int64_t row = blockIdx.x / ntiles;
   const int c0 = (int)(blockIdx.x % ntiles) * kCW;
@@ -528,6 +534,7 @@ col_relax_transposed(int op, const float* __restrict__ lw, const float* __restri
                      float* __restrict__ o_lw, float* __restrict__ o_uw, float* __restrict__ o_lb,
                      float* __restrict__ o_ub, int64_t ncols, int Di, int words, int p, float eps,
                      int* __restrict__ violation) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const int64_t col = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
   if (col >= ncols) return;
@@ -612,6 +619,7 @@ struct ConcretizeOne {
 template <int VEC>
 __global__ void __launch_bounds__(kThreads)
 concretize_native(const ConcretizeOne first, const ConcretizeOne second, int64_t n_first, int Di, int words, int p, float eps) {
+  pdl_sync();
   __shared__ float s_red[2 * 8 * kCW];
   const bool is_first = blockIdx.x < n_first;
   const ConcretizeOne& q = is_first ? first : second;
@@ -637,6 +645,7 @@ concretize_native(const ConcretizeOne first, const ConcretizeOne second, int64_t
 template <int VEC>
 __global__ void __launch_bounds__(kThreads)
 concretize_transposed(const ConcretizeOne first, const ConcretizeOne second, int64_t n_first, int Di, int words, int p, float eps) {
+  pdl_sync();
   const bool is_first = blockIdx.x < n_first;
   const ConcretizeOne& q = is_first ? first : second;
   const int64_t col = (is_first ? blockIdx.x : blockIdx.x - n_first) * (kThreads / 32) + (threadIdx.x >> 5);
@@ -655,7 +664,7 @@ int launch_concretize(ConcretizeOne first, ConcretizeOne second, int Di, int wor
     vec = vec && (Di / words) % 4 == 0;
     const int64_t n1 = ceil_div(first.rows * first.Do, kThreads / 32), blocks = n1 + ceil_div(second.rows * second.Do, kThreads / 32);
     if (blocks > 0x7fffffff) return FB_ERR_SHAPE;
-    (vec ? concretize_transposed<4> : concretize_transposed<1>)<<<(unsigned)blocks, kThreads, 0, st>>>(first, second, n1, Di, words, p,
+    fb::launch_k((vec ? concretize_transposed<4> : concretize_transposed<1>), (unsigned)blocks, kThreads, 0, st, first, second, n1, Di, words, p,
                                                                                                      eps);
   } else {
     vec = vec && first.Do % 4 == 0 && (second.rows == 0 || second.Do % 4 == 0);
@@ -663,7 +672,7 @@ int launch_concretize(ConcretizeOne first, ConcretizeOne second, int Di, int wor
     second.ntiles = std::max(1, (int)ceil_div(second.Do, kCW));
     const int64_t n1 = first.rows * first.ntiles, blocks = n1 + second.rows * second.ntiles;
     if (blocks > 0x7fffffff) return FB_ERR_SHAPE;
-    (vec ? concretize_native<4> : concretize_native<1>)<<<(unsigned)blocks, kThreads, 0, st>>>(first, second, n1, Di, words, p, eps);
+    fb::launch_k((vec ? concretize_native<4> : concretize_native<1>), (unsigned)blocks, kThreads, 0, st, first, second, n1, Di, words, p, eps);
   }
   FB_LAUNCH_OK();
   return FB_OK;
@@ -691,7 +700,7 @@ int launch_relax(int op, const float* lw, const float* uw, const float* lb, cons
     const bool held = vec && words == 1 && Di <= 512;
     auto kern = !vec ? col_relax_transposed<1, 0> : !held ? col_relax_transposed<4, 0> : Di <= 128 ? col_relax_transposed<4, 1>
                 : Di <= 256 ? col_relax_transposed<4, 2> : col_relax_transposed<4, 4>;
-    kern<<<(unsigned)blocks, kThreads, 0, st>>>(op, lw, uw, lb, ub, o_lw, o_uw, o_lb, o_ub, ncols, Di, words, p, eps, violation);
+    fb::launch_k(kern, (unsigned)blocks, kThreads, 0, st, op, lw, uw, lb, ub, o_lw, o_uw, o_lb, o_ub, ncols, Di, words, p, eps, violation);
     FB_LAUNCH_OK();
     return FB_OK;
   }
@@ -711,7 +720,7 @@ int launch_relax(int op, const float* lw, const float* uw, const float* lb, cons
   do {                                                                                                     \
     int rc_ = ensure_smem(col_relax_native<V, S>, smem);                                                   \
     if (rc_ != FB_OK) return rc_;                                                                          \
-    col_relax_native<V, S><<<(unsigned)blocks, kThreads, smem, st>>>(op, lw, uw, lb, ub, o_lw, o_uw, o_lb, \
+    fb::launch_k(col_relax_native<V, S>, (unsigned)blocks, kThreads, smem, st, op, lw, uw, lb, ub, o_lw, o_uw, o_lb, \
                                                                      o_ub, Di, Do, ntiles, words, p, eps,  \
                                                                      violation);                           \
   } while (0)
@@ -731,6 +740,7 @@ __global__ void __launch_bounds__(256)
 relax_coef_given_kernel(int op, const float* __restrict__ lb, const float* __restrict__ ub, const float* __restrict__ l,
                         const float* __restrict__ u, float* __restrict__ c_l, float* __restrict__ c_u,
                         float* __restrict__ o_lb, float* __restrict__ o_ub, int64_t n, int* __restrict__ violation) {
+  pdl_sync();
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
     bool bad = false;
     const ColCoef c = relax_column(op, l[t], u[t], lb[t], ub[t], bad);
@@ -811,7 +821,7 @@ extern "C" int fb_mul_bounds_f32(const float* x_lw, const float* x_uw, const flo
   do {                                                                                                       \
     int rc_ = ensure_smem(col_mul_bounds_native<V, S>, smem);                                                \
     if (rc_ != FB_OK) return rc_;                                                                            \
-    col_mul_bounds_native<V, S><<<(unsigned)blocks, kThreads, smem, st>>>(x_lw, x_uw, x_lb, x_ub, y_lw, y_uw, \
+    fb::launch_k(col_mul_bounds_native<V, S>, (unsigned)blocks, kThreads, smem, st, x_lw, x_uw, x_lb, x_ub, y_lw, y_uw, \
                                                                           y_lb, y_ub, z_lw, z_uw, z_lb, z_ub, \
                                                                           Di, Do, ntiles, words, p, eps);     \
   } while (0)
@@ -859,8 +869,8 @@ extern "C" int fb_norm_partials_f32(const float* lw, const float* uw, float* par
     count_launches(1);
     return FB_OK;
   }
-  if (vec) col_norm_partials_native<4><<<(unsigned)blocks, kThreads, smem, (cudaStream_t)stream>>>(lw, uw, part_l, part_u, Di_local, Do, ntiles, p);
-  else col_norm_partials_native<1><<<(unsigned)blocks, kThreads, smem, (cudaStream_t)stream>>>(lw, uw, part_l, part_u, Di_local, Do, ntiles, p);
+  if (vec) fb::launch_k(col_norm_partials_native<4>, (unsigned)blocks, kThreads, smem, (cudaStream_t)stream, lw, uw, part_l, part_u, Di_local, Do, ntiles, p);
+  else fb::launch_k(col_norm_partials_native<1>, (unsigned)blocks, kThreads, smem, (cudaStream_t)stream, lw, uw, part_l, part_u, Di_local, Do, ntiles, p);
   FB_LAUNCH_OK();
   return FB_OK;
 }
@@ -881,8 +891,8 @@ extern "C" int fb_relax_with_norms_f32(int op, const float* lw, const float* uw,
   ProfileScope prof(PK_RELAX, 2.0 * mw, 4.0 * (4 * mw + 6.0 * rows * Do), stream);
   const bool vec = Do % 4 == 0 && aligned16(lw) && aligned16(uw) && aligned16(out_lw) && aligned16(out_uw);
   cudaStream_t st = (cudaStream_t)stream;
-  if (vec) col_relax_apply_native<4><<<(unsigned)blocks, kThreads, 0, st>>>(op, lw, uw, lb, ub, norm_l, norm_u, out_lw, out_uw, out_lb, out_ub, Di_local, Do, ntiles, p, eps, violation);
-  else col_relax_apply_native<1><<<(unsigned)blocks, kThreads, 0, st>>>(op, lw, uw, lb, ub, norm_l, norm_u, out_lw, out_uw, out_lb, out_ub, Di_local, Do, ntiles, p, eps, violation);
+  if (vec) fb::launch_k(col_relax_apply_native<4>, (unsigned)blocks, kThreads, 0, st, op, lw, uw, lb, ub, norm_l, norm_u, out_lw, out_uw, out_lb, out_ub, Di_local, Do, ntiles, p, eps, violation);
+  else fb::launch_k(col_relax_apply_native<1>, (unsigned)blocks, kThreads, 0, st, op, lw, uw, lb, ub, norm_l, norm_u, out_lw, out_uw, out_lb, out_ub, Di_local, Do, ntiles, p, eps, violation);
   FB_LAUNCH_OK();
   return FB_OK;
 }
@@ -919,7 +929,7 @@ extern "C" int fb_relax_coef_given_f32(int op, const float* lb, const float* ub,
   const int64_t n = rows * Do;
   ProfileScope prof(PK_RELAX, 8.0 * n, 4.0 * 8 * n, stream);
   const int64_t want = ceil_div(n, 256), cap = (int64_t)device_info().sms * 16;
-  relax_coef_given_kernel<<<(unsigned)(want < cap ? want : cap), 256, 0, (cudaStream_t)stream>>>(op, lb, ub, l, u, c_l, c_u,
+  fb::launch_k(relax_coef_given_kernel, (unsigned)(want < cap ? want : cap), 256, 0, (cudaStream_t)stream, op, lb, ub, l, u, c_l, c_u,
                                                                                                 out_lb, out_ub, n, violation);
   FB_LAUNCH_OK();
   return FB_OK;

@@ -37,6 +37,24 @@ const DeviceInfo& device_info();
 
 void count_launches(int n);
 
+// A launch whose blocks may become resident while the launch before on the stream still drains (programmatic dependent launch):
+// the passes over one sentence are chains of kernels of 3 to 10 us with 2 us between them, most of it launch latency and
+// prologues (barriers, tensor memory, tensor maps).  The kernel must call pdl_sync() first thing.
+template <typename... P, typename... A>
+inline void launch_k(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);   // (errors are picked up by FB_LAUNCH_OK)
+}
+
 // Hint for the tensor-core GEMM (thread-local, set by the encoder driver around the projections of the first layer):
 // the operand has M rows in blocks of Di per (sentence, position) pair, L positions per sentence, and only the
 // blocks of the perturbed positions are non-zero (the input bound is an identity at those positions and zero
@@ -158,6 +176,12 @@ __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b)
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdiv_rn(a, b); }
+
+// Every kernel launched through launch_k calls this before it reads or writes anything another launch may touch: it waits for
+// the launches before to complete, and lets the next one start its prologue.
+__device__ __forceinline__ void pdl_sync() {
+  asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // Two FP32 multiply-adds per instruction (fma.rn.f32x2), lanes in a 64-bit register pair.
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {

@@ -51,6 +51,7 @@ __device__ __forceinline__ void lds128(uint32_t a, uint64_t& v, uint64_t& w) {
 template <int CPT, int PX, int KS, int ST>
 __global__ void __launch_bounds__(kConvThreads)
 conv_bounds_kernel(const ConvArgs q) {
+  pdl_sync();
   static_assert(CPT % 2 == 0 && 32 % CPT == 0, "two channels per read; every thread stages the weights of one channel");
   extern __shared__ __align__(16) float smem[];
   const int Kh = KS ? KS : q.Kh, Kw = KS ? KS : q.Kw, taps = Kh * Kw, co_n = q.G * CPT;
@@ -227,7 +228,7 @@ int launch_conv_t(const ConvArgs& q, int64_t blocks, size_t smem, cudaStream_t s
   auto kern = ks == 3 ? FB_CONV_ST(3) : ks == 5 ? FB_CONV_ST(5) : FB_CONV_ST(0);
 #undef FB_CONV_ST
   if (int rc = ensure_dynamic_smem(kern, smem)) return rc;
-  kern<<<(unsigned)blocks, q.G * 32, smem, st>>>(q);
+  fb::launch_k(kern, (unsigned)blocks, q.G * 32, smem, st, q);
   FB_LAUNCH_OK();
   return FB_OK;
 }
@@ -276,6 +277,7 @@ identity_conv_columns_kernel(int op, const float* __restrict__ x_lb, const float
                              float* __restrict__ k_l, float* __restrict__ k_u, float scale, int Cin, int H, int W, int Cout,
                              int Kh_arg, int Kw_arg, int stride, int pad, int Ho, int Wo, int p, float eps,
                              int* __restrict__ violation) {
+  pdl_sync();
   const int Kh = KS ? KS : Kh_arg, Kw = KS ? KS : Kw_arg;
   const int64_t n = (int64_t)Cout * Ho * Wo;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
@@ -334,6 +336,7 @@ __global__ void __launch_bounds__(256)
 identity_conv_rows_kernel(const float* __restrict__ Wt, const float* __restrict__ k_l, const float* __restrict__ k_u,
                           float* __restrict__ y_lw, float* __restrict__ y_uw, float scale, int64_t row_start, int Cin,
                           int H, int W, int Cout, int Kh, int Kw, int stride, int pad, int Ho, int Wo) {
+  pdl_sync();
   const int64_t r = row_start + blockIdx.x;
   const int xi = (int)(r % W), yi = (int)((r / W) % H), ci = (int)(r / ((int64_t)W * H));
   const unsigned n = (unsigned)Cout * Ho * Wo, uWo = Wo, uHo = Ho;
@@ -371,6 +374,7 @@ conv_window_kernel(const float* __restrict__ x_lo, const float* __restrict__ x_u
                    float* __restrict__ y_lo, float* __restrict__ y_up, int64_t row_start, int H0, int W0,
                    const ConvChain ch, int Cin, int H, int W, int Cout, int Kh, int Kw, int stride, int pad, int Ho,
                    int Wo, int win_h, int win_w, int out_h, int out_w) {
+  pdl_sync();
   extern __shared__ float win_smem[];
   float* s_c = win_smem;
   float* s_r = s_c + Cin * win_h * win_w;
@@ -468,7 +472,7 @@ int launch_identity_columns(int op, const float* x_lb, const float* x_ub, const 
   const int64_t ncol = (int64_t)Cout * Ho * Wo;
   const int64_t want = ceil_div(ncol, 128), cap = (int64_t)device_info().sms * 16;
   auto kern = Kh == 3 && Kw == 3 ? identity_conv_columns_kernel<3> : identity_conv_columns_kernel<0>;
-  kern<<<(unsigned)(want < cap ? want : cap), 128, 0, st>>>(op, x_lb, x_ub, Wt, bias, y_lb, y_ub, k_l, k_u, scale, Cin, H, W, Cout, Kh, Kw,
+  fb::launch_k(kern, (unsigned)(want < cap ? want : cap), 128, 0, st, op, x_lb, x_ub, Wt, bias, y_lb, y_ub, k_l, k_u, scale, Cin, H, W, Cout, Kh, Kw,
                                                             stride, pad, Ho, Wo, p, eps, violation);
   FB_LAUNCH_OK();
   return FB_OK;
@@ -500,10 +504,10 @@ extern "C" int fb_conv2d_identity_relax_f32(int op, const float* x_lb, const flo
   if (rows > 0x7fffffff) return FB_ERR_SHAPE;
   if (ncol > 0x7fffffff) return FB_ERR_SHAPE;
   if (Wo % 4 == 0 && fb::aligned16(y_lw) && fb::aligned16(y_uw))
-    fb::identity_conv_rows_kernel<4><<<(unsigned)rows, 256, 0, st>>>(Wt, k_l, k_u, y_lw, y_uw, scale, row_start, Cin, H, W,
+    fb::launch_k(fb::identity_conv_rows_kernel<4>, (unsigned)rows, 256, 0, st, Wt, k_l, k_u, y_lw, y_uw, scale, row_start, Cin, H, W,
                                                                        Cout, Kh, Kw, stride, pad, Ho, Wo);
   else
-    fb::identity_conv_rows_kernel<1><<<(unsigned)rows, 256, 0, st>>>(Wt, k_l, k_u, y_lw, y_uw, scale, row_start, Cin, H, W,
+    fb::launch_k(fb::identity_conv_rows_kernel<1>, (unsigned)rows, 256, 0, st, Wt, k_l, k_u, y_lw, y_uw, scale, row_start, Cin, H, W,
                                                                        Cout, Kh, Kw, stride, pad, Ho, Wo);
   FB_LAUNCH_OK();
   return FB_OK;
@@ -557,7 +561,7 @@ extern "C" int fb_conv2d_windowed_f32(const float* x_lw, const float* x_uw, cons
   if (int rc = fb::ensure_dynamic_smem(kern, smem)) return rc;
   fb::ProfileScope prof(fb::PK_CONV, 8.0 * rows * Cout * out_h * out_w * Cin * Kh * Kw,
                         4.0 * (2.0 * rows * Cin * win_h * win_w + 2.0 * rows * ncol), stream);
-  kern<<<(unsigned)rows, 256, smem, st>>>(x_lw, x_uw, Wt, y_lw, y_uw, row_start, H0, W0, ch, Cin, H, W, Cout, Kh, Kw, stride, pad,
+  fb::launch_k(kern, (unsigned)rows, 256, smem, st, x_lw, x_uw, Wt, y_lw, y_uw, row_start, H0, W0, ch, Cin, H, W, Cout, Kh, Kw, stride, pad,
                                           Ho, Wo, win_h, win_w, out_h, out_w);
   FB_LAUNCH_OK();
   return FB_OK;

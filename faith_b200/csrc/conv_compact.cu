@@ -51,6 +51,7 @@ __global__ void __launch_bounds__(256)
 cw_identity_rows_kernel(const float* __restrict__ Wt, const float* __restrict__ k_l, const float* __restrict__ k_u,
                         float* __restrict__ z_lw, float* __restrict__ z_uw, float scale, int64_t rows, int64_t row_start,
                         int Cin, int H, int W, int Cout, int Kh, int Kw, int stride, int pad, int Ho, int Wo, int wh, int ww) {
+  pdl_sync();
   const int64_t per_row = (int64_t)Cout * wh * ww;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < rows * per_row; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t lr = t / per_row;
@@ -129,6 +130,7 @@ cw_conv_kernel(const __grid_constant__ CwConvArgs q) {
   extern __shared__ __align__(16) float cw_smem[];
   __shared__ CwRow s_row[kCwMaxRows];
   touch_params(q);
+  pdl_sync();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x, nwarps = nthr >> 5;
   const int Kh = KS ? KS : q.Kh, Kw = KS ? KS : q.Kw, taps = Kh * Kw;
   if ((int)blockIdx.x < q.blocks_bias) {   // an ordinary convolution of one image, a thread per output
@@ -375,6 +377,7 @@ cw_norm_kernel(int op, const float* __restrict__ z_lw, const float* __restrict__
                float* __restrict__ part_u, const float* __restrict__ lb, const float* __restrict__ ub, float* __restrict__ out_lb,
                float* __restrict__ out_ub, float* __restrict__ coef, int64_t rows, int64_t row_start, int Cin0, const __grid_constant__ CwShape g, int p,
                float eps, int* __restrict__ violation) {
+  pdl_sync();
   __shared__ float s_part[2][kCwNormWarps][32];
   const int y = blockIdx.x / g.W, x = blockIdx.x - y * g.W, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.y * 32 + lane;
@@ -429,6 +432,7 @@ __global__ void __launch_bounds__(256)
 cw_relax_columns_kernel(int op, const float* __restrict__ lb, const float* __restrict__ ub, const float* __restrict__ norm_l,
                         const float* __restrict__ norm_u, float* __restrict__ out_lb, float* __restrict__ out_ub,
                         float* __restrict__ coef, int C, int64_t hw, int p, float eps, int* __restrict__ violation) {
+  pdl_sync();
   const int64_t ncol = C * hw;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < ncol; t += (int64_t)gridDim.x * blockDim.x)
     cw_relax_column(op, lb[t], ub[t], norm_l[t], norm_u[t], p, eps, t, (t % hw) * C + t / hw, ncol, out_lb, out_ub, coef, violation);
@@ -439,6 +443,7 @@ cw_relax_columns_kernel(int op, const float* __restrict__ lb, const float* __res
 __global__ void __launch_bounds__(256)
 cw_rescale_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw, const float* __restrict__ coef,
                   float* __restrict__ o_lw, float* __restrict__ o_uw, int64_t rows, int64_t row_start, const CwShape g) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const int64_t lr = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (lr >= rows) return;
@@ -487,6 +492,7 @@ template <int NB>
 __global__ void __launch_bounds__(kCwLinThreads)
 cw_linear_kernel(const __grid_constant__ CwLinearArgs q) {
   touch_params(q);
+  pdl_sync();
   constexpr int LDN = NB + 2, LDP = 32 * LDN + 2;   // the lanes' 64-bit reads, along the channels, and the stores, along the
                                                     // positions, fall on different banks
   extern __shared__ __align__(16) float cw_smem[];
@@ -642,6 +648,7 @@ cw_linear_kernel(const __grid_constant__ CwLinearArgs q) {
 __global__ void __launch_bounds__(64)
 cw_linear_range_kernel(const float* __restrict__ part, const float* __restrict__ lb, const float* __restrict__ ub, float* __restrict__ l,
                        float* __restrict__ u, int tiles, int N, int p, float eps) {
+  pdl_sync();
   const int lane = threadIdx.x & 31, side = threadIdx.x >> 5, n = blockIdx.x;
   float a = 0.f;
 #pragma unroll 4
@@ -658,6 +665,7 @@ cw_linear_range_kernel(const float* __restrict__ part, const float* __restrict__
 __global__ void __launch_bounds__(256)
 cw_expand_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw, float* __restrict__ y_lw,
                  float* __restrict__ y_uw, int64_t row_start, const CwShape g) {
+  pdl_sync();
   const int64_t r = row_start + blockIdx.x;
   int yi, xi;
   pixel_of_row(r, g.H0, g.W0, yi, xi);
@@ -775,7 +783,7 @@ int cw_conv_ex(const float* z_lo, const float* z_up, const float* W1, const floa
   if (int rc = ensure_dynamic_smem(kern, bytes() + kCwStatic)) return rc;   // (48 KB without the attribute hold the static part too)
   ProfileScope prof(PK_CONV, 8.0 * rows * Cout * go.wh * go.ww * Cin * Kh * Kw,
                     4.0 * 2.0 * rows * ((double)Cin * gi.wh * gi.ww + (double)Cout * go.wh * go.ww), (void*)st);
-  kern<<<(unsigned)blocks, threads, bytes(), st>>>(q);
+  fb::launch_k(kern, (unsigned)blocks, threads, bytes(), st, q);
   FB_LAUNCH_OK();
   return FB_OK;
 }
@@ -817,14 +825,14 @@ int cw_linear_ex(const float* z_lw, const float* z_uw, const float* coef, const 
   if (int rc = ensure_dynamic_smem(kern, smem + kCwStatic)) return rc;
   ProfileScope prof(PK_MATMUL, 8.0 * rows * C * q.g.wh * q.g.ww * N,
                     4.0 * (2.0 * rows * C * q.g.wh * q.g.ww + 2.0 * rows * N + (double)C * H * W * N), (void*)st);
-  kern<<<dim3((unsigned)blocks, (unsigned)groups), kCwLinThreads, smem, st>>>(q);
+  fb::launch_k(kern, dim3((unsigned)blocks, (unsigned)groups), kCwLinThreads, smem, st, q);
   FB_LAUNCH_OK();
   return FB_OK;
 }
 
 int cw_linear_range(const float* part, const float* lb, const float* ub, float* l, float* u, int H0, int W0, int N, int p, float eps,
                     cudaStream_t st) {
-  cw_linear_range_kernel<<<(unsigned)N, 64, 0, st>>>(part, lb, ub, l, u, (int)cw_linear_tiles(H0, W0), N, p, eps);
+  fb::launch_k(cw_linear_range_kernel, (unsigned)N, 64, 0, st, part, lb, ub, l, u, (int)cw_linear_tiles(H0, W0), N, p, eps);
   FB_LAUNCH_OK();
   return FB_OK;
 }
@@ -839,15 +847,14 @@ int cw_norm_ex(int op, const float* z_lw, const float* z_uw, float* part_l, floa
   if (rc != FB_OK) return rc;
   if (ceil_div(C, 32) > 65535 || (int64_t)Cin0 * H0 * W0 > 0x7fffffff) return FB_ERR_SHAPE;
   ProfileScope prof(PK_RELAX, 4.0 * rows * C * g.wh * g.ww, 4.0 * (2.0 * rows * C * g.wh * g.ww + 2.0 * C * H * W), (void*)st);
-  cw_norm_kernel<<<dim3((unsigned)(H * W), (unsigned)ceil_div(C, 32)), 32 * kCwNormWarps, 0, st>>>(
-      op, z_lw, z_uw, part_l, part_u, lb, ub, out_lb, out_ub, coef, rows, row_start, Cin0, g, p, eps, violation);
+  fb::launch_k(cw_norm_kernel, dim3((unsigned)(H * W), (unsigned)ceil_div(C, 32)), 32 * kCwNormWarps, 0, st, op, z_lw, z_uw, part_l, part_u, lb, ub, out_lb, out_ub, coef, rows, row_start, Cin0, g, p, eps, violation);
   FB_LAUNCH_OK();
   return FB_OK;
 }
 
 int cw_relax_columns(int op, const float* lb, const float* ub, const float* norm_l, const float* norm_u, float* out_lb, float* out_ub,
                      float* coef, int C, int64_t hw, int p, float eps, int* violation, cudaStream_t st) {
-  cw_relax_columns_kernel<<<grid_for(C * hw, 256), 256, 0, st>>>(op, lb, ub, norm_l, norm_u, out_lb, out_ub, coef, C, hw, p, eps, violation);
+  fb::launch_k(cw_relax_columns_kernel, grid_for(C * hw, 256), 256, 0, st, op, lb, ub, norm_l, norm_u, out_lb, out_ub, coef, C, hw, p, eps, violation);
   FB_LAUNCH_OK();
   return FB_OK;
 }
@@ -857,7 +864,7 @@ int cw_rescale_rows(const float* z_lw, const float* z_uw, const float* coef, flo
   CwShape g;
   int rc = make_shape(chain, n_chain, H0, W0, C, H, W, g);
   if (rc != FB_OK || rows == 0) return rc;
-  cw_rescale_kernel<<<(unsigned)ceil_div(rows, 8), 256, 0, st>>>(z_lw, z_uw, coef, out_lw, out_uw, rows, row_start, g);
+  fb::launch_k(cw_rescale_kernel, (unsigned)ceil_div(rows, 8), 256, 0, st, z_lw, z_uw, coef, out_lw, out_uw, rows, row_start, g);
   FB_LAUNCH_OK();
   return FB_OK;
 }
@@ -903,7 +910,7 @@ extern "C" int fb_cw_identity_relax_f32(int op, const float* x_lb, const float* 
   rc = launch_identity_columns(op, x_lb, x_ub, Wt, bias, y_lb, y_ub, k_l, k_u, scale, Cin, H, W, Cout, Kh, Kw, stride, pad, Ho, Wo, p, eps,
                                violation, st);
   if (rc != FB_OK || rows == 0) return rc;
-  cw_identity_rows_kernel<<<grid_for(rows * Cout * g.wh * g.ww, 256), 256, 0, st>>>(Wt, k_l, k_u, z_lw, z_uw, scale, rows, row_start,
+  fb::launch_k(cw_identity_rows_kernel, grid_for(rows * Cout * g.wh * g.ww, 256), 256, 0, st, Wt, k_l, k_u, z_lw, z_uw, scale, rows, row_start,
                                                                                    Cin, H, W, Cout, Kh, Kw, stride, pad, Ho, Wo,
                                                                                    g.wh, g.ww);
   FB_LAUNCH_OK();
@@ -962,7 +969,7 @@ extern "C" int fb_cw_expand_f32(const float* z_lw, const float* z_uw, float* y_l
   if (rows == 0) return FB_OK;
   if (rows > 0x7fffffff) return FB_ERR_SHAPE;
   ProfileScope prof(PK_ELEMENTWISE, 0.0, 4.0 * 2.0 * rows * C * H * W, stream);
-  cw_expand_kernel<<<(unsigned)rows, 256, 0, (cudaStream_t)stream>>>(z_lw, z_uw, y_lw, y_uw, row_start, g);
+  fb::launch_k(cw_expand_kernel, (unsigned)rows, 256, 0, (cudaStream_t)stream, z_lw, z_uw, y_lw, y_uw, row_start, g);
   FB_LAUNCH_OK();
   return FB_OK;
 }

@@ -32,6 +32,7 @@ dot_bias_kernel(const float* __restrict__ x_lb, const float* __restrict__ x_ub, 
                 const float* __restrict__ y_ub, const float* __restrict__ x_l, const float* __restrict__ y_l,
                 const float* __restrict__ y_u, float* __restrict__ z_lb, float* __restrict__ z_ub,
                 int64_t total, int Lx, int Ly, int K, float out_scale, int heads) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (kThreads / 32);
   for (int64_t o = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5); o < total; o += warps) {
@@ -176,6 +177,7 @@ __device__ __forceinline__ void dot_bias_tile(const DotBias& q, int w, float* sm
 
 template <int RI>
 __global__ void __launch_bounds__(kThreads) dot_bias_tiled(const DotBias q) {
+  pdl_sync();
   __shared__ float smem[dot_bias_smem_floats(RI)];
   dot_bias_tile<RI>(q, blockIdx.x, smem);
 }
@@ -225,6 +227,7 @@ dot_weight_native(const float* __restrict__ x_lw, const float* __restrict__ x_uw
                   const float* __restrict__ y_uw, const float* __restrict__ x_l, const float* __restrict__ y_l,
                   const float* __restrict__ y_u, float* __restrict__ z_lw, float* __restrict__ z_uw,
                   int Lx, int Ly, int Di, int K, int n_it, int n_jt, int n_mt, float out_scale) {
+  pdl_sync();
   extern __shared__ __align__(16) float smem[];
   float* s_xl = smem;
   float* s_xu = s_xl + XT;
@@ -329,6 +332,7 @@ dot_weight_rows_kernel(const float* __restrict__ x_lw, const float* __restrict__
                        const float* __restrict__ y_uw, const float* __restrict__ x_l, const float* __restrict__ y_l,
                        const float* __restrict__ y_u, float* __restrict__ z_lw, float* __restrict__ z_uw, int64_t total,
                        int Lx, int Ly, int Di, int K, float out_scale, int merge_heads, int y_kmajor) {
+  pdl_sync();
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int j = (int)(t % Ly), m = (int)((t / Ly) % Di), i = (int)((t / ((int64_t)Ly * Di)) % Lx);
     const int64_t b = t / ((int64_t)Ly * Di * Lx);
@@ -368,7 +372,7 @@ int launch_dot_weight_rows(const float* x_lw, const float* x_uw, const float* y_
                            float out_scale, int merge_heads, int y_kmajor, cudaStream_t st) {
   const int64_t total = (int64_t)B * Lx * Di * Ly;
   const int64_t want = ceil_div(total, 256), cap = (int64_t)device_info().sms * 64;
-  dot_weight_rows_kernel<<<(unsigned)(want < cap ? want : cap), 256, 0, st>>>(x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, total,
+  fb::launch_k(dot_weight_rows_kernel, (unsigned)(want < cap ? want : cap), 256, 0, st, x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, total,
                                                                              Lx, Ly, Di, K, out_scale, merge_heads, y_kmajor);
   FB_LAUNCH_OK();
   return FB_OK;
@@ -383,16 +387,16 @@ int launch_dot_bias(const float* x_lb, const float* x_ub, const float* y_lb, con
   DotBias q = {x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u, z_lb, z_ub, Lx, Ly, K, 0, n_jt, heads, y_kmajor, ranges_kmajor, out_scale};
   if (b32 < 2 * (int64_t)device_info().sms && b8 <= 0x7fffffff) {
     q.n_it = (int)ceil_div(Lx, 8);
-    dot_bias_tiled<8><<<(unsigned)b8, kThreads, 0, st>>>(q);
+    fb::launch_k(dot_bias_tiled<8>, (unsigned)b8, kThreads, 0, st, q);
   } else if (b32 <= 0x7fffffff) {
     q.n_it = (int)ceil_div(Lx, 32);
-    dot_bias_tiled<32><<<(unsigned)b32, kThreads, 0, st>>>(q);
+    fb::launch_k(dot_bias_tiled<32>, (unsigned)b32, kThreads, 0, st, q);
   } else {
     if (y_kmajor || ranges_kmajor) return FB_ERR_SHAPE;
     const int64_t total = (int64_t)B * Lx * Ly;
     const int64_t want = ceil_div(total, kThreads / 32);
     const int64_t cap = (int64_t)device_info().sms * 32;
-    dot_bias_kernel<<<(unsigned)(want < cap ? want : cap), kThreads, 0, st>>>(x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u, z_lb, z_ub, total,
+    fb::launch_k(dot_bias_kernel, (unsigned)(want < cap ? want : cap), kThreads, 0, st, x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u, z_lb, z_ub, total,
                                                                               Lx, Ly, K, out_scale, heads);
   }
   FB_LAUNCH_OK();
@@ -504,11 +508,10 @@ int fb::dot_product_ex(const float* x_lw, const float* x_uw, const float* x_lb, 
       const size_t psmem = sizeof(float) * kDotPipeSmemFloats;
       if (int rc = ensure_dynamic_smem(dot_weight_native_pipelined, psmem)) return rc;
       const int64_t sms = device_info().sms;
-      dot_weight_native_pipelined<<<(unsigned)(blocks < sms ? blocks : sms), kThreads, psmem, st>>>(
-          x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, Lx, Ly, Di, K, n_it, n_jt, n_mt, n_kc, n_items, out_scale, merge_heads);
+      fb::launch_k(dot_weight_native_pipelined, (unsigned)(blocks < sms ? blocks : sms), kThreads, psmem, st, x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, Lx, Ly, Di, K, n_it, n_jt, n_mt, n_kc, n_items, out_scale, merge_heads);
     } else {
       if (int rc = ensure_dynamic_smem(dot_weight_native<false>, smem)) return rc;
-      dot_weight_native<false><<<(unsigned)blocks, kThreads, smem, st>>>(x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw,
+      fb::launch_k(dot_weight_native<false>, (unsigned)blocks, kThreads, smem, st, x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw,
                                                                          z_uw, Lx, Ly, Di, K, n_it, n_jt, n_mt, out_scale);
     }
   }
@@ -552,6 +555,7 @@ namespace fb {
 namespace {
 // In-place transposition of [B][R][C] -> [B][C][R] for small matrices (R * C <= 4096): one block per b.
 __global__ void __launch_bounds__(256) transpose_small_inplace(float* a, float* b2, int R, int C) {
+  pdl_sync();
   __shared__ float t[2][4096];
   float* pa = a + (int64_t)blockIdx.x * R * C;
   float* pb = b2 + (int64_t)blockIdx.x * R * C;
@@ -636,7 +640,7 @@ int fb::context_ex(const float* x_lw, const float* x_uw, const float* x_lb, cons
   if (rc != FB_OK) return rc;
   const bool transpose = transposed_ranges || !tc || tc32;
   if (transpose) {
-    transpose_small_inplace<<<(unsigned)B, 256, 0, st>>>(y_l, y_u, K, Ly);
+    fb::launch_k(transpose_small_inplace, (unsigned)B, 256, 0, st, y_l, y_u, K, Ly);
     FB_LAUNCH_OK();
   }
   rc = launch_dot_bias(x_lb, x_ub, v_lb, v_ub, x_l, y_l, y_u, z_lb, z_ub, B, Lx, Ly, K, out_scale, merge_heads, 1, transpose ? 0 : 1, st);

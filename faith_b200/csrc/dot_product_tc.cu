@@ -125,6 +125,7 @@ dot_weight_tc(const __grid_constant__ CUtensorMap tm_xl, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_sync();
 
   // coordinates of tile t of this CTA
   auto tile_coords = [&](int t, int& b, int& i0, int& m0) {
@@ -498,8 +499,7 @@ int launch_dot_weight_tc(const float* x_lw, const float* x_uw, const float* y_lw
   });
   FB_CUDA_OK(attr_err);
   const int sms = device_info().sms;
-  dot_weight_tc<<<(unsigned)(total < sms ? total : sms), kDtThreads, kDtSmemBytes, st>>>(
-      tm_xl, tm_xu, tm_yl, tm_yu, tm_lx, tm_ly, tm_uy, tm_zl, tm_zu, Lx, Ly, n_ib, n_mb, total, out_scale, heads, y_kmajor, tc_status_sink());
+  fb::launch_k(dot_weight_tc, (unsigned)(total < sms ? total : sms), kDtThreads, kDtSmemBytes, st, tm_xl, tm_xu, tm_yl, tm_yu, tm_lx, tm_ly, tm_uy, tm_zl, tm_zu, Lx, Ly, n_ib, n_mb, total, out_scale, heads, y_kmajor, tc_status_sink());
   FB_LAUNCH_OK();
   return FB_OK;
 }

@@ -161,6 +161,7 @@ dot_weight_tc_any(const __grid_constant__ CUtensorMap tm_xl, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_sync();
 
   // 16 columns of X or Y: the sum of its two accumulators
   auto load_acc = [](uint32_t addr, uint32_t (&v)[16]) {
@@ -503,8 +504,7 @@ template <bool kTmaIn, bool kVecOut, bool kMulti>
 int launch_variant(const CUtensorMap (&tm)[4], const DotArgs& a, cudaStream_t st) {
   const int sms = device_info().sms;
   if (int rc = ensure_dynamic_smem(dot_weight_tc_any<kTmaIn, kVecOut, kMulti>, kDaSmemBytes)) return rc;
-  dot_weight_tc_any<kTmaIn, kVecOut, kMulti><<<(unsigned)(a.total_tiles < sms ? a.total_tiles : sms), kDaThreads, kDaSmemBytes, st>>>(
-      tm[0], tm[1], tm[2], tm[3], a, tc_status_sink());
+  fb::launch_k(dot_weight_tc_any<kTmaIn, kVecOut, kMulti>, (unsigned)(a.total_tiles < sms ? a.total_tiles : sms), kDaThreads, kDaSmemBytes, st, tm[0], tm[1], tm[2], tm[3], a, tc_status_sink());
   FB_LAUNCH_OK();
   return FB_OK;
 }

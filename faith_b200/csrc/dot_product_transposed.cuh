@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(DotTransposedTile<WI, WJ, WK>::kThr, 1)
 dot_weight_transposed(const float* __restrict__ x_lw, const float* __restrict__ x_uw, const float* __restrict__ y_lw,
                       const float* __restrict__ y_uw, float* __restrict__ z_lw, float* __restrict__ z_uw, const DotBias q, int Di,
                       int n_bias, int n_it, int n_jt, int n_mt) {
+  pdl_sync();
   using T = DotTransposedTile<WI, WJ, WK>;
   constexpr int KS = T::KS, TK = T::kTK, M = kDotTransposedM;
   extern __shared__ __align__(16) float smem[];
@@ -214,7 +215,7 @@ int launch_dot_transposed_t(const float* x_lw, const float* x_uw, const float* y
   if (blocks > 0x7fffffff) return FB_ERR_SHAPE;
   auto kern = dot_weight_transposed<WI, WJ, WK, VEC>;
   if (int rc = ensure_dynamic_smem(kern, T::kSmem)) return rc;
-  kern<<<(unsigned)blocks, T::kThr, T::kSmem, st>>>(x_lw, x_uw, y_lw, y_uw, z_lw, z_uw, q, Di, (int)n_bias, n_it, n_jt, n_mt);
+  fb::launch_k(kern, (unsigned)blocks, T::kThr, T::kSmem, st, x_lw, x_uw, y_lw, y_uw, z_lw, z_uw, q, Di, (int)n_bias, n_it, n_jt, n_mt);
   FB_LAUNCH_OK();
   return FB_OK;
 }

@@ -29,6 +29,7 @@ struct OutLines {
 template <int VEC>
 __global__ void __launch_bounds__(kThreads)
 add_kernel(Lines xw, Lines yw, OutLines zw, Lines xb, Lines yb, OutLines zb, int64_t nv, int64_t nb) {
+  pdl_sync();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv + nb; i += stride) {
     if (i >= nv) {
@@ -53,6 +54,7 @@ add_kernel(Lines xw, Lines yw, OutLines zw, Lines xb, Lines yb, OutLines zb, int
 template <int VEC>
 __global__ void __launch_bounds__(kThreads)
 scale_kernel(Lines xw, OutLines zw, Lines xb, OutLines zb, float c, int64_t nv, int64_t nb) {
+  pdl_sync();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv + nb; i += stride) {
     if (i >= nv) {
@@ -97,6 +99,7 @@ __global__ void __launch_bounds__(kThreads)
 rowsum_kernel(const float* __restrict__ x_lw, const float* __restrict__ x_uw, const float* __restrict__ x_lb,
               const float* __restrict__ x_ub, float* __restrict__ z_lw, float* __restrict__ z_uw,
               float* __restrict__ z_lb, float* __restrict__ z_ub, int64_t n_w, int64_t n_b, int Do) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (kThreads / 32);
   for (int64_t row = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5); row < n_w + n_b; row += warps) {
@@ -122,6 +125,7 @@ layernorm_novar_kernel(const float* __restrict__ x_lw, const float* __restrict__
                        const float* __restrict__ gamma, const float* __restrict__ beta,
                        float* __restrict__ z_lw, float* __restrict__ z_uw, float* __restrict__ z_lb,
                        float* __restrict__ z_ub, int64_t n_w, int64_t n_b, int Do) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (kThreads / 32);
   const float inv_n = 1.0f / (float)Do;
@@ -171,6 +175,7 @@ layernorm_novar_row128_kernel(const float* __restrict__ x_lw, const float* __res
                               const float* __restrict__ gamma, const float* __restrict__ beta,
                               float* __restrict__ z_lw, float* __restrict__ z_uw, float* __restrict__ z_lb,
                               float* __restrict__ z_ub, int64_t n_w, int64_t n_b, float* __restrict__ rowsum) {
+  pdl_sync();
   constexpr int Do = 128;
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (kThreads / 32);
@@ -254,6 +259,7 @@ __device__ __forceinline__ void permute_item(Index i, Index M, Index L, Index H,
 template <int VEC, bool SPLIT, typename Index>
 __global__ void __launch_bounds__(kThreads)
 heads_permute_kernel(Lines src_w, OutLines dst_w, Lines src_b, OutLines dst_b, Index n_w, Index n_b, int L, int M, int H, int d) {
+  pdl_sync();
   const bool up = blockIdx.y != 0;
   const float* const sw = up ? src_w.u : src_w.l;
   const float* const sb = up ? src_b.u : src_b.l;
@@ -278,6 +284,7 @@ heads_permute_kernel(Lines src_w, OutLines dst_w, Lines src_b, OutLines dst_b, I
 // (along d) and the writes (along L) are contiguous.
 __global__ void __launch_bounds__(kThreads)
 heads_split_transpose_kernel(const float* __restrict__ src, float* __restrict__ dst, int B, int L, int M, int H, int d) {
+  pdl_sync();
   __shared__ float tile[32][33];
   const int64_t bid = blockIdx.x;
   const int m = (int)(bid % M);
@@ -311,6 +318,7 @@ __device__ __forceinline__ void mul_feature(float wv, float a, float b, float& z
 template <int VEC>
 __global__ void __launch_bounds__(kThreads)
 mul_features_kernel(Lines xw, OutLines zw, Lines xb, OutLines zb, const float* __restrict__ w, int64_t nv, int64_t nb, int Do) {
+  pdl_sync();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv + nb; i += stride) {
     // (every element is read before it is written: z may alias x)
@@ -344,6 +352,7 @@ mul_features_kernel(Lines xw, OutLines zw, Lines xb, OutLines zb, const float* _
 __global__ void __launch_bounds__(kThreads)
 interval_mul_kernel(const float* __restrict__ xl, const float* __restrict__ xu, const float* __restrict__ yl,
                     const float* __restrict__ yu, float* __restrict__ zl, float* __restrict__ zu, int64_t n) {
+  pdl_sync();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     const float p1 = fmul(xl[i], yl[i]), p2 = fmul(xl[i], yu[i]), p3 = fmul(xu[i], yl[i]), p4 = fmul(xu[i], yu[i]);
@@ -358,6 +367,7 @@ __global__ void __launch_bounds__(kThreads)
 interval_dot_kernel(const float* __restrict__ xl, const float* __restrict__ xu, const float* __restrict__ yl,
                     const float* __restrict__ yu, float* __restrict__ zl, float* __restrict__ zu, int64_t n_out, int Lx,
                     int Ly, int K) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t o = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; o < n_out; o += warps) {
@@ -407,8 +417,8 @@ extern "C" int fb_add_f32(const float* x_lw, const float* x_uw, const float* x_l
                   aligned16(z_lw) && aligned16(z_uw);
   const Lines xw = {x_lw, x_uw}, yw = {y_lw, y_uw}, xb = {x_lb, x_ub}, yb = {y_lb, y_ub};
   const OutLines zw = {z_lw, z_uw}, zb = {z_lb, z_ub};
-  if (vw) add_kernel<4><<<stream_blocks(nw / 4 + nb), kThreads, 0, st>>>(xw, yw, zw, xb, yb, zb, nw / 4, nb);
-  else add_kernel<1><<<stream_blocks(nw + nb), kThreads, 0, st>>>(xw, yw, zw, xb, yb, zb, nw, nb);
+  if (vw) fb::launch_k(add_kernel<4>, stream_blocks(nw / 4 + nb), kThreads, 0, st, xw, yw, zw, xb, yb, zb, nw / 4, nb);
+  else fb::launch_k(add_kernel<1>, stream_blocks(nw + nb), kThreads, 0, st, xw, yw, zw, xb, yb, zb, nw, nb);
   FB_LAUNCH_OK();
   return FB_OK;
 }
@@ -432,8 +442,8 @@ extern "C" int fb_scale_f32(const float* x_lw, const float* x_uw, const float* x
   const bool vw = nw % 4 == 0 && aligned16(x_lw) && aligned16(x_uw) && aligned16(z_lw) && aligned16(z_uw);
   const Lines xw = {s_lw, s_uw}, xb = {s_lb, s_ub};
   const OutLines zw = {z_lw, z_uw}, zb = {z_lb, z_ub};
-  if (vw) scale_kernel<4><<<stream_blocks(nw / 4 + nb), kThreads, 0, st>>>(xw, zw, xb, zb, c, nw / 4, nb);
-  else scale_kernel<1><<<stream_blocks(nw + nb), kThreads, 0, st>>>(xw, zw, xb, zb, c, nw, nb);
+  if (vw) fb::launch_k(scale_kernel<4>, stream_blocks(nw / 4 + nb), kThreads, 0, st, xw, zw, xb, zb, c, nw / 4, nb);
+  else fb::launch_k(scale_kernel<1>, stream_blocks(nw + nb), kThreads, 0, st, xw, zw, xb, zb, c, nw, nb);
   FB_LAUNCH_OK();
   return FB_OK;
 }
@@ -446,8 +456,7 @@ extern "C" int fb_rowsum_f32(const float* x_lw, const float* x_uw, const float* 
   if (rows == 0 || Do == 0) return FB_OK;
   const int64_t n_w = rows * Di, n_b = rows;
   ProfileScope prof(PK_ELEMENTWISE, 2.0 * (n_w + n_b) * Do, 4.0 * 4 * (n_w + n_b) * Do, stream);
-  rowsum_kernel<<<stream_blocks((n_w + n_b) * 32), kThreads, 0, (cudaStream_t)stream>>>(
-      x_lw, x_uw, x_lb, x_ub, z_lw, z_uw, z_lb, z_ub, n_w, n_b, Do);
+  fb::launch_k(rowsum_kernel, stream_blocks((n_w + n_b) * 32), kThreads, 0, (cudaStream_t)stream, x_lw, x_uw, x_lb, x_ub, z_lw, z_uw, z_lb, z_ub, n_w, n_b, Do);
   FB_LAUNCH_OK();
   return FB_OK;
 }
@@ -474,13 +483,13 @@ int fb::layernorm_novar_rowsum(const float* x_lw, const float* x_uw, const float
   const unsigned blocks = stream_blocks((n_w + n_b) * 32);
   cudaStream_t st = (cudaStream_t)stream;
   if (row128 && r_lw)
-    layernorm_novar_row128_kernel<true><<<blocks, kThreads, 0, st>>>(x_lw, x_uw, x_lb, x_ub, r_lw, r_uw, r_lb, r_ub, gamma,
+    fb::launch_k(layernorm_novar_row128_kernel<true>, blocks, kThreads, 0, st, x_lw, x_uw, x_lb, x_ub, r_lw, r_uw, r_lb, r_ub, gamma,
                                                                       beta, z_lw, z_uw, z_lb, z_ub, n_w, n_b, rowsum);
   else if (row128)
-    layernorm_novar_row128_kernel<false><<<blocks, kThreads, 0, st>>>(x_lw, x_uw, x_lb, x_ub, r_lw, r_uw, r_lb, r_ub, gamma,
+    fb::launch_k(layernorm_novar_row128_kernel<false>, blocks, kThreads, 0, st, x_lw, x_uw, x_lb, x_ub, r_lw, r_uw, r_lb, r_ub, gamma,
                                                                        beta, z_lw, z_uw, z_lb, z_ub, n_w, n_b, rowsum);
   else
-    layernorm_novar_kernel<<<blocks, kThreads, 0, st>>>(x_lw, x_uw, x_lb, x_ub, r_lw, r_uw, r_lb, r_ub, gamma, beta, z_lw,
+    fb::launch_k(layernorm_novar_kernel, blocks, kThreads, 0, st, x_lw, x_uw, x_lb, x_ub, r_lw, r_uw, r_lb, r_ub, gamma, beta, z_lw,
                                                         z_uw, z_lb, z_ub, n_w, n_b, Do);
   FB_LAUNCH_OK();
   return FB_OK;
@@ -504,7 +513,7 @@ int permute_heads(Lines xw, Lines xb, OutLines zw, OutLines zb, int B, int L, in
   const int64_t nw = (int64_t)B * L * Di * H * d / (vec ? 4 : 1), nb = (int64_t)B * L * H * d;
   const dim3 grid(stream_blocks(nw + nb), (unsigned)lines);
   const bool small = nw + nb + (int64_t)grid.x * kThreads < (1ll << 32);
-#define FB_PERMUTE(V, I) heads_permute_kernel<V, SPLIT, I><<<grid, kThreads, 0, st>>>(xw, zw, xb, zb, (I)nw, (I)nb, L, Di, H, d)
+#define FB_PERMUTE(V, I) fb::launch_k(heads_permute_kernel<V, SPLIT, I>, grid, kThreads, 0, st, xw, zw, xb, zb, (I)nw, (I)nb, L, Di, H, d)
   if (vec && small) FB_PERMUTE(4, uint32_t);
   else if (vec) FB_PERMUTE(4, uint64_t);
   else if (small) FB_PERMUTE(1, uint32_t);
@@ -516,8 +525,8 @@ int permute_heads(Lines xw, Lines xb, OutLines zw, OutLines zb, int B, int L, in
 int split_transpose(const float* x_w, const float* x_b, float* z_w, float* z_b, int B, int L, int Di, int H, int d, cudaStream_t st) {
   const int64_t bw = (int64_t)B * H * Di, bb = (int64_t)B * H;
   FB_REQUIRE(bw <= 0x7fffffff, FB_ERR_SHAPE);
-  heads_split_transpose_kernel<<<(unsigned)bw, kThreads, 0, st>>>(x_w, z_w, B, L, Di, H, d);
-  heads_split_transpose_kernel<<<(unsigned)bb, kThreads, 0, st>>>(x_b, z_b, B, L, 1, H, d);
+  fb::launch_k(heads_split_transpose_kernel, (unsigned)bw, kThreads, 0, st, x_w, z_w, B, L, Di, H, d);
+  fb::launch_k(heads_split_transpose_kernel, (unsigned)bb, kThreads, 0, st, x_b, z_b, B, L, 1, H, d);
   FB_LAUNCH_OK_N(2);
   return FB_OK;
 }
@@ -579,8 +588,8 @@ extern "C" int fb_mul_features_f32(const float* x_lw, const float* x_uw, const f
   const Lines xw = {x_lw, x_uw}, xb = {x_lb, x_ub};
   const OutLines zw = {z_lw, z_uw}, zb = {z_lb, z_ub};
   const bool vw = Do % 4 == 0 && aligned16(x_lw) && aligned16(x_uw) && aligned16(z_lw) && aligned16(z_uw);
-  if (vw) mul_features_kernel<4><<<stream_blocks(nw / 4 + nb), kThreads, 0, st>>>(xw, zw, xb, zb, w, nw / 4, nb, Do);
-  else mul_features_kernel<1><<<stream_blocks(nw + nb), kThreads, 0, st>>>(xw, zw, xb, zb, w, nw, nb, Do);
+  if (vw) fb::launch_k(mul_features_kernel<4>, stream_blocks(nw / 4 + nb), kThreads, 0, st, xw, zw, xb, zb, w, nw / 4, nb, Do);
+  else fb::launch_k(mul_features_kernel<1>, stream_blocks(nw + nb), kThreads, 0, st, xw, zw, xb, zb, w, nw, nb, Do);
   FB_LAUNCH_OK();
   return FB_OK;
 }
@@ -590,7 +599,7 @@ extern "C" int fb_interval_mul_f32(const float* x_l, const float* x_u, const flo
   FB_REQUIRE(x_l && x_u && y_l && y_u && z_l && z_u && n >= 0, FB_ERR_ARG);
   if (n == 0) return FB_OK;
   ProfileScope prof(PK_MUL, 4.0 * n, 4.0 * 6 * n, stream);
-  interval_mul_kernel<<<stream_blocks(n), kThreads, 0, (cudaStream_t)stream>>>(x_l, x_u, y_l, y_u, z_l, z_u, n);
+  fb::launch_k(interval_mul_kernel, stream_blocks(n), kThreads, 0, (cudaStream_t)stream, x_l, x_u, y_l, y_u, z_l, z_u, n);
   FB_LAUNCH_OK();
   return FB_OK;
 }
@@ -602,7 +611,7 @@ extern "C" int fb_interval_dot_f32(const float* x_l, const float* x_u, const flo
   const int64_t n_out = (int64_t)B * Lx * Ly;
   if (n_out == 0) return FB_OK;
   ProfileScope prof(PK_DOT, 8.0 * n_out * K, 4.0 * (2.0 * B * (Lx + Ly) * K + 2.0 * n_out), stream);
-  interval_dot_kernel<<<stream_blocks(n_out * 32), kThreads, 0, (cudaStream_t)stream>>>(x_l, x_u, y_l, y_u, z_l, z_u, n_out,
+  fb::launch_k(interval_dot_kernel, stream_blocks(n_out * 32), kThreads, 0, (cudaStream_t)stream, x_l, x_u, y_l, y_u, z_l, z_u, n_out,
                                                                                          Lx, Ly, K);
   FB_LAUNCH_OK();
   return FB_OK;

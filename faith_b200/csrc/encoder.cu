@@ -89,6 +89,7 @@ __global__ void __launch_bounds__(256)
 input_bounds_kernel(const float* __restrict__ emb, float* __restrict__ lw, float* __restrict__ uw,
                     float* __restrict__ lb, float* __restrict__ ub, int64_t n_w, int64_t n_b, int L, int D, int words,
                     Positions pos, const int* __restrict__ inst_pos, const float* __restrict__ inst_eps) {
+  pdl_sync();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int Di = words * D;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_w; i += stride) {
@@ -119,6 +120,7 @@ input_bounds_norm128_kernel(const float* __restrict__ emb, const float* __restri
                             float* __restrict__ lw, float* __restrict__ uw, float* __restrict__ lb, float* __restrict__ ub,
                             int64_t n_w_rows, int64_t n_b_rows, int L, int words, Positions pos,
                             const int* __restrict__ inst_pos, const float* __restrict__ inst_eps, float* __restrict__ rowsum) {
+  pdl_sync();
   constexpr int D = 128;
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * 8;
@@ -187,6 +189,7 @@ input_bounds_norm128_kernel(const float* __restrict__ emb, const float* __restri
 __global__ void __launch_bounds__(256)
 mean_pool_kernel(const float* __restrict__ x_lo, const float* __restrict__ x_up, float* __restrict__ z_lo,
                  float* __restrict__ z_up, int64_t total, int64_t inner, int L) {
+  pdl_sync();
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t sidx = t / inner, r = t - sidx * inner;
     const float* pl = x_lo + sidx * L * inner + r;
@@ -203,6 +206,7 @@ mean_pool_kernel(const float* __restrict__ x_lo, const float* __restrict__ x_up,
 // (VerifierForward.py:289-292)
 __global__ void fold_classifier_kernel(const float* __restrict__ cls_w, const float* __restrict__ cls_b,
                                        float* __restrict__ w, float* __restrict__ b, int D) {
+  pdl_sync();
   for (int j = threadIdx.x; j < D; j += blockDim.x) w[j] = fsub(cls_w[j], cls_w[D + j]);
   if (threadIdx.x == 0) b[0] = fsub(cls_b[0], cls_b[1]);
 }
@@ -303,15 +307,14 @@ static int encoder_forward_impl(const fb_encoder* enc, const float* emb, int S, 
       const int64_t n_w_rows = rows * Di, n_b_rows = rows;
       const int64_t want = ceil_div(n_w_rows + n_b_rows, 8), cap = (int64_t)device_info().sms * 16;
       // (without encoder layers the pooler reads both buffers, so both are written)
-      input_bounds_norm128_kernel<<<(unsigned)(want < cap ? want : cap), 256, 0, st>>>(
-          emb, enc->emb_ln_g, enc->emb_ln_b, slot[A].lw, enc->layers == 0 ? slot[A].uw : slot[A].lw, slot[A].lb, slot[A].ub,
+      fb::launch_k(input_bounds_norm128_kernel, (unsigned)(want < cap ? want : cap), 256, 0, st, emb, enc->emb_ln_g, enc->emb_ln_b, slot[A].lw, enc->layers == 0 ? slot[A].uw : slot[A].lw, slot[A].lb, slot[A].ub,
           n_w_rows, n_b_rows, L, words, pos, inst_pos, inst_eps, fuse_ln ? rs_in : nullptr);
       FB_LAUNCH_OK();
     } else {
       fuse_ln = false;   // (the row sums of the layer input come from the fused input kernel)
       const int64_t n_w = rows * Di * D, n_b = rows * D;
       const int64_t want = ceil_div(n_w, 256), cap = (int64_t)device_info().sms * 16;
-      input_bounds_kernel<<<(unsigned)(want < cap ? want : cap), 256, 0, st>>>(emb, slot[B].lw, slot[B].uw, slot[B].lb,
+      fb::launch_k(input_bounds_kernel, (unsigned)(want < cap ? want : cap), 256, 0, st, emb, slot[B].lw, slot[B].uw, slot[B].lb,
                                                                                slot[B].ub, n_w, n_b, L, D, words, pos, inst_pos, inst_eps);
       FB_LAUNCH_OK();
       FB_TRY(norm_residual(enc, slot[B], nullptr, enc->emb_ln_g, enc->emb_ln_b, slot[A], rows, Di, D, stream));
@@ -609,7 +612,7 @@ static int encoder_forward_impl(const fb_encoder* enc, const float* emb, int S, 
     const BoundSet &T1 = slot[C], &T2 = slot[Dd];
     FB_TRY(dense(first_token, enc->pool_w, enc->pool_b, T2, S, Di, D, D, stream));
     FB_TRY(relax(FB_TANH, T2, T1, S, Di, D, words, p, eps, nullptr, stream));
-    fold_classifier_kernel<<<1, 128, 0, st>>>(enc->cls_w, enc->cls_b, fold_w, fold_b, D);
+    fb::launch_k(fold_classifier_kernel, 1, 128, 0, st, enc->cls_w, enc->cls_b, fold_w, fold_b, D);
     FB_LAUNCH_OK();
     FB_TRY(dense(T1, fold_w, fold_b, T2, S, Di, D, 1, stream));
     FB_TRY(fb_concretize_f32(T2.lw, T2.uw, T2.lb, T2.ub, out_l, out_u, S, Di, 1, words, p, eps, FB_NATIVE, stream));
@@ -618,9 +621,9 @@ static int encoder_forward_impl(const fb_encoder* enc, const float* emb, int S, 
     if (enc->pooling == 1) {
       // mean over the positions: [S, 1, Di, D]
       const int64_t nw = (int64_t)S * Di * D, nb = (int64_t)S * D, cap = (int64_t)device_info().sms * 32;
-      mean_pool_kernel<<<(unsigned)std::min(ceil_div(nw, 256), cap), 256, 0, st>>>(X.lw, X.uw, T1.lw, T1.uw, nw, (int64_t)Di * D, L);
+      fb::launch_k(mean_pool_kernel, (unsigned)std::min(ceil_div(nw, 256), cap), 256, 0, st, X.lw, X.uw, T1.lw, T1.uw, nw, (int64_t)Di * D, L);
       FB_LAUNCH_OK();
-      mean_pool_kernel<<<(unsigned)std::min(ceil_div(nb, 256), cap), 256, 0, st>>>(X.lb, X.ub, T1.lb, T1.ub, nb, (int64_t)D, L);
+      fb::launch_k(mean_pool_kernel, (unsigned)std::min(ceil_div(nb, 256), cap), 256, 0, st, X.lb, X.ub, T1.lb, T1.ub, nb, (int64_t)D, L);
       FB_LAUNCH_OK();
     } else {
     // first token of every sentence: [S, 1, Di, D]
@@ -635,7 +638,7 @@ static int encoder_forward_impl(const fb_encoder* enc, const float* emb, int S, 
     }
     FB_TRY(dense(T1, enc->pool_w, enc->pool_b, T2, S, Di, D, D, stream));
     FB_TRY(relax(FB_TANH, T2, T1, S, Di, D, words, p, eps, nullptr, stream));
-    fold_classifier_kernel<<<1, 128, 0, st>>>(enc->cls_w, enc->cls_b, fold_w, fold_b, D);
+    fb::launch_k(fold_classifier_kernel, 1, 128, 0, st, enc->cls_w, enc->cls_b, fold_w, fold_b, D);
     FB_LAUNCH_OK();
     FB_TRY(dense(T1, fold_w, fold_b, T2, S, Di, D, 1, stream));
     FB_TRY(fb_concretize_f32(T2.lw, T2.uw, T2.lb, T2.ub, out_l, out_u, S, Di, 1, words, p, eps, FB_NATIVE, stream));

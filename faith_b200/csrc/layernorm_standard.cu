@@ -61,6 +61,7 @@ layernorm_standard_kernel(const float* __restrict__ x_lw, const float* __restric
                           const float* __restrict__ x_ub, const float* __restrict__ gamma, const float* __restrict__ beta,
                           float* __restrict__ z_lw, float* __restrict__ z_uw, float* __restrict__ z_lb, float* __restrict__ z_ub,
                           int Di, int Do, int words, int p, float eps, int* __restrict__ violation) {
+  pdl_sync();
   extern __shared__ __align__(16) float smem[];
   const int rows = Di + 1;                         // the weight rows and, last, the bias row
   float* s_mu = smem;                              // [2][rows] row means of lw and uw
@@ -268,11 +269,9 @@ extern "C" int fb_layernorm_standard_f32(const float* x_lw, const float* x_uw, c
                         : ensure_dynamic_smem(layernorm_standard_kernel<false>, smem);
   if (rc != FB_OK) return rc;
   if (staged)
-    layernorm_standard_kernel<true><<<(unsigned)rows, kT, smem, (cudaStream_t)stream>>>(
-        x_lw, x_uw, x_lb, x_ub, gamma, beta, z_lw, z_uw, z_lb, z_ub, Di, Do, words, p, eps, violation);
+    fb::launch_k(layernorm_standard_kernel<true>, (unsigned)rows, kT, smem, (cudaStream_t)stream, x_lw, x_uw, x_lb, x_ub, gamma, beta, z_lw, z_uw, z_lb, z_ub, Di, Do, words, p, eps, violation);
   else
-    layernorm_standard_kernel<false><<<(unsigned)rows, kT, smem, (cudaStream_t)stream>>>(
-        x_lw, x_uw, x_lb, x_ub, gamma, beta, z_lw, z_uw, z_lb, z_ub, Di, Do, words, p, eps, violation);
+    fb::launch_k(layernorm_standard_kernel<false>, (unsigned)rows, kT, smem, (cudaStream_t)stream, x_lw, x_uw, x_lb, x_ub, gamma, beta, z_lw, z_uw, z_lb, z_ub, Di, Do, words, p, eps, violation);
   FB_LAUNCH_OK();
   return FB_OK;
 }

@@ -51,6 +51,7 @@ ranges_from_norms_kernel(float* __restrict__ lb, float* __restrict__ ub, const f
                          const float* __restrict__ plain_ub, const float* __restrict__ norm_lo,
                          const float* __restrict__ norm_up, float* __restrict__ out_l, float* __restrict__ out_u,
                          int64_t total, int L, int heads, int d, int words, float eps) {
+  pdl_sync();
   const int Dy = heads * d;
   const int dv = d / VEC;
   for (int64_t tv = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; tv < total / VEC; tv += (int64_t)gridDim.x * blockDim.x) {
@@ -228,10 +229,10 @@ extern "C" int fb_matmul_heads_ranges_f32(const float* x_lw, const float* x_uw, 
   const int64_t want = fb::ceil_div(vec ? total / 4 : total, 256), cap = (int64_t)fb::device_info().sms * 8;
   const unsigned blocks = (unsigned)(want < cap ? want : cap);
   if (vec)
-    fb::ranges_from_norms_kernel<4><<<blocks, 256, 0, st>>>(y_lb, y_ub, plain_lb, plain_ub, norm_lo, norm_up, y_l, y_u, total, L,
+    fb::launch_k(fb::ranges_from_norms_kernel<4>, blocks, 256, 0, st, y_lb, y_ub, plain_lb, plain_ub, norm_lo, norm_up, y_l, y_u, total, L,
                                                             heads, d, words, eps);
   else
-    fb::ranges_from_norms_kernel<1><<<blocks, 256, 0, st>>>(y_lb, y_ub, plain_lb, plain_ub, norm_lo, norm_up, y_l, y_u, total, L,
+    fb::launch_k(fb::ranges_from_norms_kernel<1>, blocks, 256, 0, st, y_lb, y_ub, plain_lb, plain_ub, norm_lo, norm_up, y_l, y_u, total, L,
                                                             heads, d, words, eps);
   FB_LAUNCH_OK();
   return FB_OK;

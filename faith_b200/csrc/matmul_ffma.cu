@@ -30,6 +30,7 @@ split_sign_gemm_ffma(const float* __restrict__ a_lo, const float* __restrict__ a
                      const float* __restrict__ W, const float* __restrict__ bias,
                      float* __restrict__ c_lo, float* __restrict__ c_up, int64_t M, int N, int K, int split_rows,
                      int split_d) {
+  pdl_sync();
   extern __shared__ __align__(16) float smem[];
   const int tid = threadIdx.x;
   const int tx = tid & 15, ty = tid >> 4;
@@ -176,6 +177,7 @@ __global__ void __launch_bounds__(kThreads)
 split_sign_gemv_rows(const float* __restrict__ a_lo, const float* __restrict__ a_up,
                      const float* __restrict__ W, const float* __restrict__ bias,
                      float* __restrict__ c_lo, float* __restrict__ c_up, int64_t M, int N, int K) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (kThreads / 32);
   for (int64_t m = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5); m < M; m += warps) {
@@ -232,6 +234,7 @@ __global__ void __launch_bounds__(kThreads)
 split_sign_gemv_tiled(const float* __restrict__ a_lo, const float* __restrict__ a_up,
                       const float* __restrict__ W, const float* __restrict__ bias,
                       float* __restrict__ c_lo, float* __restrict__ c_up, int64_t M, int N, int K) {
+  pdl_sync();
   extern __shared__ __align__(16) float gemv_sw[];   // [2][NMAX][kGemvChunk]
   constexpr int J = kGemvChunk / 128;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -326,6 +329,7 @@ template <int NMAX>
 __global__ void __launch_bounds__(kThreads)
 split_sign_gemv_block(const float* __restrict__ a_lo, const float* __restrict__ a_up, const float* __restrict__ W,
                       const float* __restrict__ bias, float* __restrict__ c_lo, float* __restrict__ c_up, int N, int K) {
+  pdl_sync();
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ float s_red[2][kThreads / 32][NMAX];
@@ -398,6 +402,7 @@ __global__ void __launch_bounds__(kThreads)
 split_sign_gemm_small(const float* __restrict__ a_lo, const float* __restrict__ a_up, const float* __restrict__ W,
                       const float* __restrict__ bias, float* __restrict__ c_lo, float* __restrict__ c_up, int64_t M, int N, int K,
                       int split_rows, int split_d) {
+  pdl_sync();
   extern __shared__ __align__(16) float smem[];
   float* const s_c = smem;                                  // [kSmRows][kSmChunk] centres
   float* const s_r = s_c + kSmRows * kSmChunk;              // radii
@@ -513,7 +518,7 @@ int launch_split_sign_ffma(const float* a_lo, const float* a_up, const float* W,
       ceil_div(M, kThreads / 32) <= 0x7fffffff) {
     const size_t gemv_smem = sizeof(float) * 2 * 16 * kGemvChunk;
     if (int rc = ensure_dynamic_smem(split_sign_gemv_tiled<16>, gemv_smem)) return rc;
-    split_sign_gemv_tiled<16><<<(unsigned)ceil_div(M, kThreads / 32), kThreads, gemv_smem, st>>>(a_lo, a_up, W, bias, c_lo, c_up, M, N, K);
+    fb::launch_k(split_sign_gemv_tiled<16>, (unsigned)ceil_div(M, kThreads / 32), kThreads, gemv_smem, st, a_lo, a_up, W, bias, c_lo, c_up, M, N, K);
     FB_LAUNCH_OK();
     return FB_OK;
   }
@@ -521,7 +526,7 @@ int launch_split_sign_ffma(const float* a_lo, const float* a_up, const float* W,
     const int64_t want = ceil_div(M, kThreads / 32);
     const int64_t cap = (int64_t)device_info().sms * 16;
     const unsigned blocks = (unsigned)(want < cap ? want : cap);
-    split_sign_gemv_rows<16><<<blocks, kThreads, 0, st>>>(a_lo, a_up, W, bias, c_lo, c_up, M, N, K);
+    fb::launch_k(split_sign_gemv_rows<16>, blocks, kThreads, 0, st, a_lo, a_up, W, bias, c_lo, c_up, M, N, K);
     FB_LAUNCH_OK();
     return FB_OK;
   }
@@ -531,18 +536,18 @@ int launch_split_sign_ffma(const float* a_lo, const float* a_up, const float* W,
   const bool vec = K % 4 == 0 && aligned16(a_lo) && aligned16(a_up) && aligned16(W);
   if (gm * gn < device_info().sms) {   // the 128 x 128 tiles would not fill the machine once
     const dim3 grid((unsigned)ceil_div(M, kSmRows), (unsigned)ceil_div(N, kSmCols));
-    if (vec) split_sign_gemm_small<true><<<grid, kThreads, kSmSmem, st>>>(a_lo, a_up, W, bias, c_lo, c_up, M, N, K, split_rows, split_d);
-    else split_sign_gemm_small<false><<<grid, kThreads, kSmSmem, st>>>(a_lo, a_up, W, bias, c_lo, c_up, M, N, K, split_rows, split_d);
+    if (vec) fb::launch_k(split_sign_gemm_small<true>, grid, kThreads, kSmSmem, st, a_lo, a_up, W, bias, c_lo, c_up, M, N, K, split_rows, split_d);
+    else fb::launch_k(split_sign_gemm_small<false>, grid, kThreads, kSmSmem, st, a_lo, a_up, W, bias, c_lo, c_up, M, N, K, split_rows, split_d);
     FB_LAUNCH_OK();
     return FB_OK;
   }
   const size_t smem = sizeof(float) * 2 * kStageFloats;
   if (vec) {
     if (int rc = ensure_dynamic_smem(split_sign_gemm_ffma<true>, smem)) return rc;
-    split_sign_gemm_ffma<true><<<dim3((unsigned)gm, gn), kThreads, smem, st>>>(a_lo, a_up, W, bias, c_lo, c_up, M, N, K, split_rows, split_d);
+    fb::launch_k(split_sign_gemm_ffma<true>, dim3((unsigned)gm, gn), kThreads, smem, st, a_lo, a_up, W, bias, c_lo, c_up, M, N, K, split_rows, split_d);
   } else {
     if (int rc = ensure_dynamic_smem(split_sign_gemm_ffma<false>, smem)) return rc;
-    split_sign_gemm_ffma<false><<<dim3((unsigned)gm, gn), kThreads, smem, st>>>(a_lo, a_up, W, bias, c_lo, c_up, M, N, K, split_rows, split_d);
+    fb::launch_k(split_sign_gemm_ffma<false>, dim3((unsigned)gm, gn), kThreads, smem, st, a_lo, a_up, W, bias, c_lo, c_up, M, N, K, split_rows, split_d);
   }
   FB_LAUNCH_OK();
   return FB_OK;

@@ -223,6 +223,30 @@ split_sign_gemm_tc(const __grid_constant__ CUtensorMap tm_lo, const __grid_const
   const int my_tiles = (int)((total_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);
   const int total_it = my_tiles * nkb;   // k-blocks this CTA walks, across all its tiles
 
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kRawStages; ++s) {
+      mbar_init(bar_full + 8 * s, 1);
+      mbar_init(bar_raw_empty + 8 * s, kGroupWarps);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(bar_ops_ready + 8 * s, kGroupWarps);
+      mbar_init(bar_mma_done + 8 * s, kIssuers);
+    }
+    mbar_init(bar_acc_ready, kIssuers);
+    mbar_init(bar_acc_free, kEpiWarps);
+    mbar_init(bar_conv, kEpiWarps);
+    mbar_init(bar_res, 1);
+    mbar_init(bar_mu, kConvWarps);
+    mbar_init(bar_mu + 8, kConvWarps);
+    *cta_abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {  // one warp allocates all of tensor memory for this CTA
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
+    tmem_relinquish();
+  }
+  pdl_sync();   // (everything above needs nothing of the launches before)
+
   // Liveness of this CTA's tiles, worked out once by all threads into a bitmap (every role of every tile asks; the
   // divisions and the position loads of the direct form, 28 warps x 100+ tiles, cost more than the zero tiles themselves).
   uint32_t* live_bits = reinterpret_cast<uint32_t*>(base_ptr + SharedLayout::bars() + 256);
@@ -244,24 +268,6 @@ split_sign_gemm_tc(const __grid_constant__ CUtensorMap tm_lo, const __grid_const
     return tile_live_slow((int)blockIdx.x + ti * (int)gridDim.x);
   };
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < kRawStages; ++s) {
-      mbar_init(bar_full + 8 * s, 1);
-      mbar_init(bar_raw_empty + 8 * s, kGroupWarps);
-    }
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(bar_ops_ready + 8 * s, kGroupWarps);
-      mbar_init(bar_mma_done + 8 * s, kIssuers);
-    }
-    mbar_init(bar_acc_ready, kIssuers);
-    mbar_init(bar_acc_free, kEpiWarps);
-    mbar_init(bar_conv, kEpiWarps);
-    mbar_init(bar_res, 1);
-    mbar_init(bar_mu, kConvWarps);
-    mbar_init(bar_mu + 8, kConvWarps);
-    *cta_abort = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
   float* const ln_smem = reinterpret_cast<float*>(base_ptr + SharedLayout::bars() + 256 + kLiveWords * 4);
   if (kLN) {
     // column means of W and |W|, the gain split by sign as the layer-norm kernel splits it.  The rows of W are dealt
@@ -309,10 +315,6 @@ split_sign_gemm_tc(const __grid_constant__ CUtensorMap tm_lo, const __grid_const
       for (int n = 0; n < N && bias_b != nullptr; ++n) sb = fmaf(__ldg(bias_b + n), inv_n, sb);
       ln_smem[kLnOffBiasMean / 4] = sb;
     }
-  }
-  if (warp == 1) {  // one warp allocates all of tensor memory for this CTA
-    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
-    tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
@@ -1006,21 +1008,21 @@ int launch_split_sign_tc(const float* a_lo, const float* a_up, const float* W, c
 #define FB_TC_ARGS tm_lo, tm_up, tm_w, tm_out_lo, tm_out_up, tm_res_lo, tm_res_up, tm_b_lo, tm_b_up, tm_bout_lo, tm_bout_up, tm_bres_lo, \
                    tm_bres_up, bias, bias_b, (int)main_tiles, same_b, M, N, K, gn, total_tiles, split_rows, split_d
   if (ln != nullptr && coef_l != nullptr)
-    split_sign_gemm_tc<true, false, true, false, true><<<grid, kThreads, kSmemBytes + kLnSmemBytes, st>>>(FB_TC_ARGS, coef_l, coef_u, coef_di, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_k(split_sign_gemm_tc<true, false, true, false, true>, grid, kThreads, kSmemBytes + kLnSmemBytes, st, FB_TC_ARGS, coef_l, coef_u, coef_di, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
   else if (ln != nullptr)
-    split_sign_gemm_tc<false, false, true, false, true><<<grid, kThreads, kSmemBytes + kLnSmemBytes, st>>>(FB_TC_ARGS, nullptr, nullptr, 1, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_k(split_sign_gemm_tc<false, false, true, false, true>, grid, kThreads, kSmemBytes + kLnSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
   else if (coef_l != nullptr && res_lo != nullptr)
-    split_sign_gemm_tc<true, false, true, false, false><<<grid, kThreads, kSmemBytes, st>>>(FB_TC_ARGS, coef_l, coef_u, coef_di, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_k(split_sign_gemm_tc<true, false, true, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, coef_l, coef_u, coef_di, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
   else if (coef_l != nullptr)
-    split_sign_gemm_tc<true, false, false, false, false><<<grid, kThreads, kSmemBytes, st>>>(FB_TC_ARGS, coef_l, coef_u, coef_di, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_k(split_sign_gemm_tc<true, false, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, coef_l, coef_u, coef_di, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
   else if (norm_lo != nullptr && a_lo == a_up)   // one tensor as both lines: zero radius
-    split_sign_gemm_tc<false, true, false, true, false><<<grid, kThreads, kSmemBytes, st>>>(FB_TC_ARGS, nullptr, nullptr, 1, norm_lo, norm_up, norm_p, status, tries, skip, live, c_lo == c_up ? 1 : 0, FB_TC_TAIL);
+    fb::launch_k(split_sign_gemm_tc<false, true, false, true, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, norm_lo, norm_up, norm_p, status, tries, skip, live, c_lo == c_up ? 1 : 0, FB_TC_TAIL);
   else if (norm_lo != nullptr)
-    split_sign_gemm_tc<false, true, false, false, false><<<grid, kThreads, kSmemBytes, st>>>(FB_TC_ARGS, nullptr, nullptr, 1, norm_lo, norm_up, norm_p, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_k(split_sign_gemm_tc<false, true, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, norm_lo, norm_up, norm_p, status, tries, skip, no_live, 0, FB_TC_TAIL);
   else if (res_lo != nullptr)
-    split_sign_gemm_tc<false, false, true, false, false><<<grid, kThreads, kSmemBytes, st>>>(FB_TC_ARGS, nullptr, nullptr, 1, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_k(split_sign_gemm_tc<false, false, true, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
   else
-    split_sign_gemm_tc<false, false, false, false, false><<<grid, kThreads, kSmemBytes, st>>>(FB_TC_ARGS, nullptr, nullptr, 1, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_k(split_sign_gemm_tc<false, false, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
 #undef FB_TC_ARGS
 #undef FB_TC_TAIL
   FB_LAUNCH_OK();
@@ -1074,6 +1076,7 @@ __device__ __forceinline__ void mma_tf32_ss(uint32_t d_tmem, uint64_t adesc, uin
 }
 
 __global__ void __launch_bounds__(128, 1) tf32_peak_kernel(int iters, int* __restrict__ status) {
+  pdl_sync();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -1129,7 +1132,7 @@ extern "C" int fb_bench_tf32(int iters, double* flops, void* stream) {
   });
   FB_CUDA_OK(attr_err);
   const int blocks = fb::device_info().sms;
-  fb::tf32_peak_kernel<<<blocks, 128, fb::kPeakSmem, (cudaStream_t)stream>>>(iters, fb::t_status_sink);
+  fb::launch_k(fb::tf32_peak_kernel, blocks, 128, fb::kPeakSmem, (cudaStream_t)stream, iters, fb::t_status_sink);
   FB_LAUNCH_OK();
   *flops = 2.0 * 128.0 * 256.0 * 8.0 * 8.0 * (double)iters * blocks;
   return FB_OK;

@@ -40,6 +40,7 @@ softmax_bounds_kernel(const float* __restrict__ lw, const float* __restrict__ uw
                       float* __restrict__ o_lb, float* __restrict__ o_ub, float* __restrict__ o_l,
                       float* __restrict__ o_u, int Di, int Do, int ld, int words, float eps,
                       int* __restrict__ violation) {
+  pdl_sync();
   constexpr int p = kP;
   constexpr int CVL = kCW / 4, RG = kThreads / CVL;   // column lanes (float4) x row groups
   extern __shared__ __align__(16) float smem[];
@@ -313,6 +314,7 @@ softmax_bounds_regs(const float* __restrict__ lw, const float* __restrict__ uw, 
                     const float* __restrict__ ub, float* __restrict__ o_lw, float* __restrict__ o_uw,
                     float* __restrict__ o_lb, float* __restrict__ o_ub, float* __restrict__ o_l, float* __restrict__ o_u,
                     int Do, int ld, int words, float eps, int vec, int* __restrict__ violation) {
+  pdl_sync();
   constexpr int p = kP, CVL = kCW / 4, RG = T / CVL, W = T / 32, Di = RG * KR;
   __shared__ float4 s_part[2][W][CVL];     // column partials of the warps, lower and upper line
   __shared__ float s_col[5][kCW];          // slopes, bias terms and lower range of exp
@@ -556,7 +558,7 @@ int fb::softmax_ex(const float* lw, const float* uw, const float* lb, const floa
     return FB_OK;                                                                                                      \
   }
 #define FB_SOFTMAX_REGS_LAUNCH(P, C, T, K)                                                                             \
-  softmax_bounds_regs<P, C, T, K><<<(unsigned)rows, T, 0, (cudaStream_t)stream>>>(                                     \
+  fb::launch_k(softmax_bounds_regs<P, C, T, K>, (unsigned)rows, T, 0, (cudaStream_t)stream, \
       lw, uw, lb, ub, out_lw, out_uw, out_lb, out_ub, out_l, out_u, Do, ld, words, eps, vec ? 1 : 0, violation)
   FB_SOFTMAX_REGS(32, 256, 4)    // Di 128
   FB_SOFTMAX_REGS(32, 256, 2)    // Di 64
@@ -568,7 +570,7 @@ int fb::softmax_ex(const float* lw, const float* uw, const float* lb, const floa
 #define FB_SOFTMAX_LAUNCH(P, C, V)                                                                                    \
   do {                                                                                                                \
     if (int rc_ = ensure_dynamic_smem(softmax_bounds_kernel<P, C, V>, smem)) return rc_;                               \
-    softmax_bounds_kernel<P, C, V><<<(unsigned)rows, kThreads, smem, (cudaStream_t)stream>>>(                          \
+    fb::launch_k(softmax_bounds_kernel<P, C, V>, (unsigned)rows, kThreads, smem, (cudaStream_t)stream, \
         lw, uw, lb, ub, out_lw, out_uw, out_lb, out_ub, out_l, out_u, Di, Do, ld, words, eps, violation);              \
   } while (0)
 #define FB_SOFTMAX_NORM(C, V)                                  \
