@@ -39,7 +39,9 @@ void count_launches(int n);
 
 // A launch whose blocks may become resident while the launch before on the stream still drains (programmatic dependent launch):
 // the passes over one sentence are chains of kernels of 3 to 10 us with 2 us between them, most of it launch latency and
-// prologues (barriers, tensor memory, tensor maps).  The kernel must call pdl_sync() first thing.
+// prologues (barriers, tensor memory, tensor maps).  The kernel must call pdl_sync() first thing.  Grids of many waves keep the
+// plain launch: the gap before them is nothing beside them, and the hand-over cost the 4096 blocks of a relaxation 2 % of
+// 135 us.
 template <typename... P, typename... A>
 inline void launch_k(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
   cudaLaunchAttribute attr;
@@ -51,7 +53,7 @@ inline void launch_k(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cud
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = (int64_t)grid.x * grid.y * grid.z <= 4 * (int64_t)device_info().sms ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);   // (errors are picked up by FB_LAUNCH_OK)
 }
 
