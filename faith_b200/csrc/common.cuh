@@ -127,6 +127,34 @@ int cw_linear_ex(const float* z_lw, const float* z_uw, const float* coef, const 
 int cw_linear_range(const float* part, const float* lb, const float* ub, float* l, float* u, int H0, int W0, int N, int p, float eps,
                     cudaStream_t st);
 
+// What the product of a few bias rows does with its result besides storing it (matmul_ffma.cu): the concretised range, from the
+// column norms [row * words + w][N] of the weight rows, to out_l / out_u in the layout of the result or (transposed) as
+// [group * head][feature][row in group]; with op >= 0 the slopes k_l, k_u and the relaxed bias terms r_lb, r_ub of that
+// relaxation, [M, N], as fb_relax_coef_given_f32 returns them.
+struct RangeEpilogue {
+  const float *norm_lo, *norm_up;
+  float *out_l, *out_u;
+  int words;
+  float eps;
+  int transposed, op;
+  float *k_l, *k_u, *r_lb, *r_ub;
+  int* violation;
+};
+bool small_product(int64_t M, int N);   // whether the kernel for few rows takes a product of that size
+int launch_split_sign_small(const float* a_lo, const float* a_up, const float* W, const float* bias, float* c_lo, float* c_up, int64_t M,
+                            int N, int K, cudaStream_t st, int split_rows, int split_d, const RangeEpilogue* range);
+// matmul.cu: fb_matmul_heads_ranges_f32 with the wishes of the driver: ranges transposed, relaxation coefficients of the result.
+// Both are extras of the kernel for few bias rows; `granted` tells whether they were done.
+struct RangeWishes {
+  int transposed, op;
+  float *k_l, *k_u, *r_lb, *r_ub;
+  int* violation;
+  bool granted;
+};
+int matmul_ranges_ex(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub, const float* W, const float* bias,
+                     float* y_lw, float* y_uw, float* y_lb, float* y_ub, float* y_l, float* y_u, float* norm_ws, int64_t rows, int Di,
+                     int Do, int Dy, int L, int heads, int words, int p, float eps, RangeWishes* wishes, void* stream);
+
 // softmax.cu: fb_softmax_ranges_f32 with rows `ld` floats apart.
 int softmax_ex(const float* lw, const float* uw, const float* lb, const float* ub, float* out_lw, float* out_uw, float* out_lb,
                float* out_ub, float* out_l, float* out_u, int64_t rows, int Di, int Do, int ld, int words, int p, float eps,

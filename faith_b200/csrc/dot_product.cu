@@ -603,12 +603,15 @@ extern "C" int fb_context_given_f32(const float* x_lw, const float* x_uw, const 
 }
 
 // The general form: any shape, x rows ldx floats apart (0: contiguous).  transposed_ranges: the value ranges end up as
-// [B, Ly, K] in y_l / y_u (small matrices only), as the entry points above document; otherwise they stay [B, K, Ly].
+// [B, Ly, K] in y_l / y_u (small matrices only), as the entry points above document; otherwise they stay [B, K, Ly].  given:
+// bit 2 = the given ranges of the values are [B, Ly, K] already.
 int fb::context_ex(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub, const float* v_lw, const float* v_uw,
                    const float* v_lb, const float* v_ub, float* z_lw, float* z_uw, float* z_lb, float* z_ub, float* x_l, float* x_u,
                    float* y_l, float* y_u, int B, int Lx, int Ly, int Di, int K, int words, int p, float eps, float out_scale,
                    int merge_heads, int given, int ldx, bool transposed_ranges, void* stream) {
-  if (given < 0 || given > 3) return FB_ERR_ARG;
+  const bool given_transposed = (given & 4) != 0;
+  if (given < 0 || given > 7 || (given_transposed && !(given & 2))) return FB_ERR_ARG;
+  given &= 3;
   if (!x_lw || !x_uw || !x_lb || !x_ub || !v_lw || !v_uw || !v_lb || !v_ub || !z_lw || !z_uw || !z_lb || !z_ub ||
       !x_l || !x_u || !y_l || !y_u)
     return FB_ERR_ARG;
@@ -638,8 +641,8 @@ int fb::context_ex(const float* x_lw, const float* x_uw, const float* x_lb, cons
   else if (given == 1)
     rc = fb_concretize_f32(v_lw, v_uw, v_lb, v_ub, y_l, y_u, (int64_t)B * K, Di, Ly, words, p, eps, FB_NATIVE, stream);
   if (rc != FB_OK) return rc;
-  const bool transpose = transposed_ranges || !tc || tc32;
-  if (transpose) {
+  const bool transpose = transposed_ranges || !tc || tc32 || given_transposed;
+  if (transpose && !given_transposed) {
     fb::launch_k(transpose_small_inplace, (unsigned)B, 256, 0, st, y_l, y_u, K, Ly);
     FB_LAUNCH_OK();
   }

@@ -492,10 +492,12 @@ static int encoder_forward_impl(const fb_encoder* enc, const float* emb, int S, 
       int vgiven = pgiven;
       BoundSet Vh = T3;
       if (li == 0) Vh.uw = Vh.lw;
-      const int vrc = fb_matmul_heads_ranges_f32(Xin.lw, Xin.uw, Xin.lb, Xin.ub, ly.v_w, ly.v_b, Vh.lw, Vh.uw, T3.lb, T3.ub, range[2],
-                                                 range[3], norm_ws, rows, Di, D, D, L, H, words, p, eps, stream);
+      RangeWishes vw = {1, -1, nullptr, nullptr, nullptr, nullptr, nullptr, false};   // the products read the value ranges transposed
+      const int vrc = matmul_ranges_ex(Xin.lw, Xin.uw, Xin.lb, Xin.ub, ly.v_w, ly.v_b, Vh.lw, Vh.uw, T3.lb, T3.ub, range[2], range[3],
+                                       norm_ws, rows, Di, D, D, L, H, words, p, eps, &vw, stream);
       if (vrc == FB_OK) {
         vgiven |= 2;
+        if (vw.granted) vgiven |= 4;
       } else if (vrc == FB_ERR_SHAPE) {
         Vh = T3;
         FB_TRY(fb_matmul_heads_f32(Xin.lw, Xin.uw, Xin.lb, Xin.ub, ly.v_w, ly.v_b, T3.lw, T3.uw, T3.lb, T3.ub, rows, Di, D, D, L, H,
@@ -554,9 +556,11 @@ static int encoder_forward_impl(const fb_encoder* enc, const float* emb, int S, 
     // slot of the layer input and the second product applies them while it reads the hidden bounds.  The
     // first product hands over the concretised range of the hidden bounds (into the unused lb / ub of
     // that slot), so the slopes need no pass over the hidden weights either.
-    int frc = fb_matmul_heads_ranges_f32(T3.lw, T3.uw, T3.lb, T3.ub, ly.f1_w, ly.f1_b, T1.lw, T1.uw, T1.lb, T1.ub, X.lb, X.ub,
-                                         norm_ws, rows, Di, D, F, L, 1, words, p, eps, stream);
-    if (frc == FB_OK) {
+    RangeWishes fw = {0, FB_RELU, X.lw, X.uw, T2.lb, T2.ub, violation, false};
+    int frc = matmul_ranges_ex(T3.lw, T3.uw, T3.lb, T3.ub, ly.f1_w, ly.f1_b, T1.lw, T1.uw, T1.lb, T1.ub, X.lb, X.ub, norm_ws, rows, Di, D, F,
+                               L, 1, words, p, eps, &fw, stream);
+    if (frc == FB_OK && fw.granted) {
+    } else if (frc == FB_OK) {
       frc = fb_relax_coef_given_f32(FB_RELU, T1.lb, T1.ub, X.lb, X.ub, X.lw, X.uw, T2.lb, T2.ub, rows, F, violation, stream);
     } else if (frc == FB_ERR_SHAPE) {
       FB_TRY(dense(T3, ly.f1_w, ly.f1_b, T1, rows, Di, D, F, stream));

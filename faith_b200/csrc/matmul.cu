@@ -184,6 +184,14 @@ extern "C" int fb_matmul_heads_ranges_f32(const float* x_lw, const float* x_uw, 
                                           const float* W, const float* bias, float* y_lw, float* y_uw, float* y_lb,
                                           float* y_ub, float* y_l, float* y_u, float* norm_ws, int64_t rows, int Di,
                                           int Do, int Dy, int L, int heads, int words, int p, float eps, void* stream) {
+  return fb::matmul_ranges_ex(x_lw, x_uw, x_lb, x_ub, W, bias, y_lw, y_uw, y_lb, y_ub, y_l, y_u, norm_ws, rows, Di, Do, Dy, L, heads, words,
+                              p, eps, nullptr, stream);
+}
+
+int fb::matmul_ranges_ex(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub, const float* W, const float* bias,
+                         float* y_lw, float* y_uw, float* y_lb, float* y_ub, float* y_l, float* y_u, float* norm_ws, int64_t rows, int Di,
+                         int Do, int Dy, int L, int heads, int words, int p, float eps, RangeWishes* wishes, void* stream) {
+  if (wishes != nullptr) wishes->granted = false;
   if (!x_lw || !x_uw || !x_lb || !x_ub || !W || !y_lw || !y_uw || !y_lb || !y_ub || !y_l || !y_u || !norm_ws)
     return FB_ERR_ARG;
   if (rows < 0 || Di <= 0 || Do <= 0 || Dy <= 0 || words <= 0 || heads < 1 || !fb::valid_norm(p)) return FB_ERR_ARG;
@@ -219,6 +227,15 @@ extern "C" int fb_matmul_heads_ranges_f32(const float* x_lw, const float* x_uw, 
     plain_lb = b_lo;
     plain_ub = b_up;
     rc = fb::launch_split_sign_tc(x_lb, x_ub, W, bias, plain_lb, plain_ub, rows, Dy, Do, st, 0, 0);
+  } else if (!fb::tc_gemm_supported(x_lb, x_ub, W, y_lb, y_ub, rows, Dy, Do) && fb::small_product(rows, Dy)) {
+    fb::RangeEpilogue rg = {norm_lo, norm_up, y_l, y_u, words, eps, 0, -1, nullptr, nullptr, nullptr, nullptr, nullptr};
+    if (wishes != nullptr) {
+      rg.transposed = wishes->transposed && heads > 1;
+      rg.op = wishes->op;
+      rg.k_l = wishes->k_l, rg.k_u = wishes->k_u, rg.r_lb = wishes->r_lb, rg.r_ub = wishes->r_ub, rg.violation = wishes->violation;
+      wishes->granted = true;
+    }
+    return fb::launch_split_sign_small(x_lb, x_ub, W, bias, y_lb, y_ub, rows, Dy, Do, st, heads > 1 ? L : 0, heads > 1 ? d : 0, &rg);
   } else {
     rc = fb::split_sign_gemm(x_lb, x_ub, W, bias, y_lb, y_ub, rows, Dy, Do, st, heads > 1 ? L : 0, heads > 1 ? d : 0);
   }

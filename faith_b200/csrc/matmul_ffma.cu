@@ -394,14 +394,15 @@ split_sign_gemv_block(const float* __restrict__ a_lo, const float* __restrict__ 
 // block owns 8 rows x 32 columns and its eight warps split K, a contiguous part each: centre and radius of the rows are
 // staged in shared memory and read as broadcasts, a lane owns one column and streams its part of that row of W with
 // 128-bit loads (whole sectors), the eight partial sums of an output are added in warp order.  Bound by the latency of one
-// pass over the operands: 4.0 us resp. 9.0 us at the sizes above.
+// pass over the operands: 4.0 us resp. 9.0 us at the sizes above.  The concretised range of the rows and the coefficients of a
+// relaxation follow in the same launch where the caller wants them (two launches of 2 to 3 us each otherwise).
 constexpr int kSmRows = 8, kSmCols = 32, kSmWarps = kThreads / 32, kSmChunk = 512;
 constexpr uint32_t kSmSmem = sizeof(float) * (2 * kSmRows * kSmChunk + 2 * kSmWarps * kSmRows * kSmCols);
 template <bool VEC>
 __global__ void __launch_bounds__(kThreads)
 split_sign_gemm_small(const float* __restrict__ a_lo, const float* __restrict__ a_up, const float* __restrict__ W,
                       const float* __restrict__ bias, float* __restrict__ c_lo, float* __restrict__ c_up, int64_t M, int N, int K,
-                      int split_rows, int split_d) {
+                      int split_rows, int split_d, const RangeEpilogue rg) {
   pdl_sync();
   extern __shared__ __align__(16) float smem[];
   float* const s_c = smem;                                  // [kSmRows][kSmChunk] centres
@@ -483,16 +484,48 @@ split_sign_gemm_small(const float* __restrict__ a_lo, const float* __restrict__ 
   }
   float lo = fsub(c, r), up = fadd(c, r);
   if (bias != nullptr) { lo = fadd(lo, bias[n]); up = fadd(up, bias[n]); }
-  int64_t o = m * N + n;
+  int64_t o = m * N + n, ot = o;
   if (split_rows > 0) {
-    const int64_t g = m / split_rows, rr = m % split_rows;
-    o = ((g * (N / split_d) + n / split_d) * split_rows + rr) * split_d + n % split_d;
+    const int64_t g = m / split_rows, rr = m % split_rows, gh = g * (N / split_d) + n / split_d;
+    o = (gh * split_rows + rr) * split_d + n % split_d;
+    ot = (gh * split_d + n % split_d) * split_rows + rr;
   }
   c_lo[o] = lo;
   c_up[o] = up;
+  if (rg.norm_lo == nullptr) return;
+  const float lb = lo, ub = up;
+  for (int w = 0; w < rg.words; ++w) {
+    const int64_t at = (m * rg.words + w) * N + n;
+    lo = fadd(lo, fmul(-rg.eps, __ldg(rg.norm_lo + at)));
+    up = fadd(up, fmul(rg.eps, __ldg(rg.norm_up + at)));
+  }
+  rg.out_l[rg.transposed ? ot : o] = lo;
+  rg.out_u[rg.transposed ? ot : o] = up;
+  if (rg.op < 0) return;
+  bool bad = false;
+  const ColCoef k = relax_column(rg.op, lo, up, lb, ub, bad);
+  if (rg.violation != nullptr && (bad || k.c_lu != 0.f || k.c_ul != 0.f)) atomicOr(rg.violation, bad ? 1 : 2);
+  rg.k_l[m * N + n] = k.c_ll;
+  rg.k_u[m * N + n] = k.c_uu;
+  rg.r_lb[m * N + n] = k.nlb;
+  rg.r_ub[m * N + n] = k.nub;
 }
 
 }  // namespace
+
+// (below that many 128 x 128 tiles the kernel above would not fill the machine once)
+bool small_product(int64_t M, int N) { return N > 16 && ceil_div(M, BM) * ceil_div(N, BN) < device_info().sms; }
+
+int launch_split_sign_small(const float* a_lo, const float* a_up, const float* W, const float* bias, float* c_lo, float* c_up, int64_t M,
+                            int N, int K, cudaStream_t st, int split_rows, int split_d, const RangeEpilogue* range) {
+  const bool vec = K % 4 == 0 && aligned16(a_lo) && aligned16(a_up) && aligned16(W);
+  const dim3 grid((unsigned)ceil_div(M, kSmRows), (unsigned)ceil_div(N, kSmCols));
+  const RangeEpilogue rg = range != nullptr ? *range : RangeEpilogue{};
+  launch_k(vec ? split_sign_gemm_small<true> : split_sign_gemm_small<false>, grid, kThreads, kSmSmem, st, a_lo, a_up, W, bias, c_lo, c_up, M,
+           N, K, split_rows, split_d, rg);
+  FB_LAUNCH_OK();
+  return FB_OK;
+}
 
 // One split-sign GEMM: (a_lo, a_up) [M, K] x W[N, K]^T (+ bias) -> (c_lo, c_up) [M, N].
 int launch_split_sign_ffma(const float* a_lo, const float* a_up, const float* W, const float* bias, float* c_lo,
@@ -534,13 +567,8 @@ int launch_split_sign_ffma(const float* a_lo, const float* a_up, const float* W,
   const int gn = (int)ceil_div(N, BN);
   if (gm > 0x7fffffff || gn > 65535) return FB_ERR_SHAPE;
   const bool vec = K % 4 == 0 && aligned16(a_lo) && aligned16(a_up) && aligned16(W);
-  if (gm * gn < device_info().sms) {   // the 128 x 128 tiles would not fill the machine once
-    const dim3 grid((unsigned)ceil_div(M, kSmRows), (unsigned)ceil_div(N, kSmCols));
-    if (vec) fb::launch_k(split_sign_gemm_small<true>, grid, kThreads, kSmSmem, st, a_lo, a_up, W, bias, c_lo, c_up, M, N, K, split_rows, split_d);
-    else fb::launch_k(split_sign_gemm_small<false>, grid, kThreads, kSmSmem, st, a_lo, a_up, W, bias, c_lo, c_up, M, N, K, split_rows, split_d);
-    FB_LAUNCH_OK();
-    return FB_OK;
-  }
+  if (gm * gn < device_info().sms)
+    return launch_split_sign_small(a_lo, a_up, W, bias, c_lo, c_up, M, N, K, st, split_rows, split_d, nullptr);
   const size_t smem = sizeof(float) * 2 * kStageFloats;
   if (vec) {
     if (int rc = ensure_dynamic_smem(split_sign_gemm_ffma<true>, smem)) return rc;
