@@ -19,11 +19,12 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "dot_bias.cuh"
 
 namespace fb {
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = kDotBiasThreads;
 
 // ---------------------------------------------------------------- bias part
 // One warp per output element (b, i, j); lanes across k.
@@ -74,103 +75,6 @@ dot_bias_kernel(const float* __restrict__ x_lb, const float* __restrict__ x_ub, 
       const int64_t i_ = bi % Lx, od = (((b / heads) * Lx + i_) * heads + b % heads) * Ly + j;
       z_lb[od] = fmul(fadd(fadd(fadd(fadd(gl, l1), l2), l3), l4), out_scale);
       z_ub[od] = fmul(fadd(fadd(fadd(fadd(gu, u1), u2), u3), u4), out_scale);
-    }
-  }
-}
-
-// Tiled version of the bias part: one block per (b, RI i, 32 j) tile; the seven row tiles are staged in shared memory (row
-// stride 33 floats: conflict-free both for the row-wise fill and for the column-wise reads), K in chunks of 32 whose global
-// loads are issued before the arithmetic of the chunk before; a thread owns the outputs (warp + 8 c, lane),
-// c = 0 .. RI / 8 - 1.  Same partial sums and the same final order of additions as dot_bias_kernel.  RI = 8 where 32-row
-// tiles would leave SMs idle: the kernel is bound by the latency of one chunk, and four blocks of 32 rows (one sentence, four
-// heads) took 7.5 us.
-// y_kmajor: y_lb / y_ub are stored [b, k, j] instead of [b, j, k]; ranges_kmajor: y_l / y_u likewise.
-struct DotBias {
-  const float *x_lb, *x_ub, *y_lb, *y_ub, *x_l, *y_l, *y_u;
-  float *z_lb, *z_ub;
-  int Lx, Ly, K, n_it, n_jt, heads, y_kmajor, ranges_kmajor;
-  float out_scale;
-};
-__host__ __device__ constexpr int dot_bias_smem_floats(int ri) { return (3 * ri + 4 * 32) * 33; }
-
-template <int RI>
-__device__ __forceinline__ void dot_bias_tile(const DotBias& q, int w, float* smem) {
-  constexpr int C = RI / 8;
-  float (*sx)[RI][33] = reinterpret_cast<float (*)[RI][33]>(smem);                  // x_lb, x_ub, x_l
-  float (*sy)[32][33] = reinterpret_cast<float (*)[32][33]>(smem + 3 * RI * 33);    // y_lb, y_ub, y_l, y_u
-  const int jt = w % q.n_jt; w /= q.n_jt;
-  const int it = w % q.n_it;
-  const int64_t b = w / q.n_it;
-  const int i0 = it * RI, j0 = jt * 32;
-  const int tid = threadIdx.x, warp = tid >> 5, j = tid & 31;
-  float gl[C], gu[C], l1[C], l2[C], l3[C], l4[C], u1[C], u2[C], u3[C], u4[C];
-#pragma unroll
-  for (int c = 0; c < C; ++c) gl[c] = gu[c] = l1[c] = l2[c] = l3[c] = l4[c] = u1[c] = u2[c] = u3[c] = u4[c] = 0.f;
-  float vx[3][C], vy[4][4];
-  auto load = [&](int k0) {
-    const float* const xs[3] = {q.x_lb, q.x_ub, q.x_l};
-    const float* const ys[4] = {q.y_lb, q.y_ub, q.y_l, q.y_u};
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-      for (int c = 0; c < C; ++c) {
-        const int r = warp + 8 * c;
-        vx[a][c] = (i0 + r < q.Lx && k0 + j < q.K) ? xs[a][((int64_t)b * q.Lx + i0 + r) * q.K + k0 + j] : 0.f;
-      }
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const bool km = a < 2 ? q.y_kmajor != 0 : q.ranges_kmajor != 0;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int hi = warp + 8 * c, r = km ? j : hi, k = km ? hi : j;   // the fast index is the contiguous one
-        const int64_t idx = km ? ((int64_t)b * q.K + k0 + k) * q.Ly + j0 + r : ((int64_t)b * q.Ly + j0 + r) * q.K + k0 + k;
-        vy[a][c] = (j0 + r < q.Ly && k0 + k < q.K) ? ys[a][idx] : 0.f;
-      }
-    }
-  };
-  load(0);
-  for (int k0 = 0; k0 < q.K; k0 += 32) {
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-      for (int c = 0; c < C; ++c) sx[a][warp + 8 * c][j] = vx[a][c];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const bool km = a < 2 ? q.y_kmajor != 0 : q.ranges_kmajor != 0;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int hi = warp + 8 * c;
-        sy[a][km ? j : hi][km ? hi : j] = vy[a][c];
-      }
-    }
-    __syncthreads();
-    if (k0 + 32 < q.K) load(k0 + 32);
-#pragma unroll 4
-    for (int k = 0; k < 32; ++k) {
-      const float yl = sy[0][j][k], yu = sy[1][j][k], ly = sy[2][j][k], uy = sy[3][j][k];
-      const float lyp = ly > 0.f ? ly : 0.f, lyn = ly < 0.f ? ly : 0.f;
-      const float uyp = uy > 0.f ? uy : 0.f, uyn = uy < 0.f ? uy : 0.f;
-#pragma unroll
-      for (int c = 0; c < C; ++c) {
-        const float xl = sx[0][warp + 8 * c][k], xu = sx[1][warp + 8 * c][k], lx = sx[2][warp + 8 * c][k];
-        const float lxp = lx > 0.f ? lx : 0.f, lxn = lx < 0.f ? lx : 0.f;
-        gl[c] = fadd(gl[c], fmul(-ly, lx));
-        gu[c] = fadd(gu[c], fmul(-uy, lx));
-        l1[c] = fmaf(xl, lyp, l1[c]); l2[c] = fmaf(xu, lyn, l2[c]); l3[c] = fmaf(yl, lxp, l3[c]); l4[c] = fmaf(yu, lxn, l4[c]);
-        u1[c] = fmaf(xu, uyp, u1[c]); u2[c] = fmaf(xl, uyn, u2[c]); u3[c] = fmaf(yu, lxp, u3[c]); u4[c] = fmaf(yl, lxn, u4[c]);
-      }
-    }
-    __syncthreads();
-  }
-  if (j0 + j >= q.Ly) return;
-#pragma unroll
-  for (int c = 0; c < C; ++c) {
-    const int i = i0 + warp + 8 * c;
-    if (i < q.Lx) {
-      // heads > 1: head-merged output [S, Lx, heads * Ly]
-      const int64_t od = (((b / q.heads) * q.Lx + i) * q.heads + b % q.heads) * q.Ly + j0 + j;
-      q.z_lb[od] = fmul(fadd(fadd(fadd(fadd(gl[c], l1[c]), l2[c]), l3[c]), l4[c]), q.out_scale);
-      q.z_ub[od] = fmul(fadd(fadd(fadd(fadd(gu[c], u1[c]), u2[c]), u3[c]), u4[c]), q.out_scale);
     }
   }
 }
@@ -379,25 +283,21 @@ int launch_dot_weight_rows(const float* x_lw, const float* x_uw, const float* y_
 }
 
 
-int launch_dot_bias(const float* x_lb, const float* x_ub, const float* y_lb, const float* y_ub, const float* x_l, const float* y_l,
-                    const float* y_u, float* z_lb, float* z_ub, int B, int Lx, int Ly, int K, float out_scale, int heads,
-                    int y_kmajor, int ranges_kmajor, cudaStream_t st) {
-  const int n_jt = (int)ceil_div(Ly, 32);
-  const int64_t b32 = (int64_t)B * ceil_div(Lx, 32) * n_jt, b8 = (int64_t)B * ceil_div(Lx, 8) * n_jt;
-  DotBias q = {x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u, z_lb, z_ub, Lx, Ly, K, 0, n_jt, heads, y_kmajor, ranges_kmajor, out_scale};
+int launch_dot_bias(DotBias q, int B, cudaStream_t st) {
+  const int Lx = q.Lx, Ly = q.Ly, K = q.K;
+  const int64_t b32 = (int64_t)B * ceil_div(Lx, 32) * q.n_jt, b8 = (int64_t)B * ceil_div(Lx, 8) * q.n_jt;
   if (b32 < 2 * (int64_t)device_info().sms && b8 <= 0x7fffffff) {
-    q.n_it = (int)ceil_div(Lx, 8);
     fb::launch_k(dot_bias_tiled<8>, (unsigned)b8, kThreads, 0, st, q);
   } else if (b32 <= 0x7fffffff) {
     q.n_it = (int)ceil_div(Lx, 32);
     fb::launch_k(dot_bias_tiled<32>, (unsigned)b32, kThreads, 0, st, q);
   } else {
-    if (y_kmajor || ranges_kmajor) return FB_ERR_SHAPE;
+    if (q.y_kmajor || q.ranges_kmajor) return FB_ERR_SHAPE;
     const int64_t total = (int64_t)B * Lx * Ly;
     const int64_t want = ceil_div(total, kThreads / 32);
     const int64_t cap = (int64_t)device_info().sms * 32;
-    fb::launch_k(dot_bias_kernel, (unsigned)(want < cap ? want : cap), kThreads, 0, st, x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u, z_lb, z_ub, total,
-                                                                              Lx, Ly, K, out_scale, heads);
+    fb::launch_k(dot_bias_kernel, (unsigned)(want < cap ? want : cap), kThreads, 0, st, q.x_lb, q.x_ub, q.y_lb, q.y_ub, q.x_l, q.y_l, q.y_u, q.z_lb,
+                 q.z_ub, total, Lx, Ly, K, q.out_scale, q.heads);
   }
   FB_LAUNCH_OK();
   return FB_OK;
@@ -415,12 +315,13 @@ bool dot_tc_supported(const float* x_lw, const float* x_uw, const float* y_lw, c
                       int Di, int K, int heads);
 int launch_dot_weight_tc(const float* x_lw, const float* x_uw, const float* y_lw, const float* y_uw, const float* x_l,
                          const float* y_l, const float* y_u, float* z_lw, float* z_uw, int B, int Lx, int Ly, int Di,
-                         float out_scale, int heads, int y_kmajor, cudaStream_t st);
+                         float out_scale, int heads, int y_kmajor, cudaStream_t st, const DotBias& bias, bool& bias_done);
 // dot_product_tc_any.cu
 bool dot_tc_any_supported(int B, int Lx, int Ly, int Di, int K);
 int launch_dot_weight_tc_any(const float* x_lw, const float* x_uw, const float* y_lw, const float* y_uw, const float* x_l,
                              const float* y_l, const float* y_u, float* z_lw, float* z_uw, int B, int Lx, int Ly, int Di, int K,
-                             float out_scale, int heads, int y_kmajor, int y_ranges_kmajor, int ldx, int ldz, cudaStream_t st);
+                             float out_scale, int heads, int y_kmajor, int y_ranges_kmajor, int ldx, int ldz, cudaStream_t st,
+                             const DotBias& bias, bool& bias_done);
 namespace {
 // FB_DOT_IMPL=ffma in the environment keeps the dot product on the CUDA-core kernels (exact fp32 products)
 bool dot_force_cuda_cores() {
@@ -474,21 +375,25 @@ int fb::dot_product_ex(const float* x_lw, const float* x_uw, const float* x_lb, 
   else if (given == 1)
     rc = fb_concretize_f32(y_lw, y_uw, y_lb, y_ub, y_l, y_u, (int64_t)B * Ly, Di, K, words, p, eps, layout, stream);
   if (rc != FB_OK) return rc;
-  if (layout == FB_TRANSPOSED && ldz == 0) {
-    const DotBias q = {x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u, z_lb, z_ub, Lx, Ly, K, (int)ceil_div(Lx, 8), (int)ceil_div(Ly, 32), 1, 0, 0,
-                       out_scale};
-    return launch_dot_transposed(x_lw, x_uw, y_lw, y_uw, z_lw, z_uw, q, B, Di, st);
-  }
-  rc = launch_dot_bias(x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u, z_lb, z_ub, B, Lx, Ly, K, out_scale, merge_heads, 0, 0, st);
-  if (rc != FB_OK) return rc;
+  const DotBias q = {x_lb, x_ub, y_lb, y_ub, x_l, y_l, y_u, z_lb, z_ub, Lx, Ly, K, (int)ceil_div(Lx, 8), (int)ceil_div(Ly, 32), merge_heads, 0, 0,
+                     out_scale};
+  if (layout == FB_TRANSPOSED && ldz == 0) return launch_dot_transposed(x_lw, x_uw, y_lw, y_uw, z_lw, z_uw, q, B, Di, st);
   // Tensor-core kernels: the one for the attention shapes with lengths that are multiples of 32 (5.6 TB/s on a large batch,
   // where the other reaches 4.8), else the one for any shape of the native layout; a few query rows would be padded to 32 there.
-  if (layout == FB_NATIVE && !dot_force_cuda_cores() && ldz == 0 &&
-      dot_tc_supported(x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, K, merge_heads))
-    return launch_dot_weight_tc(x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, out_scale, merge_heads, 0, st);
-  if (layout == FB_NATIVE && !dot_force_cuda_cores() && Lx > kFewRows && dot_tc_any_supported(B, Lx, Ly, Di, K))
-    return launch_dot_weight_tc_any(x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, K, out_scale, merge_heads, 0, 0,
-                                    0, ldz, st);
+  bool bias_done = false;
+  if (layout == FB_NATIVE && !dot_force_cuda_cores()) {
+    const bool tc32 = ldz == 0 && dot_tc_supported(x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, K, merge_heads);
+    if (tc32 || (Lx > kFewRows && dot_tc_any_supported(B, Lx, Ly, Di, K))) {
+      rc = tc32 ? launch_dot_weight_tc(x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, out_scale, merge_heads, 0, st, q,
+                                       bias_done)
+                : launch_dot_weight_tc_any(x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, K, out_scale, merge_heads, 0,
+                                           0, 0, ldz, st, q, bias_done);
+      if (rc != FB_OK || bias_done) return rc;
+      return launch_dot_bias(q, B, st);
+    }
+  }
+  rc = launch_dot_bias(q, B, st);
+  if (rc != FB_OK) return rc;
   if (ldz != 0) return FB_ERR_SHAPE;
   if (layout == FB_NATIVE && Lx <= kFewRows)
     return launch_dot_weight_rows(x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, K, out_scale, merge_heads, 0, st);
@@ -646,13 +551,18 @@ int fb::context_ex(const float* x_lw, const float* x_uw, const float* x_lb, cons
     fb::launch_k(transpose_small_inplace, (unsigned)B, 256, 0, st, y_l, y_u, K, Ly);
     FB_LAUNCH_OK();
   }
-  rc = launch_dot_bias(x_lb, x_ub, v_lb, v_ub, x_l, y_l, y_u, z_lb, z_ub, B, Lx, Ly, K, out_scale, merge_heads, 1, transpose ? 0 : 1, st);
-  if (rc != FB_OK) return rc;
+  const DotBias q = {x_lb, x_ub, v_lb, v_ub, x_l, y_l, y_u, z_lb, z_ub, Lx, Ly, K, (int)ceil_div(Lx, 8), (int)ceil_div(Ly, 32), merge_heads, 1,
+                     transpose ? 0 : 1, out_scale};
+  bool bias_done = false;
   if (!tc)
-    return launch_dot_weight_rows(x_lw, x_uw, v_lw, v_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, K, out_scale, merge_heads, 1, st);
-  if (tc32) return launch_dot_weight_tc(x_lw, x_uw, v_lw, v_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, out_scale, merge_heads, 1, st);
-  return launch_dot_weight_tc_any(x_lw, x_uw, v_lw, v_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, K, out_scale, merge_heads, 1,
-                                  transpose ? 0 : 1, ldx, 0, st);
+    rc = launch_dot_weight_rows(x_lw, x_uw, v_lw, v_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, K, out_scale, merge_heads, 1, st);
+  else if (tc32)
+    rc = launch_dot_weight_tc(x_lw, x_uw, v_lw, v_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, out_scale, merge_heads, 1, st, q, bias_done);
+  else
+    rc = launch_dot_weight_tc_any(x_lw, x_uw, v_lw, v_uw, x_l, y_l, y_u, z_lw, z_uw, B, Lx, Ly, Di, K, out_scale, merge_heads, 1,
+                                  transpose ? 0 : 1, ldx, 0, st, q, bias_done);
+  if (rc != FB_OK || bias_done) return rc;
+  return launch_dot_bias(q, B, st);
 }
 
 extern "C" int fb_context_f32(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub,

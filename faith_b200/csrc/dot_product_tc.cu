@@ -40,6 +40,7 @@
 #include <unordered_map>
 
 #include "common.cuh"
+#include "dot_bias.cuh"
 
 namespace fb {
 namespace {
@@ -88,8 +89,14 @@ dot_weight_tc(const __grid_constant__ CUtensorMap tm_xl, const __grid_constant__
               const __grid_constant__ CUtensorMap tm_lx, const __grid_constant__ CUtensorMap tm_ly,
               const __grid_constant__ CUtensorMap tm_uy, const __grid_constant__ CUtensorMap tm_zl,
               const __grid_constant__ CUtensorMap tm_zu, int Lx, int Ly, int n_ib, int n_mb, int total_tiles,
-              float out_scale, int heads, int y_kmajor, int* __restrict__ status) {
+              float out_scale, int heads, int y_kmajor, int* __restrict__ status, const DotBias bias, int n_bias) {
   extern __shared__ uint8_t smem_raw[];
+  const int grid = (int)gridDim.x - n_bias;   // blocks of the weight part; the rest take a tile of the bias part each
+  if ((int)blockIdx.x >= grid) {
+    pdl_sync();
+    if (threadIdx.x < kDotBiasThreads) dot_bias_tile<8>(bias, (int)blockIdx.x - grid, reinterpret_cast<float*>(smem_raw));
+    return;
+  }
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t bar0 = base + kDtOffBars;
@@ -103,7 +110,7 @@ dot_weight_tc(const __grid_constant__ CUtensorMap tm_xl, const __grid_constant__
   volatile int* cta_abort = reinterpret_cast<volatile int*>(base_ptr + kDtOffBars + 72);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int my_tiles = (total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int my_tiles = (total_tiles - (int)blockIdx.x + grid - 1) / grid;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) {
@@ -129,7 +136,7 @@ dot_weight_tc(const __grid_constant__ CUtensorMap tm_xl, const __grid_constant__
 
   // coordinates of tile t of this CTA
   auto tile_coords = [&](int t, int& b, int& i0, int& m0) {
-    const int tile = (int)blockIdx.x + t * (int)gridDim.x;
+    const int tile = (int)blockIdx.x + t * grid;
     const int mb = tile % n_mb, rest = tile / n_mb;
     m0 = mb * 4;
     i0 = (rest % n_ib) * 32;
@@ -478,7 +485,7 @@ int* tc_status_sink();
 
 int launch_dot_weight_tc(const float* x_lw, const float* x_uw, const float* y_lw, const float* y_uw, const float* x_l,
                          const float* y_l, const float* y_u, float* z_lw, float* z_uw, int B, int Lx, int Ly, int Di,
-                         float out_scale, int heads, int y_kmajor, cudaStream_t st) {
+                         float out_scale, int heads, int y_kmajor, cudaStream_t st, const DotBias& bias, bool& bias_done) {
   CUtensorMap tm_xl, tm_xu, tm_yl, tm_yu, tm_lx, tm_ly, tm_uy, tm_zl, tm_zu;
   const uint64_t S = (uint64_t)(B / heads);
   if (!make_map3(&tm_xl, x_lw, 32, (uint64_t)Di, (uint64_t)B * Lx) || !make_map3(&tm_xu, x_uw, 32, (uint64_t)Di, (uint64_t)B * Lx) ||
@@ -499,7 +506,12 @@ int launch_dot_weight_tc(const float* x_lw, const float* x_uw, const float* y_lw
   });
   FB_CUDA_OK(attr_err);
   const int sms = device_info().sms;
-  fb::launch_k(dot_weight_tc, (unsigned)(total < sms ? total : sms), kDtThreads, kDtSmemBytes, st, tm_xl, tm_xu, tm_yl, tm_yu, tm_lx, tm_ly, tm_uy, tm_zl, tm_zu, Lx, Ly, n_ib, n_mb, total, out_scale, heads, y_kmajor, tc_status_sink());
+  // the bias part goes along where that leaves a block per SM: a launch of 4 us for one sentence of four heads
+  const int64_t n_bias = (int64_t)B * bias.n_it * bias.n_jt;
+  bias_done = total + n_bias <= sms;
+  const int extra = bias_done ? (int)n_bias : 0;
+  launch_k(dot_weight_tc, (unsigned)((total < sms ? total : sms) + extra), kDtThreads, kDtSmemBytes, st, tm_xl, tm_xu, tm_yl, tm_yu, tm_lx, tm_ly,
+           tm_uy, tm_zl, tm_zu, Lx, Ly, n_ib, n_mb, total, out_scale, heads, y_kmajor, tc_status_sink(), bias, extra);
   FB_LAUNCH_OK();
   return FB_OK;
 }

@@ -51,6 +51,7 @@
 #include <unordered_map>
 
 #include "common.cuh"
+#include "dot_bias.cuh"
 
 namespace fb {
 int* tc_status_sink();   // matmul_tc.cu: the status word of the pass being enqueued, if any
@@ -114,8 +115,14 @@ template <bool kTmaIn, bool kVecOut, bool kMulti>
 __global__ void __launch_bounds__(kDaThreads, 1)
 dot_weight_tc_any(const __grid_constant__ CUtensorMap tm_xl, const __grid_constant__ CUtensorMap tm_xu,
               const __grid_constant__ CUtensorMap tm_yl, const __grid_constant__ CUtensorMap tm_yu, const DotArgs A,
-              int* __restrict__ status) {
+              int* __restrict__ status, const DotBias bias, int n_bias) {
   extern __shared__ uint8_t smem_raw[];
+  const int grid = (int)gridDim.x - n_bias;   // blocks of the weight part; the rest take a tile of the bias part each
+  if ((int)blockIdx.x >= grid) {
+    pdl_sync();
+    if (threadIdx.x < kDotBiasThreads) dot_bias_tile<8>(bias, (int)blockIdx.x - grid, reinterpret_cast<float*>(smem_raw));
+    return;
+  }
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t bar0 = base + kDaOffBars;
@@ -133,8 +140,8 @@ dot_weight_tc_any(const __grid_constant__ CUtensorMap tm_xl, const __grid_consta
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // tiles of this CTA: a contiguous range in the order (b, i block, j block, m block), m fastest
-  const int first_tile = (int)((int64_t)blockIdx.x * A.total_tiles / gridDim.x);
-  const int my_tiles = (int)((int64_t)(blockIdx.x + 1) * A.total_tiles / gridDim.x) - first_tile;
+  const int first_tile = (int)((int64_t)blockIdx.x * A.total_tiles / grid);
+  const int my_tiles = (int)((int64_t)(blockIdx.x + 1) * A.total_tiles / grid) - first_tile;
   const int n_kc = kMulti ? A.n_kc : 1;
   const int n_items = my_tiles * n_kc;   // item = chunk of a tile
 
@@ -501,10 +508,11 @@ bool make_in_map(CUtensorMap* map, const float* ptr, uint64_t C, uint64_t Di, ui
   return get_map(map, MapKey{ptr, {C, Di, R, B, 1}, {ld * 4, Di * ld * 4, R * Di * ld * 4, 0}, {32, 4, 32, 1, 1}, 4});
 }
 template <bool kTmaIn, bool kVecOut, bool kMulti>
-int launch_variant(const CUtensorMap (&tm)[4], const DotArgs& a, cudaStream_t st) {
+int launch_variant(const CUtensorMap (&tm)[4], const DotArgs& a, cudaStream_t st, const DotBias& bias, int n_bias) {
   const int sms = device_info().sms;
   if (int rc = ensure_dynamic_smem(dot_weight_tc_any<kTmaIn, kVecOut, kMulti>, kDaSmemBytes)) return rc;
-  fb::launch_k(dot_weight_tc_any<kTmaIn, kVecOut, kMulti>, (unsigned)(a.total_tiles < sms ? a.total_tiles : sms), kDaThreads, kDaSmemBytes, st, tm[0], tm[1], tm[2], tm[3], a, tc_status_sink());
+  fb::launch_k(dot_weight_tc_any<kTmaIn, kVecOut, kMulti>, (unsigned)((a.total_tiles < sms ? a.total_tiles : sms) + n_bias), kDaThreads, kDaSmemBytes,
+               st, tm[0], tm[1], tm[2], tm[3], a, tc_status_sink(), bias, n_bias);
   FB_LAUNCH_OK();
   return FB_OK;
 }
@@ -521,7 +529,8 @@ bool dot_tc_any_supported(int B, int Lx, int Ly, int Di, int K) {
 // are [B, K, Ly] instead of [B, Ly, K].
 int launch_dot_weight_tc_any(const float* x_lw, const float* x_uw, const float* y_lw, const float* y_uw, const float* x_l,
                          const float* y_l, const float* y_u, float* z_lw, float* z_uw, int B, int Lx, int Ly, int Di, int K,
-                         float out_scale, int heads, int y_kmajor, int y_ranges_kmajor, int ldx, int ldz, cudaStream_t st) {
+                         float out_scale, int heads, int y_kmajor, int y_ranges_kmajor, int ldx, int ldz, cudaStream_t st,
+                             const DotBias& bias, bool& bias_done) {
   DotArgs a = {x_lw, x_uw, y_lw, y_uw, x_l, y_l, y_u, z_lw, z_uw, Lx, Ly, Di, K, 0, 0, 0, 0, 0, 0, 0, 0, heads, y_kmajor,
                y_ranges_kmajor, out_scale};
   a.ldx = ldx > 0 ? ldx : K;
@@ -542,7 +551,11 @@ int launch_dot_weight_tc_any(const float* x_lw, const float* x_uw, const float* 
         !make_in_map(&tm[2], y_lw, yc, Di, yr, B, a.ldy) || !make_in_map(&tm[3], y_uw, yc, Di, yr, B, a.ldy))
       return FB_ERR_CUDA;
   }
-#define FB_DOT_VARIANT(I, O) return a.n_kc > 1 ? launch_variant<I, O, true>(tm, a, st) : launch_variant<I, O, false>(tm, a, st)
+  // the bias part goes along where that leaves a block per SM (as in the kernel for lengths of 32)
+  const int64_t bias_blocks = (int64_t)B * bias.n_it * bias.n_jt;
+  bias_done = a.total_tiles + bias_blocks <= device_info().sms;
+  const int n_bias = bias_done ? (int)bias_blocks : 0;
+#define FB_DOT_VARIANT(I, O) return a.n_kc > 1 ? launch_variant<I, O, true>(tm, a, st, bias, n_bias) : launch_variant<I, O, false>(tm, a, st, bias, n_bias)
   if (tma_in && vec_out) FB_DOT_VARIANT(true, true);
   if (tma_in) FB_DOT_VARIANT(true, false);
   if (vec_out) FB_DOT_VARIANT(false, true);
