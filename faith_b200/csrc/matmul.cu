@@ -1,5 +1,6 @@
 // fb_matmul_f32: bounds x constant weight.  Dispatches to the split-sign GEMM kernels.
 #include "common.cuh"
+#include "matmul_small.cuh"
 
 #include <cstdlib>
 #include <cstring>
@@ -13,7 +14,7 @@ int launch_split_sign_tc(const float* a_lo, const float* a_up, const float* W, c
                          const float* coef_l = nullptr, const float* coef_u = nullptr, int coef_di = 1,
                          float* norm_lo = nullptr, float* norm_up = nullptr, int norm_p = 0,
                          const float* res_lo = nullptr, const float* res_up = nullptr, const TcBiasRows* br = nullptr,
-                         const TcLnArgs* ln = nullptr);
+                         const TcLnArgs* ln = nullptr, const SmallProduct* few = nullptr, bool* few_done = nullptr);
 bool tc_bias_rows_mergeable(const float* a_lo, const float* a_up, const float* b_lo, const float* b_up, const float* W,
                             const float* cb_lo, const float* cb_up, int64_t Mb, int N, int K, bool with_norms);
 int launch_split_sign_ffma(const float* a_lo, const float* a_up, const float* W, const float* bias, float* c_lo,
@@ -108,6 +109,13 @@ ranges_from_norms_kernel(float* __restrict__ lb, float* __restrict__ ub, const f
 }
 }  // namespace fb
 
+// Whether the bias rows of a product go to the kernel for few rows, in the form that can ride in the tensor-core launch.
+static bool small_bias_rows(const float* x_lb, const float* x_ub, const float* W, const float* y_lb, const float* y_ub, int64_t rows, int Dy,
+                            int Do) {
+  return rows > 0 && !fb::tc_gemm_supported(x_lb, x_ub, W, y_lb, y_ub, rows, Dy, Do) && fb::small_product(rows, Dy) && Do % 4 == 0 &&
+         fb::aligned16(x_lb) && fb::aligned16(x_ub) && fb::aligned16(W);
+}
+
 static int matmul_impl(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub, const float* W,
                        const float* bias, float* y_lw, float* y_uw, float* y_lb, float* y_ub, int64_t rows, int Di,
                        int Do, int Dy, int L, int heads, void* stream) {
@@ -126,10 +134,21 @@ static int matmul_impl(const float* x_lw, const float* x_uw, const float* x_lb, 
     return fb::launch_split_sign_tc(x_lw, x_uw, W, nullptr, y_lw, y_uw, Mw, Dy, Do, st, 0, 0, nullptr, nullptr, 1, nullptr,
                                     nullptr, 0, nullptr, nullptr, &br);
   }
-  // weight rows: [rows * Di, Do] -> [rows * Di, Dy]; no bias on the symbolic part
-  int rc = fb::split_sign_gemm(x_lw, x_uw, W, nullptr, y_lw, y_uw, rows * (int64_t)Di, Dy, Do, st,
-                               heads > 1 ? L * Di : 0, d);
-  if (rc != FB_OK) return rc;
+  // weight rows: [rows * Di, Do] -> [rows * Di, Dy]; no bias on the symbolic part.  On the tensor cores they take the bias rows
+  // along where those go to the kernel for few rows and SMs are left for them.
+  const int split_rows = heads > 1 ? L * Di : 0;
+  bool bias_done = false;
+  int rc;
+  if (Mw > 0 && fb::use_tensor_cores() && fb::tc_gemm_supported(x_lw, x_uw, W, y_lw, y_uw, Mw, Dy, Do) &&
+      (split_rows == 0 || fb::tc_split_supported(Mw, Dy, split_rows, d))) {
+    const fb::SmallProduct few = {x_lb, x_ub, W, bias, y_lb, y_ub, rows, Dy, Do, heads > 1 ? L : 0, d};
+    const bool takes = small_bias_rows(x_lb, x_ub, W, y_lb, y_ub, rows, Dy, Do);
+    rc = fb::launch_split_sign_tc(x_lw, x_uw, W, nullptr, y_lw, y_uw, Mw, Dy, Do, st, split_rows, d, nullptr, nullptr, 1, nullptr, nullptr, 0,
+                                  nullptr, nullptr, nullptr, nullptr, takes ? &few : nullptr, &bias_done);
+  } else {
+    rc = fb::split_sign_gemm(x_lw, x_uw, W, nullptr, y_lw, y_uw, Mw, Dy, Do, st, split_rows, d);
+  }
+  if (rc != FB_OK || bias_done) return rc;
   // bias rows: [rows, Do] -> [rows, Dy], + bias
   return fb::split_sign_gemm(x_lb, x_ub, W, bias, y_lb, y_ub, rows, Dy, Do, st, heads > 1 ? L : 0, d);
 }
@@ -168,9 +187,12 @@ extern "C" int fb_matmul_coef_f32(const float* x_lw, const float* x_uw, const fl
   fb::ProfileScope prof(fb::PK_MATMUL, 8.0 * Mt * Do * Dy, 4.0 * (2 * Mt * Do + 2 * Mt * Dy + (double)Do * Dy + Dy), stream);
   const fb::TcBiasRows br = {x_lb, x_ub, bias, y_lb, y_ub, rows, nullptr, nullptr};
   const bool merged = fb::tc_bias_rows_mergeable(x_lw, x_uw, x_lb, x_ub, W, y_lb, y_ub, rows, Dy, Do, false);
+  const fb::SmallProduct few = {x_lb, x_ub, W, bias, y_lb, y_ub, rows, Dy, Do, 0, 0};
+  const bool takes = !merged && small_bias_rows(x_lb, x_ub, W, y_lb, y_ub, rows, Dy, Do);
+  bool few_done = false;
   int rc = fb::launch_split_sign_tc(x_lw, x_uw, W, nullptr, y_lw, y_uw, M, Dy, Do, st, 0, 0, c_l, c_u, Di, nullptr, nullptr, 0,
-                                    nullptr, nullptr, merged ? &br : nullptr);
-  if (rc != FB_OK || merged) return rc;
+                                    nullptr, nullptr, merged ? &br : nullptr, nullptr, takes ? &few : nullptr, &few_done);
+  if (rc != FB_OK || merged || few_done) return rc;
   return fb::split_sign_gemm(x_lb, x_ub, W, bias, y_lb, y_ub, rows, Dy, Do, st);
 }
 

@@ -14,6 +14,7 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "matmul_small.cuh"
 
 namespace fb {
 namespace {
@@ -389,126 +390,11 @@ split_sign_gemv_block(const float* __restrict__ a_lo, const float* __restrict__ 
   cluster.sync();   // the other blocks' shared memory stays alive until block 0 has read it
 }
 
-// Few output tiles (the bias rows of a sentence, the pooler: M of 1 to a few hundred): the 128 x 128 tiles above would leave all
-// but a handful of SMs idle, each walking K alone (32 x 128 x 128 on one block: 28 us, 32 x 512 -> 128: 99 us).  Here a
-// block owns 8 rows x 32 columns and its eight warps split K, a contiguous part each: centre and radius of the rows are
-// staged in shared memory and read as broadcasts, a lane owns one column and streams its part of that row of W with
-// 128-bit loads (whole sectors), the eight partial sums of an output are added in warp order.  Bound by the latency of one
-// pass over the operands: 4.0 us resp. 9.0 us at the sizes above.  The concretised range of the rows and the coefficients of a
-// relaxation follow in the same launch where the caller wants them (two launches of 2 to 3 us each otherwise).
-constexpr int kSmRows = 8, kSmCols = 32, kSmWarps = kThreads / 32, kSmChunk = 512;
-constexpr uint32_t kSmSmem = sizeof(float) * (2 * kSmRows * kSmChunk + 2 * kSmWarps * kSmRows * kSmCols);
 template <bool VEC>
-__global__ void __launch_bounds__(kThreads)
-split_sign_gemm_small(const float* __restrict__ a_lo, const float* __restrict__ a_up, const float* __restrict__ W,
-                      const float* __restrict__ bias, float* __restrict__ c_lo, float* __restrict__ c_up, int64_t M, int N, int K,
-                      int split_rows, int split_d, const RangeEpilogue rg) {
+__global__ void __launch_bounds__(kSmThreads) split_sign_gemm_small(const SmallProduct q, const RangeEpilogue rg) {
   pdl_sync();
   extern __shared__ __align__(16) float smem[];
-  float* const s_c = smem;                                  // [kSmRows][kSmChunk] centres
-  float* const s_r = s_c + kSmRows * kSmChunk;              // radii
-  float* const s_red = s_r + kSmRows * kSmChunk;            // [2][warps][rows][cols]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t m0 = (int64_t)blockIdx.x * kSmRows;
-  const int n = blockIdx.y * kSmCols + lane;
-  const float* const wrow = W + (int64_t)(n < N ? n : N - 1) * K;   // (a column beyond N computes what is not stored)
-  float sc[kSmRows], sr[kSmRows];
-#pragma unroll
-  for (int i = 0; i < kSmRows; ++i) { sc[i] = 0.f; sr[i] = 0.f; }
-  for (int k0 = 0; k0 < K; k0 += kSmChunk) {
-    const int kc = min(kSmChunk, K - k0), quads = (kc + 3) / 4;
-    if (k0 > 0) __syncthreads();
-    for (int f = tid; f < kSmRows * quads; f += kThreads) {
-      const int i = f / quads, q = f % quads;
-      const int64_t m = m0 + i;
-      float lo[4] = {0.f, 0.f, 0.f, 0.f}, up[4] = {0.f, 0.f, 0.f, 0.f};
-      if (m < M) {
-        const float* pl = a_lo + m * K + k0 + 4 * q;
-        const float* pu = a_up + m * K + k0 + 4 * q;
-        if (VEC) {
-          *reinterpret_cast<float4*>(lo) = __ldg(reinterpret_cast<const float4*>(pl));
-          *reinterpret_cast<float4*>(up) = __ldg(reinterpret_cast<const float4*>(pu));
-        } else {
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            if (4 * q + e < kc) { lo[e] = __ldg(pl + e); up[e] = __ldg(pu + e); }
-        }
-      }
-      float4 c, r;
-      c.x = fmul(fadd(lo[0], up[0]), 0.5f); r.x = fmul(fsub(up[0], lo[0]), 0.5f);
-      c.y = fmul(fadd(lo[1], up[1]), 0.5f); r.y = fmul(fsub(up[1], lo[1]), 0.5f);
-      c.z = fmul(fadd(lo[2], up[2]), 0.5f); r.z = fmul(fsub(up[2], lo[2]), 0.5f);
-      c.w = fmul(fadd(lo[3], up[3]), 0.5f); r.w = fmul(fsub(up[3], lo[3]), 0.5f);
-      *reinterpret_cast<float4*>(s_c + i * kSmChunk + 4 * q) = c;
-      *reinterpret_cast<float4*>(s_r + i * kSmChunk + 4 * q) = r;
-    }
-    __syncthreads();
-    const int per = (quads + kSmWarps - 1) / kSmWarps;
-    const int q_end = min(quads, (warp + 1) * per);
-#pragma unroll 4
-    for (int q = warp * per; q < q_end; ++q) {
-      float w[4] = {0.f, 0.f, 0.f, 0.f};
-      const float* pw = wrow + k0 + 4 * q;
-      if (VEC) {
-        *reinterpret_cast<float4*>(w) = __ldg(reinterpret_cast<const float4*>(pw));
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (4 * q + e < kc) w[e] = __ldg(pw + e);
-      }
-#pragma unroll
-      for (int i = 0; i < kSmRows; ++i) {
-        const float4 c = *reinterpret_cast<const float4*>(s_c + i * kSmChunk + 4 * q);
-        const float4 r = *reinterpret_cast<const float4*>(s_r + i * kSmChunk + 4 * q);
-        sc[i] = fmaf(c.x, w[0], sc[i]); sr[i] = fmaf(r.x, fabsf(w[0]), sr[i]);
-        sc[i] = fmaf(c.y, w[1], sc[i]); sr[i] = fmaf(r.y, fabsf(w[1]), sr[i]);
-        sc[i] = fmaf(c.z, w[2], sc[i]); sr[i] = fmaf(r.z, fabsf(w[2]), sr[i]);
-        sc[i] = fmaf(c.w, w[3], sc[i]); sr[i] = fmaf(r.w, fabsf(w[3]), sr[i]);
-      }
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < kSmRows; ++i) {
-    s_red[(warp * kSmRows + i) * kSmCols + lane] = sc[i];
-    s_red[((kSmWarps + warp) * kSmRows + i) * kSmCols + lane] = sr[i];
-  }
-  __syncthreads();
-  // thread (row i = warp, column = lane)
-  const int64_t m = m0 + warp;
-  if (m >= M || n >= N) return;
-  float c = s_red[warp * kSmCols + lane], r = s_red[(kSmWarps * kSmRows + warp) * kSmCols + lane];
-#pragma unroll
-  for (int w = 1; w < kSmWarps; ++w) {
-    c = fadd(c, s_red[(w * kSmRows + warp) * kSmCols + lane]);
-    r = fadd(r, s_red[((kSmWarps + w) * kSmRows + warp) * kSmCols + lane]);
-  }
-  float lo = fsub(c, r), up = fadd(c, r);
-  if (bias != nullptr) { lo = fadd(lo, bias[n]); up = fadd(up, bias[n]); }
-  int64_t o = m * N + n, ot = o;
-  if (split_rows > 0) {
-    const int64_t g = m / split_rows, rr = m % split_rows, gh = g * (N / split_d) + n / split_d;
-    o = (gh * split_rows + rr) * split_d + n % split_d;
-    ot = (gh * split_d + n % split_d) * split_rows + rr;
-  }
-  c_lo[o] = lo;
-  c_up[o] = up;
-  if (rg.norm_lo == nullptr) return;
-  const float lb = lo, ub = up;
-  for (int w = 0; w < rg.words; ++w) {
-    const int64_t at = (m * rg.words + w) * N + n;
-    lo = fadd(lo, fmul(-rg.eps, __ldg(rg.norm_lo + at)));
-    up = fadd(up, fmul(rg.eps, __ldg(rg.norm_up + at)));
-  }
-  rg.out_l[rg.transposed ? ot : o] = lo;
-  rg.out_u[rg.transposed ? ot : o] = up;
-  if (rg.op < 0) return;
-  bool bad = false;
-  const ColCoef k = relax_column(rg.op, lo, up, lb, ub, bad);
-  if (rg.violation != nullptr && (bad || k.c_lu != 0.f || k.c_ul != 0.f)) atomicOr(rg.violation, bad ? 1 : 2);
-  rg.k_l[m * N + n] = k.c_ll;
-  rg.k_u[m * N + n] = k.c_uu;
-  rg.r_lb[m * N + n] = k.nlb;
-  rg.r_ub[m * N + n] = k.nub;
+  small_product_block<VEC>(q, rg, blockIdx.x, blockIdx.y, smem);
 }
 
 }  // namespace
@@ -521,8 +407,8 @@ int launch_split_sign_small(const float* a_lo, const float* a_up, const float* W
   const bool vec = K % 4 == 0 && aligned16(a_lo) && aligned16(a_up) && aligned16(W);
   const dim3 grid((unsigned)ceil_div(M, kSmRows), (unsigned)ceil_div(N, kSmCols));
   const RangeEpilogue rg = range != nullptr ? *range : RangeEpilogue{};
-  launch_k(vec ? split_sign_gemm_small<true> : split_sign_gemm_small<false>, grid, kThreads, kSmSmem, st, a_lo, a_up, W, bias, c_lo, c_up, M,
-           N, K, split_rows, split_d, rg);
+  const SmallProduct q = {a_lo, a_up, W, bias, c_lo, c_up, M, N, K, split_rows, split_d};
+  launch_k(vec ? split_sign_gemm_small<true> : split_sign_gemm_small<false>, grid, kSmThreads, kSmSmem, st, q, rg);
   FB_LAUNCH_OK();
   return FB_OK;
 }

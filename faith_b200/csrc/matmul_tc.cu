@@ -53,6 +53,7 @@
 #include <unordered_map>
 
 #include "common.cuh"
+#include "matmul_small.cuh"
 
 namespace fb {
 namespace {
@@ -139,6 +140,11 @@ struct SharedLayout {
   __host__ __device__ static constexpr uint32_t bars() { return out() + kOutStageBytes; }
 };
 
+// (a call, not inlined: the registers of the tiles' roles stay as they are)
+__device__ __noinline__ void few_rows(const SmallProduct& q, int bx, int by, float* smem) {
+  small_product_block<true>(q, RangeEpilogue{}, bx, by, smem);
+}
+
 // kCoef: column slopes of a relaxation are applied to the operands on the fly (a separate instantiation, so
 // that the plain kernel keeps its register allocation).
 // kNorm: the epilogue also writes the dual norm over the 128 rows of every output column of the tile,
@@ -183,10 +189,17 @@ split_sign_gemm_tc(const __grid_constant__ CUtensorMap tm_lo, const __grid_const
                    const float* __restrict__ coef_l, const float* __restrict__ coef_u, int coef_di,
                    float* __restrict__ norm_lo, float* __restrict__ norm_up, int norm_p,
                    int* __restrict__ status, uint32_t wait_tries, int skip_it, const LiveRows live_rows, int same_out,
-                   const TcLnArgs ln_args, int64_t Mb) {
+                   const TcLnArgs ln_args, int64_t Mb, const SmallProduct small, int n_small) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
+  const int grid = (int)gridDim.x - n_small;   // CTAs of the tiles; the others take a block of the product of few rows each
+  if (!kNorm && !kResid && (int)blockIdx.x >= grid) {
+    pdl_sync();
+    const int e = (int)blockIdx.x - grid, gx = (int)((small.M + kSmRows - 1) / kSmRows);
+    if (threadIdx.x < kSmThreads) few_rows(small, e % gx, e / gx, reinterpret_cast<float*>(base_ptr));
+    return;
+  }
   // Row blocks known to be zero (live_rows.L > 0; zero-radius instantiation only): a tile of such a block is not
   // loaded, converted or multiplied; the issuers only signal "ready" and the epilogue stores zeros (and zero norms).
   const bool use_live = kPoint && kNorm && !kCoef && !kResid && live_rows.L > 0;
@@ -217,10 +230,10 @@ split_sign_gemm_tc(const __grid_constant__ CUtensorMap tm_lo, const __grid_const
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nkb = (K + BK - 1) / BK;
-  // tiles of this CTA: blockIdx.x + i * gridDim.x, i = 0 .. my_tiles-1; n is the fast tile index
+  // tiles of this CTA: blockIdx.x + i * grid, i = 0 .. my_tiles-1; n is the fast tile index
   // (the host side guarantees that tile and k-block counts fit 32 bits: 64-bit loop counters and a
   // 64-bit division per k-block cost more instructions than the conversion itself)
-  const int my_tiles = (int)((total_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);
+  const int my_tiles = (int)((total_tiles - blockIdx.x + grid - 1) / grid);
   const int total_it = my_tiles * nkb;   // k-blocks this CTA walks, across all its tiles
 
   if (threadIdx.x == 0) {
@@ -256,16 +269,16 @@ split_sign_gemm_tc(const __grid_constant__ CUtensorMap tm_lo, const __grid_const
       uint32_t bits = 0;
       for (int k = 0; k < 32; ++k) {
         const int ti = w * 32 + k;
-        if (ti < my_tiles && tile_live_slow((int)blockIdx.x + ti * (int)gridDim.x)) bits |= 1u << k;
+        if (ti < my_tiles && tile_live_slow((int)blockIdx.x + ti * grid)) bits |= 1u << k;
       }
       live_bits[w] = bits;
     }
   }
-  // ti: index among this CTA's tiles (tile = blockIdx.x + ti * gridDim.x)
+  // ti: index among this CTA's tiles (tile = blockIdx.x + ti * grid)
   auto tile_live = [&](int ti) -> bool {
     if (!use_live) return true;
     if (live_map) return (live_bits[ti >> 5] >> (ti & 31)) & 1u;
-    return tile_live_slow((int)blockIdx.x + ti * (int)gridDim.x);
+    return tile_live_slow((int)blockIdx.x + ti * grid);
   };
 
   float* const ln_smem = reinterpret_cast<float*>(base_ptr + SharedLayout::bars() + 256 + kLiveWords * 4);
@@ -329,7 +342,7 @@ split_sign_gemm_tc(const __grid_constant__ CUtensorMap tm_lo, const __grid_const
     int it = 0;
     bool ok = true;
     for (int ti = 0; ti < my_tiles && ok; ++ti) {
-      const int tile = blockIdx.x + ti * gridDim.x;
+      const int tile = blockIdx.x + ti * grid;
       if (!tile_live(ti)) continue;
       const bool bseg = tile >= main_tiles;            // a tile of the bias rows
       const int stile = bseg ? tile - main_tiles : tile;
@@ -426,7 +439,7 @@ split_sign_gemm_tc(const __grid_constant__ CUtensorMap tm_lo, const __grid_const
     bool staging_zero = false;   // the staging buffer holds zeros (left there by a tile of a zero row block)
     int le = 0;                  // tiles read out of tensor memory so far (the issuers count the same tiles)
     for (int e = 0; e < my_tiles && ok; ++e) {
-      const int etile = blockIdx.x + e * gridDim.x;
+      const int etile = blockIdx.x + e * grid;
       const bool elive = tile_live(e);
       const bool bseg = etile >= main_tiles;           // a tile of the bias rows: maps and bias of its own, plain store, no norms
       const int stile = bseg ? etile - main_tiles : etile;
@@ -695,7 +708,7 @@ split_sign_gemm_tc(const __grid_constant__ CUtensorMap tm_lo, const __grid_const
       }
       if (kCoef) {
         while (c_kb >= nkb) { c_kb -= nkb; ++c_ti; }
-        const int tile = blockIdx.x + c_ti * gridDim.x;
+        const int tile = blockIdx.x + c_ti * grid;
         if (tile >= main_tiles) {
           // bias rows carry no slopes (the relaxed bias terms are given as they are): a factor of one is exact
 #pragma unroll
@@ -915,7 +928,8 @@ bool tc_gemm_supported(const float* a_lo, const float* a_up, const float* W, con
 int launch_split_sign_tc(const float* a_lo, const float* a_up, const float* W, const float* bias, float* c_lo,
                          float* c_up, int64_t M, int N, int K, cudaStream_t st, int split_rows, int split_d,
                          const float* coef_l, const float* coef_u, int coef_di, float* norm_lo, float* norm_up,
-                         int norm_p, const float* res_lo, const float* res_up, const TcBiasRows* br, const TcLnArgs* ln) {
+                         int norm_p, const float* res_lo, const float* res_up, const TcBiasRows* br, const TcLnArgs* ln,
+                         const SmallProduct* few, bool* few_done) {
   // Bias rows in the same grid (br != nullptr): they must take the same instantiation as the weight rows (zero
   // radius or not, residual or not); the caller checks tc_bias_rows_mergeable first.
   if (br != nullptr && ((br->res_lo != nullptr) != (res_lo != nullptr) || (br->res_lo != nullptr) != (br->res_up != nullptr) ||
@@ -988,7 +1002,20 @@ int launch_split_sign_tc(const float* a_lo, const float* a_up, const float* W, c
   FB_CUDA_OK(attr_err);
   // persistent: one CTA per SM (tensor memory and shared memory allow exactly one)
   const int64_t sms = device_info().sms;
-  const unsigned grid = (unsigned)(total_tiles < sms ? total_tiles : sms);
+  unsigned grid = (unsigned)(total_tiles < sms ? total_tiles : sms);
+  // A product of few rows (the bias part) goes along in blocks of its own where the tiles leave an SM for each of them: a launch of
+  // 4 us (K = 128) to 9 us (K = 512) less.
+  SmallProduct small = {};
+  int n_small = 0;
+  if (few != nullptr && norm_lo == nullptr && res_lo == nullptr) {
+    const int64_t blocks = ceil_div(few->M, kSmRows) * ceil_div(few->N, kSmCols);
+    if (total_tiles + blocks <= sms) {
+      small = *few;
+      n_small = (int)blocks;
+      grid += (unsigned)blocks;
+      *few_done = true;
+    }
+  }
   int* status = t_status_sink;
   const uint32_t tries = g_wait_tries;
   const int skip = g_skip_it;
@@ -1004,7 +1031,7 @@ int launch_split_sign_tc(const float* a_lo, const float* a_up, const float* W, c
     ln_args.w_raw = W;
   }
   const int64_t Mb = br != nullptr ? br->M : 0;
-#define FB_TC_TAIL ln_args, Mb
+#define FB_TC_TAIL ln_args, Mb, small, n_small
 #define FB_TC_ARGS tm_lo, tm_up, tm_w, tm_out_lo, tm_out_up, tm_res_lo, tm_res_up, tm_b_lo, tm_b_up, tm_bout_lo, tm_bout_up, tm_bres_lo, \
                    tm_bres_up, bias, bias_b, (int)main_tiles, same_b, M, N, K, gn, total_tiles, split_rows, split_d
   if (ln != nullptr && coef_l != nullptr)
@@ -1161,7 +1188,7 @@ extern "C" int fb_tc_selftest_timeout(const float* x_lw, const float* x_uw, cons
   int* const saved_sink = fb::t_status_sink;
   fb::t_status_sink = status;
   rc = fb::launch_split_sign_tc(x_lw, x_uw, W, nullptr, y_lw, y_uw, M, N, K, (cudaStream_t)stream, 0, 0, nullptr, nullptr, 1,
-                                nullptr, nullptr, 0, nullptr, nullptr, nullptr, nullptr);
+                                nullptr, nullptr, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
   fb::t_status_sink = saved_sink;
   fb::g_wait_tries = fb::kMaxTries;
   fb::g_skip_it = -1;
