@@ -238,6 +238,111 @@ col_relax_native(int op, const float* __restrict__ lw, const float* __restrict__
                             s_l, s_u, s_coef);
 }
 
+// The same for tiles that fit into the block's registers: a thread holds its N rows of four columns of either line, so that the
+// tile is read once, with all its loads in flight at once, and written from registers.  Di <= 32 * N, and word blocks of a
+// multiple of 32 rows (a thread's row i then lies in word 32 i / blk for every thread).
+// Bound by HBM.  relu on [8, 64, 64, 512]: 63.3 us staged in shared memory, 54.7 us held (N = 2, 64 registers).  With N = 4 (98
+// registers, Di 128) and N = 8 (119, Di 256) too few blocks are left to hide the column's scalar chain: tanh on
+// [8, 64, 128, 256] 100 us against 73 us staged, on [8, 64, 256, 256] 136 us against 137 us with the second pass through L2.
+template <int N>
+__global__ void __launch_bounds__(kThreads)
+col_relax_held(int op, const float* __restrict__ lw, const float* __restrict__ uw, const float* __restrict__ lb,
+               const float* __restrict__ ub, float* __restrict__ o_lw, float* __restrict__ o_uw, float* __restrict__ o_lb,
+               float* __restrict__ o_ub, int Di, int Do, int ntiles, int words, int p, float eps, int* __restrict__ violation) {
+  pdl_sync();
+  __shared__ float s_red[2 * 8 * kCW], s_coef[4 * kCW];
+  const int64_t row = blockIdx.x / ntiles;
+  const int c0 = (int)(blockIdx.x % ntiles) * kCW;
+  const int tid = threadIdx.x, cvl = tid & 7, rg = tid >> 3, warp = tid >> 5, lane = tid & 31;
+  const int col = c0 + cvl * 4;
+  const bool col_ok = col < Do;   // (Do is a multiple of four)
+  const size_t base = (size_t)row * Di * Do + col;
+  float4 vl[N], vu[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int r = rg + 32 * i;
+    vl[i] = vu[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (col_ok && r < Di) {
+      vl[i] = __ldg(reinterpret_cast<const float4*>(lw + base + (size_t)r * Do));
+      vu[i] = __ldg(reinterpret_cast<const float4*>(uw + base + (size_t)r * Do));
+    }
+  }
+  const bool mine = tid < kCW && c0 + tid < Do;
+  float lbv = 0.f, ubv = 0.f;
+  if (mine) {
+    lbv = lb[(size_t)row * Do + c0 + tid];
+    ubv = ub[(size_t)row * Do + c0 + tid];
+  }
+  float l = lbv, u = ubv;
+  const int blk = Di / words;
+  for (int w = 0; w < words; ++w) {
+    float al[4] = {0.f, 0.f, 0.f, 0.f}, au[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (32 * i >= w * blk && 32 * i < (w + 1) * blk) {   // (a zero beyond Di leaves every norm as it is)
+        al[0] = norm_accum(p, al[0], vl[i].x); al[1] = norm_accum(p, al[1], vl[i].y);
+        al[2] = norm_accum(p, al[2], vl[i].z); al[3] = norm_accum(p, al[3], vl[i].w);
+        au[0] = norm_accum(p, au[0], vu[i].x); au[1] = norm_accum(p, au[1], vu[i].y);
+        au[2] = norm_accum(p, au[2], vu[i].z); au[3] = norm_accum(p, au[3], vu[i].w);
+      }
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+      for (int s = 8; s < 32; s <<= 1) {
+        al[e] = norm_combine(p, al[e], __shfl_xor_sync(0xffffffffu, al[e], s));
+        au[e] = norm_combine(p, au[e], __shfl_xor_sync(0xffffffffu, au[e], s));
+      }
+    if (w > 0) __syncthreads();
+    if (lane < 8) {
+      *reinterpret_cast<float4*>(s_red + warp * kCW + lane * 4) = make_float4(al[0], al[1], al[2], al[3]);
+      *reinterpret_cast<float4*>(s_red + (8 + warp) * kCW + lane * 4) = make_float4(au[0], au[1], au[2], au[3]);
+    }
+    __syncthreads();
+    if (tid < kCW) {
+      float sl = s_red[tid], su = s_red[8 * kCW + tid];
+#pragma unroll
+      for (int k = 1; k < 8; ++k) {
+        sl = norm_combine(p, sl, s_red[k * kCW + tid]);
+        su = norm_combine(p, su, s_red[(8 + k) * kCW + tid]);
+      }
+      l = fadd(l, fmul(-eps, norm_finish(p, sl)));
+      u = fadd(u, fmul(eps, norm_finish(p, su)));
+    }
+  }
+  if (tid < kCW) {
+    ColCoef c = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (mine) {
+      bool bad = false;
+      c = relax_column(op, l, u, lbv, ubv, bad);
+      if (bad && violation != nullptr) *violation = 1;
+      o_lb[(size_t)row * Do + c0 + tid] = c.nlb;
+      o_ub[(size_t)row * Do + c0 + tid] = c.nub;
+    }
+    s_coef[0 * kCW + tid] = c.c_ll;
+    s_coef[1 * kCW + tid] = c.c_lu;
+    s_coef[2 * kCW + tid] = c.c_ul;
+    s_coef[3 * kCW + tid] = c.c_uu;
+  }
+  __syncthreads();
+  if (!col_ok) return;
+  const float4 ll = *reinterpret_cast<const float4*>(s_coef + cvl * 4), lu = *reinterpret_cast<const float4*>(s_coef + kCW + cvl * 4),
+               ul = *reinterpret_cast<const float4*>(s_coef + 2 * kCW + cvl * 4),
+               uu = *reinterpret_cast<const float4*>(s_coef + 3 * kCW + cvl * 4);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int r = rg + 32 * i;
+    if (r >= Di) break;
+    const float4 a = vl[i], b = vu[i];
+    float4 x, y;
+    x.x = fmaf(ll.x, a.x, fmul(lu.x, b.x)); y.x = fmaf(uu.x, b.x, fmul(ul.x, a.x));
+    x.y = fmaf(ll.y, a.y, fmul(lu.y, b.y)); y.y = fmaf(uu.y, b.y, fmul(ul.y, a.y));
+    x.z = fmaf(ll.z, a.z, fmul(lu.z, b.z)); y.z = fmaf(uu.z, b.z, fmul(ul.z, a.z));
+    x.w = fmaf(ll.w, a.w, fmul(lu.w, b.w)); y.w = fmaf(uu.w, b.w, fmul(ul.w, a.w));
+    *reinterpret_cast<float4*>(o_lw + base + (size_t)r * Do) = x;
+    *reinterpret_cast<float4*>(o_uw + base + (size_t)r * Do) = y;
+  }
+}
+
 // McCormick product of two bounded operands: both are concretised in the same block, the four
 // input tiles stay in shared memory (or are re-read) for the combination pass.
 template <int VEC, bool STAGED>
@@ -709,6 +814,12 @@ int launch_relax(int op, const float* lw, const float* uw, const float* lb, cons
   if (blocks > 0x7fffffff) return FB_ERR_SHAPE;
   const bool vec = Do % 4 == 0 && aligned16(lw) && aligned16(uw) &&
                    (op >= OP_COEF_ONLY || (aligned16(o_lw) && aligned16(o_uw)));
+  // a tile that fits into registers without costing occupancy
+  if (vec && op < OP_COEF_ONLY && Di <= 64 && (words == 1 || (Di / words) % 32 == 0)) {
+    launch_k(col_relax_held<2>, (unsigned)blocks, kThreads, 0, st, op, lw, uw, lb, ub, o_lw, o_uw, o_lb, o_ub, Di, Do, ntiles, words, p, eps, violation);
+    FB_LAUNCH_OK();
+    return FB_OK;
+  }
   // Keep the tile in shared memory when a few blocks per SM still fit; the coefficient-only mode has no second pass and never
   // stages.
   const size_t staged_bytes = relax_smem_bytes(Di, true, 2);

@@ -1129,3 +1129,16 @@ def test_conv_of_many_images_tiles(N, C, H, W, Co, kh, kw, s, p):
     r = ops.conv2d((lw.to(DEV), uw.to(DEV), lb.to(DEV), ub.to(DEV)), wt.to(DEV), bias.to(DEV), s, p)
     for got, k in zip(r, ("lw", "uw", "lb", "ub")):
         helpers.assert_arbitrated(got, getattr(o, k), getattr(o64, k), "conv %s %s" % ((N, C, H, W, Co, kh, kw, s, p), k))
+
+
+@pytest.mark.parametrize("Di,Do,words", [(32, 4, 1), (33, 36, 1), (64, 40, 2), (64, 64, 1), (5, 8, 1), (60, 32, 1)])
+@pytest.mark.parametrize("p", [1.0, 2.0, float("inf")])
+def test_relax_of_short_columns_held_in_registers(Di, Do, words, p):
+    from faith_b200 import ops
+    from faith_b200._lib import FB_TANH
+    t = cases.rand_bounds(423, 2, 3, Di, Do, -0.7, 0.2)
+    o = O.OBounds(p, 0.02, *t, words=words).tanh()
+    lw, lb, uw, ub = [v.to(DEV) for v in t]
+    z = ops.relax(FB_TANH, lw, uw, lb, ub, p, 0.02, words)
+    for got, name in zip(z, ("lw", "uw", "lb", "ub")):
+        helpers.assert_close(got, getattr(o, name), name)
