@@ -175,7 +175,8 @@ __device__ __noinline__ void few_rows(const SmallProduct& q, int bx, int by, flo
 // status: device word of the caller (may be null); bit 2 is set when a bounded wait of this launch expired.
 // wait_tries: bound of every mbarrier wait in tries of ~20 us.  skip_it >= 0 makes the producer of CTA 0 leave
 // out the loads of that k-block: the self-test of the give-up path (fb_tc_selftest_timeout), never set otherwise.
-template <bool kCoef, bool kNorm, bool kResid, bool kPoint, bool kLN>
+// kFew: blocks of the product of few rows ride along (an instantiation of its own: the others keep their registers).
+template <bool kCoef, bool kNorm, bool kResid, bool kPoint, bool kLN, bool kFew>
 __global__ void __launch_bounds__(kThreads, 1)
 split_sign_gemm_tc(const __grid_constant__ CUtensorMap tm_lo, const __grid_constant__ CUtensorMap tm_up,
                    const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_out_lo,
@@ -193,8 +194,8 @@ split_sign_gemm_tc(const __grid_constant__ CUtensorMap tm_lo, const __grid_const
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
-  const int grid = (int)gridDim.x - n_small;   // CTAs of the tiles; the others take a block of the product of few rows each
-  if (!kNorm && !kResid && (int)blockIdx.x >= grid) {
+  const int grid = kFew ? (int)gridDim.x - n_small : (int)gridDim.x;   // CTAs of the tiles; the others take a block of few rows each
+  if (kFew && (int)blockIdx.x >= grid) {
     pdl_sync();
     const int e = (int)blockIdx.x - grid, gx = (int)((small.M + kSmRows - 1) / kSmRows);
     if (threadIdx.x < kSmThreads) few_rows(small, e % gx, e / gx, reinterpret_cast<float*>(base_ptr));
@@ -982,22 +983,26 @@ int launch_split_sign_tc(const float* a_lo, const float* a_up, const float* W, c
   cudaError_t attr_err = cudaSuccess;
   std::call_once(attr_once[dev & 63], [&]() {
     const int bytes = (int)kSmemBytes;
-    attr_err = cudaFuncSetAttribute(split_sign_gemm_tc<false, false, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    attr_err = cudaFuncSetAttribute(split_sign_gemm_tc<false, false, false, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (attr_err == cudaSuccess)
-      attr_err = cudaFuncSetAttribute(split_sign_gemm_tc<true, false, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+      attr_err = cudaFuncSetAttribute(split_sign_gemm_tc<true, false, false, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (attr_err == cudaSuccess)
-      attr_err = cudaFuncSetAttribute(split_sign_gemm_tc<false, true, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+      attr_err = cudaFuncSetAttribute(split_sign_gemm_tc<false, true, false, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (attr_err == cudaSuccess)
-      attr_err = cudaFuncSetAttribute(split_sign_gemm_tc<false, false, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+      attr_err = cudaFuncSetAttribute(split_sign_gemm_tc<false, false, true, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (attr_err == cudaSuccess)
-      attr_err = cudaFuncSetAttribute(split_sign_gemm_tc<true, false, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+      attr_err = cudaFuncSetAttribute(split_sign_gemm_tc<true, false, true, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (attr_err == cudaSuccess)
-      attr_err = cudaFuncSetAttribute(split_sign_gemm_tc<false, true, false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+      attr_err = cudaFuncSetAttribute(split_sign_gemm_tc<false, true, false, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (attr_err == cudaSuccess)
+      attr_err = cudaFuncSetAttribute(split_sign_gemm_tc<false, false, false, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (attr_err == cudaSuccess)
+      attr_err = cudaFuncSetAttribute(split_sign_gemm_tc<true, false, false, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     const int ln_bytes = (int)(kSmemBytes + kLnSmemBytes);
     if (attr_err == cudaSuccess)
-      attr_err = cudaFuncSetAttribute(split_sign_gemm_tc<false, false, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ln_bytes);
+      attr_err = cudaFuncSetAttribute(split_sign_gemm_tc<false, false, true, false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, ln_bytes);
     if (attr_err == cudaSuccess)
-      attr_err = cudaFuncSetAttribute(split_sign_gemm_tc<true, false, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ln_bytes);
+      attr_err = cudaFuncSetAttribute(split_sign_gemm_tc<true, false, true, false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, ln_bytes);
   });
   FB_CUDA_OK(attr_err);
   // persistent: one CTA per SM (tensor memory and shared memory allow exactly one)
@@ -1035,21 +1040,21 @@ int launch_split_sign_tc(const float* a_lo, const float* a_up, const float* W, c
 #define FB_TC_ARGS tm_lo, tm_up, tm_w, tm_out_lo, tm_out_up, tm_res_lo, tm_res_up, tm_b_lo, tm_b_up, tm_bout_lo, tm_bout_up, tm_bres_lo, \
                    tm_bres_up, bias, bias_b, (int)main_tiles, same_b, M, N, K, gn, total_tiles, split_rows, split_d
   if (ln != nullptr && coef_l != nullptr)
-    fb::launch_k(split_sign_gemm_tc<true, false, true, false, true>, grid, kThreads, kSmemBytes + kLnSmemBytes, st, FB_TC_ARGS, coef_l, coef_u, coef_di, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_k(split_sign_gemm_tc<true, false, true, false, true, false>, grid, kThreads, kSmemBytes + kLnSmemBytes, st, FB_TC_ARGS, coef_l, coef_u, coef_di, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
   else if (ln != nullptr)
-    fb::launch_k(split_sign_gemm_tc<false, false, true, false, true>, grid, kThreads, kSmemBytes + kLnSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_k(split_sign_gemm_tc<false, false, true, false, true, false>, grid, kThreads, kSmemBytes + kLnSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
   else if (coef_l != nullptr && res_lo != nullptr)
-    fb::launch_k(split_sign_gemm_tc<true, false, true, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, coef_l, coef_u, coef_di, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_k(split_sign_gemm_tc<true, false, true, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, coef_l, coef_u, coef_di, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
   else if (coef_l != nullptr)
-    fb::launch_k(split_sign_gemm_tc<true, false, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, coef_l, coef_u, coef_di, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_k(n_small > 0 ? split_sign_gemm_tc<true, false, false, false, false, true> : split_sign_gemm_tc<true, false, false, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, coef_l, coef_u, coef_di, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
   else if (norm_lo != nullptr && a_lo == a_up)   // one tensor as both lines: zero radius
-    fb::launch_k(split_sign_gemm_tc<false, true, false, true, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, norm_lo, norm_up, norm_p, status, tries, skip, live, c_lo == c_up ? 1 : 0, FB_TC_TAIL);
+    fb::launch_k(split_sign_gemm_tc<false, true, false, true, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, norm_lo, norm_up, norm_p, status, tries, skip, live, c_lo == c_up ? 1 : 0, FB_TC_TAIL);
   else if (norm_lo != nullptr)
-    fb::launch_k(split_sign_gemm_tc<false, true, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, norm_lo, norm_up, norm_p, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_k(split_sign_gemm_tc<false, true, false, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, norm_lo, norm_up, norm_p, status, tries, skip, no_live, 0, FB_TC_TAIL);
   else if (res_lo != nullptr)
-    fb::launch_k(split_sign_gemm_tc<false, false, true, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_k(split_sign_gemm_tc<false, false, true, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
   else
-    fb::launch_k(split_sign_gemm_tc<false, false, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_k(n_small > 0 ? split_sign_gemm_tc<false, false, false, false, false, true> : split_sign_gemm_tc<false, false, false, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
 #undef FB_TC_ARGS
 #undef FB_TC_TAIL
   FB_LAUNCH_OK();
