@@ -184,6 +184,38 @@ input_bounds_norm128_kernel(const float* __restrict__ emb, const float* __restri
   }
 }
 
+// The rows of the first token of every sentence, both lines and both bias terms in one launch (as four strided copies they took
+// 1.5 us each and as much again between them).  VEC: floats per access.
+template <int VEC>
+__global__ void __launch_bounds__(256)
+first_token_kernel(const BoundSet x, const BoundSet y, int64_t n_w, int64_t n_b, int L, int64_t total) {
+  pdl_sync();
+  // per sentence: lw, uw (n_w floats each), lb, ub (n_b floats each)
+  const int64_t per = 2 * (n_w + n_b) / VEC;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t s = t / per;
+    int64_t e = (t - s * per) * VEC;
+    const bool w = e < 2 * n_w;
+    if (!w) e -= 2 * n_w;
+    const int64_t n = w ? n_w : n_b;
+    const bool up = e >= n;
+    if (up) e -= n;
+    const float* src = (w ? (up ? x.uw : x.lw) : (up ? x.ub : x.lb)) + s * L * n + e;
+    float* dst = (w ? (up ? y.uw : y.lw) : (up ? y.ub : y.lb)) + s * n + e;
+    if (VEC == 4) *reinterpret_cast<float4*>(dst) = __ldg(reinterpret_cast<const float4*>(src));
+    else *dst = __ldg(src);
+  }
+}
+
+int copy_first_tokens(const BoundSet& x, const BoundSet& y, int S, int L, int Di, int D, cudaStream_t st) {
+  const int64_t n_w = (int64_t)Di * D, n_b = D;
+  const bool vec = D % 4 == 0;   // (the arena's buffers are 256-byte aligned)
+  const int64_t total = S * 2 * (n_w + n_b) / (vec ? 4 : 1), cap = (int64_t)device_info().sms * 16;
+  launch_k(vec ? first_token_kernel<4> : first_token_kernel<1>, (unsigned)std::min(ceil_div(total, 256), cap), 256, 0, st, x, y, n_w, n_b, L, total);
+  FB_LAUNCH_OK();
+  return FB_OK;
+}
+
 // Mean over the positions: z[s, r] = (sum_l x[s, l, r]) / L for the inner[-sized] slab r of every sentence (r runs over
 // Di * D weight entries resp. D bias entries); lanes along r, the L terms added in order.
 __global__ void __launch_bounds__(256)
@@ -349,12 +381,7 @@ static int encoder_forward_impl(const fb_encoder* enc, const float* emb, int S, 
       if (fits) {
         const BoundSet Kh = slot[Dd], Vd = slot[C];
         // the first token's rows of the layer input
-        FB_CUDA_OK(cudaMemcpy2DAsync(Xq.lw, (size_t)Di * D * 4, X.lw, (size_t)L * Di * D * 4, (size_t)Di * D * 4, S,
-                                     cudaMemcpyDeviceToDevice, st));
-        FB_CUDA_OK(cudaMemcpy2DAsync(Xq.uw, (size_t)Di * D * 4, X.uw, (size_t)L * Di * D * 4, (size_t)Di * D * 4, S,
-                                     cudaMemcpyDeviceToDevice, st));
-        FB_CUDA_OK(cudaMemcpy2DAsync(Xq.lb, (size_t)D * 4, X.lb, (size_t)L * D * 4, (size_t)D * 4, S, cudaMemcpyDeviceToDevice, st));
-        FB_CUDA_OK(cudaMemcpy2DAsync(Xq.ub, (size_t)D * 4, X.ub, (size_t)L * D * 4, (size_t)D * 4, S, cudaMemcpyDeviceToDevice, st));
+        FB_TRY(copy_first_tokens(X, Xq, S, L, Di, D, st));
         // query of token 0 [S*H, 1, Di, d], keys of every token [S*H, L, Di, d] (with their ranges from the GEMM's
         // epilogue where the shapes allow it), scores [S*H, 1, Di, L]
         FB_TRY(fb_matmul_heads_f32(Xq.lw, Xq.uw, Xq.lb, Xq.ub, ly.q_w, ly.q_b, Qh.lw, Qh.uw, Qh.lb, Qh.ub, S, Di, D, D, 1, H, stream));
@@ -630,15 +657,8 @@ static int encoder_forward_impl(const fb_encoder* enc, const float* emb, int S, 
       fb::launch_k(mean_pool_kernel, (unsigned)std::min(ceil_div(nb, 256), cap), 256, 0, st, X.lb, X.ub, T1.lb, T1.ub, nb, (int64_t)D, L);
       FB_LAUNCH_OK();
     } else {
-    // first token of every sentence: [S, 1, Di, D]
-    FB_CUDA_OK(cudaMemcpy2DAsync(T1.lw, (size_t)Di * D * 4, X.lw, (size_t)L * Di * D * 4, (size_t)Di * D * 4, S,
-                                 cudaMemcpyDeviceToDevice, st));
-    FB_CUDA_OK(cudaMemcpy2DAsync(T1.uw, (size_t)Di * D * 4, X.uw, (size_t)L * Di * D * 4, (size_t)Di * D * 4, S,
-                                 cudaMemcpyDeviceToDevice, st));
-    FB_CUDA_OK(cudaMemcpy2DAsync(T1.lb, (size_t)D * 4, X.lb, (size_t)L * D * 4, (size_t)D * 4, S,
-                                 cudaMemcpyDeviceToDevice, st));
-    FB_CUDA_OK(cudaMemcpy2DAsync(T1.ub, (size_t)D * 4, X.ub, (size_t)L * D * 4, (size_t)D * 4, S,
-                                 cudaMemcpyDeviceToDevice, st));
+      // first token of every sentence: [S, 1, Di, D]
+      FB_TRY(copy_first_tokens(X, T1, S, L, Di, D, st));
     }
     FB_TRY(dense(T1, enc->pool_w, enc->pool_b, T2, S, Di, D, D, stream));
     FB_TRY(relax(FB_TANH, T2, T1, S, Di, D, words, p, eps, nullptr, stream));
