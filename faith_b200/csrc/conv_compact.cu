@@ -88,7 +88,7 @@ cw_identity_rows_kernel(const float* __restrict__ Wt, const float* __restrict__ 
 // The input comes from compact rows, or (W1 != nullptr) is the first convolution and its relaxation, evaluated from the filter
 // while it is staged: those rows are never written.  The first blocks compute the bias image.
 // Bound by latency and shared-memory reads: 3072 rows, 16 -> 32 channels, 3 x 3 stride 2 took 35 us with a thread per output of
-// one row, whose tap bounds differ from lane to lane, and 8 us before it to write its input.
+// one row, whose tap bounds differ from lane to lane, and 8 us before it to write its input; 20 us now for both.
 constexpr int kCwR = 8;             // rows per thread
 constexpr int kCwConvThreads = 512;   // at most; the items of a block in one round where that is possible
 constexpr int kCwMaxRows = 32;      // rows per block at most: one per lane
@@ -354,7 +354,7 @@ cw_conv_kernel(const __grid_constant__ CwConvArgs q) {
 // op < 0: the unfinished accumulations go to part_l / part_u.  Otherwise the relaxation's coefficients follow at once (no
 // exchange between ranks in between): out_lb / out_ub receive the relaxed bias terms, coef as cw_relax_columns_kernel writes it.
 // 3072 rows of 3 x 3 x 32 windows, 8192 columns: 13 us with a warp per column of channel-major rows, whose 32 lanes touch 32
-// sectors per load.
+// sectors per load; 5 us now, coefficients included.
 constexpr int kCwNormWarps = 16, kCwNormLoads = 4;
 
 __device__ __forceinline__ void cw_relax_column(int op, float lbv, float ubv, float nl, float nu, int p, float eps, int64_t dense,
@@ -474,7 +474,7 @@ cw_rescale_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw
 // Where this is the last layer (part != nullptr), the rows are not written: what is left of them is their dual norm, one partial
 // accumulation per block, tile and output.  The first bias_blocks blocks compute the bias part, an output each.
 // Bound by L2 reads: with W^T in global memory every row read its own copy of the weights (20 us and 2 us for the transpose at
-// 3072 rows, 288 elements, 10 outputs, and 9 us to write the rescaled rows first).
+// 3072 rows, 288 elements, 10 outputs, and 9 us to write the rescaled rows first; 12 us now).
 constexpr int kCwPx = 8, kCwLinWarps = 24, kCwLinThreads = 32 * kCwLinWarps;   // 24: the rows of 8 pixels of 3 channels
 
 struct CwLinearArgs {
