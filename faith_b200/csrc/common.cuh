@@ -39,11 +39,11 @@ void count_launches(int n);
 
 // A launch whose blocks may become resident while the launch before on the stream still drains (programmatic dependent launch):
 // the passes over one sentence are chains of kernels of 3 to 10 us with 2 us between them, most of it launch latency and
-// prologues (barriers, tensor memory, tensor maps).  The kernel must call pdl_sync() first thing.  Grids of many waves keep the
-// plain launch: the gap before them is nothing beside them, and the hand-over cost the 4096 blocks of a relaxation 2 % of
-// 135 us.
+// prologues (barriers, tensor memory, tensor maps).  The kernel must call pdl_sync() first thing.  Work of many waves keeps the
+// plain launch: the gap before it is nothing beside it, and the hand-over cost the 4096 blocks of a relaxation 2 % of 135 us.
+// tiles: what a persistent kernel walks, the number of blocks for any other.
 template <typename... P, typename... A>
-inline void launch_k(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+inline void launch_tiles(int64_t tiles, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -53,8 +53,12 @@ inline void launch_k(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cud
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = &attr;
-  cfg.numAttrs = (int64_t)grid.x * grid.y * grid.z <= 4 * (int64_t)device_info().sms ? 1 : 0;
+  cfg.numAttrs = tiles <= 4 * (int64_t)device_info().sms ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);   // (errors are picked up by FB_LAUNCH_OK)
+}
+template <typename... P, typename... A>
+inline void launch_k(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  launch_tiles((int64_t)grid.x * grid.y * grid.z, kern, grid, block, smem, st, args...);
 }
 
 // Hint for the tensor-core GEMM (thread-local, set by the encoder driver around the projections of the first layer):

@@ -510,7 +510,7 @@ int launch_dot_weight_tc(const float* x_lw, const float* x_uw, const float* y_lw
   const int64_t n_bias = (int64_t)B * bias.n_it * bias.n_jt;
   bias_done = total + n_bias <= sms;
   const int extra = bias_done ? (int)n_bias : 0;
-  launch_k(dot_weight_tc, (unsigned)((total < sms ? total : sms) + extra), kDtThreads, kDtSmemBytes, st, tm_xl, tm_xu, tm_yl, tm_yu, tm_lx, tm_ly,
+  launch_tiles(total, dot_weight_tc, (unsigned)((total < sms ? total : sms) + extra), kDtThreads, kDtSmemBytes, st, tm_xl, tm_xu, tm_yl, tm_yu, tm_lx, tm_ly,
            tm_uy, tm_zl, tm_zu, Lx, Ly, n_ib, n_mb, total, out_scale, heads, y_kmajor, tc_status_sink(), bias, extra);
   FB_LAUNCH_OK();
   return FB_OK;

@@ -511,7 +511,7 @@ template <bool kTmaIn, bool kVecOut, bool kMulti>
 int launch_variant(const CUtensorMap (&tm)[4], const DotArgs& a, cudaStream_t st, const DotBias& bias, int n_bias) {
   const int sms = device_info().sms;
   if (int rc = ensure_dynamic_smem(dot_weight_tc_any<kTmaIn, kVecOut, kMulti>, kDaSmemBytes)) return rc;
-  fb::launch_k(dot_weight_tc_any<kTmaIn, kVecOut, kMulti>, (unsigned)((a.total_tiles < sms ? a.total_tiles : sms) + n_bias), kDaThreads, kDaSmemBytes,
+  fb::launch_tiles(a.total_tiles, dot_weight_tc_any<kTmaIn, kVecOut, kMulti>, (unsigned)((a.total_tiles < sms ? a.total_tiles : sms) + n_bias), kDaThreads, kDaSmemBytes,
                st, tm[0], tm[1], tm[2], tm[3], a, tc_status_sink(), bias, n_bias);
   FB_LAUNCH_OK();
   return FB_OK;

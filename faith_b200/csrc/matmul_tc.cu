@@ -1040,21 +1040,21 @@ int launch_split_sign_tc(const float* a_lo, const float* a_up, const float* W, c
 #define FB_TC_ARGS tm_lo, tm_up, tm_w, tm_out_lo, tm_out_up, tm_res_lo, tm_res_up, tm_b_lo, tm_b_up, tm_bout_lo, tm_bout_up, tm_bres_lo, \
                    tm_bres_up, bias, bias_b, (int)main_tiles, same_b, M, N, K, gn, total_tiles, split_rows, split_d
   if (ln != nullptr && coef_l != nullptr)
-    fb::launch_k(split_sign_gemm_tc<true, false, true, false, true, false>, grid, kThreads, kSmemBytes + kLnSmemBytes, st, FB_TC_ARGS, coef_l, coef_u, coef_di, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_tiles(total_tiles, split_sign_gemm_tc<true, false, true, false, true, false>, grid, kThreads, kSmemBytes + kLnSmemBytes, st, FB_TC_ARGS, coef_l, coef_u, coef_di, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
   else if (ln != nullptr)
-    fb::launch_k(split_sign_gemm_tc<false, false, true, false, true, false>, grid, kThreads, kSmemBytes + kLnSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_tiles(total_tiles, split_sign_gemm_tc<false, false, true, false, true, false>, grid, kThreads, kSmemBytes + kLnSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
   else if (coef_l != nullptr && res_lo != nullptr)
-    fb::launch_k(split_sign_gemm_tc<true, false, true, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, coef_l, coef_u, coef_di, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_tiles(total_tiles, split_sign_gemm_tc<true, false, true, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, coef_l, coef_u, coef_di, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
   else if (coef_l != nullptr)
-    fb::launch_k(n_small > 0 ? split_sign_gemm_tc<true, false, false, false, false, true> : split_sign_gemm_tc<true, false, false, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, coef_l, coef_u, coef_di, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_tiles(total_tiles, n_small > 0 ? split_sign_gemm_tc<true, false, false, false, false, true> : split_sign_gemm_tc<true, false, false, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, coef_l, coef_u, coef_di, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
   else if (norm_lo != nullptr && a_lo == a_up)   // one tensor as both lines: zero radius
-    fb::launch_k(split_sign_gemm_tc<false, true, false, true, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, norm_lo, norm_up, norm_p, status, tries, skip, live, c_lo == c_up ? 1 : 0, FB_TC_TAIL);
+    fb::launch_tiles(total_tiles, split_sign_gemm_tc<false, true, false, true, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, norm_lo, norm_up, norm_p, status, tries, skip, live, c_lo == c_up ? 1 : 0, FB_TC_TAIL);
   else if (norm_lo != nullptr)
-    fb::launch_k(split_sign_gemm_tc<false, true, false, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, norm_lo, norm_up, norm_p, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_tiles(total_tiles, split_sign_gemm_tc<false, true, false, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, norm_lo, norm_up, norm_p, status, tries, skip, no_live, 0, FB_TC_TAIL);
   else if (res_lo != nullptr)
-    fb::launch_k(split_sign_gemm_tc<false, false, true, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_tiles(total_tiles, split_sign_gemm_tc<false, false, true, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
   else
-    fb::launch_k(n_small > 0 ? split_sign_gemm_tc<false, false, false, false, false, true> : split_sign_gemm_tc<false, false, false, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
+    fb::launch_tiles(total_tiles, n_small > 0 ? split_sign_gemm_tc<false, false, false, false, false, true> : split_sign_gemm_tc<false, false, false, false, false, false>, grid, kThreads, kSmemBytes, st, FB_TC_ARGS, nullptr, nullptr, 1, nullptr, nullptr, 0, status, tries, skip, no_live, 0, FB_TC_TAIL);
 #undef FB_TC_ARGS
 #undef FB_TC_TAIL
   FB_LAUNCH_OK();

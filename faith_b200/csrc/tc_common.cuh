@@ -121,10 +121,6 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
       ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar)
       : "memory");
 }
-__device__ __forceinline__ void tma_store_5d(const CUtensorMap* map, int x, int y, int z, int w, int v, uint32_t src) {
-  asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4, %5}], [%6];"
-               ::"l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(v), "r"(src) : "memory");
-}
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // waits until the bulk stores committed so far have finished READING shared memory
 __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
