@@ -1142,3 +1142,17 @@ def test_relax_of_short_columns_held_in_registers(Di, Do, words, p):
     z = ops.relax(FB_TANH, lw, uw, lb, ub, p, 0.02, words)
     for got, name in zip(z, ("lw", "uw", "lb", "ub")):
         helpers.assert_close(got, getattr(o, name), name)
+
+
+@pytest.mark.parametrize("L,Di,Do,p,words", [(80, 24, 40, 1.0, 2), (80, 256, 128, 2.0, 2), (37, 48, 32, float("inf"), 3),
+                                             (18, 64, 20, 2.0, 1), (2, 64, 2100, float("inf"), 1)])
+def test_standard_layer_norm_by_number_of_rows(L, Di, Do, p, words):
+    """A block per row (many rows) and clusters of 2 to 8 blocks per row, tile in shared memory or not."""
+    test_standard_layer_norm_in_one_kernel(L, Di, Do, p, words)
+
+
+@pytest.mark.parametrize("Di,Do,words", [(256, 21, 2), (256, 32, 1), (256, 17, 4)])
+@pytest.mark.parametrize("p", [1.0, 2.0, float("inf")])
+def test_fused_softmax_of_wide_inputs(Di, Do, words, p):
+    """Eight rows of dim_in per thread."""
+    test_fused_softmax_of_any_length(Di, Do, words, p)
