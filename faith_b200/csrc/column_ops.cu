@@ -178,6 +178,42 @@ __device__ __forceinline__ void tile_rescale(const float* __restrict__ gl, const
   }
 }
 
+// The tangent points of tanh for a block's kCW columns by all of its warps, l and u being known to thread c < kCW of column c:
+// one thread per column walked twenty dependent evaluations (a third of the block's lifetime, with seven warps waiting).  The two
+// searches go to different warps, and three warps each evaluate the middle and both middles that can follow, i.e. two steps
+// of ten at a time; the moves and their rounding are those of tanh_point.  tanh on [8, 64, 128, 256]: 79 -> 72 us.  Every thread
+// calls; point[2] is valid in threads < kCW, where `mine`.
+__device__ __forceinline__ void tanh_points(float l, float u, bool mine, float point[2]) {
+  static_assert(kCW == 32 && kThreads == 256 && kTanhSteps % 2 == 0, "a lane per column, a warp per evaluation");
+  __shared__ float s_range[2][kCW];
+  __shared__ float s_point[2][kCW];
+  __shared__ bool s_right[2][2][3][kCW];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid < kCW) { s_range[0][tid] = mine ? l : 0.f; s_range[1][tid] = mine ? u : 0.f; }
+  __syncthreads();
+  const float cl = s_range[0][lane], cu = s_range[1][lane];
+  const bool search = (cl > 0.f) == (cu < 0.f);   // the range crosses zero (as relax_column tells it)
+  const bool upper = warp & 1;
+  const int node = warp >> 1;      // 0: d, 1: what follows a step to the right, 2: to the left, 3: none
+  const float x = upper ? cl : cu, tx = tanhf(x);
+  TanhSearch q = tanh_search(upper, cl, cu);
+#pragma unroll 1
+  for (int t = 0; t < kTanhSteps / 2; ++t) {
+    if (node < 3 && search) {
+      const float d = node == 0 ? q.d : tanh_move(q, node == 1).d;
+      s_right[t & 1][upper][node][lane] = tanh_right_of(upper, d, x, tx);
+    }
+    __syncthreads();
+    if (search) {
+      const bool first = s_right[t & 1][upper][0][lane], second = s_right[t & 1][upper][first ? 1 : 2][lane];
+      q = tanh_move(tanh_move(q, first), second);
+    }
+  }
+  if (node == 0) s_point[upper][lane] = q.d;
+  __syncthreads();
+  if (tid < kCW) { point[0] = s_point[0][tid]; point[1] = s_point[1][tid]; }
+}
+
 template <int VEC, bool STAGED>
 __global__ void __launch_bounds__(kThreads)
 col_relax_native(int op, const float* __restrict__ lw, const float* __restrict__ uw,
@@ -204,12 +240,15 @@ col_relax_native(int op, const float* __restrict__ lw, const float* __restrict__
   }
   float l, u;
   tile_concretize<VEC, STAGED>(gl, gu, Di, Do, c0, words, p, eps, s_l, s_u, s_red, lbv, ubv, l, u);
+  const bool tanh_op = (op >= OP_COEF_ONLY ? op - OP_COEF_ONLY : op) == FB_TANH;
+  float point[2] = {0.f, 0.f};
+  if (tanh_op) tanh_points(l, u, mine, point);
   if (op >= OP_COEF_ONLY) {
     // coefficients only: o_lw / o_uw are [rows, Do] arrays that receive the own-side slopes; a column
     // with a cross term (possible only for an inverted range l > u) raises bit 1 of the flag
     if (mine) {
       bool bad = false;
-      const ColCoef c = relax_column(op - OP_COEF_ONLY, l, u, lbv, ubv, bad);
+      const ColCoef c = relax_column(op - OP_COEF_ONLY, l, u, lbv, ubv, bad, tanh_op ? point : nullptr);
       if (violation != nullptr && (bad || c.c_lu != 0.f || c.c_ul != 0.f)) atomicOr(violation, bad ? 1 : 2);
       const size_t o = (size_t)row * Do + c0 + tid;
       o_lw[o] = c.c_ll;
@@ -223,7 +262,7 @@ col_relax_native(int op, const float* __restrict__ lw, const float* __restrict__
     ColCoef c = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (mine) {
       bool bad = false;
-      c = relax_column(op, l, u, lbv, ubv, bad);
+      c = relax_column(op, l, u, lbv, ubv, bad, tanh_op ? point : nullptr);
       if (bad && violation != nullptr) *violation = 1;
       o_lb[(size_t)row * Do + c0 + tid] = c.nlb;
       o_ub[(size_t)row * Do + c0 + tid] = c.nub;
@@ -241,16 +280,18 @@ col_relax_native(int op, const float* __restrict__ lw, const float* __restrict__
 // The same for tiles that fit into the block's registers: a thread holds its N rows of four columns of either line, so that the
 // tile is read once, with all its loads in flight at once, and written from registers.  Di <= 32 * N, and word blocks of a
 // multiple of 32 rows (a thread's row i then lies in word 32 i / blk for every thread).
-// Bound by HBM.  relu on [8, 64, 64, 512]: 63.3 us staged in shared memory, 54.7 us held (N = 2, 64 registers).  With N = 4 (98
-// registers, Di 128) and N = 8 (119, Di 256) too few blocks are left to hide the column's scalar chain: tanh on
-// [8, 64, 128, 256] 100 us against 73 us staged, on [8, 64, 256, 256] 136 us against 137 us with the second pass through L2.
+// Bound by HBM.  relu on [8, 64, 64, 512]: 63.3 us staged in shared memory, 54.7 us held (N = 2, 64 registers).  N = 8 (Di 256)
+// leaves two blocks per SM, which read once what would otherwise come twice, the second time from L2: [8, 64, 256, 256] relu
+// 111 -> 87 us, tanh 129 -> 107 us.  N = 4 (Di 128) has too few blocks to hide the column's scalar chain beside a tile that fits
+// into shared memory six times: tanh on [8, 64, 128, 256] 89 us against 72 us staged.
 template <int N>
 __global__ void __launch_bounds__(kThreads)
 col_relax_held(int op, const float* __restrict__ lw, const float* __restrict__ uw, const float* __restrict__ lb,
                const float* __restrict__ ub, float* __restrict__ o_lw, float* __restrict__ o_uw, float* __restrict__ o_lb,
                float* __restrict__ o_ub, int Di, int Do, int ntiles, int words, int p, float eps, int* __restrict__ violation) {
   pdl_sync();
-  __shared__ float s_red[2 * 8 * kCW], s_coef[4 * kCW];
+  constexpr int kWords = 4;   // word blocks between two barriers
+  __shared__ float s_red_all[kWords * 2 * 8 * kCW], s_coef[4 * kCW];
   const int64_t row = blockIdx.x / ntiles;
   const int c0 = (int)(blockIdx.x % ntiles) * kCW;
   const int tid = threadIdx.x, cvl = tid & 7, rg = tid >> 3, warp = tid >> 5, lane = tid & 31;
@@ -292,28 +333,35 @@ col_relax_held(int op, const float* __restrict__ lw, const float* __restrict__ u
         al[e] = norm_combine(p, al[e], __shfl_xor_sync(0xffffffffu, al[e], s));
         au[e] = norm_combine(p, au[e], __shfl_xor_sync(0xffffffffu, au[e], s));
       }
-    if (w > 0) __syncthreads();
+    if (w > 0 && w % kWords == 0) __syncthreads();
+    float* const s_red = s_red_all + (w % kWords) * (2 * 8 * kCW);
     if (lane < 8) {
       *reinterpret_cast<float4*>(s_red + warp * kCW + lane * 4) = make_float4(al[0], al[1], al[2], al[3]);
       *reinterpret_cast<float4*>(s_red + (8 + warp) * kCW + lane * 4) = make_float4(au[0], au[1], au[2], au[3]);
     }
+    if (w + 1 < words && (w + 1) % kWords != 0) continue;
     __syncthreads();
     if (tid < kCW) {
-      float sl = s_red[tid], su = s_red[8 * kCW + tid];
+      for (int q = 0; q <= w % kWords; ++q) {
+        const float* const red = s_red_all + q * (2 * 8 * kCW);
+        float sl = red[tid], su = red[8 * kCW + tid];
 #pragma unroll
-      for (int k = 1; k < 8; ++k) {
-        sl = norm_combine(p, sl, s_red[k * kCW + tid]);
-        su = norm_combine(p, su, s_red[(8 + k) * kCW + tid]);
+        for (int k = 1; k < 8; ++k) {
+          sl = norm_combine(p, sl, red[k * kCW + tid]);
+          su = norm_combine(p, su, red[(8 + k) * kCW + tid]);
+        }
+        l = fadd(l, fmul(-eps, norm_finish(p, sl)));
+        u = fadd(u, fmul(eps, norm_finish(p, su)));
       }
-      l = fadd(l, fmul(-eps, norm_finish(p, sl)));
-      u = fadd(u, fmul(eps, norm_finish(p, su)));
     }
   }
+  float point[2] = {0.f, 0.f};
+  if (op == FB_TANH) tanh_points(l, u, mine, point);
   if (tid < kCW) {
     ColCoef c = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (mine) {
       bool bad = false;
-      c = relax_column(op, l, u, lbv, ubv, bad);
+      c = relax_column(op, l, u, lbv, ubv, bad, op == FB_TANH ? point : nullptr);
       if (bad && violation != nullptr) *violation = 1;
       o_lb[(size_t)row * Do + c0 + tid] = c.nlb;
       o_ub[(size_t)row * Do + c0 + tid] = c.nub;
@@ -814,9 +862,10 @@ int launch_relax(int op, const float* lw, const float* uw, const float* lb, cons
   if (blocks > 0x7fffffff) return FB_ERR_SHAPE;
   const bool vec = Do % 4 == 0 && aligned16(lw) && aligned16(uw) &&
                    (op >= OP_COEF_ONLY || (aligned16(o_lw) && aligned16(o_uw)));
-  // a tile that fits into registers without costing occupancy
-  if (vec && op < OP_COEF_ONLY && Di <= 64 && (words == 1 || (Di / words) % 32 == 0)) {
-    launch_k(col_relax_held<2>, (unsigned)blocks, kThreads, 0, st, op, lw, uw, lb, ub, o_lw, o_uw, o_lb, o_ub, Di, Do, ntiles, words, p, eps, violation);
+  // a tile that fits into registers without costing occupancy, or that is too large for shared memory (figures at the kernel)
+  if (vec && op < OP_COEF_ONLY && (Di <= 64 || (Di > 128 && Di <= 256)) && (words == 1 || (Di / words) % 32 == 0)) {
+    auto kern = Di <= 64 ? col_relax_held<2> : col_relax_held<8>;
+    launch_k(kern, (unsigned)blocks, kThreads, 0, st, op, lw, uw, lb, ub, o_lw, o_uw, o_lb, o_ub, Di, Do, ntiles, words, p, eps, violation);
     FB_LAUNCH_OK();
     return FB_OK;
   }

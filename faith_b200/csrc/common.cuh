@@ -294,9 +294,39 @@ __device__ __forceinline__ float exp_capped(float x) {
   return fmul(expf(thres), fadd(fsub(x, thres), 1.f));
 }
 
+// Tangent points of tanh on a range that crosses zero (Bounds.py:1027-1103): upper = false: the point in [l, 0] whose tangent
+// passes through (u, tanh u), else the point in [0, u] whose tangent passes through (l, tanh l); ten bisection steps.  One step
+// is an evaluation of tanh_right_of and a move of (d, lo, hi).
+struct TanhSearch {
+  float d, lo, hi;
+};
+__device__ __forceinline__ TanhSearch tanh_search(bool upper, float l, float u) {
+  return upper ? TanhSearch{fmul(u, 0.5f), 0.f, u} : TanhSearch{fmul(l, 0.5f), l, 0.f};
+}
+// does the search go on to the right of d?  x, tx: the point the tangent has to meet (u for the lower line, l for the upper)
+__device__ __forceinline__ bool tanh_right_of(bool upper, float d, float x, float tx) {
+  const float td = tanhf(d);
+  const float v = upper ? fsub(fdiv(fsub(td, tx), fadd(fsub(d, x), kGuard)), dtanh_ref(d))
+                        : fsub(fdiv(fsub(tx, td), fadd(fsub(x, d), kGuard)), dtanh_ref(d));
+  return upper ? !(v > 0.f) : v > 0.f;
+}
+__device__ __forceinline__ TanhSearch tanh_move(TanhSearch q, bool right) {
+  if (right) return TanhSearch{fmul(fadd(q.d, q.hi), 0.5f), q.d, q.hi};
+  return TanhSearch{fmul(fadd(q.d, q.lo), 0.5f), q.lo, q.d};
+}
+constexpr int kTanhSteps = 10;
+__device__ __forceinline__ float tanh_point(bool upper, float l, float u) {
+  const float x = upper ? l : u, tx = tanhf(x);
+  TanhSearch q = tanh_search(upper, l, u);
+#pragma unroll 1
+  for (int t = 0; t < kTanhSteps; ++t) q = tanh_move(q, tanh_right_of(upper, q.d, x, tx));
+  return q.d;
+}
+
 // Per-column relaxation: from the concretised range (l, u) and the bias terms (lb, ub) to
-// the column coefficients.  `bad` is set when FB_RECIPROCAL sees l < 1e-12.
-__device__ inline ColCoef relax_column(int op, float l, float u, float lb, float ub, bool& bad) {
+// the column coefficients.  `bad` is set when FB_RECIPROCAL sees l < 1e-12.  tangent: the two tangent points of tanh where
+// the caller has them already (lower line, upper line), else they are searched here.
+__device__ inline ColCoef relax_column(int op, float l, float u, float lb, float ub, bool& bad, const float* tangent = nullptr) {
   ColCoef c = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (op >= FB_INTERVAL) {
     // interval form (the reference's `ibp` branches): constant bounds, no dependence on the weights
@@ -398,25 +428,11 @@ __device__ inline ColCoef relax_column(int op, float l, float u, float lb, float
   }
   if (both != 0.f) {
     const float tu = tanhf(u), tl = tanhf(l);
-    // lower line: tangent point in [l, 0] whose tangent passes through (u, tanh u)
-    float d = fmul(l, 0.5f), lo = l, hi = 0.f;
-#pragma unroll 1
-    for (int t = 0; t < 10; ++t) {
-      const float v = fsub(fdiv(fsub(tu, tanhf(d)), fadd(fsub(u, d), kGuard)), dtanh_ref(d));
-      if (v > 0.f) { lo = d; d = fmul(fadd(d, hi), 0.5f); }
-      else         { hi = d; d = fmul(fadd(d, lo), 0.5f); }
-    }
+    float d = tangent != nullptr ? tangent[0] : tanh_point(false, l, u);
     float td = tanhf(d);
     float k = fdiv(fsub(td, tu), fadd(fsub(d, u), kGuard));
     add_line(c, both, true, k, d, td, lb, ub);
-    // upper line: tangent point in [0, u] whose tangent passes through (l, tanh l)
-    d = fmul(u, 0.5f); lo = 0.f; hi = u;
-#pragma unroll 1
-    for (int t = 0; t < 10; ++t) {
-      const float v = fsub(fdiv(fsub(tanhf(d), tl), fadd(fsub(d, l), kGuard)), dtanh_ref(d));
-      if (v > 0.f) { hi = d; d = fmul(fadd(d, lo), 0.5f); }
-      else         { lo = d; d = fmul(fadd(d, hi), 0.5f); }
-    }
+    d = tangent != nullptr ? tangent[1] : tanh_point(true, l, u);
     td = tanhf(d);
     k = fdiv(fsub(td, tl), fadd(fsub(d, l), kGuard));
     add_line(c, both, false, k, d, td, lb, ub);

@@ -1156,3 +1156,9 @@ def test_standard_layer_norm_by_number_of_rows(L, Di, Do, p, words):
 def test_fused_softmax_of_wide_inputs(Di, Do, words, p):
     """Eight rows of dim_in per thread."""
     test_fused_softmax_of_any_length(Di, Do, words, p)
+
+
+@pytest.mark.parametrize("Di,Do,words", [(129, 36, 1), (160, 32, 5), (256, 40, 8), (256, 64, 1), (255, 4, 1)])
+@pytest.mark.parametrize("p", [1.0, 2.0, float("inf")])
+def test_relax_of_wide_columns_held_in_registers(Di, Do, words, p):
+    test_relax_of_short_columns_held_in_registers(Di, Do, words, p)
