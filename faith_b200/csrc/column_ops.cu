@@ -291,7 +291,7 @@ col_relax_held(int op, const float* __restrict__ lw, const float* __restrict__ u
                float* __restrict__ o_ub, int Di, int Do, int ntiles, int words, int p, float eps, int* __restrict__ violation) {
   pdl_sync();
   constexpr int kWords = 4;   // word blocks between two barriers
-  __shared__ float s_red_all[kWords * 2 * 8 * kCW], s_coef[4 * kCW];
+  __shared__ float s_red[kWords * 2 * 8 * kCW], s_norm[2 * kWords][kCW], s_coef[4 * kCW];
   const int64_t row = blockIdx.x / ntiles;
   const int c0 = (int)(blockIdx.x % ntiles) * kCW;
   const int tid = threadIdx.x, cvl = tid & 7, rg = tid >> 3, warp = tid >> 5, lane = tid & 31;
@@ -326,32 +326,34 @@ col_relax_held(int op, const float* __restrict__ lw, const float* __restrict__ u
         au[0] = norm_accum(p, au[0], vu[i].x); au[1] = norm_accum(p, au[1], vu[i].y);
         au[2] = norm_accum(p, au[2], vu[i].z); au[3] = norm_accum(p, au[3], vu[i].w);
       }
+    // the four row groups of a warp: every lane gives away the values it does not keep (6 shuffles where a butterfly of every
+    // value takes 16), ending with two columns of one line
+    const bool up8 = lane & 8, up16 = lane & 16;
+    float h[4], g[2];
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
+    for (int e = 0; e < 4; ++e) h[e] = norm_combine(p, up8 ? au[e] : al[e], __shfl_xor_sync(0xffffffffu, up8 ? al[e] : au[e], 8));
 #pragma unroll
-      for (int s = 8; s < 32; s <<= 1) {
-        al[e] = norm_combine(p, al[e], __shfl_xor_sync(0xffffffffu, al[e], s));
-        au[e] = norm_combine(p, au[e], __shfl_xor_sync(0xffffffffu, au[e], s));
-      }
+    for (int e = 0; e < 2; ++e)
+      g[e] = norm_combine(p, up16 ? h[2 + e] : h[e], __shfl_xor_sync(0xffffffffu, up16 ? h[e] : h[2 + e], 16));
     if (w > 0 && w % kWords == 0) __syncthreads();
-    float* const s_red = s_red_all + (w % kWords) * (2 * 8 * kCW);
-    if (lane < 8) {
-      *reinterpret_cast<float4*>(s_red + warp * kCW + lane * 4) = make_float4(al[0], al[1], al[2], al[3]);
-      *reinterpret_cast<float4*>(s_red + (8 + warp) * kCW + lane * 4) = make_float4(au[0], au[1], au[2], au[3]);
-    }
+    *reinterpret_cast<float2*>(s_red + (((w % kWords) * 2 + (up8 ? 1 : 0)) * 8 + warp) * kCW + cvl * 4 + (up16 ? 2 : 0)) = make_float2(g[0], g[1]);
     if (w + 1 < words && (w + 1) % kWords != 0) continue;
+    __syncthreads();
+    {   // a warp per word block and line, a lane per column
+      static_assert(kWords * 2 * kCW == kThreads, "a thread per word block, line and column");
+      if (warp < 2 * (w % kWords + 1)) {
+        const float* const red = s_red + warp * 8 * kCW + lane;
+        float v = red[0];
+#pragma unroll
+        for (int k = 1; k < 8; ++k) v = norm_combine(p, v, red[k * kCW]);
+        s_norm[warp][lane] = norm_finish(p, v);
+      }
+    }
     __syncthreads();
     if (tid < kCW) {
       for (int q = 0; q <= w % kWords; ++q) {
-        const float* const red = s_red_all + q * (2 * 8 * kCW);
-        float sl = red[tid], su = red[8 * kCW + tid];
-#pragma unroll
-        for (int k = 1; k < 8; ++k) {
-          sl = norm_combine(p, sl, red[k * kCW + tid]);
-          su = norm_combine(p, su, red[(8 + k) * kCW + tid]);
-        }
-        l = fadd(l, fmul(-eps, norm_finish(p, sl)));
-        u = fadd(u, fmul(eps, norm_finish(p, su)));
+        l = fadd(l, fmul(-eps, s_norm[2 * q][tid]));
+        u = fadd(u, fmul(eps, s_norm[2 * q + 1][tid]));
       }
     }
   }
