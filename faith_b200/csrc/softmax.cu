@@ -361,6 +361,18 @@ softmax_bounds_regs(const float* __restrict__ lw, const float* __restrict__ uw, 
         nu[e] = norm_accum(p, nu[e], y[k][e]);
       }
     }
+    if constexpr (CVL == 8) {
+      // every lane gives away the values it does not keep and ends with two columns of one line: 6 shuffles instead of 16
+      const bool up8 = lane & 8, up16 = lane & 16;
+      float h[4], g[2];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) h[e] = norm_combine(p, up8 ? nu[e] : nl[e], __shfl_xor_sync(0xffffffffu, up8 ? nl[e] : nu[e], 8));
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        g[e] = norm_combine(p, up16 ? h[2 + e] : h[e], __shfl_xor_sync(0xffffffffu, up16 ? h[e] : h[2 + e], 16));
+      reinterpret_cast<float2*>(&s_part[up8 ? 1 : 0][warp][cvl])[up16 ? 1 : 0] = make_float2(g[0], g[1]);
+      return;
+    }
 #pragma unroll
     for (int e = 0; e < 4; ++e)
 #pragma unroll
@@ -409,19 +421,38 @@ softmax_bounds_regs(const float* __restrict__ lw, const float* __restrict__ uw, 
       b[k][0] = fmul(b[k][0], ku.x); b[k][1] = fmul(b[k][1], ku.y); b[k][2] = fmul(b[k][2], ku.z); b[k][3] = fmul(b[k][3], ku.w);
     }
   }
-  float rs[KR][2];   // row sums of exp of this thread's rows
+  // row sums of exp over the CVL lanes of a row, to s_row
 #pragma unroll
-  for (int k = 0; k < KR; ++k) {
-    float sa = fadd(fadd(a[k][0], a[k][1]), fadd(a[k][2], a[k][3]));
-    float sb = fadd(fadd(b[k][0], b[k][1]), fadd(b[k][2], b[k][3]));
+  for (int k0 = 0; k0 < KR; k0 += 4) {
+    constexpr int NK = KR < 4 ? KR : 4;
+    float v[4][2];
 #pragma unroll
-    for (int s = 1; s < CVL; s <<= 1) {
-      sa += __shfl_xor_sync(0xffffffffu, sa, s);
-      sb += __shfl_xor_sync(0xffffffffu, sb, s);
+    for (int k = 0; k < NK; ++k) {
+      v[k][0] = fadd(fadd(a[k0 + k][0], a[k0 + k][1]), fadd(a[k0 + k][2], a[k0 + k][3]));
+      v[k][1] = fadd(fadd(b[k0 + k][0], b[k0 + k][1]), fadd(b[k0 + k][2], b[k0 + k][3]));
     }
-    rs[k][0] = sa;
-    rs[k][1] = sb;
-    if (cvl == 0) { s_row[0][k * RG + rg] = sa; s_row[1][k * RG + rg] = sb; }
+    if constexpr (NK == 4 && CVL == 8) {   // eight sums over eight lanes: a lane ends with one of them, 7 shuffles instead of 24
+      const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4;
+      float x[2][2], y[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) x[k][e] = (b0 ? v[2 + k][e] : v[k][e]) + __shfl_xor_sync(0xffffffffu, b0 ? v[k][e] : v[2 + k][e], 1);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) y[e] = (b1 ? x[1][e] : x[0][e]) + __shfl_xor_sync(0xffffffffu, b1 ? x[0][e] : x[1][e], 2);
+      const float z = (b2 ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, b2 ? y[0] : y[1], 4);
+      s_row[b2 ? 1 : 0][(k0 + (b0 ? 2 : 0) + (b1 ? 1 : 0)) * RG + rg] = z;
+    } else {
+#pragma unroll
+      for (int k = 0; k < NK; ++k) {
+#pragma unroll
+        for (int s = 1; s < CVL; s <<= 1) {
+          v[k][0] += __shfl_xor_sync(0xffffffffu, v[k][0], s);
+          v[k][1] += __shfl_xor_sync(0xffffffffu, v[k][1], s);
+        }
+        if (cvl == 0) { s_row[0][(k0 + k) * RG + rg] = v[k][0]; s_row[1][(k0 + k) * RG + rg] = v[k][1]; }
+      }
+    }
   }
   float la = mine ? s_col[2][tid] : 0.f;
   for (int w = 0; w < words; ++w) {
@@ -469,7 +500,7 @@ softmax_bounds_regs(const float* __restrict__ lw, const float* __restrict__ uw, 
   const float be[4] = {be4.x, be4.y, be4.z, be4.w};
 #pragma unroll
   for (int k = 0; k < KR; ++k) {
-    const float r_l = fmul(rs[k][1], kl_r), r_u = fmul(rs[k][0], ku_r);
+    const float r_l = fmul(s_row[1][k * RG + rg], kl_r), r_u = fmul(s_row[0][k * RG + rg], ku_r);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float e_l = a[k][e], e_u = b[k][e];
@@ -549,7 +580,8 @@ int fb::softmax_ex(const float* lw, const float* uw, const float* lb, const floa
   // The tile in registers: rows split evenly over the threads, word blocks over the row groups; blocks of up to 256 threads
   // (512, for dim_in 256 or lengths above 32, leave one block per SM and take 456 instead of 256 us for 8064 rows; 256 threads
   // with eight rows each, two blocks per SM: 2016 rows of [256, 21] 86 -> 76 us).
-  // 32768 rows of [128, 32]: 483 -> 448 us; 6144 rows of [128, 12]: 88 -> 46 us.
+  // 32768 rows of [128, 32]: 483 -> 448 us, 437 -> 427 us with the exchanges that give values away; 6144 rows of [128, 12]: 88 ->
+  // 46 us.
 #define FB_SOFTMAX_REGS(C, T, K)                                                                                       \
   if (cw == C && Di == T / (C / 4) * K && K % words == 0) {                                                            \
     if (p == FB_PINF) FB_SOFTMAX_REGS_LAUNCH(FB_PINF, C, T, K);                                                        \
