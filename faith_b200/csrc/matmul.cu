@@ -251,13 +251,15 @@ int fb::matmul_ranges_ex(const float* x_lw, const float* x_uw, const float* x_lb
     rc = fb::launch_split_sign_tc(x_lb, x_ub, W, bias, plain_lb, plain_ub, rows, Dy, Do, st, 0, 0);
   } else if (!fb::tc_gemm_supported(x_lb, x_ub, W, y_lb, y_ub, rows, Dy, Do) && fb::small_product(rows, Dy)) {
     fb::RangeEpilogue rg = {norm_lo, norm_up, y_l, y_u, words, eps, 0, -1, nullptr, nullptr, nullptr, nullptr, nullptr};
+    bool split = heads > 1;
     if (wishes != nullptr) {
-      rg.transposed = wishes->transposed && heads > 1;
+      rg.transposed = wishes->transposed;
+      split = split || wishes->transposed;   // (transposed ranges are addressed by the split, also by that into one head)
       rg.op = wishes->op;
       rg.k_l = wishes->k_l, rg.k_u = wishes->k_u, rg.r_lb = wishes->r_lb, rg.r_ub = wishes->r_ub, rg.violation = wishes->violation;
       wishes->granted = true;
     }
-    return fb::launch_split_sign_small(x_lb, x_ub, W, bias, y_lb, y_ub, rows, Dy, Do, st, heads > 1 ? L : 0, heads > 1 ? d : 0, &rg);
+    return fb::launch_split_sign_small(x_lb, x_ub, W, bias, y_lb, y_ub, rows, Dy, Do, st, split ? L : 0, split ? d : 0, &rg);
   } else {
     rc = fb::split_sign_gemm(x_lb, x_ub, W, bias, y_lb, y_ub, rows, Dy, Do, st, heads > 1 ? L : 0, heads > 1 ? d : 0);
   }

@@ -1080,6 +1080,23 @@ def test_encoder_of_a_length_that_is_not_a_multiple_of_four(L, words):
     helpers.assert_within_noise(u, u32, u64, "u")
 
 
+# One head: the driver asks the kernel for few rows for the value ranges in the layout of the context product, with a split of
+# one head.  A radius at which the probabilities are wide: value ranges in the wrong order move the result by some hundred
+# times the noise (at 1e-3 they hide in it).
+@pytest.mark.parametrize("S,L,words,layers", [(1, 32, 1, 1), (1, 21, 2, 2), (3, 21, 1, 1), (7, 32, 1, 2), (1, 6, 1, 2), (2, 36, 1, 1), (9, 32, 1, 1)])
+def test_encoder_with_one_head(S, L, words, layers):
+    import faith_b200
+    model = O.make_encoder(9, layers=layers, d_model=128, heads=1, ffn=512)
+    emb = torch.randn(S, L, 128, generator=torch.Generator().manual_seed(10))
+    pos, p, eps = [1, 4][:words], 2.0, 0.1
+    l32, u32 = O.encoder_forward(model, emb, pos, p, eps)
+    l64, u64 = O.encoder_forward(O.model_to(model, torch.float64), emb.double(), pos, p, eps)
+    l, u, viol = faith_b200.EncoderVerifier(model, DEV).forward(emb.to(DEV), pos, p, eps)
+    assert int(viol.item()) == 0
+    helpers.assert_within_noise(l, l32, l64, "l, one head")
+    helpers.assert_within_noise(u, u32, u64, "u, one head")
+
+
 # (one coordinate past a 64-wide tile, odd dim_in, K past the 128 values staged at a time, a tile of one row, both block
 # shapes)
 @pytest.mark.parametrize("B,Lx,Ly,Di,K", [(1, 1, 3, 2, 1), (1, 5, 9, 65, 130), (2, 9, 4, 66, 7), (4, 33, 31, 128, 33), (2, 40, 48, 250, 150)])
