@@ -360,7 +360,8 @@ static int encoder_forward_impl(const fb_encoder* enc, const float* emb, int S, 
       // ---- last layer, first token only (the pooler reads nothing else of its output, VerifierForward.py:269-287).
       // Keys and values at every position; query, attention row, attention output, feed-forward block at position 0.
       // Plain operator calls throughout: the tensors on the query side are 1/L of the usual size.
-      const BoundSet X = slot[A];
+      BoundSet X = slot[A];
+      if (li == 0) { X.uw = X.lw; X.ub = X.lb; }   // (the lines of the input coincide, and only lw has been written)
       char* bump = reinterpret_cast<char*>(slot[B].lw);
       char* const bump_end = bump + plan.slot_bytes;
       bool fits = true;

@@ -308,6 +308,28 @@ def test_last_layer_for_the_first_token_only_gives_the_same_bounds(full_size):
     helpers.assert_within_noise(u2, u32, u64, "u instances")
 
 
+@pytest.mark.parametrize("S,L,heads,inst", [(2, 16, 8, False), (1, 9, 1, True), (9, 32, 4, False), (3, 33, 4, True)])
+def test_first_token_only_of_a_single_layer(S, L, heads, inst):
+    """The last layer is then the first one as well: of its input only one line is in memory (the lines coincide).  The arena
+    is filled with NaN beforehand, so that a line that nothing has written cannot go unnoticed."""
+    import faith_b200
+    model = O.make_encoder(12, layers=1, heads=heads)
+    emb = torch.randn(S, L, 128, generator=torch.Generator().manual_seed(13))
+    p, eps = 2.0, 0.1
+    ver = faith_b200.EncoderVerifier(model, DEV, first_token_only=True)
+    ver._ws = torch.full((ver.workspace_bytes(S, L, 1),), 255, dtype=torch.uint8, device=DEV)
+    if inst:
+        l, u, viol = ver.forward_instances(emb.to(DEV), torch.full((S, 1), 2, dtype=torch.int32, device=DEV), p,
+                                           torch.full((S,), eps, device=DEV))
+    else:
+        l, u, viol = ver.forward(emb.to(DEV), [2], p, eps)
+    assert ver.check_status(viol) == 0
+    l32, u32 = O.encoder_forward(model, emb, [2], p, eps)
+    l64, u64 = O.encoder_forward(O.model_to(model, torch.float64), emb.double(), [2], p, eps)
+    helpers.assert_within_noise(l, l32, l64, "l")
+    helpers.assert_within_noise(u, u32, u64, "u")
+
+
 def test_mean_pooling_option():
     """pooling = "mean" (the pooling the benchmark description names; the reference pools the first token): mean over the
     positions -> dense -> tanh.  Against the oracle's restatement (no reference implementation exists: unpinned), and
