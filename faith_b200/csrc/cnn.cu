@@ -120,10 +120,12 @@ extern "C" int fb_cnn_forward_f32(const fb_cnn* net, const float* image, int p, 
       const int ho = (h + 2 * ly.pad - ly.kh) / ly.stride + 1, wo = (w + 2 * ly.pad - ly.kw) / ly.stride + 1;
       rc = launch_identity_columns(op, image, image, ly.weight, ly.bias, x.lb, x.ub, col_ws, col_ws + (int64_t)ly.cout * ho * wo, 1.0f, c, h, w,
                                    ly.cout, ly.kh, ly.kw, ly.stride, ly.pad, ho, wo, p, eps, violation, st);
+    } else if (cw) {
+      rc = cw_identity_rows(op, image, ly.weight, ly.bias, x.lw, x.uw, x.lb, x.ub, col_ws, rows, row_start, c, h, w, ly.cout, ly.kh, ly.kw,
+                            ly.stride, ly.pad, p, eps, violation, st);
     } else {
-      rc = (cw ? fb_cw_identity_relax_f32 : fb_conv2d_identity_relax_f32)(op, image, image, ly.weight, ly.bias, 1.0f, x.lw, x.uw, x.lb, x.ub,
-                                                                          col_ws, rows, row_start, c, h, w, ly.cout, ly.kh, ly.kw,
-                                                                          ly.stride, ly.pad, p, eps, violation, stream);
+      rc = fb_conv2d_identity_relax_f32(op, image, image, ly.weight, ly.bias, 1.0f, x.lw, x.uw, x.lb, x.ub, col_ws, rows, row_start, c, h, w,
+                                        ly.cout, ly.kh, ly.kw, ly.stride, ly.pad, p, eps, violation, stream);
     }
     if (rc != FB_OK) return rc;
     chain[0] = ly.kh, chain[1] = ly.kw, chain[2] = ly.stride, chain[3] = ly.pad;
@@ -143,7 +145,7 @@ extern "C" int fb_cnn_forward_f32(const fb_cnn* net, const float* image, int p, 
       std::swap(x.uw, y.uw);
       rescaled = false;
     }
-    int rc = fb_cw_expand_f32(x.lw, x.uw, y.lw, y.uw, rows, row_start, net->h, net->w, chain, n_chain, c, h, w, stream);
+    int rc = cw_expand_rows(x.lw, x.uw, y.lw, y.uw, rows, row_start, net->h, net->w, chain, n_chain, c, h, w, st);
     if (rc != FB_OK) return rc;
     std::swap(x.lw, y.lw);
     std::swap(x.uw, y.uw);

@@ -112,7 +112,12 @@ int concretize_pair(const float* x_lw, const float* x_uw, const float* x_lb, con
                     int x_do, const float* y_lw, const float* y_uw, const float* y_lb, const float* y_ub, float* y_l, float* y_u,
                     int64_t y_rows, int y_do, int Di, int words, int p, float eps, int layout, cudaStream_t st);
 
-// conv_compact.cu: the operators on compact rows with the options of the CNN driver (see the definitions).
+// conv_compact.cu: the operators on compact rows in the CNN driver's form and with its options (see the definitions).
+int cw_identity_rows(int op, const float* x, const float* Wt, const float* bias, float* z_lw, float* z_uw, float* y_lb, float* y_ub,
+                     float* col_ws, int64_t rows, int64_t row_start, int Cin, int H, int W, int Cout, int Kh, int Kw, int stride, int pad,
+                     int p, float eps, int* violation, cudaStream_t st);
+int cw_expand_rows(const float* z_lw, const float* z_uw, float* y_lw, float* y_uw, int64_t rows, int64_t row_start, int H0, int W0,
+                   const int* chain, int n_chain, int C, int H, int W, cudaStream_t st);
 int cw_conv_ex(const float* z_lo, const float* z_up, const float* W1, const float* k_l, const float* k_u, float scale, int Cin0,
                const float* Wt, float* y_lo, float* y_up, const float* b_lo, const float* b_up, const float* bias, float* yb_lo,
                float* yb_up, int64_t rows, int64_t row_start, int H0, int W0, const int* chain, int n_chain, int Cin, int H, int W,

@@ -5,10 +5,12 @@
 // The dense-row kernels of conv.cu still write and read those zeros: [rows, C, H, W] per tensor, 98 % zeros for the
 // benchmark CNN.  Here a row is kept as its window only:
 //
-//     z[r, dy, dx, c] = row r at (c, wy.lo(r) + dy, wx.lo(r) + dx),   dy < wh, dx < ww,
+//     z[r, c, dy, dx] = row r at (c, wy.lo(r) + dy, wx.lo(r) + dx),   dy < wh, dx < ww,
 //
-// (channels innermost: the kernels have their lanes on the channels, and their loads and stores of rows are whole sectors)
-// with (wh, ww) the largest window over all pixels (fb_cw_extent); where a pixel's own window is smaller nothing is written.
+// with (wh, ww) the largest window over all pixels (fb_cw_extent) and zeros where a pixel's own window is smaller: the form of
+// the C ABI (kAbi = true below).  Between its layers the CNN driver keeps the rows as z[r, dy, dx, c] (kAbi = false): the kernels
+// have their lanes on the channels, so that their loads and stores of rows are whole sectors; its windows are cut to the last map
+// only (CwAxis), and where a pixel's own window is smaller nothing is written.
 // The origin (wy.lo, wx.lo) is recomputed from the pixel and the chain wherever it is needed.  Every operator of the
 // CNN pass has a compact form: first convolution + relaxation, later convolutions, the column norms over dim_in
 // (a gather over the rows whose window holds the column, in row order: deterministic), the rescale of a relaxation,
@@ -27,10 +29,32 @@
 namespace fb {
 namespace {
 
-// Geometry of a compact tensor: its windows and its dense shape.
-struct CwShape {
+// Geometry of a compact tensor: its windows, its dense shape and the order of a row's elements.
+template <bool kAbi>
+struct CwShape;
+
+template <>
+struct CwShape<false> {
   CwAxis y, x;
   int H0, W0, C, H, W, wh, ww;
+  __device__ __forceinline__ Span rows(int yi) const { return {y.lo(yi), y.hi(yi)}; }
+  __device__ __forceinline__ Span cols(int xi) const { return {x.lo(xi), x.hi(xi)}; }
+  // elements between neighbouring columns and between neighbouring channels
+  __device__ __forceinline__ int step_x() const { return C; }
+  __device__ __forceinline__ int step_c() const { return 1; }
+  // element e of a row
+  __device__ __forceinline__ void split(int e, int& c, int& dy, int& dx) const { c = e % C, dx = (e / C) % ww, dy = e / (C * ww); }
+};
+
+template <>
+struct CwShape<true> : CwShape<false> {   // (y and x: windows that hold these, for the ranges of loops)
+  ConvChain ch;
+  bool same;   // y and x are these windows, as behind most chains: no walk along the chain (norms of 3072 rows: 12.3 -> 5.5 us)
+  __device__ __forceinline__ Span rows(int yi) const { return same ? CwShape<false>::rows(yi) : chain_span(ch, ch.kh, ch.n, H0, yi); }
+  __device__ __forceinline__ Span cols(int xi) const { return same ? CwShape<false>::cols(xi) : chain_span(ch, ch.kw, ch.n, W0, xi); }
+  __device__ __forceinline__ int step_x() const { return 1; }
+  __device__ __forceinline__ int step_c() const { return wh * ww; }
+  __device__ __forceinline__ void split(int e, int& c, int& dy, int& dx) const { dx = e % ww, dy = (e / ww) % wh, c = e / (ww * wh); }
 };
 
 __device__ __forceinline__ void pixel_of_row(int64_t r, int H0, int W0, int& yi, int& xi) {
@@ -46,7 +70,9 @@ __device__ __forceinline__ void touch_params(const Args& q) {
   if (at < sizeof(Args) / 4) asm volatile("" ::"r"(reinterpret_cast<const int*>(&q)[at]));
 }
 
-// First convolution (+ relaxation) of the identity input, compact: one thread per element of z.
+// First convolution (+ relaxation) of the identity input, compact: one thread per element of z.  (Behind a single convolution the
+// two forms have the same windows.)
+template <bool kAbi>
 __global__ void __launch_bounds__(256)
 cw_identity_rows_kernel(const float* __restrict__ Wt, const float* __restrict__ k_l, const float* __restrict__ k_u,
                         float* __restrict__ z_lw, float* __restrict__ z_uw, float scale, int64_t rows, int64_t row_start,
@@ -56,7 +82,7 @@ cw_identity_rows_kernel(const float* __restrict__ Wt, const float* __restrict__ 
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < rows * per_row; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t lr = t / per_row;
     const int e = (int)(t - lr * per_row);
-    const int co = e % Cout, dx = (e / Cout) % ww, dy = e / (Cout * ww);
+    const int co = kAbi ? e / (ww * wh) : e % Cout, dx = kAbi ? e % ww : (e / Cout) % ww, dy = kAbi ? (e / ww) % wh : e / (Cout * ww);
     const int64_t r = row_start + lr;
     const int xi = (int)(r % W), yi = (int)((r / W) % H), ci = (int)(r / ((int64_t)W * H));
     Span sy = {yi, yi}, sx = {xi, xi};
@@ -112,6 +138,13 @@ struct CwConvArgs {
   CwAxis iy, ix, oy, ox;                       // input and output windows
 };
 
+template <bool kAbi>
+struct CwConvParams : CwConvArgs {};
+template <>
+struct CwConvParams<true> : CwConvArgs {
+  ConvChain ch;   // up to and including this convolution
+};
+
 struct __align__(16) CwRow {
   int lr, yi, xi, ci;      // local row (-1: none), pixel
   int uy, ux;              // input window without borders: first row and column
@@ -124,9 +157,9 @@ struct __align__(16) CwRow {
 // KS: filter size when it is the same in both directions and known at compile time (3), 0 = from the arguments.
 // CPT: output channels per thread (2 where Cout is even: the pairs of a tap are one 128-bit read, and the inputs, which every lane
 // reads, serve twice the multiply-adds).
-template <int KS, int CPT>
+template <int KS, int CPT, bool kAbi>
 __global__ void __launch_bounds__(kCwConvThreads)
-cw_conv_kernel(const __grid_constant__ CwConvArgs q) {
+cw_conv_kernel(const __grid_constant__ CwConvParams<kAbi> q) {
   extern __shared__ __align__(16) float cw_smem[];
   __shared__ CwRow s_row[kCwMaxRows];
   touch_params(q);
@@ -185,12 +218,22 @@ cw_conv_kernel(const __grid_constant__ CwConvArgs q) {
       }
       live = r.lr >= 0;
       r.uy = vy + q.stride * ky, r.ux = vx + q.stride * kx;
-      r.iy = max(0, r.uy), r.ix = max(0, r.ux);
-      r.ih = min(q.H, r.uy + ih) - r.iy, r.iw = min(q.W, r.ux + iw) - r.ix;
-      const int oy = max(0, wy + ky), ox = max(0, wx + kx);
-      r.oh = live ? max(0, min(q.Ho, wy + ky + oh) - oy) : 0, r.ow = live ? max(0, min(q.Wo, wx + kx + ow) - ox) : 0;
+      int oy, ox;
+      if constexpr (kAbi) {
+        const Span sy = chain_span(q.ch, q.ch.kh, q.ch.n - 1, q.H0, r.yi), sx = chain_span(q.ch, q.ch.kw, q.ch.n - 1, q.W0, r.xi);
+        const Span ty = chain_span(q.ch, q.ch.kh, q.ch.n, q.H0, r.yi), tx = chain_span(q.ch, q.ch.kw, q.ch.n, q.W0, r.xi);
+        r.iy = sy.lo, r.ix = sx.lo, r.ih = sy.hi - sy.lo + 1, r.iw = sx.hi - sx.lo + 1;
+        oy = ty.lo, ox = tx.lo;
+        r.oh = live ? max(0, ty.hi - oy + 1) : 0, r.ow = live ? max(0, tx.hi - ox + 1) : 0;
+      } else {
+        r.iy = max(0, r.uy), r.ix = max(0, r.ux);
+        r.ih = min(q.H, r.uy + ih) - r.iy, r.iw = min(q.W, r.ux + iw) - r.ix;
+        oy = max(0, wy + ky), ox = max(0, wx + kx);
+        r.oh = live ? max(0, min(q.Ho, wy + ky + oh) - oy) : 0, r.ow = live ? max(0, min(q.Wo, wx + kx + ow) - ox) : 0;
+      }
       r.py = oy - wy - ky, r.px = ox - wx - kx;
-      r.base = (((int64_t)r.lr * q.owh - r.py) * q.oww - r.px) * q.Cout;
+      r.base = kAbi ? (int64_t)r.lr * q.Cout * q.owh * q.oww - r.py * q.oww - r.px
+                    : (((int64_t)r.lr * q.owh - r.py) * q.oww - r.px) * q.Cout;
       s_row[tid] = r;
     }
     if (!__syncthreads_or(live)) return;
@@ -257,19 +300,22 @@ cw_conv_kernel(const __grid_constant__ CwConvArgs q) {
               }
             }
         } else {
-          // lanes along the channel: neighbouring words of a row
+          // lanes along the channel: neighbouring words of a row of the driver
           for (int v = warp; v < ih * n_rows; v += nwarps) {
             const int uy = v / n_rows, t = v - uy * n_rows;
             const CwRow& r = s_row[t];
             const int dy = r.uy + uy - r.iy, dx0 = r.ux - r.ix;
             const bool in_y = r.lr >= 0 && dy >= 0 && dy < r.ih;
-            const int64_t o = (((int64_t)r.lr * q.iwh + dy) * q.iww + dx0) * q.Cin + c0;
+            const int step_x = kAbi ? 1 : q.Cin, step_c = kAbi ? q.iwh * q.iww : 1;
+            const int64_t o = kAbi ? ((int64_t)r.lr * q.Cin + c0) * step_c + dy * q.iww + dx0
+                                   : (((int64_t)r.lr * q.iwh + dy) * q.iww + dx0) * q.Cin + c0;
             for (int c = lane; c < cc; c += 32) {
               float2* dst = s_x + (c * q.uih + uy) * q.uiw * n_rows + t;
 #pragma unroll 3
               for (int ux = 0; ux < iw; ++ux) {
                 const bool in = in_y && dx0 + ux >= 0 && dx0 + ux < r.iw;
-                const float lo = in ? __ldg(q.z_lo + o + ux * q.Cin + c) : 0.f, up = in ? __ldg(q.z_up + o + ux * q.Cin + c) : 0.f;
+                const int64_t at = o + ux * step_x + c * step_c;
+                const float lo = in ? __ldg(q.z_lo + at) : 0.f, up = in ? __ldg(q.z_up + at) : 0.f;
                 dst[ux * n_rows] = make_float2(fmul(fadd(lo, up), 0.5f), fmul(fsub(up, lo), 0.5f));
               }
             }
@@ -335,12 +381,13 @@ cw_conv_kernel(const __grid_constant__ CwConvArgs q) {
       for (int j = 0; j < kCwR; ++j) {
         const CwRow& r = s_row[g * kCwR + j];
         if ((unsigned)(py - r.py) < (unsigned)r.oh && (unsigned)(px - r.px) < (unsigned)r.ow) {
-          const int64_t o = r.base + (int64_t)(py * q.oww + px) * q.Cout + co;
+          const int step_c = kAbi ? q.owh * q.oww : 1;
+          const int64_t o = r.base + (int64_t)(py * q.oww + px) * (kAbi ? 1 : q.Cout) + (int64_t)co * step_c;
 #pragma unroll
           for (int e = 0; e < CPT; ++e) {
             const float2 v = unpack2(acc[j][e]);
-            q.y_lo[o + e] = fsub(v.x, v.y);
-            q.y_up[o + e] = fadd(v.x, v.y);
+            q.y_lo[o + e * step_c] = fsub(v.x, v.y);
+            q.y_up[o + e * step_c] = fadd(v.x, v.y);
           }
         }
       }
@@ -372,10 +419,11 @@ __device__ __forceinline__ void cw_relax_column(int op, float lbv, float ubv, fl
   coef[3 * ncol + at] = c.c_uu;
 }
 
+template <bool kAbi>
 __global__ void __launch_bounds__(32 * kCwNormWarps)
 cw_norm_kernel(int op, const float* __restrict__ z_lw, const float* __restrict__ z_uw, float* __restrict__ part_l,
                float* __restrict__ part_u, const float* __restrict__ lb, const float* __restrict__ ub, float* __restrict__ out_lb,
-               float* __restrict__ out_ub, float* __restrict__ coef, int64_t rows, int64_t row_start, int Cin0, const __grid_constant__ CwShape g, int p,
+               float* __restrict__ out_ub, float* __restrict__ coef, int64_t rows, int64_t row_start, int Cin0, const __grid_constant__ CwShape<kAbi> g, int p,
                float eps, int* __restrict__ violation) {
   pdl_sync();
   __shared__ float s_part[2][kCwNormWarps][32];
@@ -389,14 +437,17 @@ cw_norm_kernel(int op, const float* __restrict__ z_lw, const float* __restrict__
     for (int k = warp; k < Cin0 * ny; k += kCwNormWarps) {
       const int ci = k / ny, yi = y0 + k - ci * ny;
       const int64_t lr0 = ((int64_t)ci * g.H0 + yi) * g.W0 + x0 - row_start;
-      const int dy = y - g.y.lo(yi);
+      const Span wy = g.rows(yi);
+      const int dy = y - wy.lo;
+      const bool in_y = !kAbi || (y >= wy.lo && y <= wy.hi);
       for (int kx = 0; kx < nx; kx += kCwNormLoads) {
         float vl[kCwNormLoads], vu[kCwNormLoads];   // zeros leave every norm as it is
 #pragma unroll
         for (int e = 0; e < kCwNormLoads; ++e) {
           const int64_t lr = lr0 + kx + e;
-          const bool in = kx + e < nx && lr >= 0 && lr < rows && c < g.C;
-          const int64_t o = in ? ((lr * g.wh + dy) * g.ww + (x - g.x.lo(x0 + kx + e))) * g.C + c : 0;
+          const Span wx = g.cols(x0 + kx + e);
+          const bool in = kx + e < nx && lr >= 0 && lr < rows && c < g.C && in_y && (!kAbi || (x >= wx.lo && x <= wx.hi));
+          const int64_t o = !in ? 0 : kAbi ? ((lr * g.C + c) * g.wh + dy) * g.ww + (x - wx.lo) : ((lr * g.wh + dy) * g.ww + (x - wx.lo)) * g.C + c;
           vl[e] = in ? __ldg(z_lw + o) : 0.f;
           vu[e] = in ? __ldg(z_uw + o) : 0.f;
         }
@@ -427,7 +478,9 @@ cw_norm_kernel(int op, const float* __restrict__ z_lw, const float* __restrict__
   }
 }
 
-// Relaxation coefficients per column from the (reduced) norms, coef [4][H * W][C]; the relaxed bias terms go to out_lb / out_ub.
+// Relaxation coefficients per column from the (reduced) norms, in the order of the rows' elements: coef [4][H * W][C], or (kAbi)
+// [4][C][H * W]; the relaxed bias terms go to out_lb / out_ub.
+template <bool kAbi>
 __global__ void __launch_bounds__(256)
 cw_relax_columns_kernel(int op, const float* __restrict__ lb, const float* __restrict__ ub, const float* __restrict__ norm_l,
                         const float* __restrict__ norm_u, float* __restrict__ out_lb, float* __restrict__ out_ub,
@@ -435,14 +488,15 @@ cw_relax_columns_kernel(int op, const float* __restrict__ lb, const float* __res
   pdl_sync();
   const int64_t ncol = C * hw;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < ncol; t += (int64_t)gridDim.x * blockDim.x)
-    cw_relax_column(op, lb[t], ub[t], norm_l[t], norm_u[t], p, eps, t, (t % hw) * C + t / hw, ncol, out_lb, out_ub, coef, violation);
+    cw_relax_column(op, lb[t], ub[t], norm_l[t], norm_u[t], p, eps, t, kAbi ? t : (t % hw) * C + t / hw, ncol, out_lb, out_ub, coef, violation);
 }
 
 // Rescale of a relaxation on compact rows: out_lw = c_ll lw + c_lu uw, out_uw = c_uu uw + c_ul lw (the expressions of
 // the dense kernel).  A warp per row: the window is worked out once, the lanes interleave over its elements.
+template <bool kAbi>
 __global__ void __launch_bounds__(256)
 cw_rescale_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw, const float* __restrict__ coef,
-                  float* __restrict__ o_lw, float* __restrict__ o_uw, int64_t rows, int64_t row_start, const CwShape g) {
+                  float* __restrict__ o_lw, float* __restrict__ o_uw, int64_t rows, int64_t row_start, const __grid_constant__ CwShape<kAbi> g) {
   pdl_sync();
   const int lane = threadIdx.x & 31;
   const int64_t lr = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -451,12 +505,13 @@ cw_rescale_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw
   const int64_t ncol = (int64_t)g.C * g.H * g.W;
   int yi, xi;
   pixel_of_row(row_start + lr, g.H0, g.W0, yi, xi);
-  const int ylo = g.y.lo(yi), xlo = g.x.lo(xi), ah = g.y.hi(yi) - ylo + 1, aw = g.x.hi(xi) - xlo + 1;
+  const Span wy = g.rows(yi), wx = g.cols(xi);
   for (int e = lane; e < per_row; e += 32) {
-    const int c = e % g.C, dx = (e / g.C) % g.ww, dy = e / (g.C * g.ww);
+    int c, dy, dx;
+    g.split(e, c, dy, dx);
     float lo = 0.f, up = 0.f;
-    if (dy < ah && dx < aw) {
-      const int64_t col = ((int64_t)(ylo + dy) * g.W + xlo + dx) * g.C + c;
+    if (wy.lo + dy <= wy.hi && wx.lo + dx <= wx.hi) {
+      const int64_t pos = (int64_t)(wy.lo + dy) * g.W + wx.lo + dx, col = kAbi ? (int64_t)c * g.H * g.W + pos : pos * g.C + c;
       const float a = z_lw[lr * per_row + e], b = z_uw[lr * per_row + e];
       lo = fmaf(coef[col], a, fmul(coef[ncol + col], b));
       up = fmaf(coef[3 * ncol + col], b, fmul(coef[2 * ncol + col], a));
@@ -477,6 +532,7 @@ cw_rescale_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw
 // 3072 rows, 288 elements, 10 outputs, and 9 us to write the rescaled rows first; 12 us now).
 constexpr int kCwPx = 8, kCwLinWarps = 24, kCwLinThreads = 32 * kCwLinWarps;   // 24: the rows of 8 pixels of 3 channels
 
+template <bool kAbi>
 struct CwLinearArgs {
   const float *z_lw, *z_uw, *coef, *W;
   float *y_lw, *y_uw, *part;
@@ -485,12 +541,12 @@ struct CwLinearArgs {
   int bias_blocks;
   int64_t rows, row_start;
   int ci0, n_ci, N, nb, ny_max, nx_max, p;
-  CwShape g;
+  CwShape<kAbi> g;
 };
 
-template <int NB>
+template <int NB, bool kAbi>
 __global__ void __launch_bounds__(kCwLinThreads)
-cw_linear_kernel(const __grid_constant__ CwLinearArgs q) {
+cw_linear_kernel(const __grid_constant__ CwLinearArgs<kAbi> q) {
   touch_params(q);
   pdl_sync();
   constexpr int LDN = NB + 2, LDP = 32 * LDN + 2;   // the lanes' 64-bit reads, along the channels, and the stores, along the
@@ -498,7 +554,7 @@ cw_linear_kernel(const __grid_constant__ CwLinearArgs q) {
   extern __shared__ __align__(16) float cw_smem[];
   __shared__ float s_red[2][kCwLinWarps][16];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const CwShape& g = q.g;
+  const CwShape<kAbi>& g = q.g;
   const int64_t ncol = (int64_t)g.C * g.H * g.W;
   if ((int)blockIdx.x < q.bias_blocks) {
     if (blockIdx.y > 0) return;
@@ -530,7 +586,8 @@ cw_linear_kernel(const __grid_constant__ CwLinearArgs q) {
   const int n0 = blockIdx.y * q.nb, nb = min(q.nb, q.N - n0);
   // the union of the windows (their ends do not decrease along the pixels)
   const int ylo = g.y.lo(yi), yhi = g.y.hi(yi), xl = g.x.lo(x0), nxr = max(0, g.x.hi(x0 + npx - 1) - xl + 1), rows_here = npx * q.n_ci;
-  const int64_t per_pos = g.C, per_row = (int64_t)g.wh * g.ww * g.C;
+  const int64_t per_pos = g.step_x(), per_row = (int64_t)g.wh * g.ww * g.C;
+  const Span wy = kAbi ? g.rows(yi) : Span{ylo, yhi};   // window rows of the tile's pixels
   float pl = 0.f, pu = 0.f;   // accumulated norms of this lane's output
   for (int r0 = 0; r0 < rows_here; r0 += kCwLinWarps) {
     float sc[NB], sr[NB];
@@ -538,7 +595,8 @@ cw_linear_kernel(const __grid_constant__ CwLinearArgs q) {
     for (int n = 0; n < NB; ++n) sc[n] = sr[n] = 0.f;
     const int t = r0 + warp, px = t % npx, ci = q.ci0 + t / npx;
     int64_t lr = -1;
-    const int wlo = g.x.lo(x0 + px), aw = g.x.hi(x0 + px) - wlo + 1;
+    const Span wx = g.cols(x0 + px);
+    const int wlo = wx.lo, aw = wx.hi - wlo + 1;
     if (t < rows_here) {
       const int64_t l = ((int64_t)ci * g.H0 + yi) * g.W0 + x0 + px - q.row_start;
       if (l >= 0 && l < q.rows) lr = l;
@@ -561,11 +619,12 @@ cw_linear_kernel(const __grid_constant__ CwLinearArgs q) {
         }
         // the row's elements, three at a time: those of the next step are loaded before the arithmetic of this one
         const bool mine = lr >= 0 && c < g.C && aw > 0;
-        const int steps_x = (aw + 2) / 3, steps = mine ? (yb - ya + 1) * steps_x : 0;
+        const int y_first = kAbi ? max(ya, wy.lo) : ya, y_last = kAbi ? min(yb, wy.hi) : yb;
+        const int steps_x = (aw + 2) / 3, steps = mine ? max(0, y_last - y_first + 1) * steps_x : 0;
         float zl[3], zu[3], kf[4][3];
-        int sy = ya, sx = 0;   // the next step: row, first column of the window
+        int sy = y_first, sx = 0;   // the next step: row, first column of the window
         auto load = [&] {
-          const int64_t zb = lr * per_row + ((int64_t)(sy - ylo) * g.ww + sx) * per_pos + c, cb = ((int64_t)sy * g.W + wlo + sx) * g.C + c;
+          const int64_t zb = lr * per_row + ((int64_t)(sy - wy.lo) * g.ww + sx) * per_pos + (int64_t)c * g.step_c(), cb = ((int64_t)sy * g.W + wlo + sx) * g.C + c;
 #pragma unroll
           for (int e = 0; e < 3; ++e) {
             const bool in = sx + e < aw;
@@ -662,14 +721,15 @@ cw_linear_range_kernel(const float* __restrict__ part, const float* __restrict__
 }
 
 // Dense rows from compact ones: one block per row, zeros outside the window.
+template <bool kAbi>
 __global__ void __launch_bounds__(256)
 cw_expand_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw, float* __restrict__ y_lw,
-                 float* __restrict__ y_uw, int64_t row_start, const CwShape g) {
+                 float* __restrict__ y_uw, int64_t row_start, const __grid_constant__ CwShape<kAbi> g) {
   pdl_sync();
   const int64_t r = row_start + blockIdx.x;
   int yi, xi;
   pixel_of_row(r, g.H0, g.W0, yi, xi);
-  const int ylo = g.y.lo(yi), yhi = g.y.hi(yi), xlo = g.x.lo(xi), xhi = g.x.hi(xi);
+  const Span wy = g.rows(yi), wx = g.cols(xi);
   const int per_row = g.C * g.wh * g.ww;
   const unsigned n = (unsigned)g.C * g.H * g.W, uW = g.W, uH = g.H;
   const float* zl = z_lw + (int64_t)blockIdx.x * per_row;
@@ -679,8 +739,8 @@ cw_expand_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw,
   for (unsigned t = threadIdx.x; t < n; t += blockDim.x) {
     const unsigned q = t / uW, x = t - q * uW, c = q / uH, y = q - c * uH;
     float lo = 0.f, up = 0.f;
-    if ((int)y >= ylo && (int)y <= yhi && (int)x >= xlo && (int)x <= xhi) {
-      const int e = (((int)y - ylo) * g.ww + ((int)x - xlo)) * g.C + (int)c;
+    if ((int)y >= wy.lo && (int)y <= wy.hi && (int)x >= wx.lo && (int)x <= wx.hi) {
+      const int e = (((int)y - wy.lo) * g.ww + ((int)x - wx.lo)) * g.step_x() + (int)c * g.step_c();
       lo = zl[e];
       up = zu[e];
     }
@@ -689,7 +749,8 @@ cw_expand_kernel(const float* __restrict__ z_lw, const float* __restrict__ z_uw,
   }
 }
 
-int make_shape(const int* chain, int n_chain, int H0, int W0, int C, int H, int W, CwShape& g) {
+template <bool kAbi>
+int make_shape(const int* chain, int n_chain, int H0, int W0, int C, int H, int W, CwShape<kAbi>& g) {
   int h, w;
   ConvChain ch;
   int rc = chain_from_host(chain, n_chain, H0, W0, ch, h, w);
@@ -699,7 +760,13 @@ int make_shape(const int* chain, int n_chain, int H0, int W0, int C, int H, int 
   rc = axis_from_chain(ch, ch.kh, H, g.y);
   if (rc == FB_OK) rc = axis_from_chain(ch, ch.kw, W, g.x);
   if (rc != FB_OK) return rc;
-  g.wh = axis_extent(g.y, H0), g.ww = axis_extent(g.x, W0);
+  if constexpr (kAbi) {
+    g.ch = ch;
+    g.wh = chain_extent(ch, ch.kh, H0), g.ww = chain_extent(ch, ch.kw, W0);
+    g.same = axis_is_chain(g.y, ch, ch.kh, H0) && axis_is_chain(g.x, ch, ch.kw, W0);
+  } else {
+    g.wh = axis_extent(g.y, H0), g.ww = axis_extent(g.x, W0);
+  }
   if ((int64_t)C * H * W > 0x7fffffff || (int64_t)C * g.wh * g.ww > 0x7fffffff) return FB_ERR_SHAPE;
   return FB_OK;
 }
@@ -716,18 +783,17 @@ inline void row_channels(int64_t row_start, int64_t rows, int H0, int W0, int& c
   n_ci = (int)((row_start + rows - 1) / hw) - ci0 + 1;
 }
 
-}  // namespace
-
 // z_lo == nullptr: the rows of the first convolution, from its filter W1 and the slopes k_l, k_u (chain has one entry).
 // b_lo != nullptr: the bias image goes along (b_lo, b_up [Cin, H, W] -> yb_lo, yb_up).
-int cw_conv_ex(const float* z_lo, const float* z_up, const float* W1, const float* k_l, const float* k_u, float scale, int Cin0,
+template <bool kAbi>
+int conv_rows(const float* z_lo, const float* z_up, const float* W1, const float* k_l, const float* k_u, float scale, int Cin0,
                const float* Wt, float* y_lo, float* y_up, const float* b_lo, const float* b_up, const float* bias, float* yb_lo,
                float* yb_up, int64_t rows, int64_t row_start, int H0, int W0, const int* chain, int n_chain, int Cin, int H, int W,
                int Cout, int Kh, int Kw, int stride, int pad, cudaStream_t st) {
   if (rows < 0 || row_start < 0 || Cin <= 0 || Cout <= 0 || Kh <= 0 || Kw <= 0 || stride <= 0 || pad < 0 || n_chain < 1)
     return FB_ERR_ARG;
   if (n_chain >= kMaxChain) return FB_ERR_SHAPE;
-  CwShape gi, go;
+  CwShape<kAbi> gi, go;
   int rc = make_shape(chain, n_chain, H0, W0, Cin, H, W, gi);
   if (rc != FB_OK) return rc;
   const int Ho = (H + 2 * pad - Kh) / stride + 1, Wo = (W + 2 * pad - Kw) / stride + 1;
@@ -740,7 +806,8 @@ int cw_conv_ex(const float* z_lo, const float* z_up, const float* W1, const floa
   if (rows == 0) return FB_OK;
   if (rows > 0x7fffffff) return FB_ERR_SHAPE;
 
-  CwConvArgs q = {};
+  CwConvParams<kAbi> q = {};
+  if constexpr (kAbi) q.ch = go.ch;
   q.z_lo = z_lo, q.z_up = z_up, q.W1 = W1, q.k_l = k_l, q.k_u = k_u, q.scale = scale, q.Cin0 = Cin0;
   q.Wt = Wt, q.y_lo = y_lo, q.y_up = y_up;
   q.b_lo = b_lo, q.b_up = b_up, q.bias = bias, q.yb_lo = yb_lo, q.yb_up = yb_up;
@@ -778,25 +845,31 @@ int cw_conv_ex(const float* z_lo, const float* z_up, const float* W1, const floa
   q.blocks_bias = b_lo != nullptr ? (int)std::min<int64_t>(ceil_div(out, threads), device_info().sms) : 0;
   const int64_t blocks = q.blocks_bias + (int64_t)cls_y * q.cls_x * q.per_class;
   if (blocks > 0x7fffffff) return FB_ERR_SHAPE;
-  auto kern = Kh == 3 && Kw == 3 ? (cpt == 2 ? cw_conv_kernel<3, 2> : cw_conv_kernel<3, 1>)
-                                 : (cpt == 2 ? cw_conv_kernel<0, 2> : cw_conv_kernel<0, 1>);
+  auto kern = Kh == 3 && Kw == 3 ? (cpt == 2 ? cw_conv_kernel<3, 2, kAbi> : cw_conv_kernel<3, 1, kAbi>)
+                                 : (cpt == 2 ? cw_conv_kernel<0, 2, kAbi> : cw_conv_kernel<0, 1, kAbi>);
   if (int rc = ensure_dynamic_smem(kern, bytes() + kCwStatic)) return rc;   // (48 KB without the attribute hold the static part too)
   ProfileScope prof(PK_CONV, 8.0 * rows * Cout * go.wh * go.ww * Cin * Kh * Kw,
                     4.0 * 2.0 * rows * ((double)Cin * gi.wh * gi.ww + (double)Cout * go.wh * go.ww), (void*)st);
+  if (kAbi) {   // (the kernel stores the pixels' own windows)
+    const size_t n = sizeof(float) * (size_t)rows * Cout * go.wh * go.ww;
+    FB_CUDA_OK(cudaMemsetAsync(y_lo, 0, n, st));
+    FB_CUDA_OK(cudaMemsetAsync(y_up, 0, n, st));
+  }
   fb::launch_k(kern, (unsigned)blocks, threads, bytes(), st, q);
   FB_LAUNCH_OK();
   return FB_OK;
 }
 
-int64_t cw_linear_tiles(int H0, int W0) { return (int64_t)H0 * ceil_div(W0, kCwPx); }
+inline int64_t linear_tiles(int H0, int W0) { return (int64_t)H0 * ceil_div(W0, kCwPx); }
 
 // coef != nullptr: the rows go through that rescale first.  part != nullptr: no rows are written, but the partial norms
-// [cw_linear_tiles][2][N].  lb != nullptr: the bias part goes along.
-int cw_linear_ex(const float* z_lw, const float* z_uw, const float* coef, const float* Wl, float* y_lw, float* y_uw, float* part,
+// [linear_tiles][2][N].  lb != nullptr: the bias part goes along.
+template <bool kAbi>
+int linear_rows(const float* z_lw, const float* z_uw, const float* coef, const float* Wl, float* y_lw, float* y_uw, float* part,
                  const float* lb, const float* ub, const float* bias, float* y_lb, float* y_ub, int64_t rows, int64_t row_start, int H0,
                  int W0, const int* chain, int n_chain, int C, int H, int W, int N, int p, cudaStream_t st) {
   if (rows < 0 || row_start < 0 || N <= 0) return FB_ERR_ARG;
-  CwLinearArgs q = {};
+  CwLinearArgs<kAbi> q = {};
   int rc = make_shape(chain, n_chain, H0, W0, C, H, W, q.g);
   if (rc != FB_OK) return rc;
   if (rows == 0) return FB_OK;
@@ -818,16 +891,125 @@ int cw_linear_ex(const float* z_lw, const float* z_uw, const float* coef, const 
   q.nb = (int)ceil_div(N, groups);
   NB = (int)ceil_div(q.nb, 4) * 4;
   q.ny_max = (int)std::max<int64_t>(1, std::min<int64_t>(q.g.wh, (int64_t)(limit / 2 / row_bytes())));   // two blocks per SM where that is possible
-  const int64_t blocks = q.bias_blocks + cw_linear_tiles(H0, W0);
+  const int64_t blocks = q.bias_blocks + linear_tiles(H0, W0);
   if (blocks > 0x7fffffff || groups > 65535) return FB_ERR_SHAPE;
   const size_t smem = row_bytes() * q.ny_max;
-  auto kern = NB == 4 ? cw_linear_kernel<4> : NB == 8 ? cw_linear_kernel<8> : NB == 12 ? cw_linear_kernel<12> : cw_linear_kernel<16>;
+  auto kern = NB == 4    ? cw_linear_kernel<4, kAbi>
+              : NB == 8  ? cw_linear_kernel<8, kAbi>
+              : NB == 12 ? cw_linear_kernel<12, kAbi>
+                         : cw_linear_kernel<16, kAbi>;
   if (int rc = ensure_dynamic_smem(kern, smem + kCwStatic)) return rc;
   ProfileScope prof(PK_MATMUL, 8.0 * rows * C * q.g.wh * q.g.ww * N,
                     4.0 * (2.0 * rows * C * q.g.wh * q.g.ww + 2.0 * rows * N + (double)C * H * W * N), (void*)st);
   fb::launch_k(kern, dim3((unsigned)blocks, (unsigned)groups), kCwLinThreads, smem, st, q);
   FB_LAUNCH_OK();
   return FB_OK;
+}
+
+// op < 0: partial accumulations to part_l / part_u; else the coefficients of the relaxation and the relaxed bias terms.
+template <bool kAbi>
+int norm_columns(int op, const float* z_lw, const float* z_uw, float* part_l, float* part_u, const float* lb, const float* ub, float* out_lb,
+               float* out_ub, float* coef, int64_t rows, int64_t row_start, int Cin0, int H0, int W0, const int* chain, int n_chain, int C,
+               int H, int W, int p, float eps, int* violation, cudaStream_t st) {
+  if (rows < 0 || row_start < 0 || Cin0 <= 0 || !valid_norm(p) || row_start + rows > (int64_t)Cin0 * H0 * W0) return FB_ERR_ARG;
+  CwShape<kAbi> g;
+  int rc = make_shape(chain, n_chain, H0, W0, C, H, W, g);
+  if (rc != FB_OK) return rc;
+  if (ceil_div(C, 32) > 65535 || (int64_t)Cin0 * H0 * W0 > 0x7fffffff) return FB_ERR_SHAPE;
+  ProfileScope prof(PK_RELAX, 4.0 * rows * C * g.wh * g.ww, 4.0 * (2.0 * rows * C * g.wh * g.ww + 2.0 * C * H * W), (void*)st);
+  fb::launch_k(cw_norm_kernel<kAbi>, dim3((unsigned)(H * W), (unsigned)ceil_div(C, 32)), 32 * kCwNormWarps, 0, st, op, z_lw, z_uw, part_l, part_u, lb, ub, out_lb, out_ub, coef, rows, row_start, Cin0, g, p, eps, violation);
+  FB_LAUNCH_OK();
+  return FB_OK;
+}
+
+template <bool kAbi>
+int relax_columns(int op, const float* lb, const float* ub, const float* norm_l, const float* norm_u, float* out_lb, float* out_ub,
+                  float* coef, int C, int64_t hw, int p, float eps, int* violation, cudaStream_t st) {
+  fb::launch_k(cw_relax_columns_kernel<kAbi>, grid_for(C * hw, 256), 256, 0, st, op, lb, ub, norm_l, norm_u, out_lb, out_ub, coef, C, hw, p, eps, violation);
+  FB_LAUNCH_OK();
+  return FB_OK;
+}
+
+template <bool kAbi>
+int rescale_rows(const float* z_lw, const float* z_uw, const float* coef, float* out_lw, float* out_uw, int64_t rows, int64_t row_start,
+                    int H0, int W0, const int* chain, int n_chain, int C, int H, int W, cudaStream_t st) {
+  CwShape<kAbi> g;
+  int rc = make_shape(chain, n_chain, H0, W0, C, H, W, g);
+  if (rc != FB_OK || rows == 0) return rc;
+  fb::launch_k(cw_rescale_kernel<kAbi>, (unsigned)ceil_div(rows, 8), 256, 0, st, z_lw, z_uw, coef, out_lw, out_uw, rows, row_start, g);
+  FB_LAUNCH_OK();
+  return FB_OK;
+}
+
+// First convolution and relaxation (op < 0: none): the columns' slopes, then the rows.
+template <bool kAbi>
+int identity_rows(int op, const float* x_lb, const float* x_ub, const float* Wt, const float* bias, float scale, float* z_lw, float* z_uw,
+                  float* y_lb, float* y_ub, float* col_ws, int64_t rows, int64_t row_start, int Cin, int H, int W, int Cout, int Kh, int Kw,
+                  int stride, int pad, int p, float eps, int* violation, cudaStream_t st) {
+  if (rows < 0 || row_start < 0 || Cin <= 0 || H <= 0 || W <= 0 || Cout <= 0 || Kh <= 0 || Kw <= 0 || stride <= 0 || pad < 0 ||
+      !valid_norm(p) || row_start + rows > (int64_t)Cin * H * W)
+    return FB_ERR_ARG;
+  if (op >= 0 && !(op >= FB_RELU && op <= FB_SQRT)) return FB_ERR_ARG;
+  const int chain[4] = {Kh, Kw, stride, pad};
+  CwShape<kAbi> g;
+  const int Ho = (H + 2 * pad - Kh) / stride + 1, Wo = (W + 2 * pad - Kw) / stride + 1;
+  if (Ho <= 0 || Wo <= 0) return FB_ERR_SHAPE;
+  int rc = make_shape(chain, 1, H, W, Cout, Ho, Wo, g);
+  if (rc != FB_OK) return rc;
+  const int64_t ncol = (int64_t)Cout * Ho * Wo;
+  ProfileScope prof(PK_CONV, 2.0 * rows * Cout * g.wh * g.ww, 4.0 * 2.0 * rows * Cout * g.wh * g.ww, (void*)st);
+  float* k_l = col_ws;
+  float* k_u = col_ws + ncol;
+  rc = launch_identity_columns(op, x_lb, x_ub, Wt, bias, y_lb, y_ub, k_l, k_u, scale, Cin, H, W, Cout, Kh, Kw, stride, pad, Ho, Wo, p, eps,
+                               violation, st);
+  if (rc != FB_OK || rows == 0) return rc;
+  fb::launch_k(cw_identity_rows_kernel<kAbi>, grid_for(rows * Cout * g.wh * g.ww, 256), 256, 0, st, Wt, k_l, k_u, z_lw, z_uw, scale, rows, row_start,
+                                                                                   Cin, H, W, Cout, Kh, Kw, stride, pad, Ho, Wo,
+                                                                                   g.wh, g.ww);
+  FB_LAUNCH_OK();
+  return FB_OK;
+}
+
+// Dense rows [rows, C, H, W].
+template <bool kAbi>
+int expand_rows(const float* z_lw, const float* z_uw, float* y_lw, float* y_uw, int64_t rows, int64_t row_start, int H0, int W0,
+                const int* chain, int n_chain, int C, int H, int W, cudaStream_t st) {
+  if (rows < 0 || row_start < 0) return FB_ERR_ARG;
+  CwShape<kAbi> g;
+  int rc = make_shape(chain, n_chain, H0, W0, C, H, W, g);
+  if (rc != FB_OK) return rc;
+  if (rows == 0) return FB_OK;
+  if (rows > 0x7fffffff) return FB_ERR_SHAPE;
+  ProfileScope prof(PK_ELEMENTWISE, 0.0, 4.0 * 2.0 * rows * C * H * W, (void*)st);
+  fb::launch_k(cw_expand_kernel<kAbi>, (unsigned)rows, 256, 0, st, z_lw, z_uw, y_lw, y_uw, row_start, g);
+  FB_LAUNCH_OK();
+  return FB_OK;
+}
+
+}  // namespace
+
+int cw_identity_rows(int op, const float* x, const float* Wt, const float* bias, float* z_lw, float* z_uw, float* y_lb, float* y_ub,
+                     float* col_ws, int64_t rows, int64_t row_start, int Cin, int H, int W, int Cout, int Kh, int Kw, int stride, int pad,
+                     int p, float eps, int* violation, cudaStream_t st) {
+  return identity_rows<false>(op, x, x, Wt, bias, 1.0f, z_lw, z_uw, y_lb, y_ub, col_ws, rows, row_start, Cin, H, W, Cout, Kh, Kw, stride, pad,
+                              p, eps, violation, st);
+}
+
+int cw_conv_ex(const float* z_lo, const float* z_up, const float* W1, const float* k_l, const float* k_u, float scale, int Cin0,
+               const float* Wt, float* y_lo, float* y_up, const float* b_lo, const float* b_up, const float* bias, float* yb_lo,
+               float* yb_up, int64_t rows, int64_t row_start, int H0, int W0, const int* chain, int n_chain, int Cin, int H, int W,
+               int Cout, int Kh, int Kw, int stride, int pad, cudaStream_t st) {
+  return conv_rows<false>(z_lo, z_up, W1, k_l, k_u, scale, Cin0, Wt, y_lo, y_up, b_lo, b_up, bias, yb_lo, yb_up, rows, row_start, H0, W0,
+                          chain, n_chain, Cin, H, W, Cout, Kh, Kw, stride, pad, st);
+}
+
+int64_t cw_linear_tiles(int H0, int W0) { return linear_tiles(H0, W0); }
+
+int cw_linear_ex(const float* z_lw, const float* z_uw, const float* coef, const float* Wl, float* y_lw, float* y_uw, float* part,
+                 const float* lb, const float* ub, const float* bias, float* y_lb, float* y_ub, int64_t rows, int64_t row_start, int H0,
+                 int W0, const int* chain, int n_chain, int C, int H, int W, int N, int p, cudaStream_t st) {
+  return linear_rows<false>(z_lw, z_uw, coef, Wl, y_lw, y_uw, part, lb, ub, bias, y_lb, y_ub, rows, row_start, H0, W0, chain, n_chain, C, H,
+                            W, N, p, st);
 }
 
 int cw_linear_range(const float* part, const float* lb, const float* ub, float* l, float* u, int H0, int W0, int N, int p, float eps,
@@ -837,36 +1019,26 @@ int cw_linear_range(const float* part, const float* lb, const float* ub, float* 
   return FB_OK;
 }
 
-// op < 0: partial accumulations to part_l / part_u; else the coefficients of the relaxation and the relaxed bias terms.
 int cw_norm_ex(int op, const float* z_lw, const float* z_uw, float* part_l, float* part_u, const float* lb, const float* ub, float* out_lb,
                float* out_ub, float* coef, int64_t rows, int64_t row_start, int Cin0, int H0, int W0, const int* chain, int n_chain, int C,
                int H, int W, int p, float eps, int* violation, cudaStream_t st) {
-  if (rows < 0 || row_start < 0 || Cin0 <= 0 || !valid_norm(p) || row_start + rows > (int64_t)Cin0 * H0 * W0) return FB_ERR_ARG;
-  CwShape g;
-  int rc = make_shape(chain, n_chain, H0, W0, C, H, W, g);
-  if (rc != FB_OK) return rc;
-  if (ceil_div(C, 32) > 65535 || (int64_t)Cin0 * H0 * W0 > 0x7fffffff) return FB_ERR_SHAPE;
-  ProfileScope prof(PK_RELAX, 4.0 * rows * C * g.wh * g.ww, 4.0 * (2.0 * rows * C * g.wh * g.ww + 2.0 * C * H * W), (void*)st);
-  fb::launch_k(cw_norm_kernel, dim3((unsigned)(H * W), (unsigned)ceil_div(C, 32)), 32 * kCwNormWarps, 0, st, op, z_lw, z_uw, part_l, part_u, lb, ub, out_lb, out_ub, coef, rows, row_start, Cin0, g, p, eps, violation);
-  FB_LAUNCH_OK();
-  return FB_OK;
+  return norm_columns<false>(op, z_lw, z_uw, part_l, part_u, lb, ub, out_lb, out_ub, coef, rows, row_start, Cin0, H0, W0, chain, n_chain, C,
+                             H, W, p, eps, violation, st);
 }
 
 int cw_relax_columns(int op, const float* lb, const float* ub, const float* norm_l, const float* norm_u, float* out_lb, float* out_ub,
                      float* coef, int C, int64_t hw, int p, float eps, int* violation, cudaStream_t st) {
-  fb::launch_k(cw_relax_columns_kernel, grid_for(C * hw, 256), 256, 0, st, op, lb, ub, norm_l, norm_u, out_lb, out_ub, coef, C, hw, p, eps, violation);
-  FB_LAUNCH_OK();
-  return FB_OK;
+  return relax_columns<false>(op, lb, ub, norm_l, norm_u, out_lb, out_ub, coef, C, hw, p, eps, violation, st);
 }
 
 int cw_rescale_rows(const float* z_lw, const float* z_uw, const float* coef, float* out_lw, float* out_uw, int64_t rows, int64_t row_start,
                     int H0, int W0, const int* chain, int n_chain, int C, int H, int W, cudaStream_t st) {
-  CwShape g;
-  int rc = make_shape(chain, n_chain, H0, W0, C, H, W, g);
-  if (rc != FB_OK || rows == 0) return rc;
-  fb::launch_k(cw_rescale_kernel, (unsigned)ceil_div(rows, 8), 256, 0, st, z_lw, z_uw, coef, out_lw, out_uw, rows, row_start, g);
-  FB_LAUNCH_OK();
-  return FB_OK;
+  return rescale_rows<false>(z_lw, z_uw, coef, out_lw, out_uw, rows, row_start, H0, W0, chain, n_chain, C, H, W, st);
+}
+
+int cw_expand_rows(const float* z_lw, const float* z_uw, float* y_lw, float* y_uw, int64_t rows, int64_t row_start, int H0, int W0,
+                   const int* chain, int n_chain, int C, int H, int W, cudaStream_t st) {
+  return expand_rows<false>(z_lw, z_uw, y_lw, y_uw, rows, row_start, H0, W0, chain, n_chain, C, H, W, st);
 }
 
 }  // namespace fb
@@ -879,11 +1051,7 @@ extern "C" int fb_cw_extent(int H0, int W0, const int* chain, int n_chain, int* 
   int h, w;
   int rc = chain_from_host(chain, n_chain, H0, W0, ch, h, w);
   if (rc != FB_OK) return rc;
-  CwAxis y, x;
-  rc = axis_from_chain(ch, ch.kh, h, y);
-  if (rc == FB_OK) rc = axis_from_chain(ch, ch.kw, w, x);
-  if (rc != FB_OK) return rc;
-  *wh = axis_extent(y, H0), *ww = axis_extent(x, W0);
+  *wh = chain_extent(ch, ch.kh, H0), *ww = chain_extent(ch, ch.kw, W0);
   return FB_OK;
 }
 
@@ -892,45 +1060,24 @@ extern "C" int fb_cw_identity_relax_f32(int op, const float* x_lb, const float* 
                                         int64_t rows, int64_t row_start, int Cin, int H, int W, int Cout, int Kh, int Kw,
                                         int stride, int pad, int p, float eps, int* violation, void* stream) {
   if (!x_lb || !x_ub || !Wt || !z_lw || !z_uw || !y_lb || !y_ub || !col_ws) return FB_ERR_ARG;
-  if (rows < 0 || row_start < 0 || Cin <= 0 || H <= 0 || W <= 0 || Cout <= 0 || Kh <= 0 || Kw <= 0 || stride <= 0 || pad < 0 ||
-      !valid_norm(p) || row_start + rows > (int64_t)Cin * H * W)
-    return FB_ERR_ARG;
-  if (op >= 0 && !(op >= FB_RELU && op <= FB_SQRT)) return FB_ERR_ARG;
-  const int chain[4] = {Kh, Kw, stride, pad};
-  CwShape g;
-  const int Ho = (H + 2 * pad - Kh) / stride + 1, Wo = (W + 2 * pad - Kw) / stride + 1;
-  if (Ho <= 0 || Wo <= 0) return FB_ERR_SHAPE;
-  int rc = make_shape(chain, 1, H, W, Cout, Ho, Wo, g);
-  if (rc != FB_OK) return rc;
-  cudaStream_t st = (cudaStream_t)stream;
-  const int64_t ncol = (int64_t)Cout * Ho * Wo;
-  ProfileScope prof(PK_CONV, 2.0 * rows * Cout * g.wh * g.ww, 4.0 * 2.0 * rows * Cout * g.wh * g.ww, stream);
-  float* k_l = col_ws;
-  float* k_u = col_ws + ncol;
-  rc = launch_identity_columns(op, x_lb, x_ub, Wt, bias, y_lb, y_ub, k_l, k_u, scale, Cin, H, W, Cout, Kh, Kw, stride, pad, Ho, Wo, p, eps,
-                               violation, st);
-  if (rc != FB_OK || rows == 0) return rc;
-  fb::launch_k(cw_identity_rows_kernel, grid_for(rows * Cout * g.wh * g.ww, 256), 256, 0, st, Wt, k_l, k_u, z_lw, z_uw, scale, rows, row_start,
-                                                                                   Cin, H, W, Cout, Kh, Kw, stride, pad, Ho, Wo,
-                                                                                   g.wh, g.ww);
-  FB_LAUNCH_OK();
-  return FB_OK;
+  return identity_rows<true>(op, x_lb, x_ub, Wt, bias, scale, z_lw, z_uw, y_lb, y_ub, col_ws, rows, row_start, Cin, H, W, Cout, Kh, Kw,
+                             stride, pad, p, eps, violation, (cudaStream_t)stream);
 }
 
 extern "C" int fb_cw_conv2d_f32(const float* x_lw, const float* x_uw, const float* Wt, float* y_lw, float* y_uw, int64_t rows,
                                 int64_t row_start, int H0, int W0, const int* chain, int n_chain, int Cin, int H, int W,
                                 int Cout, int Kh, int Kw, int stride, int pad, void* stream) {
   if (!x_lw || !x_uw || !Wt || !y_lw || !y_uw) return FB_ERR_ARG;
-  return cw_conv_ex(x_lw, x_uw, nullptr, nullptr, nullptr, 1.f, 0, Wt, y_lw, y_uw, nullptr, nullptr, nullptr, nullptr, nullptr, rows,
-                    row_start, H0, W0, chain, n_chain, Cin, H, W, Cout, Kh, Kw, stride, pad, (cudaStream_t)stream);
+  return conv_rows<true>(x_lw, x_uw, nullptr, nullptr, nullptr, 1.f, 0, Wt, y_lw, y_uw, nullptr, nullptr, nullptr, nullptr, nullptr, rows,
+                         row_start, H0, W0, chain, n_chain, Cin, H, W, Cout, Kh, Kw, stride, pad, (cudaStream_t)stream);
 }
 
 extern "C" int fb_cw_norm_partials_f32(const float* z_lw, const float* z_uw, float* part_l, float* part_u, int64_t rows,
                                        int64_t row_start, int Cin0, int H0, int W0, const int* chain, int n_chain, int C, int H,
                                        int W, int p, void* stream) {
   if (!z_lw || !z_uw || !part_l || !part_u) return FB_ERR_ARG;
-  return cw_norm_ex(-1, z_lw, z_uw, part_l, part_u, nullptr, nullptr, nullptr, nullptr, nullptr, rows, row_start, Cin0, H0, W0, chain,
-                    n_chain, C, H, W, p, 0.f, nullptr, (cudaStream_t)stream);
+  return norm_columns<true>(-1, z_lw, z_uw, part_l, part_u, nullptr, nullptr, nullptr, nullptr, nullptr, rows, row_start, Cin0, H0, W0, chain,
+                            n_chain, C, H, W, p, 0.f, nullptr, (cudaStream_t)stream);
 }
 
 extern "C" int fb_cw_relax_apply_f32(int op, const float* z_lw, const float* z_uw, const float* lb, const float* ub,
@@ -941,35 +1088,26 @@ extern "C" int fb_cw_relax_apply_f32(int op, const float* z_lw, const float* z_u
   if (op < FB_RELU || op > FB_SQRT) return FB_ERR_ARG;
   if (!z_lw || !z_uw || !lb || !ub || !norm_l || !norm_u || !out_lw || !out_uw || !out_lb || !out_ub || !coef_ws) return FB_ERR_ARG;
   if (rows < 0 || row_start < 0 || !valid_norm(p)) return FB_ERR_ARG;
-  CwShape g;
+  CwShape<true> g;
   int rc = make_shape(chain, n_chain, H0, W0, C, H, W, g);
   if (rc != FB_OK) return rc;
   const int64_t ncol = (int64_t)C * H * W, per_row = (int64_t)C * g.wh * g.ww;
   ProfileScope prof(PK_RELAX, 4.0 * rows * per_row, 4.0 * (4.0 * rows * per_row + 10.0 * ncol), stream);
-  rc = cw_relax_columns(op, lb, ub, norm_l, norm_u, out_lb, out_ub, coef_ws, C, (int64_t)H * W, p, eps, violation, (cudaStream_t)stream);
+  rc = relax_columns<true>(op, lb, ub, norm_l, norm_u, out_lb, out_ub, coef_ws, C, (int64_t)H * W, p, eps, violation, (cudaStream_t)stream);
   if (rc != FB_OK) return rc;
-  return cw_rescale_rows(z_lw, z_uw, coef_ws, out_lw, out_uw, rows, row_start, H0, W0, chain, n_chain, C, H, W, (cudaStream_t)stream);
+  return rescale_rows<true>(z_lw, z_uw, coef_ws, out_lw, out_uw, rows, row_start, H0, W0, chain, n_chain, C, H, W, (cudaStream_t)stream);
 }
 
 extern "C" int fb_cw_linear_f32(const float* z_lw, const float* z_uw, const float* Wl, float* y_lw, float* y_uw, float* wt_ws,
                                 int64_t rows, int64_t row_start, int H0, int W0, const int* chain, int n_chain, int C, int H,
                                 int W, int N, void* stream) {
   if (!z_lw || !z_uw || !Wl || !y_lw || !y_uw || !wt_ws) return FB_ERR_ARG;
-  return cw_linear_ex(z_lw, z_uw, nullptr, Wl, y_lw, y_uw, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, rows, row_start, H0, W0,
-                      chain, n_chain, C, H, W, N, FB_PINF, (cudaStream_t)stream);
+  return linear_rows<true>(z_lw, z_uw, nullptr, Wl, y_lw, y_uw, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, rows, row_start, H0, W0,
+                           chain, n_chain, C, H, W, N, FB_PINF, (cudaStream_t)stream);
 }
 
 extern "C" int fb_cw_expand_f32(const float* z_lw, const float* z_uw, float* y_lw, float* y_uw, int64_t rows, int64_t row_start,
                                 int H0, int W0, const int* chain, int n_chain, int C, int H, int W, void* stream) {
   if (!z_lw || !z_uw || !y_lw || !y_uw) return FB_ERR_ARG;
-  if (rows < 0 || row_start < 0) return FB_ERR_ARG;
-  CwShape g;
-  int rc = make_shape(chain, n_chain, H0, W0, C, H, W, g);
-  if (rc != FB_OK) return rc;
-  if (rows == 0) return FB_OK;
-  if (rows > 0x7fffffff) return FB_ERR_SHAPE;
-  ProfileScope prof(PK_ELEMENTWISE, 0.0, 4.0 * 2.0 * rows * C * H * W, stream);
-  fb::launch_k(cw_expand_kernel, (unsigned)rows, 256, 0, (cudaStream_t)stream, z_lw, z_uw, y_lw, y_uw, row_start, g);
-  FB_LAUNCH_OK();
-  return FB_OK;
+  return expand_rows<true>(z_lw, z_uw, y_lw, y_uw, rows, row_start, H0, W0, chain, n_chain, C, H, W, (cudaStream_t)stream);
 }

@@ -29,17 +29,31 @@ __host__ __device__ inline Span span_after_conv(Span s, int k, int stride, int p
   return o;
 }
 
+// Window, along one axis (k: the filter sizes of the chain along it) and in the coordinates of the output of the first n
+// convolutions, reached by pixel i of n0.
+__host__ __device__ inline Span chain_span(const ConvChain& ch, const int* k, int n, int n0, int i) {
+  Span s = {i, i};
+  for (int j = 0; j < n; ++j) {
+    n0 = (n0 + 2 * ch.pad[j] - k[j]) / ch.stride[j] + 1;
+    s = span_after_conv(s, k[j], ch.stride[j], ch.pad[j], n0);
+  }
+  return s;
+}
+
 // Window (in the coordinates of the chain's last output) reached by pixel (yi, xi) of the H0 x W0 image.
 __host__ __device__ inline void chain_window(const ConvChain& ch, int H0, int W0, int yi, int xi, Span& wy, Span& wx) {
-  wy.lo = wy.hi = yi;
-  wx.lo = wx.hi = xi;
-  int h = H0, w = W0;
-  for (int i = 0; i < ch.n; ++i) {
-    h = (h + 2 * ch.pad[i] - ch.kh[i]) / ch.stride[i] + 1;
-    w = (w + 2 * ch.pad[i] - ch.kw[i]) / ch.stride[i] + 1;
-    wy = span_after_conv(wy, ch.kh[i], ch.stride[i], ch.pad[i], h);
-    wx = span_after_conv(wx, ch.kw[i], ch.stride[i], ch.pad[i], w);
+  wy = chain_span(ch, ch.kh, ch.n, H0, yi);
+  wx = chain_span(ch, ch.kw, ch.n, W0, xi);
+}
+
+// Largest window along one axis that any pixel of n0 reaches through the chain (at least 1).
+inline int chain_extent(const ConvChain& ch, const int* k, int n0) {
+  int win = 1;
+  for (int i = 0; i < n0; ++i) {
+    const Span s = chain_span(ch, k, ch.n, n0, i);
+    win = std::max(win, s.hi - s.lo + 1);
   }
+  return win;
 }
 
 // Host side: the chain as the C ABI passes it (n x 4 ints: kernel height, kernel width, stride, padding).  Fills `ch`
@@ -59,8 +73,8 @@ inline int chain_from_host(const int* chain, int n_chain, int H0, int W0, ConvCh
   return FB_OK;
 }
 
-// The same for the compact rows (conv_compact.cu), along one axis.  Without the borders of the maps the nested divisions of a
-// chain collapse into one: pixel i reaches [ceil((i + A) / S), floor((i + B) / S)], S the product of the strides, so that a shift
+// The same for the compact rows of the CNN driver (conv_compact.cu), along one axis.  Without the borders of the maps the nested
+// divisions of a chain collapse into one: pixel i reaches [ceil((i + A) / S), floor((i + B) / S)], S the product of the strides, so that a shift
 // of the pixel by S shifts the window by one; the compact window is that interval cut to the map.  (It holds the window above,
 // and is larger only where a padding exceeds its filter or a stride its filter; what is more is zero.)  Turned round, output y is
 // reached by the pixels [y S - B, y S - A].
@@ -93,6 +107,15 @@ inline int axis_extent(const CwAxis& ax, int n0) {
   int win = 1;
   for (int i = 0; i < n0; ++i) win = std::max(win, ax.hi(i) - ax.lo(i) + 1);
   return win;
+}
+
+// Whether these are the windows of chain_span for every pixel of n0.
+inline bool axis_is_chain(const CwAxis& ax, const ConvChain& ch, const int* k, int n0) {
+  for (int i = 0; i < n0; ++i) {
+    const Span s = chain_span(ch, k, ch.n, n0, i);
+    if (ax.lo(i) != s.lo || ax.hi(i) != s.hi) return false;
+  }
+  return true;
 }
 
 // Bias part, slopes and relaxed bias terms of the first convolution and the relaxation behind it, per output column (conv.cu).

@@ -134,7 +134,7 @@ def _chain_arr(chain):
 
 
 def cw_extent(H0, W0, chain):
-    """Largest window (wh, ww) any pixel of an H0 x W0 image reaches through `chain`: the middle dimensions of a compact
+    """Largest window (wh, ww) any pixel of an H0 x W0 image reaches through `chain`: the trailing dimensions of a compact
     tensor (fb_cw_extent)."""
     wh, ww = ctypes.c_int(0), ctypes.c_int(0)
     check(load().fb_cw_extent(H0, W0, _chain_arr(chain), len(chain), ctypes.byref(wh), ctypes.byref(ww)), "fb_cw_extent")
@@ -142,13 +142,13 @@ def cw_extent(H0, W0, chain):
 
 
 def cw_identity_relax(op, image_lb, image_ub, weight, bias, rows, row_start, stride, pad, p, eps, scale=1.0):
-    """conv_identity_relax with compact rows: z_lw, z_uw [rows, wh, ww, Cout] (fb_cw_identity_relax_f32)."""
+    """conv_identity_relax with compact rows: z_lw, z_uw [rows, Cout, wh, ww] (fb_cw_identity_relax_f32)."""
     dev = ops._chk(image_lb, image_ub, weight, bias)
     C, H, W = image_lb.shape[-3:]
     Co, _, Kh, Kw = weight.shape
     Ho, Wo = (H + 2 * pad - Kh) // stride + 1, (W + 2 * pad - Kw) // stride + 1
     wh, ww = cw_extent(H, W, [(Kh, Kw, stride, pad)])
-    z_lw = torch.empty(rows, wh, ww, Co, device=dev)
+    z_lw = torch.empty(rows, Co, wh, ww, device=dev)
     z_uw = torch.empty_like(z_lw)
     y_lb = torch.empty(1, Co, Ho, Wo, device=dev)
     y_ub = torch.empty_like(y_lb)
@@ -165,10 +165,10 @@ def cw_identity_relax(op, image_lb, image_ub, weight, bias, rows, row_start, str
 def cw_conv(z_lw, z_uw, weight, stride, pad, row_start, H0, W0, chain, H, W):
     """Weight part of a later convolution on compact rows (fb_cw_conv2d_f32); `chain` leads to the input [Cin, H, W]."""
     dev = ops._chk(z_lw, z_uw, weight)
-    rows, C = z_lw.shape[0], z_lw.shape[3]
+    rows, C = z_lw.shape[:2]
     Co, _, Kh, Kw = weight.shape
     wh, ww = cw_extent(H0, W0, list(chain) + [(Kh, Kw, stride, pad)])
-    y_lw = torch.empty(rows, wh, ww, Co, device=dev)
+    y_lw = torch.empty(rows, Co, wh, ww, device=dev)
     y_uw = torch.empty_like(y_lw)
     with torch.cuda.device(dev):
         check(load().fb_cw_conv2d_f32(z_lw.data_ptr(), z_uw.data_ptr(), weight.data_ptr(), y_lw.data_ptr(), y_uw.data_ptr(), rows,
@@ -180,7 +180,7 @@ def cw_conv(z_lw, z_uw, weight, stride, pad, row_start, H0, W0, chain, H, W):
 def cw_norm_partials(z_lw, z_uw, row_start, Cin0, H0, W0, chain, H, W, p):
     """Unfinished dual-norm accumulation of every dense column over the rows of a compact tensor (fb_cw_norm_partials_f32)."""
     dev = ops._chk(z_lw, z_uw)
-    rows, C = z_lw.shape[0], z_lw.shape[3]
+    rows, C = z_lw.shape[:2]
     part_l = torch.empty(C * H * W, device=dev)
     part_u = torch.empty_like(part_l)
     with torch.cuda.device(dev):
@@ -193,7 +193,7 @@ def cw_norm_partials(z_lw, z_uw, row_start, Cin0, H0, W0, chain, H, W, p):
 def cw_relax_apply(op, z_lw, z_uw, lb, ub, norm_l, norm_u, row_start, H0, W0, chain, H, W, p, eps):
     """Relaxation of compact rows from given (reduced) norm accumulations (fb_cw_relax_apply_f32)."""
     dev = ops._chk(z_lw, z_uw, lb, ub, norm_l, norm_u)
-    rows, C = z_lw.shape[0], z_lw.shape[3]
+    rows, C = z_lw.shape[:2]
     o_lw, o_uw, o_lb, o_ub = torch.empty_like(z_lw), torch.empty_like(z_uw), torch.empty_like(lb), torch.empty_like(ub)
     coef = torch.empty(4 * C * H * W, device=dev)
     with torch.cuda.device(dev):
@@ -207,14 +207,13 @@ def cw_relax_apply(op, z_lw, z_uw, lb, ub, norm_l, norm_u, row_start, H0, W0, ch
 def cw_linear(z_lw, z_uw, weight, row_start, H0, W0, chain, H, W):
     """Weight rows of the linear layer that ends the spatial part, from compact rows: [rows, N] (fb_cw_linear_f32)."""
     dev = ops._chk(z_lw, z_uw, weight)
-    rows, C = z_lw.shape[0], z_lw.shape[3]
+    rows, C = z_lw.shape[:2]
     N = weight.shape[0]
     y_lw = torch.empty(rows, N, device=dev)
     y_uw = torch.empty_like(y_lw)
-    wt_ws = torch.empty(weight.numel(), device=dev)
     with torch.cuda.device(dev):
         check(load().fb_cw_linear_f32(z_lw.data_ptr(), z_uw.data_ptr(), weight.data_ptr(), y_lw.data_ptr(), y_uw.data_ptr(),
-                                      wt_ws.data_ptr(), rows,
+                                      y_lw.data_ptr(), rows,   # (the scratch argument is not used)
                                       row_start, H0, W0, _chain_arr(chain), len(chain), C, H, W, N, ops._stream()),
               "fb_cw_linear_f32")
     return y_lw, y_uw
@@ -223,7 +222,7 @@ def cw_linear(z_lw, z_uw, weight, row_start, H0, W0, chain, H, W):
 def cw_expand(z_lw, z_uw, row_start, H0, W0, chain, H, W):
     """Dense rows [rows, C, H, W] of a compact tensor (fb_cw_expand_f32)."""
     dev = ops._chk(z_lw, z_uw)
-    rows, C = z_lw.shape[0], z_lw.shape[3]
+    rows, C = z_lw.shape[:2]
     y_lw = torch.empty(rows, C, H, W, device=dev)
     y_uw = torch.empty_like(y_lw)
     with torch.cuda.device(dev):

@@ -534,8 +534,8 @@ int fb_concretize_sharded_f32(fb_comm* c, int algo,
 
 /* ---- compact rows for the convolutions behind an identity input ---------------------------
  * Row r of such a CNN is zero outside the window its pixel reaches (fb_conv2d_windowed_f32 above); here a row is stored
- * as that window only, z [rows, wh, ww, C] with z[r, dy, dx, c] = row r at (c, y_lo(r) + dy, x_lo(r) + dx),
- * (wh, ww) the largest window over all pixels (fb_cw_extent); what lies beyond a pixel's own window is not defined.  `chain`
+ * as that window only, z [rows, C, wh, ww] with z[r, c, dy, dx] = row r at (c, y_lo(r) + dy, x_lo(r) + dx) and zeros
+ * where the pixel's own window is smaller than (wh, ww), the largest window over all pixels (fb_cw_extent).  `chain`
  * (host, n_chain x 4 ints: kernel height, kernel width, stride, padding) always lists the convolutions that lead from
  * the H0 x W0 image to the tensor in question, whose dense shape is [C, H, W].  For the benchmark CNN a row shrinks
  * from 16 384 resp. 8 192 values to 144 resp. 288.  No counterpart in the reference.
@@ -584,7 +584,7 @@ int fb_cw_expand_f32(const float* z_lw, const float* z_uw, float* y_lw, float* y
  * communicator (world > 1) the dual norms are all-reduced over the ranks by `algo` (fb_allreduce_algo) and every rank
  * gets the same range, with comm == NULL nothing is exchanged.  One call enqueues the whole pass on `stream`.
  * The first layer must be a convolution (its output, and the relaxation behind it, are written from the filter alone).
- * compact != 0 (the default of the Python layer): rows are kept as their windows only (the fb_cw_* operators above)
+ * compact != 0 (the default of the Python layer): rows are kept as their windows only (as the fb_cw_* operators above do)
  * until the first linear layer; compact == 0: dense rows, fb_conv2d_identity_relax_f32 and fb_conv2d_windowed_f32.  The reference has no CNN
  * verifier to mirror (HandTunedKernels/convolution_verification.cu:228-238 is a benchmark stub); layer semantics are
  * Bounds.matmul / Bounds.relu (Bounds.py:397-413, :921-963) with dim_in as the batch axis of the convolutions.

@@ -141,3 +141,14 @@ def assert_arbitrated(got, ref32, ref64, what, c=4.0, rtol=RTOL, atol=ATOL):
 def assert_bounds_arbitrated(g, o32, o64, what, c=4.0):
     for k in ("lw", "uw", "lb", "ub"):
         assert_arbitrated(getattr(g, k), getattr(o32, k), getattr(o64, k), "%s %s" % (what, k), c=c)
+
+
+def conv_window(n0, chain, i):
+    """Outputs [lo, hi] (along one axis) that pixel i of n0 reaches through `chain`, a list of (kernel, stride, padding): cut to
+    the map of every convolution; empty (lo > hi) where a stride steps over it."""
+    lo = hi = i
+    for k, stride, pad in chain:
+        n0 = (n0 + 2 * pad - k) // stride + 1
+        if lo <= hi:
+            lo, hi = max(0, -(-(lo + pad - (k - 1)) // stride)), min(n0 - 1, (hi + pad) // stride)
+    return lo, hi

@@ -161,6 +161,39 @@ def test_compact_window_extent_without_gpu():
     assert extent(8, 8, [(3, 3, 1, 1)] * 9)[0] == 2                            # more than eight convolutions
 
 
+def test_compact_window_extent_of_any_chain_without_gpu():
+    """The windows are cut to every map of the chain, also where a padding exceeds its filter or a stride steps over pixels."""
+    import ctypes
+    import random
+    import helpers
+    from faith_b200 import _lib
+    lib = _lib.load()
+    rng = random.Random(5)
+    tried = 0
+    while tried < 300:
+        n0 = (rng.randint(1, 24), rng.randint(1, 24))
+        chain = [(rng.choice([1, 2, 3, 5, 7]), rng.choice([1, 2, 3, 5]), rng.choice([1, 1, 2, 3, 4]), rng.choice([0, 1, 2, 4]))
+                 for _ in range(rng.randint(1, 4))]
+        want = []
+        for axis in (0, 1):
+            n, geo = n0[axis], [(c[axis], c[2], c[3]) for c in chain]
+            for k, stride, pad in geo:
+                n = (n + 2 * pad - k) // stride + 1 if n + 2 * pad >= k else 0
+                if n <= 0:
+                    break
+            if n <= 0:
+                break
+            spans = [helpers.conv_window(n0[axis], geo, i) for i in range(n0[axis])]
+            want.append(max([1] + [hi - lo + 1 for lo, hi in spans]))
+        if len(want) < 2:
+            continue
+        tried += 1
+        arr = (ctypes.c_int * (4 * len(chain)))(*[v for c in chain for v in c])
+        wh, ww = ctypes.c_int(0), ctypes.c_int(0)
+        assert lib.fb_cw_extent(n0[0], n0[1], arr, len(chain), ctypes.byref(wh), ctypes.byref(ww)) == 0
+        assert [wh.value, ww.value] == want, (n0, chain)
+
+
 def test_encoder_arena_size_without_gpu():
     """fb_encoder_workspace_bytes is host arithmetic: four bound slots sized for the widest tensor of a block, the range
     scratch of the dot products, the column-norm scratch and the row sums of the layer input; it grows with the

@@ -295,6 +295,55 @@ def test_compact_rows_of_odd_shapes(C, H, W, c1, c2, k2, s2, p2, n, start, drop)
     helpers.assert_close(yu, dl[1].reshape(rows, n), "linear uw", atol=2e-6)
 
 
+# the geometry of the benchmark CNN; odd sizes with a filter of two sizes; paddings beyond the filter; strides that step over pixels
+@pytest.mark.parametrize("C,H,W,geoms,start,drop", [
+    (3, 8, 8, [(3, 3, 1, 1), (3, 3, 2, 1)], 0, 0), (2, 9, 7, [(3, 3, 1, 1), (5, 2, 1, 2), (3, 3, 2, 0)], 11, 20),
+    (1, 6, 5, [(2, 2, 1, 3), (3, 3, 2, 3), (1, 1, 1, 0)], 0, 0), (2, 10, 9, [(1, 1, 2, 0), (2, 3, 3, 1), (3, 3, 1, 1)], 0, 3)])
+def test_compact_rows_hold_the_window_of_every_channel_and_zeros(C, H, W, geoms, start, drop):
+    """The documented form of the compact tensors, z[r, c, dy, dx] = row r at (c, y_lo + dy, x_lo + dx) and zeros beyond the
+    pixel's own window, element by element against the dense rows: first convolution, later convolutions, a relaxation."""
+    from faith_b200 import ops, sharded
+    from faith_b200._lib import FB_RELU
+    g = torch.Generator().manual_seed(47)
+    chans = [C, 5, 8, 3][:len(geoms) + 1]
+    rows, p, eps = C * H * W - start - drop, 2.0, 0.05
+    img = torch.rand(1, C, H, W, generator=g).to(DEV)
+    ws = [(torch.randn(chans[i + 1], chans[i], kh, kw, generator=g) * 0.3).to(DEV) for i, (kh, kw, _, _) in enumerate(geoms)]
+
+    def same(z, dense, chain, what):
+        wy = [helpers.conv_window(H, [(c[0], c[2], c[3]) for c in chain], i) for i in range(H)]
+        wx = [helpers.conv_window(W, [(c[1], c[2], c[3]) for c in chain], i) for i in range(W)]
+        want = torch.zeros(rows, dense.shape[1], max([1] + [b - a + 1 for a, b in wy]), max([1] + [b - a + 1 for a, b in wx]))
+        for r in range(rows):
+            (ya, yb), (xa, xb) = wy[(start + r) // W % H], wx[(start + r) % W]
+            if ya <= yb and xa <= xb:
+                want[r, :, :yb - ya + 1, :xb - xa + 1] = dense[r, :, ya:yb + 1, xa:xb + 1].cpu()
+        assert z.shape == want.shape and torch.equal(z.cpu(), want), what
+
+    _, _, s, q = geoms[0]
+    dense = sharded.conv_identity_relax(FB_RELU, img, img.clone(), ws[0], None, rows, start, s, q, p, eps)
+    z = sharded.cw_identity_relax(FB_RELU, img, img.clone(), ws[0], None, rows, start, s, q, p, eps)
+    chain = [geoms[0]]
+    for i in (0, 1):
+        same(z[i], dense[i][0], chain, "first convolution")
+    for (kh, kw, s, q), w in zip(geoms[1:], ws[1:]):
+        h, x = dense[0].shape[-2:]
+        z = sharded.cw_conv(z[0], z[1], w, s, q, start, H, W, chain, h, x)
+        dense = ops.conv2d(dense, w, None, s, q)
+        chain = chain + [(kh, kw, s, q)]
+        for i in (0, 1):
+            same(z[i], dense[i][0], chain, "convolution %d" % len(chain))
+        h, x = dense[0].shape[-2:]
+        feat = dense[2].numel()
+        nl, nu = sharded.cw_norm_partials(z[0], z[1], start, C, H, W, chain, h, x, p)
+        z = sharded.cw_relax_apply(FB_RELU, z[0], z[1], dense[2].reshape(-1), dense[3].reshape(-1), nl, nu, start, H, W, chain, h, x, p, eps)
+        o = ops.relax_with_norms(FB_RELU, dense[0].reshape(1, rows, feat), dense[1].reshape(1, rows, feat), dense[2].reshape(1, feat),
+                                 dense[3].reshape(1, feat), nl.reshape(1, feat), nu.reshape(1, feat), p, eps)
+        dense = tuple(a.view(b.shape) for a, b in zip(o, dense))
+        for i in (0, 1):
+            same(z[i], dense[i][0], chain, "relaxation %d" % len(chain))
+
+
 @pytest.mark.parametrize("C,HW,c1,c2,n,p", [(1, 16, 8, 16, 2, 1.0), (3, 23, 24, 48, 16, 2.0), (1, 21, 5, 7, 33, float("inf"))])
 def test_cnn_driver_with_the_head_reduced_to_its_norms(C, HW, c1, c2, n, p):
     from faith_b200.sharded import CnnVerifier
