@@ -154,6 +154,38 @@ struct __align__(16) CwRow {
   int64_t base;            // element (0, 0, 0) of the output row, shifted by (py, px)
 };
 
+// The bias image: an ordinary convolution, a thread per output from `first` on in steps of `step`.
+template <int KS>
+__device__ __forceinline__ void conv_bias_image(const CwConvArgs& q, int64_t first, int64_t step) {
+  const int Kh = KS ? KS : q.Kh, Kw = KS ? KS : q.Kw, taps = Kh * Kw;
+  const int64_t total = (int64_t)q.Cout * q.Ho * q.Wo;
+  for (int64_t t = first; t < total; t += step) {
+    const int ow = (int)(t % q.Wo), oh = (int)((t / q.Wo) % q.Ho), co = (int)(t / ((int64_t)q.Wo * q.Ho));
+    const int ih0 = oh * q.stride - q.pad, iw0 = ow * q.stride - q.pad;
+    float ac = 0.f, ar = 0.f;
+#pragma unroll 2
+    for (int c = 0; c < q.Cin; ++c) {
+      const float* wp = q.Wt + ((int64_t)co * q.Cin + c) * taps;
+      const int64_t plane = (int64_t)c * q.H * q.W;
+#pragma unroll
+      for (int kh = 0; kh < (KS ? KS : Kh); ++kh)
+#pragma unroll
+        for (int kw = 0; kw < (KS ? KS : Kw); ++kw) {
+          const int ih = ih0 + kh, iw = iw0 + kw;
+          const bool in = ih >= 0 && ih < q.H && iw >= 0 && iw < q.W;
+          const int64_t o = plane + (int64_t)ih * q.W + iw;
+          const float w = __ldg(wp + kh * Kw + kw), lo = in ? __ldg(q.b_lo + o) : 0.f, up = in ? __ldg(q.b_up + o) : 0.f;
+          ac = fmaf(fmul(fadd(lo, up), 0.5f), w, ac);
+          ar = fmaf(fmul(fsub(up, lo), 0.5f), fabsf(w), ar);
+        }
+    }
+    float lo = fsub(ac, ar), up = fadd(ac, ar);
+    if (q.bias != nullptr) { lo = fadd(lo, q.bias[co]); up = fadd(up, q.bias[co]); }
+    q.yb_lo[t] = lo;
+    q.yb_up[t] = up;
+  }
+}
+
 // KS: filter size when it is the same in both directions and known at compile time (3), 0 = from the arguments.
 // CPT: output channels per thread (2 where Cout is even: the pairs of a tap are one 128-bit read, and the inputs, which every lane
 // reads, serve twice the multiply-adds).
@@ -166,33 +198,8 @@ cw_conv_kernel(const __grid_constant__ CwConvParams<kAbi> q) {
   pdl_sync();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x, nwarps = nthr >> 5;
   const int Kh = KS ? KS : q.Kh, Kw = KS ? KS : q.Kw, taps = Kh * Kw;
-  if ((int)blockIdx.x < q.blocks_bias) {   // an ordinary convolution of one image, a thread per output
-    const int64_t total = (int64_t)q.Cout * q.Ho * q.Wo;
-    for (int64_t t = (int64_t)blockIdx.x * nthr + tid; t < total; t += (int64_t)q.blocks_bias * nthr) {
-      const int ow = (int)(t % q.Wo), oh = (int)((t / q.Wo) % q.Ho), co = (int)(t / ((int64_t)q.Wo * q.Ho));
-      const int ih0 = oh * q.stride - q.pad, iw0 = ow * q.stride - q.pad;
-      float ac = 0.f, ar = 0.f;
-#pragma unroll 2
-      for (int c = 0; c < q.Cin; ++c) {
-        const float* wp = q.Wt + ((int64_t)co * q.Cin + c) * taps;
-        const int64_t plane = (int64_t)c * q.H * q.W;
-#pragma unroll
-        for (int kh = 0; kh < (KS ? KS : Kh); ++kh)
-#pragma unroll
-          for (int kw = 0; kw < (KS ? KS : Kw); ++kw) {
-            const int ih = ih0 + kh, iw = iw0 + kw;
-            const bool in = ih >= 0 && ih < q.H && iw >= 0 && iw < q.W;
-            const int64_t o = plane + (int64_t)ih * q.W + iw;
-            const float w = __ldg(wp + kh * Kw + kw), lo = in ? __ldg(q.b_lo + o) : 0.f, up = in ? __ldg(q.b_up + o) : 0.f;
-            ac = fmaf(fmul(fadd(lo, up), 0.5f), w, ac);
-            ar = fmaf(fmul(fsub(up, lo), 0.5f), fabsf(w), ar);
-          }
-      }
-      float lo = fsub(ac, ar), up = fadd(ac, ar);
-      if (q.bias != nullptr) { lo = fadd(lo, q.bias[co]); up = fadd(up, q.bias[co]); }
-      q.yb_lo[t] = lo;
-      q.yb_up[t] = up;
-    }
+  if ((int)blockIdx.x < q.blocks_bias) {
+    conv_bias_image<KS>(q, (int64_t)blockIdx.x * nthr + tid, (int64_t)q.blocks_bias * nthr);
     return;
   }
   const int bid = blockIdx.x - q.blocks_bias, cls = bid / q.per_class, chunk = bid - cls * q.per_class;
@@ -392,6 +399,56 @@ cw_conv_kernel(const __grid_constant__ CwConvParams<kAbi> q) {
         }
       }
     }
+  }
+}
+
+// The same, a thread per output that reads its taps from global memory: for windows that shared memory does not hold (they are
+// taken without the borders of the maps above, so that filters larger than a small map can exceed it).
+template <bool kAbi>
+__global__ void __launch_bounds__(256)
+cw_conv_direct_kernel(const __grid_constant__ CwConvParams<kAbi> q, const __grid_constant__ CwShape<kAbi> gi,
+                      const __grid_constant__ CwShape<kAbi> go) {
+  pdl_sync();
+  if ((int)blockIdx.x < q.blocks_bias) {
+    conv_bias_image<0>(q, (int64_t)blockIdx.x * 256 + threadIdx.x, (int64_t)q.blocks_bias * 256);
+    return;
+  }
+  const int64_t per_in = (int64_t)gi.C * gi.wh * gi.ww, per_out = (int64_t)go.C * go.wh * go.ww;
+  const int64_t step = (int64_t)(gridDim.x - q.blocks_bias) * 256;
+  for (int64_t t = (int64_t)(blockIdx.x - q.blocks_bias) * 256 + threadIdx.x; t < q.rows * per_out; t += step) {
+    const int64_t lr = t / per_out, r = q.row_start + lr;
+    int co, dy, dx;
+    go.split((int)(t - lr * per_out), co, dy, dx);
+    const int xi = (int)(r % q.W0), yi = (int)((r / q.W0) % q.H0), ci = (int)(r / ((int64_t)q.W0 * q.H0));
+    const Span wy = go.rows(yi), wx = go.cols(xi), vy = gi.rows(yi), vx = gi.cols(xi);
+    if (wy.lo + dy > wy.hi || wx.lo + dx > wx.hi) continue;
+    const int y0 = (wy.lo + dy) * q.stride - q.pad, x0 = (wx.lo + dx) * q.stride - q.pad;   // first tap
+    const int ky0 = max(0, vy.lo - y0), ky1 = min(q.Kh, vy.hi + 1 - y0), kx0 = max(0, vx.lo - x0), kx1 = min(q.Kw, vx.hi + 1 - x0);
+    float ac = 0.f, ar = 0.f;
+    for (int c = 0; c < q.Cin; ++c)
+      for (int ky = ky0; ky < ky1; ++ky)
+        for (int kx = kx0; kx < kx1; ++kx) {
+          const int y = y0 + ky, x = x0 + kx;
+          float lo = 0.f, up = 0.f;
+          if (q.W1 != nullptr) {
+            const int jy = yi - (y * q.stride1 - q.pad1), jx = xi - (x * q.stride1 - q.pad1);
+            if (jy >= 0 && jy < q.kh1 && jx >= 0 && jx < q.kw1) {
+              const float tap = fmul(q.scale, __ldg(q.W1 + (((int64_t)c * q.Cin0 + ci) * q.kh1 + jy) * q.kw1 + jx));
+              const int64_t col = ((int64_t)c * q.H + y) * q.W + x;
+              lo = fmul(tap, __ldg(q.k_l + col));
+              up = fmul(tap, __ldg(q.k_u + col));
+            }
+          } else {
+            const int64_t o = lr * per_in + ((int64_t)(y - vy.lo) * gi.ww + x - vx.lo) * gi.step_x() + (int64_t)c * gi.step_c();
+            lo = __ldg(q.z_lo + o);
+            up = __ldg(q.z_up + o);
+          }
+          const float w = __ldg(q.Wt + (((int64_t)co * q.Cin + c) * q.Kh + ky) * q.Kw + kx);
+          ac = fmaf(fmul(fadd(lo, up), 0.5f), w, ac);
+          ar = fmaf(fmul(fsub(up, lo), 0.5f), fabsf(w), ar);
+        }
+    q.y_lo[t] = fsub(ac, ar);
+    q.y_up[t] = fadd(ac, ar);
   }
 }
 
@@ -837,17 +894,18 @@ int conv_rows(const float* z_lo, const float* z_up, const float* W1, const float
     if (q.CC > 1) q.CC = (q.CC + 1) / 2;
     else q.G = (q.G + 1) / 2;
   }
-  if (bytes() > limit) return FB_ERR_SHAPE;
+  const bool direct = bytes() > limit;
   q.per_class = (int)ceil_div(n_cls, (int64_t)q.G * kCwR);
   const int64_t items = (int64_t)q.G * go.wh * go.ww * (Cout / cpt);
-  const int threads = (int)(ceil_div(ceil_div(items, ceil_div(items, kCwConvThreads)), 32) * 32);
+  const int threads = direct ? 256 : (int)(ceil_div(ceil_div(items, ceil_div(items, kCwConvThreads)), 32) * 32);
   const int64_t out = (int64_t)Cout * Ho * Wo;
   q.blocks_bias = b_lo != nullptr ? (int)std::min<int64_t>(ceil_div(out, threads), device_info().sms) : 0;
-  const int64_t blocks = q.blocks_bias + (int64_t)cls_y * q.cls_x * q.per_class;
+  const int64_t blocks = q.blocks_bias + (direct ? grid_for(rows * Cout * go.wh * go.ww, 256) : (int64_t)cls_y * q.cls_x * q.per_class);
   if (blocks > 0x7fffffff) return FB_ERR_SHAPE;
   auto kern = Kh == 3 && Kw == 3 ? (cpt == 2 ? cw_conv_kernel<3, 2, kAbi> : cw_conv_kernel<3, 1, kAbi>)
                                  : (cpt == 2 ? cw_conv_kernel<0, 2, kAbi> : cw_conv_kernel<0, 1, kAbi>);
-  if (int rc = ensure_dynamic_smem(kern, bytes() + kCwStatic)) return rc;   // (48 KB without the attribute hold the static part too)
+  if (!direct)
+    if (int rc = ensure_dynamic_smem(kern, bytes() + kCwStatic)) return rc;   // (48 KB without the attribute hold the static part too)
   ProfileScope prof(PK_CONV, 8.0 * rows * Cout * go.wh * go.ww * Cin * Kh * Kw,
                     4.0 * 2.0 * rows * ((double)Cin * gi.wh * gi.ww + (double)Cout * go.wh * go.ww), (void*)st);
   if (kAbi) {   // (the kernel stores the pixels' own windows)
@@ -855,7 +913,8 @@ int conv_rows(const float* z_lo, const float* z_up, const float* W1, const float
     FB_CUDA_OK(cudaMemsetAsync(y_lo, 0, n, st));
     FB_CUDA_OK(cudaMemsetAsync(y_up, 0, n, st));
   }
-  fb::launch_k(kern, (unsigned)blocks, threads, bytes(), st, q);
+  if (direct) fb::launch_k(cw_conv_direct_kernel<kAbi>, (unsigned)blocks, threads, 0, st, q, gi, go);
+  else fb::launch_k(kern, (unsigned)blocks, threads, bytes(), st, q);
   FB_LAUNCH_OK();
   return FB_OK;
 }

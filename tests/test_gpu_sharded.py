@@ -295,10 +295,12 @@ def test_compact_rows_of_odd_shapes(C, H, W, c1, c2, k2, s2, p2, n, start, drop)
     helpers.assert_close(yu, dl[1].reshape(rows, n), "linear uw", atol=2e-6)
 
 
-# the geometry of the benchmark CNN; odd sizes with a filter of two sizes; paddings beyond the filter; strides that step over pixels
+# the geometry of the benchmark CNN; odd sizes with a filter of two sizes; paddings beyond the filter; strides that step over
+# pixels; windows beyond shared memory
 @pytest.mark.parametrize("C,H,W,geoms,start,drop", [
     (3, 8, 8, [(3, 3, 1, 1), (3, 3, 2, 1)], 0, 0), (2, 9, 7, [(3, 3, 1, 1), (5, 2, 1, 2), (3, 3, 2, 0)], 11, 20),
-    (1, 6, 5, [(2, 2, 1, 3), (3, 3, 2, 3), (1, 1, 1, 0)], 0, 0), (2, 10, 9, [(1, 1, 2, 0), (2, 3, 3, 1), (3, 3, 1, 1)], 0, 3)])
+    (1, 6, 5, [(2, 2, 1, 3), (3, 3, 2, 3), (1, 1, 1, 0)], 0, 0), (2, 10, 9, [(1, 1, 2, 0), (2, 3, 3, 1), (3, 3, 1, 1)], 0, 3),
+    (1, 7, 9, [(33, 33, 1, 16), (33, 33, 1, 16), (3, 3, 2, 1)], 5, 9)])
 def test_compact_rows_hold_the_window_of_every_channel_and_zeros(C, H, W, geoms, start, drop):
     """The documented form of the compact tensors, z[r, c, dy, dx] = row r at (c, y_lo + dy, x_lo + dx) and zeros beyond the
     pixel's own window, element by element against the dense rows: first convolution, later convolutions, a relaxation."""
@@ -342,6 +344,24 @@ def test_compact_rows_hold_the_window_of_every_channel_and_zeros(C, H, W, geoms,
         dense = tuple(a.view(b.shape) for a, b in zip(o, dense))
         for i in (0, 1):
             same(z[i], dense[i][0], chain, "relaxation %d" % len(chain))
+
+
+@pytest.mark.parametrize("chain", [[33, 33, 3], [65, 3], [3, 41, 21]])
+def test_cnn_driver_with_filters_larger_than_the_map(chain):
+    """Windows that do not fit into shared memory before they are cut to the map: the pass goes on with dense rows."""
+    from faith_b200.sharded import CnnVerifier
+    g = torch.Generator().manual_seed(48)
+    hw, c, layers = 12, 1, []
+    for i, k in enumerate(chain):
+        layers += [("conv", torch.randn(2 + i, c, k, k, generator=g) / (4 * c) ** 0.5, torch.randn(2 + i, generator=g) * 0.1, 1, k // 2), ("relu",)]
+        c = 2 + i
+    layers.append(("linear", torch.randn(4, c * hw * hw, generator=g) * 0.02, torch.randn(4, generator=g) * 0.1))
+    img = torch.rand(1, hw, hw, generator=g)
+    want = CnnVerifier(layers, DEV, compact=False).forward(img, float("inf"), 0.01)
+    got = CnnVerifier(layers, DEV).forward(img, float("inf"), 0.01)
+    scale = float(want[1].abs().max())
+    helpers.assert_close(got[0], want[0].cpu(), "l", atol=2e-6 * scale)
+    helpers.assert_close(got[1], want[1].cpu(), "u", atol=2e-6 * scale)
 
 
 @pytest.mark.parametrize("C,HW,c1,c2,n,p", [(1, 16, 8, 16, 2, 1.0), (3, 23, 24, 48, 16, 2.0), (1, 21, 5, 7, 33, float("inf"))])
