@@ -644,7 +644,7 @@ cw_linear_kernel(const __grid_constant__ CwLinearArgs<kAbi> q) {
   // the union of the windows (their ends do not decrease along the pixels)
   const int ylo = g.y.lo(yi), yhi = g.y.hi(yi), xl = g.x.lo(x0), nxr = max(0, g.x.hi(x0 + npx - 1) - xl + 1), rows_here = npx * q.n_ci;
   const int64_t per_pos = g.step_x(), per_row = (int64_t)g.wh * g.ww * g.C;
-  const Span wy = kAbi ? g.rows(yi) : Span{ylo, yhi};   // window rows of the tile's pixels
+  const int wy0 = kAbi ? g.rows(yi).lo : ylo;   // first row of the windows of the tile's pixels
   float pl = 0.f, pu = 0.f;   // accumulated norms of this lane's output
   for (int r0 = 0; r0 < rows_here; r0 += kCwLinWarps) {
     float sc[NB], sr[NB];
@@ -652,8 +652,7 @@ cw_linear_kernel(const __grid_constant__ CwLinearArgs<kAbi> q) {
     for (int n = 0; n < NB; ++n) sc[n] = sr[n] = 0.f;
     const int t = r0 + warp, px = t % npx, ci = q.ci0 + t / npx;
     int64_t lr = -1;
-    const Span wx = g.cols(x0 + px);
-    const int wlo = wx.lo, aw = wx.hi - wlo + 1;
+    const int wlo = g.cols(x0 + px).lo, aw = g.cols(x0 + px).hi - wlo + 1;
     if (t < rows_here) {
       const int64_t l = ((int64_t)ci * g.H0 + yi) * g.W0 + x0 + px - q.row_start;
       if (l >= 0 && l < q.rows) lr = l;
@@ -676,12 +675,12 @@ cw_linear_kernel(const __grid_constant__ CwLinearArgs<kAbi> q) {
         }
         // the row's elements, three at a time: those of the next step are loaded before the arithmetic of this one
         const bool mine = lr >= 0 && c < g.C && aw > 0;
-        const int y_first = kAbi ? max(ya, wy.lo) : ya, y_last = kAbi ? min(yb, wy.hi) : yb;
-        const int steps_x = (aw + 2) / 3, steps = mine ? max(0, y_last - y_first + 1) * steps_x : 0;
+        const int y_first = kAbi ? max(ya, wy0) : ya, n_y = kAbi ? max(0, min(yb, g.rows(yi).hi) - y_first + 1) : yb - ya + 1;
+        const int steps_x = (aw + 2) / 3, steps = mine ? n_y * steps_x : 0;
         float zl[3], zu[3], kf[4][3];
         int sy = y_first, sx = 0;   // the next step: row, first column of the window
         auto load = [&] {
-          const int64_t zb = lr * per_row + ((int64_t)(sy - wy.lo) * g.ww + sx) * per_pos + (int64_t)c * g.step_c(), cb = ((int64_t)sy * g.W + wlo + sx) * g.C + c;
+          const int64_t zb = lr * per_row + ((int64_t)(sy - wy0) * g.ww + sx) * per_pos + (kAbi ? (int64_t)c * g.step_c() : c), cb = ((int64_t)sy * g.W + wlo + sx) * g.C + c;
 #pragma unroll
           for (int e = 0; e < 3; ++e) {
             const bool in = sx + e < aw;
