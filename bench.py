@@ -437,13 +437,13 @@ def per_config_lines(ctx, lib, pipes, pk):
     layers = O.make_cnn(5)
     img = torch.rand(3, 32, 32, generator=torch.Generator().manual_seed(5)).pin_memory()   # 12 KB, copied every pass
     ver = CnnVerifier(layers, dev)
-    # Default route: rows kept as their windows only (fb_cw_*): 7 MB of rows instead of 600 MB; what remains is 14 small
-    # launches, so the figure is launch- and latency-bound and a roofline fraction says little (bytes: the compact rows
-    # written and read by each operator plus the 0.33 MB head weight, 2.3 GFLOP almost all in the head).
+    # Default route: rows kept as their windows only (conv_compact.cu): 7 MB of rows instead of 600 MB; what remains is five
+    # small launches, so the figure is latency-bound and a roofline fraction says little (bytes: the compact rows written
+    # and read plus the 0.33 MB head weight, 2.3 GFLOP almost all in the head).
     per = ctx.loop_ms(lambda: ver.forward(img, INF, 2.0 / 255), 10)
     out.append(roof_entry("C5 CNN pass, one image (conv3-16, relu, conv16-32 s2, relu, linear 8192-10), 1 GPU; compact rows "
                           "(default route)", per, 2.3e9, 0.06e9, ffma_alg, "ffma", hbm,
-                          {"images_per_s": 1e3 / per, "note": "latency-bound: 14 launches of a few microseconds each, replayed from a CUDA graph"}))
+                          {"images_per_s": 1e3 / per, "note": "latency-bound: five dependent launches of 5 to 20 microseconds each"}))
     # Dense rows, identity-input structure used (first convolution + relu written from the filter alone, windowed second
     # convolution): 1.41 GB moved.
     ver_rows = CnnVerifier(layers, dev, compact=False)
@@ -503,16 +503,11 @@ def cnn_sharded(ctx, lib, steps):
         ver = CnnVerifier(layers, ctx.dev, comm=comm, algo=algo, compact=compact)
         for _ in range(3):
             l, u = ver.forward(img, INF, eps, ctx.rank, ctx.world)
-        # (a single-GPU pass is replayed from a CUDA graph, which the library's launch counter does not see: the
-        # launches of one pass are counted on an uncaptured run)
-        counter = CnnVerifier(layers, ctx.dev, comm=comm, algo=algo, compact=compact, graph=False)
-        counter.forward(img, INF, eps, ctx.rank, ctx.world)
         n0 = lib.fb_launch_count()
-        counter.forward(img, INF, eps, ctx.rank, ctx.world)
+        ver.forward(img, INF, eps, ctx.rank, ctx.world)
         launches = int(lib.fb_launch_count() - n0)
         ms = ctx.timed(lambda: ver.forward(img, INF, eps, ctx.rank, ctx.world), steps)
-        res[name] = {"ms_per_image": ms / steps, "images_per_s": 1e3 * steps / ms, "launches_per_image": launches,
-                     "cuda_graph": bool(ver.graph and ctx.world == 1)}
+        res[name] = {"ms_per_image": ms / steps, "images_per_s": 1e3 * steps / ms, "launches_per_image": launches}
         if comm is not None:
             comm.check(sync=True)
         l, u = ver.forward(img, INF, eps, ctx.rank, ctx.world)

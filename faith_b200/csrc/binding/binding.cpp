@@ -630,6 +630,37 @@ FB_FN(softmax_checked) {   // x (4), p, eps, words -> None or (lw, uw, lb, ub, s
   END_HANDLE_TH_ERRORS
 }
 
+// net (address of an fb_cnn), image [C, H, W], p, eps, first row, rows, communicator (address or None), all-reduce, compact,
+// features of the last layer, arena (uint8 tensor) -> [2, features]: lower and upper ends of the range
+FB_FN(cnn_forward) {
+  HANDLE_TH_ERRORS
+  Call c(args, nargs, 11, "cnn_forward");
+  auto address = [&](int i) {
+    void* const p = PyLong_AsVoidPtr(args[i]);
+    if (p == nullptr && PyErr_Occurred()) throw python_error();
+    return p;
+  };
+  const fb_cnn* const net = static_cast<const fb_cnn*>(address(0));
+  const at::Tensor& image = c.tensor(1);
+  const int p = c.norm(2), start = c.integer(4), rows = c.integer(5), algo = c.integer(7), compact = c.integer(8), n_out = c.integer(9);
+  const float eps = c.real(3);
+  fb_comm* const comm = c.none(6) ? nullptr : static_cast<fb_comm*>(address(6));
+  if (image.numel() != (int64_t)net->cin * net->h * net->w) fail("cnn_forward: the image is not of the network's input shape");
+  if (!THPVariable_Check(args[10])) fail("cnn_forward: arena tensor required");
+  const at::Tensor& arena = THPVariable_Unpack(args[10]);
+  if (!arena.is_cuda() || arena.scalar_type() != at::kByte || arena.get_device() != c.device()) fail("cnn_forward: arena of the image's device required");
+  at::Tensor out = empty({2, n_out}, c.device());
+  int rc;
+  {
+    Launch l(c.device());
+    rc = fb_cnn_forward_f32(net, ptr(image), p, eps, start, rows, comm, algo, compact, ptr(out), ptr(out) + n_out, nullptr,
+                            arena.data_ptr(), arena.numel(), l.stream());
+  }
+  check_status(rc, "fb_cnn_forward_f32");
+  return THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
 FB_FN(setup) {   // FaithError, _lib.check
   if (nargs != 2) {
     PyErr_SetString(PyExc_TypeError, "setup takes 2 arguments");
@@ -646,7 +677,7 @@ FB_FN(setup) {   // FaithError, _lib.check
 PyMethodDef kMethods[] = {FB_DEF(setup), FB_DEF(concretize), FB_DEF(relax), FB_DEF(relax_checked), FB_DEF(matmul), FB_DEF(dot_product),
                           FB_DEF(context_kmajor), FB_DEF(context), FB_DEF(mul_bounds), FB_DEF(add), FB_DEF(scale), FB_DEF(mul_features), FB_DEF(rowsum),
                           FB_DEF(layernorm_novar), FB_DEF(layernorm_standard_checked), FB_DEF(split_heads), FB_DEF(merge_heads), FB_DEF(conv2d), FB_DEF(softmax),
-                          FB_DEF(softmax_checked), {nullptr, nullptr, 0, nullptr}};
+                          FB_DEF(softmax_checked), FB_DEF(cnn_forward), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_binding", "Native boundary of the tensor-level operators.", -1, kMethods,
                        nullptr, nullptr, nullptr, nullptr};
 

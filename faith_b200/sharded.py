@@ -242,12 +242,17 @@ class CnnVerifier:
     whole pass, the structure of the identity input is used (first convolution and its relaxation written from the
     filter alone, later convolutions windowed).  `forward(dense=True)`, and networks that start otherwise, take the
     general kernels operator by operator with the identity materialised.
+
+    `graph` is accepted and has no effect.  Single-GPU passes used to be replayed from a CUDA graph captured per shape, norm
+    and radius, which were never given up.  With five launches a pass the copies around a replay cost more than enqueueing it
+    (3 x 32 x 32 image: 49.6 us a pass replayed, 44.1 us enqueued; one pass alone 60.7 and 56.1 us), and the first pass at a
+    radius was a capture and an instantiation (0.8 ms and more; 57 us now).
     """
 
     def __init__(self, layers, device, group=None, comm=None, algo=0, compact=True, graph=True):
         self.device = torch.device(device)
-        self.graph = graph      # single-GPU passes through the driver are replayed from a CUDA graph
-        self._graphs = {}
+        self.graph = graph      # without effect (see the class)
+        self._plan = None
         self.compact = compact  # rows kept as their windows only (fb_cw_*), or dense rows (fb_conv2d_windowed_f32)
         self.group = group
         self.comm = comm        # faith_b200.comm.Comm: the all-reduces are enqueued by the library (NCCL or one-shot)
@@ -275,49 +280,28 @@ class CnnVerifier:
         self._recs = recs
         self._driver_ok = bool(self.layers) and self.layers[0][0] == "conv"
 
-    def _run_driver(self, img, p, eps, start, size, world):
-        """One fb_cnn_forward_f32 call on the current stream; img [C, H, W] on the device."""
-        C, H, W = img.shape
-        lib = load()
-        net = _lib.Cnn(len(self.layers), self._recs, C, H, W)
-        need = lib.fb_cnn_workspace_bytes(ctypes.byref(net), size)
-        if need < 0:
-            raise _lib.FaithError("fb_cnn_workspace_bytes: network not supported by the driver")
-        if self._arena is None or self._arena.numel() < need:
-            self._graphs.clear()     # captured passes point into the arena that is about to be replaced
-            self._arena = torch.empty(need, dtype=torch.uint8, device=self.device)
-        out = torch.empty(2, self._out_features(C, H, W), device=self.device)
-        comm = self.comm._h if (self.comm is not None and world > 1) else None
-        with torch.cuda.device(self.device):
-            check(lib.fb_cnn_forward_f32(ctypes.byref(net), img.data_ptr(), ops.norm_code(p), float(eps), start, size, comm,
-                                         self.algo, 1 if self.compact else 0, out[0].data_ptr(), out[1].data_ptr(), None,
-                                         self._arena.data_ptr(), self._arena.numel(), ops._stream()), "fb_cnn_forward_f32")
-        return out
+    def _plan_for(self, C, H, W, size):
+        """The network as the C driver takes it for a C x H x W image and the features of its last layer, with the arena for
+        `size` rows of dim_in at hand; kept for the shape of the last call."""
+        key = (C, H, W, size)
+        if self._plan is None or self._plan[0] != key:
+            net = _lib.Cnn(len(self.layers), self._recs, C, H, W)
+            need = load().fb_cnn_workspace_bytes(ctypes.byref(net), size)
+            if need < 0:
+                raise _lib.FaithError("fb_cnn_workspace_bytes: network not supported by the driver")
+            if self._arena is None or self._arena.numel() < need:
+                self._arena = torch.empty(need, dtype=torch.uint8, device=self.device)
+            self._plan = (key, net, self._out_features(C, H, W))
+        return self._plan
 
     def _forward_driver(self, image, p, eps, start, size, world):
-        if not self.graph or world > 1:
-            img = image.to(self.device, torch.float32, non_blocking=True).contiguous()
-            return self._run_driver(img, p, eps, start, size, world).unbind(0)
-        # Single GPU: the pass is a dozen launches of a few microseconds each, which cost more to launch than to run;
-        # they are captured once per (shape, norm, radius) into a CUDA graph that reads the image from a fixed device
-        # buffer and writes the range to fixed outputs.  (Not with a communicator: the one-shot exchange takes its
-        # epoch as a kernel argument, which a replay would repeat.)
-        key = (tuple(image.shape), float(p), float(eps), start, size)
-        ent = self._graphs.get(key)
-        if ent is None:
-            with torch.cuda.device(self.device):
-                static_img = torch.empty(tuple(image.shape), device=self.device)
-                static_img.copy_(image)
-                self._run_driver(static_img, p, eps, start, size, world)      # sizes the arena, warms every launcher
-                torch.cuda.synchronize(self.device)
-                g = torch.cuda.CUDAGraph()
-                with torch.cuda.graph(g, capture_error_mode="thread_local"):   # other threads (a collective's watchdog) stay free to call CUDA
-                    out = self._run_driver(static_img, p, eps, start, size, world)
-            ent = self._graphs[key] = (g, static_img, out)
-        g, static_img, out = ent
-        static_img.copy_(image, non_blocking=True)
-        g.replay()
-        return out.clone().unbind(0)
+        """One fb_cnn_forward_f32 call on the current stream."""
+        _, net, n_out = self._plan_for(*image.shape, size)
+        img = image.to(self.device, torch.float32, non_blocking=True).contiguous()
+        comm = self.comm._h.value if (self.comm is not None and world > 1) else None
+        out = _lib.binding().cnn_forward(ctypes.addressof(net), img, p, eps, start, size, comm, self.algo, 1 if self.compact else 0,
+                                         n_out, self._arena)
+        return out.unbind(0)
 
     def _out_features(self, C, H, W):
         c, h, w = C, H, W

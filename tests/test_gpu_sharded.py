@@ -364,6 +364,33 @@ def test_cnn_driver_with_filters_larger_than_the_map(chain):
     helpers.assert_close(got[1], want[1].cpu(), "u", atol=2e-6 * scale)
 
 
+def test_cnn_verifier_keeps_nothing_per_radius():
+    """A radius or an image that the verifier has not seen costs what a known one does: nothing is captured or allocated for it.
+    The pass can be captured by the caller."""
+    from faith_b200.sharded import CnnVerifier
+    g = torch.Generator().manual_seed(49)
+    layers = [("conv", torch.randn(4, 2, 3, 3, generator=g) * 0.3, None, 1, 1), ("relu",),
+              ("linear", torch.randn(5, 4 * 10 * 10, generator=g) * 0.05, torch.randn(5, generator=g))]
+    ver = CnnVerifier(layers, DEV)
+    imgs = [torch.rand(2, 10, 10, generator=g).to(DEV) for _ in range(8)]
+    ver.forward(imgs[0], 2.0, 0.01)
+    reserved = torch.cuda.memory_reserved()
+    for i, img in enumerate(imgs):
+        l, u = ver.forward(img, 2.0, 0.01 + 0.003 * i)
+        want = CnnVerifier(layers, DEV, graph=False).forward(img, 2.0, 0.01 + 0.003 * i)
+        assert torch.equal(l, want[0]) and torch.equal(u, want[1])
+    assert torch.cuda.memory_reserved() == reserved
+    buf = imgs[0].clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        l, u = ver.forward(buf, 2.0, 0.02)
+    for img in imgs[1:3]:
+        buf.copy_(img)
+        graph.replay()
+        want = ver.forward(img, 2.0, 0.02)
+        assert torch.equal(l, want[0]) and torch.equal(u, want[1])
+
+
 @pytest.mark.parametrize("C,HW,c1,c2,n,p", [(1, 16, 8, 16, 2, 1.0), (3, 23, 24, 48, 16, 2.0), (1, 21, 5, 7, 33, float("inf"))])
 def test_cnn_driver_with_the_head_reduced_to_its_norms(C, HW, c1, c2, n, p):
     from faith_b200.sharded import CnnVerifier
