@@ -151,10 +151,26 @@ def binding():
     if _binding_module is None:
         load()
         import torch  # noqa: F401  (the module links against torch's libraries)
-        from . import _binding
+        try:
+            from . import _binding
+        except ImportError as e:
+            raise ImportError("%s (%s)" % (e, _REBUILD)) from e
+        _check_target(_binding)
         _binding.setup(FaithError, check)
         _binding_module = _binding
     return _binding_module
+
+
+_REBUILD = "the extension module has to be built for the torch at hand: python -m faith_b200.build"
+
+
+def _check_target(module):
+    """Refuses an extension module that was built for another torch or interpreter: it uses torch's internal C++ interface."""
+    import torch
+    from .build import binding_target
+    want = binding_target(torch.__version__)
+    if getattr(module, "built_for", None) != want:
+        raise ImportError("faith_b200._binding was built for %s, this is %s (%s)" % (getattr(module, "built_for", "an unknown torch"), want, _REBUILD))
 
 
 class FaithError(RuntimeError):

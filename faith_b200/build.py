@@ -5,6 +5,7 @@ boundary faith_b200/_binding.so from csrc/binding/ with the host compiler.
     python -m faith_b200.build --force    # rebuild everything
 """
 import concurrent.futures
+import importlib.metadata
 import os
 import subprocess
 import sys
@@ -41,16 +42,32 @@ def _cuda_home():
     return os.environ.get("CUDA_HOME", "/usr/local/cuda")
 
 
+def binding_target(torch_version=None):
+    """What the extension module is built for: it uses torch's internal C++ interface, so another torch (or another
+    interpreter) needs another build.  The module holds this text as `built_for`."""
+    if torch_version is None:
+        torch_version = importlib.metadata.version("torch")   # (without the import, which takes seconds)
+    return "torch %s, %s" % (torch_version, sysconfig.get_config_var("SOABI"))
+
+
+def _binding_current(path, target):
+    newest = max(os.path.getmtime(BINDING_SRC), max(os.path.getmtime(os.path.join(INCLUDE, f)) for f in os.listdir(INCLUDE)))
+    if not os.path.exists(path) or os.path.getmtime(path) < newest:
+        return False
+    with open(path, "rb") as f:
+        return target.encode() + b"\0" in f.read()
+
+
 def _build_binding(force, verbose):
     """The extension module that faith_b200/ops.py calls: host code only, linked against the C-ABI library next to it."""
-    newest = max(os.path.getmtime(BINDING_SRC), max(os.path.getmtime(os.path.join(INCLUDE, f)) for f in os.listdir(INCLUDE)))
-    if not force and os.path.exists(BINDING) and os.path.getmtime(BINDING) >= newest:
+    if not force and _binding_current(BINDING, binding_target()):
         return
     import torch
     troot = os.path.dirname(torch.__file__)
     tlib = os.path.join(troot, "lib")
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
            "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
+           '-DFB_BUILT_FOR="%s"' % binding_target(torch.__version__),
            "-I" + INCLUDE, "-I" + os.path.join(troot, "include"),
            "-I" + os.path.join(troot, "include", "torch", "csrc", "api", "include"),
            "-I" + os.path.join(_cuda_home(), "include"), "-I" + sysconfig.get_paths()["include"],

@@ -683,4 +683,11 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_binding", "Native boundary of th
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__binding(void) { return PyModule_Create(&kModule); }
+PyMODINIT_FUNC PyInit__binding(void) {
+  PyObject* const m = PyModule_Create(&kModule);
+  if (m != nullptr && PyModule_AddStringConstant(m, "built_for", FB_BUILT_FOR) != 0) {   // (build.py: binding_target)
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}

@@ -3,6 +3,8 @@ import ctypes
 import os
 import re
 
+import pytest
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
@@ -221,3 +223,19 @@ def test_encoder_arena_size_without_gpu():
     assert lib.fb_encoder_workspace_bytes(ctypes.byref(enc()), S, L, 2) > got
     assert lib.fb_encoder_workspace_bytes(ctypes.byref(enc(d_model=130)), S, L, words) == -1
     assert lib.fb_encoder_workspace_bytes(None, S, L, words) == -1
+
+
+def test_binding_belongs_to_the_torch_at_hand():
+    """The extension module is rebuilt for, and refused with, any other torch or interpreter than its own."""
+    import types
+    import torch
+    from faith_b200 import _lib, build
+    target = build.binding_target()
+    assert target == build.binding_target(torch.__version__)
+    assert build._binding_current(build.BINDING, target)
+    assert not build._binding_current(build.BINDING, build.binding_target("0.0.1"))
+    assert _lib.binding().built_for == target
+    with pytest.raises(ImportError, match="python -m faith_b200.build"):
+        _lib._check_target(types.SimpleNamespace(built_for=build.binding_target("0.0.1")))
+    with pytest.raises(ImportError, match="python -m faith_b200.build"):
+        _lib._check_target(types.SimpleNamespace())
