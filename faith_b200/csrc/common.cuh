@@ -149,7 +149,7 @@ struct RangeEpilogue {
   float *k_l, *k_u, *r_lb, *r_ub;
   int* violation;
 };
-bool small_product(int64_t M, int N);   // whether the kernel for few rows takes a product of that size
+bool small_product(int64_t M, int N, int K);   // whether the kernel for few rows takes a product of that size
 int launch_split_sign_small(const float* a_lo, const float* a_up, const float* W, const float* bias, float* c_lo, float* c_up, int64_t M,
                             int N, int K, cudaStream_t st, int split_rows, int split_d, const RangeEpilogue* range);
 // matmul.cu: fb_matmul_heads_ranges_f32 with the wishes of the driver: ranges transposed, relaxation coefficients of the result.

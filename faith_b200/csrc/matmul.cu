@@ -112,7 +112,7 @@ ranges_from_norms_kernel(float* __restrict__ lb, float* __restrict__ ub, const f
 // Whether the bias rows of a product go to the kernel for few rows, in the form that can ride in the tensor-core launch.
 static bool small_bias_rows(const float* x_lb, const float* x_ub, const float* W, const float* y_lb, const float* y_ub, int64_t rows, int Dy,
                             int Do) {
-  return rows > 0 && !fb::tc_gemm_supported(x_lb, x_ub, W, y_lb, y_ub, rows, Dy, Do) && fb::small_product(rows, Dy) && Do % 4 == 0 &&
+  return rows > 0 && !fb::tc_gemm_supported(x_lb, x_ub, W, y_lb, y_ub, rows, Dy, Do) && fb::small_product(rows, Dy, Do) && Do % 4 == 0 &&
          fb::aligned16(x_lb) && fb::aligned16(x_ub) && fb::aligned16(W);
 }
 
@@ -249,7 +249,7 @@ int fb::matmul_ranges_ex(const float* x_lw, const float* x_uw, const float* x_lb
     plain_lb = b_lo;
     plain_ub = b_up;
     rc = fb::launch_split_sign_tc(x_lb, x_ub, W, bias, plain_lb, plain_ub, rows, Dy, Do, st, 0, 0);
-  } else if (!fb::tc_gemm_supported(x_lb, x_ub, W, y_lb, y_ub, rows, Dy, Do) && fb::small_product(rows, Dy)) {
+  } else if (!fb::tc_gemm_supported(x_lb, x_ub, W, y_lb, y_ub, rows, Dy, Do) && fb::small_product(rows, Dy, Do)) {
     fb::RangeEpilogue rg = {norm_lo, norm_up, y_l, y_u, words, eps, 0, -1, nullptr, nullptr, nullptr, nullptr, nullptr};
     bool split = heads > 1;
     if (wishes != nullptr) {

@@ -399,8 +399,21 @@ __global__ void __launch_bounds__(kSmThreads) split_sign_gemm_small(const SmallP
 
 }  // namespace
 
-// (below that many 128 x 128 tiles the kernel above would not fill the machine once)
-bool small_product(int64_t M, int N) { return N > 16 && ceil_div(M, BM) * ceil_div(N, BN) < device_info().sms; }
+// Whether a product goes to the blocks of 8 x 32 (split_sign_gemm_small) instead of the tiles of 128 x 128.  Where the tiles
+// would not fill the machine once, they take as long as one of them takes, whatever M; the small blocks take turns, each reading its
+// columns of W again.  Measured, us, tiles / small blocks at 2000 and at 4000 blocks: K = 30, N = 128 14.5 / 12.5 and 14.5 / 20.6;
+// K = 130, N = 128 39.4 / 24.7 and 40.0 / 42.7; K = 1022, N = 128 245 / 144 and 246 / 291; K = 9, N = 200 10.5 / 10.4 and
+// 10.5 / 16.6; K = 130, N = 128, 18 000 rows 41.2 / 88.1.  The rule compares the slopes of both (us; a result whose rows do not
+// take 128-bit stores costs a tile 5 more): over 680 sizes (3 <= K <= 2050, 17 <= N <= 2050) the kernel it takes is at most 15 %
+// slower than the other.
+static bool few_blocks(int64_t M, int N, int K) {
+  const int64_t sms = device_info().sms;
+  if (ceil_div(M, BM) * ceil_div(N, BN) >= sms) return false;
+  const double blocks_per_sm = (double)(ceil_div(M, kSmRows) * ceil_div(N, kSmCols)) / sms;
+  const double tile = 3.3 + 3.2 * ceil_div(K, BK) + (N > 64 && N % 4 != 0 ? 5.0 : 0.0);
+  return blocks_per_sm * (0.414 + 0.0074 * K) <= tile;
+}
+bool small_product(int64_t M, int N, int K) { return N > 16 && few_blocks(M, N, K); }
 
 int launch_split_sign_small(const float* a_lo, const float* a_up, const float* W, const float* bias, float* c_lo, float* c_up, int64_t M,
                             int N, int K, cudaStream_t st, int split_rows, int split_d, const RangeEpilogue* range) {
@@ -453,7 +466,7 @@ int launch_split_sign_ffma(const float* a_lo, const float* a_up, const float* W,
   const int gn = (int)ceil_div(N, BN);
   if (gm > 0x7fffffff || gn > 65535) return FB_ERR_SHAPE;
   const bool vec = K % 4 == 0 && aligned16(a_lo) && aligned16(a_up) && aligned16(W);
-  if (gm * gn < device_info().sms)
+  if (few_blocks(M, N, K))
     return launch_split_sign_small(a_lo, a_up, W, bias, c_lo, c_up, M, N, K, st, split_rows, split_d, nullptr);
   const size_t smem = sizeof(float) * 2 * kStageFloats;
   if (vec) {

@@ -1025,6 +1025,19 @@ def test_product_of_few_rows(B, L, Do, Dy):
     helpers.assert_bounds_arbitrated(got, o, o64, "product of few rows %d %d %d" % (B * L, Do, Dy))
 
 
+@pytest.mark.parametrize("rows,Do,Dy", [(9024, 30, 33), (9025, 30, 33), (6424, 65, 130), (6425, 65, 130), (1000, 9, 500), (1001, 9, 500)])
+def test_product_between_small_blocks_and_tiles(rows, Do, Dy):
+    """Either side of the rule that sends a product to blocks of 8 x 32 or to tiles of 128 x 128 (the sizes are those of 148 SMs)."""
+    from faith_b200 import ops
+    lw, lb, uw, ub = cases.rand_bounds(1303, 1, rows, 1, Do)
+    W, bias = cases.rand_weight(1304, Dy, Do)
+    z = ops.matmul(*[t.to(DEV) for t in (lw, uw, lb, ub)], W.to(DEV), bias.to(DEV))
+    o = O.OBounds(2.0, 0.1, lw, lb, uw, ub).dense(W, bias)
+    o64 = O.OBounds(2.0, 0.1, *[t.double() for t in (lw, lb, uw, ub)]).dense(W.double(), bias.double())
+    for got, k in zip(z, ("lw", "uw", "lb", "ub")):
+        helpers.assert_arbitrated(got, getattr(o, k), getattr(o64, k), "product of %d rows, %s" % (rows, k))
+
+
 @pytest.mark.parametrize("B,Lx,Ly,Di,K,words", [(2, 5, 5, 6, 3, 1), (3, 21, 21, 64, 32, 2), (2, 33, 40, 32, 32, 1), (1, 64, 31, 10, 64, 1),
                                                 (2, 32, 23, 16, 21, 1)])
 def test_dot_and_context_of_ragged_lengths(B, Lx, Ly, Di, K, words):
