@@ -183,7 +183,7 @@ int context_ex(const float* x_lw, const float* x_uw, const float* x_lb, const fl
                float* y_l, float* y_u, int B, int Lx, int Ly, int Di, int K, int words, int p, float eps, float out_scale,
                int merge_heads, int given, int ldx, bool transposed_ranges, void* stream);
 
-// Opts `kernel` in to `bytes` of dynamic shared memory on the current device (nothing to do up to 48 KB, or when it
+// Opts `kernel` in to `bytes` of dynamic shared memory on the current device (nothing to do up to 40 KB, or when it
 // already has that much): FB_OK or FB_ERR_CUDA.
 int ensure_dynamic_smem_impl(const void* func, size_t bytes);
 template <typename K>

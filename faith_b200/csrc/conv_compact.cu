@@ -904,7 +904,7 @@ int conv_rows(const float* z_lo, const float* z_up, const float* W1, const float
   auto kern = Kh == 3 && Kw == 3 ? (cpt == 2 ? cw_conv_kernel<3, 2, kAbi> : cw_conv_kernel<3, 1, kAbi>)
                                  : (cpt == 2 ? cw_conv_kernel<0, 2, kAbi> : cw_conv_kernel<0, 1, kAbi>);
   if (!direct)
-    if (int rc = ensure_dynamic_smem(kern, bytes() + kCwStatic)) return rc;   // (48 KB without the attribute hold the static part too)
+    if (int rc = ensure_dynamic_smem(kern, bytes())) return rc;
   ProfileScope prof(PK_CONV, 8.0 * rows * Cout * go.wh * go.ww * Cin * Kh * Kw,
                     4.0 * 2.0 * rows * ((double)Cin * gi.wh * gi.ww + (double)Cout * go.wh * go.ww), (void*)st);
   if (kAbi) {   // (the kernel stores the pixels' own windows)
@@ -956,7 +956,7 @@ int linear_rows(const float* z_lw, const float* z_uw, const float* coef, const f
               : NB == 8  ? cw_linear_kernel<8, kAbi>
               : NB == 12 ? cw_linear_kernel<12, kAbi>
                          : cw_linear_kernel<16, kAbi>;
-  if (int rc = ensure_dynamic_smem(kern, smem + kCwStatic)) return rc;
+  if (int rc = ensure_dynamic_smem(kern, smem)) return rc;
   ProfileScope prof(PK_MATMUL, 8.0 * rows * C * q.g.wh * q.g.ww * N,
                     4.0 * (2.0 * rows * C * q.g.wh * q.g.ww + 2.0 * rows * N + (double)C * H * W * N), (void*)st);
   fb::launch_k(kern, dim3((unsigned)blocks, (unsigned)groups), kCwLinThreads, smem, st, q);

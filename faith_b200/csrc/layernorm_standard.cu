@@ -133,7 +133,7 @@ layernorm_standard_kernel(const float* __restrict__ x_lw, const float* __restric
   const int cols = Do < kT ? Do : kT;
   const int groups = kT / cols;
   const int blk = Di / words;
-  __shared__ float s_red[2][kT];
+  __shared__ float s_red[2][kT];   // (beside the dynamic part: see ensure_dynamic_smem)
   bool bad = false;
   for (int c0 = 0; c0 < Do; c0 += cols) {
     const int cc = tid % cols, g = tid / cols, j = c0 + cc;

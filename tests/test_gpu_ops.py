@@ -1181,6 +1181,12 @@ def test_standard_layer_norm_by_number_of_rows(L, Di, Do, p, words):
     test_standard_layer_norm_in_one_kernel(L, Di, Do, p, words)
 
 
+@pytest.mark.parametrize("Di,Do,words", [(166, 32, 2), (160, 33, 1), (150, 36, 3), (560, 8, 2)])
+def test_standard_layer_norm_near_48_KB_of_shared_memory(Di, Do, words):
+    """Tiles that stay below 48 KB by themselves and exceed them together with the kernel's static part."""
+    test_standard_layer_norm_in_one_kernel(40, Di, Do, 2.0, words)
+
+
 @pytest.mark.parametrize("Di,Do,words", [(256, 21, 2), (256, 32, 1), (256, 17, 4)])
 @pytest.mark.parametrize("p", [1.0, 2.0, float("inf")])
 def test_fused_softmax_of_wide_inputs(Di, Do, words, p):
