@@ -181,21 +181,23 @@ __device__ __forceinline__ void tile_rescale(const float* __restrict__ gl, const
 // The tangent points of tanh for a block's kCW columns by all of its warps, l and u being known to thread c < kCW of column c:
 // one thread per column walked twenty dependent evaluations (a third of the block's lifetime, with seven warps waiting).  The two
 // searches go to different warps, and three warps each evaluate the middle and both middles that can follow, i.e. two steps
-// of ten at a time; the moves and their rounding are those of tanh_point.  tanh on [8, 64, 128, 256]: 79 -> 72 us.  Every thread
-// calls; point[2] is valid in threads < kCW, where `mine`.
+// of ten at a time; the moves and their rounding are those of tanh_point.  tanh on [8, 64, 128, 256]: 79 -> 72 us.  A block none of
+// whose columns crosses zero has nothing to search (16384 rows of [8, 8] with one column in ten crossing: 164 us with the columns
+// beyond Do searched as well, 68 us).  Every thread calls; point[2] is valid in threads < kCW whose column crosses zero.
 __device__ __forceinline__ void tanh_points(float l, float u, bool mine, float point[2]) {
   static_assert(kCW == 32 && kThreads == 256 && kTanhSteps % 2 == 0, "a lane per column, a warp per evaluation");
   __shared__ float s_range[2][kCW];
   __shared__ float s_point[2][kCW];
   __shared__ bool s_right[2][2][3][kCW];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid < kCW) { s_range[0][tid] = mine ? l : 0.f; s_range[1][tid] = mine ? u : 0.f; }
+  if (tid < kCW) { s_range[0][tid] = mine ? l : 1.f; s_range[1][tid] = mine ? u : 1.f; }   // (no search beyond the last column)
   __syncthreads();
   const float cl = s_range[0][lane], cu = s_range[1][lane];
   const bool search = (cl > 0.f) == (cu < 0.f);   // the range crosses zero (as relax_column tells it)
   const bool upper = warp & 1;
   const int node = warp >> 1;      // 0: d, 1: what follows a step to the right, 2: to the left, 3: none
   const float x = upper ? cl : cu, tx = tanhf(x);
+  if (!__any_sync(0xffffffffu, search)) return;   // (the same in every warp: a lane per column)
   TanhSearch q = tanh_search(upper, cl, cu);
 #pragma unroll 1
   for (int t = 0; t < kTanhSteps / 2; ++t) {
@@ -220,7 +222,7 @@ col_relax_native(int op, const float* __restrict__ lw, const float* __restrict__
                  const float* __restrict__ lb, const float* __restrict__ ub,
                  float* __restrict__ o_lw, float* __restrict__ o_uw, float* __restrict__ o_lb,
                  float* __restrict__ o_ub, int Di, int Do, int ntiles, int words, int p, float eps,
-                 int* __restrict__ violation) {
+                 int tanh_op, int* __restrict__ violation) {
   pdl_sync();
   extern __shared__ __align__(16) float smem[];
   float* s_red = smem;                    // [2][8][kCW]
@@ -240,7 +242,6 @@ col_relax_native(int op, const float* __restrict__ lw, const float* __restrict__
   }
   float l, u;
   tile_concretize<VEC, STAGED>(gl, gu, Di, Do, c0, words, p, eps, s_l, s_u, s_red, lbv, ubv, l, u);
-  const bool tanh_op = (op >= OP_COEF_ONLY ? op - OP_COEF_ONLY : op) == FB_TANH;
   float point[2] = {0.f, 0.f};
   if (tanh_op) tanh_points(l, u, mine, point);
   if (op >= OP_COEF_ONLY) {
@@ -283,12 +284,16 @@ col_relax_native(int op, const float* __restrict__ lw, const float* __restrict__
 // Bound by HBM.  relu on [8, 64, 64, 512]: 63.3 us staged in shared memory, 54.7 us held (N = 2, 64 registers).  N = 8 (Di 256)
 // leaves two blocks per SM, which read once what would otherwise come twice, the second time from L2: [8, 64, 256, 256] relu
 // 111 -> 87 us, tanh 129 -> 107 us.  N = 4 (Di 128) has too few blocks to hide the column's scalar chain beside a tile that fits
-// into shared memory six times: tanh on [8, 64, 128, 256] 89 us against 72 us staged.
+// into shared memory six times: tanh on [8, 64, 128, 256] 89 us against 72 us staged.  Where half of the registers hold nothing
+// the staged tile is the better one: 32 768 rows of [32, 32] relu 146 us staged, 153 us held (N = 2), tanh 204 and 219 us.  So it
+// is for tanh, whose chain is longer, with N = 8, less than 224 rows and more blocks than fit at once: 5461 rows of [192, 32], most
+// columns crossing zero, 116 us staged, 125 us held; relu 98 and 83 us; tanh on 170 rows 8.7 and 7.6 us.
 template <int N>
 __global__ void __launch_bounds__(kThreads)
 col_relax_held(int op, const float* __restrict__ lw, const float* __restrict__ uw, const float* __restrict__ lb,
                const float* __restrict__ ub, float* __restrict__ o_lw, float* __restrict__ o_uw, float* __restrict__ o_lb,
-               float* __restrict__ o_ub, int Di, int Do, int ntiles, int words, int p, float eps, int* __restrict__ violation) {
+               float* __restrict__ o_ub, int Di, int Do, int ntiles, int words, int p, float eps, int tanh_op,
+               int* __restrict__ violation) {
   pdl_sync();
   constexpr int kWords = 4;   // word blocks between two barriers
   __shared__ float s_red[kWords * 2 * 8 * kCW], s_norm[2 * kWords][kCW], s_coef[4 * kCW];
@@ -358,12 +363,12 @@ col_relax_held(int op, const float* __restrict__ lw, const float* __restrict__ u
     }
   }
   float point[2] = {0.f, 0.f};
-  if (op == FB_TANH) tanh_points(l, u, mine, point);
+  if (tanh_op) tanh_points(l, u, mine, point);
   if (tid < kCW) {
     ColCoef c = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (mine) {
       bool bad = false;
-      c = relax_column(op, l, u, lbv, ubv, bad, op == FB_TANH ? point : nullptr);
+      c = relax_column(op, l, u, lbv, ubv, bad, tanh_op ? point : nullptr);
       if (bad && violation != nullptr) *violation = 1;
       o_lb[(size_t)row * Do + c0 + tid] = c.nlb;
       o_ub[(size_t)row * Do + c0 + tid] = c.nub;
@@ -864,10 +869,12 @@ int launch_relax(int op, const float* lw, const float* uw, const float* lb, cons
   if (blocks > 0x7fffffff) return FB_ERR_SHAPE;
   const bool vec = Do % 4 == 0 && aligned16(lw) && aligned16(uw) &&
                    (op >= OP_COEF_ONLY || (aligned16(o_lw) && aligned16(o_uw)));
+  const bool tanh_op = (op >= OP_COEF_ONLY ? op - OP_COEF_ONLY : op) == FB_TANH;
   // a tile that fits into registers without costing occupancy, or that is too large for shared memory (figures at the kernel)
-  if (vec && op < OP_COEF_ONLY && (Di <= 64 || (Di > 128 && Di <= 256)) && (words == 1 || (Di / words) % 32 == 0)) {
+  const bool held = (Di > 32 && Di <= 64) || (Di > 128 && Di <= 256 && (!tanh_op || Di >= 224 || blocks <= 2 * device_info().sms));
+  if (vec && op < OP_COEF_ONLY && held && (words == 1 || (Di / words) % 32 == 0)) {
     auto kern = Di <= 64 ? col_relax_held<2> : col_relax_held<8>;
-    launch_k(kern, (unsigned)blocks, kThreads, 0, st, op, lw, uw, lb, ub, o_lw, o_uw, o_lb, o_ub, Di, Do, ntiles, words, p, eps, violation);
+    launch_k(kern, (unsigned)blocks, kThreads, 0, st, op, lw, uw, lb, ub, o_lw, o_uw, o_lb, o_ub, Di, Do, ntiles, words, p, eps, tanh_op ? 1 : 0, violation);
     FB_LAUNCH_OK();
     return FB_OK;
   }
@@ -884,7 +891,7 @@ int launch_relax(int op, const float* lw, const float* uw, const float* lb, cons
     if (rc_ != FB_OK) return rc_;                                                                          \
     fb::launch_k(col_relax_native<V, S>, (unsigned)blocks, kThreads, smem, st, op, lw, uw, lb, ub, o_lw, o_uw, o_lb, \
                                                                      o_ub, Di, Do, ntiles, words, p, eps,  \
-                                                                     violation);                           \
+                                                                     tanh_op ? 1 : 0, violation);                           \
   } while (0)
   if (vec && staged) FB_RELAX_LAUNCH(4, true);
   else if (vec) FB_RELAX_LAUNCH(4, false);

@@ -1194,6 +1194,25 @@ def test_fused_softmax_of_wide_inputs(Di, Do, words, p):
     test_fused_softmax_of_any_length(Di, Do, words, p)
 
 
+# (either side of the sizes at which the tile moves between registers and shared memory, with few and with many blocks)
+@pytest.mark.parametrize("L,Di,Do", [(3, 32, 36), (3, 33, 8), (5, 64, 40), (3, 65, 12), (3, 160, 36), (301, 160, 4), (301, 224, 4), (3, 257, 8)])
+@pytest.mark.parametrize("cross", ["none", "one", "all"])
+def test_tanh_of_blocks_with_and_without_a_search(L, Di, Do, cross):
+    """Columns that do not cross zero, one that does per row, and all of them: a block skips the bisections where none does."""
+    from faith_b200 import ops
+    from faith_b200._lib import FB_TANH
+    lw, lb, uw, ub = cases.rand_bounds(424, 1, L, Di, Do, 1.0, 0.01)
+    lb, ub = lb.abs() + 1.0, ub.abs() + 3.0
+    if cross != "none":
+        at = slice(Do - 1, Do) if cross == "one" else slice(0, Do)
+        lb[..., at] = -lb[..., at]
+    lb[:, ::2], ub[:, ::2] = -ub[:, ::2], -lb[:, ::2]
+    o = O.OBounds(2.0, 0.02, lw, lb, uw, ub).tanh()
+    z = ops.relax(FB_TANH, *[t.to(DEV) for t in (lw, uw, lb, ub)], 2.0, 0.02, 1)
+    for got, name in zip(z, ("lw", "uw", "lb", "ub")):
+        helpers.assert_close(got, getattr(o, name), name)
+
+
 @pytest.mark.parametrize("Di,Do,words", [(129, 36, 1), (160, 32, 5), (256, 40, 8), (256, 64, 1), (255, 4, 1)])
 @pytest.mark.parametrize("p", [1.0, 2.0, float("inf")])
 def test_relax_of_wide_columns_held_in_registers(Di, Do, words, p):
