@@ -206,6 +206,109 @@ dot_weight_transposed(const float* __restrict__ x_lw, const float* __restrict__ 
   }
 }
 
+// Many thin products (a few rows against any number, a large batch): a thread per coordinate and 4 x 4 outputs, operands straight
+// from global memory.  The kernel above has one block of 200 KB an SM and its ring to fill for each; here many small blocks hide
+// each other's loads.  512 products of 64 x 1 rows, K = 8, dim_in 2: 386 us above, 156 us here; 4 x 64, K = 8, dim_in 8: 299 and
+// 175 us.  With more arithmetic per loaded value the ring wins again: 512 of 4 x 16, K = 128, dim_in 16: 555 and 867 us.
+constexpr int kThinM = 128, kThinK = 128;
+__global__ void __launch_bounds__(kThinM)
+dot_weight_transposed_thin(const float* __restrict__ x_lw, const float* __restrict__ x_uw, const float* __restrict__ y_lw,
+                           const float* __restrict__ y_uw, float* __restrict__ z_lw, float* __restrict__ z_uw, const DotBias q, int Di,
+                           int n_it, int n_jt) {
+  pdl_sync();
+  __shared__ float s_lx[4][kThinK], s_ly[4][kThinK], s_uy[4][kThinK];
+  const float* __restrict__ x_l = q.x_l;
+  const float* __restrict__ y_l = q.y_l;
+  const float* __restrict__ y_u = q.y_u;
+  const int Lx = q.Lx, Ly = q.Ly, K = q.K;
+  int64_t bid = blockIdx.x;
+  const int jt = (int)(bid % n_jt); bid /= n_jt;
+  const int it = (int)(bid % n_it); bid /= n_it;
+  const int64_t b = bid;
+  const int i0 = it * 4, j0 = jt * 4;
+  const int m = blockIdx.y * kThinM + threadIdx.x;
+  const bool m_ok = m < Di;
+  float acc_l[4][4], acc_u[4][4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) { acc_l[a][c] = 0.f; acc_u[a][c] = 0.f; }
+  for (int k0 = 0; k0 < K; k0 += kThinK) {
+    const int nk = min(kThinK, K - k0);
+    for (int f = threadIdx.x; f < 4 * kThinK; f += kThinM) {
+      const int r = f / kThinK, k = f % kThinK;
+      const bool kin = k < nk;
+      s_lx[r][k] = (kin && i0 + r < Lx) ? x_l[(b * Lx + i0 + r) * (int64_t)K + k0 + k] : 0.f;
+      s_ly[r][k] = (kin && j0 + r < Ly) ? y_l[(b * Ly + j0 + r) * (int64_t)K + k0 + k] : 0.f;
+      s_uy[r][k] = (kin && j0 + r < Ly) ? y_u[(b * Ly + j0 + r) * (int64_t)K + k0 + k] : 0.f;
+    }
+    __syncthreads();
+    if (m_ok) {
+      for (int k = 0; k < nk; ++k) {
+        float xl[4], xu[4], yl[4], yu[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          const bool ok = i0 + a < Lx;
+          const int64_t o = ((b * Lx + i0 + a) * (int64_t)K + k0 + k) * Di + m;
+          xl[a] = ok ? __ldg(x_lw + o) : 0.f;
+          xu[a] = ok ? __ldg(x_uw + o) : 0.f;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const bool ok = j0 + c < Ly;
+          const int64_t o = ((b * Ly + j0 + c) * (int64_t)K + k0 + k) * Di + m;
+          yl[c] = ok ? __ldg(y_lw + o) : 0.f;
+          yu[c] = ok ? __ldg(y_uw + o) : 0.f;
+        }
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          const float lx = s_lx[a][k];
+          const float lxp = fmaxf(lx, 0.f), lxn = fminf(lx, 0.f);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const float ly = s_ly[c][k], uy = s_uy[c][k];
+            float l = acc_l[a][c], u = acc_u[a][c];
+            l = fmaf(xl[a], fmaxf(ly, 0.f), l); l = fmaf(xu[a], fminf(ly, 0.f), l);
+            l = fmaf(yl[c], lxp, l);            l = fmaf(yu[c], lxn, l);
+            u = fmaf(xu[a], fmaxf(uy, 0.f), u); u = fmaf(xl[a], fminf(uy, 0.f), u);
+            u = fmaf(yu[c], lxp, u);            u = fmaf(yl[c], lxn, u);
+            acc_l[a][c] = l; acc_u[a][c] = u;
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if (!m_ok) return;
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if (i0 + a < Lx && j0 + c < Ly) {
+        const int64_t o = ((b * Lx + i0 + a) * (int64_t)Ly + j0 + c) * Di + m;
+        z_lw[o] = fmul(acc_l[a][c], q.out_scale);
+        z_uw[o] = fmul(acc_u[a][c], q.out_scale);
+      }
+}
+
+bool dot_transposed_thin(const DotBias& q, int B, int Di) {
+  const double per_sm = (double)B * ceil_div(q.Lx, 4) * ceil_div(q.Ly, 4) * ceil_div(Di, kDotTransposedM) / device_info().sms;
+  return std::min(q.Lx, q.Ly) <= 4 && (int64_t)q.K * std::min(Di, kDotTransposedM) <= 800 &&
+         (per_sm >= 3.0 + q.K / 16.0 || (q.Lx > 32 && per_sm >= 2.0));
+}
+
+int launch_dot_transposed_thin(const float* x_lw, const float* x_uw, const float* y_lw, const float* y_uw, float* z_lw, float* z_uw,
+                               const DotBias& q, int B, int Di, cudaStream_t st) {
+  if (int rc = launch_dot_bias(q, B, st)) return rc;
+  const int n_it = (int)ceil_div(q.Lx, 4), n_jt = (int)ceil_div(q.Ly, 4);
+  const int64_t blocks = (int64_t)B * n_it * n_jt, my = ceil_div(Di, kThinM);
+  if (blocks > 0x7fffffff || my > 65535) return FB_ERR_SHAPE;
+  fb::launch_k(dot_weight_transposed_thin, dim3((unsigned)blocks, (unsigned)my), kThinM, 0, st, x_lw, x_uw, y_lw, y_uw, z_lw, z_uw, q, Di, n_it,
+               n_jt);
+  FB_LAUNCH_OK();
+  return FB_OK;
+}
+
 template <int WI, int WJ, int WK, int VEC>
 int launch_dot_transposed_t(const float* x_lw, const float* x_uw, const float* y_lw, const float* y_uw, float* z_lw, float* z_uw,
                             const DotBias& q, int B, int Di, cudaStream_t st) {
@@ -222,6 +325,7 @@ int launch_dot_transposed_t(const float* x_lw, const float* x_uw, const float* y
 
 int launch_dot_transposed(const float* x_lw, const float* x_uw, const float* y_lw, const float* y_uw, float* z_lw, float* z_uw,
                           const DotBias& q, int B, int Di, cudaStream_t st) {
+  if (dot_transposed_thin(q, B, Di)) return launch_dot_transposed_thin(x_lw, x_uw, y_lw, y_uw, z_lw, z_uw, q, B, Di, st);
   const auto aligned8 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7) == 0; };
   const bool vec = Di % 4 == 0 && aligned16(x_lw) && aligned16(x_uw) && aligned16(y_lw) && aligned16(y_uw) && aligned8(z_lw) && aligned8(z_uw);
   // Rounds of one block per SM times the arithmetic of a block (in 4 x 4 tiles over all k), the smaller tiles charged for

@@ -1127,6 +1127,12 @@ def test_dot_product_transposed_edges(B, Lx, Ly, Di, K):
         helpers.assert_arbitrated(got, getattr(o, name), getattr(o64, name), "transposed dot %s %s" % (name, (B, Lx, Ly, Di, K)))
 
 
+# (few rows against any number in a large batch: a tile of one row and of four, k past the 128 values staged at a time, odd dim_in)
+@pytest.mark.parametrize("B,Lx,Ly,Di,K", [(300, 9, 4, 5, 7), (256, 1, 33, 66, 12), (160, 40, 1, 2, 150), (700, 3, 2, 129, 6)])
+def test_dot_product_transposed_of_many_thin_products(B, Lx, Ly, Di, K):
+    test_dot_product_transposed_edges(B, Lx, Ly, Di, K)
+
+
 @pytest.mark.parametrize("Di", [1, 4, 126, 128, 132, 256, 260, 512, 516])
 @pytest.mark.parametrize("p", [1.0, 2.0, float("inf")])
 def test_relax_transposed_columns_held_in_registers(Di, p):
