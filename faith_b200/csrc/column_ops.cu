@@ -662,7 +662,6 @@ __device__ __forceinline__ void transposed_concretize(const float* __restrict__ 
   l = lbv, u = ubv;
   for (int w = 0; w < words; ++w) {
     float al = 0.f, au = 0.f;
-#pragma unroll 2
     for (int r = w * blk + lane * VEC; r < (w + 1) * blk; r += 32 * VEC) {
       if (VEC == 4) {
         const float4 a = __ldg(reinterpret_cast<const float4*>(gl + r));

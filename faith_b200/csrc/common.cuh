@@ -217,7 +217,8 @@ __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b)
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdiv_rn(a, b); }
 
 // Every kernel launched through launch_k calls this before it reads or writes anything another launch may touch: it waits for
-// the launches before to complete, and lets the next one start its prologue.
+// the launches before to complete, and lets the next one start its prologue.  Unconditional: with a test of the grid's size
+// around it, kernels overlapped the launch before them and read what it had not written yet.
 __device__ __forceinline__ void pdl_sync() {
   asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
 }
