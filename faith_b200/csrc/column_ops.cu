@@ -884,11 +884,12 @@ int launch_relax(int op, const float* lw, const float* uw, const float* lb, cons
   // re-read through L2: tanh on [8, 64, 256, 256] 0.172 ms staged, 0.137 ms not, 0.48 -> 0.60 of the HBM roof.)
   const bool staged = op < OP_COEF_ONLY && staged_bytes <= 40 * 1024;
   const size_t smem = staged ? staged_bytes : relax_smem_bytes(Di, false, 2);
+  const int64_t tiles = op < OP_COEF_ONLY && !staged && 2 * blocks > 5 * device_info().sms ? kManyTiles : blocks;
 #define FB_RELAX_LAUNCH(V, S)                                                                              \
   do {                                                                                                     \
     int rc_ = ensure_smem(col_relax_native<V, S>, smem);                                                   \
     if (rc_ != FB_OK) return rc_;                                                                          \
-    fb::launch_k(col_relax_native<V, S>, (unsigned)blocks, kThreads, smem, st, op, lw, uw, lb, ub, o_lw, o_uw, o_lb, \
+    fb::launch_tiles(tiles, col_relax_native<V, S>, (unsigned)blocks, kThreads, smem, st, op, lw, uw, lb, ub, o_lw, o_uw, o_lb, \
                                                                      o_ub, Di, Do, ntiles, words, p, eps,  \
                                                                      tanh_op ? 1 : 0, violation);                           \
   } while (0)
@@ -985,11 +986,12 @@ extern "C" int fb_mul_bounds_f32(const float* x_lw, const float* x_uw, const flo
   const size_t staged_bytes = relax_smem_bytes(Di, true, 4);
   const bool staged = staged_bytes <= 100 * 1024;
   const size_t smem = staged ? staged_bytes : relax_smem_bytes(Di, false, 4);
+  const int64_t tiles = (int64_t)Di * (Do < kCW ? Do : kCW) >= 8192 && blocks > 2 * device_info().sms ? kManyTiles : blocks;
 #define FB_MUL_LAUNCH(V, S)                                                                                  \
   do {                                                                                                       \
     int rc_ = ensure_smem(col_mul_bounds_native<V, S>, smem);                                                \
     if (rc_ != FB_OK) return rc_;                                                                            \
-    fb::launch_k(col_mul_bounds_native<V, S>, (unsigned)blocks, kThreads, smem, st, x_lw, x_uw, x_lb, x_ub, y_lw, y_uw, \
+    fb::launch_tiles(tiles, col_mul_bounds_native<V, S>, (unsigned)blocks, kThreads, smem, st, x_lw, x_uw, x_lb, x_ub, y_lw, y_uw, \
                                                                           y_lb, y_ub, z_lw, z_uw, z_lb, z_ub, \
                                                                           Di, Do, ntiles, words, p, eps);     \
   } while (0)

@@ -41,7 +41,11 @@ void count_launches(int n);
 // the passes over one sentence are chains of kernels of 3 to 10 us with 2 us between them, most of it launch latency and
 // prologues (barriers, tensor memory, tensor maps).  The kernel must call pdl_sync() first thing.  Work of many waves keeps the
 // plain launch: the gap before it is nothing beside it, and the hand-over cost the 4096 blocks of a relaxation 2 % of 135 us.
-// tiles: what a persistent kernel walks, the number of blocks for any other.
+// tiles: what a persistent kernel walks, the number of blocks for any other; kManyTiles where the blocks run long and there are more
+// of them than two an SM: those that come early fill the gaps as these appear, two more on one SM than on another, and that costs
+// more than the launch.  us plain and programmatic: product of two bounds, 420 blocks of 320 rows 22.8 and 32.4; relu, 440 blocks of
+// 384 rows re-read from L2 3.3 more, tanh 4.2 more; 16 columns of K = 400, 580 blocks 9.7 more.
+constexpr int64_t kManyTiles = INT64_MAX;
 template <typename... P, typename... A>
 inline void launch_tiles(int64_t tiles, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
   cudaLaunchAttribute attr;

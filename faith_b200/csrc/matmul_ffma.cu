@@ -458,7 +458,8 @@ int launch_split_sign_ffma(const float* a_lo, const float* a_up, const float* W,
     const int64_t want = ceil_div(M, kThreads / 32);
     const int64_t cap = (int64_t)device_info().sms * 16;
     const unsigned blocks = (unsigned)(want < cap ? want : cap);
-    fb::launch_k(split_sign_gemv_rows<16>, blocks, kThreads, 0, st, a_lo, a_up, W, bias, c_lo, c_up, M, N, K);
+    const int64_t tiles = N > 8 && blocks > 3 * device_info().sms ? kManyTiles : blocks;   // (three blocks an SM)
+    fb::launch_tiles(tiles, split_sign_gemv_rows<16>, blocks, kThreads, 0, st, a_lo, a_up, W, bias, c_lo, c_up, M, N, K);
     FB_LAUNCH_OK();
     return FB_OK;
   }
