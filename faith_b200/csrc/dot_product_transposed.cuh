@@ -328,11 +328,12 @@ int launch_dot_transposed(const float* x_lw, const float* x_uw, const float* y_l
   if (dot_transposed_thin(q, B, Di)) return launch_dot_transposed_thin(x_lw, x_uw, y_lw, y_uw, z_lw, z_uw, q, B, Di, st);
   const auto aligned8 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7) == 0; };
   const bool vec = Di % 4 == 0 && aligned16(x_lw) && aligned16(x_uw) && aligned16(y_lw) && aligned16(y_uw) && aligned8(z_lw) && aligned8(z_uw);
-  // Rounds of one block per SM times the arithmetic of a block (in 4 x 4 tiles over all k), the smaller tiles charged for
-  // reading every operand row twice and four times as often from L2.
+  // Rounds of one block per SM times what a block takes: its arithmetic (in 4 x 4 tiles), the smaller tiles charged for reading
+  // every operand row twice and four times as often from L2, and, in the same unit (90 ns), its start and the sums of its shares.
+  // Without the latter short sums went to the smallest tiles: 353 products of 12 x 10, K = 8, dim_in 32 112 us, 57 us with it.
   const int64_t sms = device_info().sms, bm = (int64_t)B * ceil_div(Di, kDotTransposedM);
   auto rounds = [&](int t) { return ceil_div(bm * ceil_div(q.Lx, t) * ceil_div(q.Ly, t), sms); };
-  const int64_t c16 = 16 * rounds(16), c8 = 5 * rounds(8), c4 = 2 * rounds(4);
+  const int64_t K = q.K, c16 = (16 * K + 70) * rounds(16), c8 = (5 * K + 40) * rounds(8), c4 = (2 * K + 26) * rounds(4);
 #define FB_DOT_T(...) (vec ? launch_dot_transposed_t<__VA_ARGS__, 4>(x_lw, x_uw, y_lw, y_uw, z_lw, z_uw, q, B, Di, st) \
                            : launch_dot_transposed_t<__VA_ARGS__, 1>(x_lw, x_uw, y_lw, y_uw, z_lw, z_uw, q, B, Di, st))
   if (c16 <= c8 && c16 <= c4) return FB_DOT_T(4, 4, 1);
