@@ -18,7 +18,7 @@ int launch_split_sign_tc(const float* a_lo, const float* a_up, const float* W, c
 bool tc_bias_rows_mergeable(const float* a_lo, const float* a_up, const float* b_lo, const float* b_up, const float* W,
                             const float* cb_lo, const float* cb_up, int64_t Mb, int N, int K, bool with_norms);
 int launch_split_sign_ffma(const float* a_lo, const float* a_up, const float* W, const float* bias, float* c_lo,
-                           float* c_up, int64_t M, int N, int K, cudaStream_t st, int split_rows, int split_d);
+                           float* c_up, int64_t M, int N, int K, cudaStream_t st, int split_rows, int split_d, int64_t rows_before);
 
 // FB_MATMUL_IMPL=ffma forces the CUDA-core kernel (exact fp32 products); default: tensor cores
 // (3xTF32) for the large weight GEMM when the shape allows it.
@@ -33,11 +33,12 @@ static bool use_tensor_cores() {
 // split_rows > 0: head-split store of the result, [group * H + head][row in group][feature in head]
 // with groups of split_rows consecutive rows and heads of split_d consecutive columns.
 static int split_sign_gemm(const float* a_lo, const float* a_up, const float* W, const float* bias, float* c_lo,
-                           float* c_up, int64_t M, int N, int K, cudaStream_t st, int split_rows = 0, int split_d = 0) {
+                           float* c_up, int64_t M, int N, int K, cudaStream_t st, int split_rows = 0, int split_d = 0,
+                           int64_t rows_before = 0) {
   if (use_tensor_cores() && tc_gemm_supported(a_lo, a_up, W, c_lo, c_up, M, N, K) &&
       (split_rows == 0 || tc_split_supported(M, N, split_rows, split_d)))
     return launch_split_sign_tc(a_lo, a_up, W, bias, c_lo, c_up, M, N, K, st, split_rows, split_d);
-  return launch_split_sign_ffma(a_lo, a_up, W, bias, c_lo, c_up, M, N, K, st, split_rows, split_d);
+  return launch_split_sign_ffma(a_lo, a_up, W, bias, c_lo, c_up, M, N, K, st, split_rows, split_d, rows_before);
 }
 
 // Ranges of a (head-split) product from the per-word-block column norms that the GEMM epilogue wrote:
@@ -150,7 +151,7 @@ static int matmul_impl(const float* x_lw, const float* x_uw, const float* x_lb, 
   }
   if (rc != FB_OK || bias_done) return rc;
   // bias rows: [rows, Do] -> [rows, Dy], + bias
-  return fb::split_sign_gemm(x_lb, x_ub, W, bias, y_lb, y_ub, rows, Dy, Do, st, heads > 1 ? L : 0, d);
+  return fb::split_sign_gemm(x_lb, x_ub, W, bias, y_lb, y_ub, rows, Dy, Do, st, heads > 1 ? L : 0, d, Mw);
 }
 
 extern "C" int fb_matmul_f32(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub,

@@ -13,6 +13,8 @@
 // into registers before the current step is computed (two shared-memory stages).
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "matmul_small.cuh"
 
@@ -426,9 +428,10 @@ int launch_split_sign_small(const float* a_lo, const float* a_up, const float* W
   return FB_OK;
 }
 
-// One split-sign GEMM: (a_lo, a_up) [M, K] x W[N, K]^T (+ bias) -> (c_lo, c_up) [M, N].
+// One split-sign GEMM: (a_lo, a_up) [M, K] x W[N, K]^T (+ bias) -> (c_lo, c_up) [M, N].  rows_before: rows of the same product in the
+// launch before this one.
 int launch_split_sign_ffma(const float* a_lo, const float* a_up, const float* W, const float* bias, float* c_lo,
-                           float* c_up, int64_t M, int N, int K, cudaStream_t st, int split_rows, int split_d) {
+                           float* c_up, int64_t M, int N, int K, cudaStream_t st, int split_rows, int split_d, int64_t rows_before) {
   if (M == 0 || N == 0) return FB_OK;
   if (N <= 16 && split_rows == 0 && K >= 2048 && M <= 32) {
     cudaLaunchConfig_t cfg = {};
@@ -458,7 +461,10 @@ int launch_split_sign_ffma(const float* a_lo, const float* a_up, const float* W,
     const int64_t want = ceil_div(M, kThreads / 32);
     const int64_t cap = (int64_t)device_info().sms * 16;
     const unsigned blocks = (unsigned)(want < cap ? want : cap);
-    const int64_t tiles = N > 8 && blocks > 3 * device_info().sms ? kManyTiles : blocks;   // (three blocks an SM)
+    // (Long blocks in number, here or in the launch before: the few bias rows would come early and crowd onto the SMs that the weight
+    // rows leave first.  Weight and bias rows of 4800 x 480 -> 16: 65 us plain, 78 us programmatic; 16 x 250 -> 7: 24.7 and 19.8 us.)
+    const int64_t tiles = (int64_t)N * K >= 1024 && std::max<int64_t>(blocks, ceil_div(rows_before, kThreads / 32)) > 2 * device_info().sms
+                              ? kManyTiles : blocks;
     fb::launch_tiles(tiles, split_sign_gemv_rows<16>, blocks, kThreads, 0, st, a_lo, a_up, W, bias, c_lo, c_up, M, N, K);
     FB_LAUNCH_OK();
     return FB_OK;
