@@ -22,7 +22,7 @@ namespace {
 // (whole rows of narrow maps, several images of small ones): a fixed 16 x 16 or 8 x 32 tile spent up to two thirds of its
 // threads on padding.  Every output accumulates over (input channel, tap row, tap column) in that order, whatever the tile.
 // 384 images, 16 -> 32 channels, 32 x 32, 3 x 3, stride 2: 100 us with one pixel x 32 channels per thread and scalar
-// multiply-adds (and 21 us more for the bias image in a launch of its own), 83 us now; 25 us are arithmetic, the staging alone
+// multiply-adds (and 21 us more for the bias image in a launch of its own), 86 us now; 25 us are arithmetic, the staging alone
 // takes 35 us and overlaps with it only across the four blocks of an SM, and the last of 1.3 rounds of blocks is thin.
 struct ConvArgs {
   const float *x_lo, *x_up, *b_lo, *b_up;   // n_img images without the bias, then n_bias with it
