@@ -21,7 +21,10 @@
 // error class of an fp32 multiplication.  The tensor core truncates when it adds to an accumulator, so few instructions may
 // add to one of full magnitude: X and Y have two accumulators each, added with round-to-nearest in the epilogue.  One
 // chunk of k: centre and radius, the small products first.  More chunks (kMulti): hh and the small products.  Error
-// against fp64 over the fp32 noise of the reference: 1.5 at K = 32 (CUDA cores 1.4), below the CUDA cores' at K = 512.
+// against fp64 over the fp32 noise of the reference: 1.3 to 1.7 at K = 32 (CUDA cores 1.4 to 1.5), below the CUDA cores' at
+// K = 512; 1.5 to 2.3 for short sums, K = 7 and 16 (CUDA cores 1.2 to 1.4).  As in every centre/radius product the error of
+// either side is relative to the larger of |lw| and |uw|, where the CUDA cores' is relative to the side itself: it tells for
+// weights whose gap is thousands of times their value, and such a bound says nothing any more.
 //
 // What bounds it: about 2.8 us per tile whatever the data, i.e. the SM's shared memory (raw tiles in and out, B operands,
 // transposition, result: 3000 cycles of its 128 bytes per cycle) and the hand-overs between the roles; with full tiles of 32
