@@ -104,6 +104,29 @@ struct TcLnArgs {
   int64_t rs_stride;
 };
 
+// A large product for the fp16-split kernels (matmul_tc_f16.cuh), as launch_split_sign_tc has checked it: operands [M, K], W [N, K],
+// results [M, N] (head-split where split_rows > 0), slopes, norms, residual and bias rows as there, null where absent.
+struct F16Product {
+  const float *a_lo, *a_up, *W, *bias;
+  float *c_lo, *c_up;
+  int64_t M;
+  int N, K, split_rows, split_d;
+  const float *coef_l, *coef_u;
+  int coef_di;
+  float *norm_lo, *norm_up;
+  int norm_p;
+  const float *res_lo, *res_up;
+  const TcBiasRows* br;
+  int* status;
+  uint32_t wait_tries;
+  int skip_it;
+  LiveRows live;
+};
+int launch_split_sign_f16(const F16Product& q, cudaStream_t st);          // K <= 128
+int launch_split_sign_f16_stream(const F16Product& q, cudaStream_t st);   // K > 128
+int f16_error_flag(int* flag);
+int f16_stream_error_flag(int* flag);
+
 // fb_layernorm_novar_f32 that can also leave the row sums of its result behind (rowsum, may be null; 128 features
 // only): [2 lines][4 partial sums][rows * (Di + 1)], of which it writes the first partial sum of each line.
 int layernorm_novar_rowsum(const float* x_lw, const float* x_uw, const float* x_lb, const float* x_ub, const float* r_lw,

@@ -14,7 +14,7 @@ int launch_split_sign_tc(const float* a_lo, const float* a_up, const float* W, c
                          const float* coef_l = nullptr, const float* coef_u = nullptr, int coef_di = 1,
                          float* norm_lo = nullptr, float* norm_up = nullptr, int norm_p = 0,
                          const float* res_lo = nullptr, const float* res_up = nullptr, const TcBiasRows* br = nullptr,
-                         const TcLnArgs* ln = nullptr, const SmallProduct* few = nullptr, bool* few_done = nullptr);
+                         const TcLnArgs* ln = nullptr, const SmallProduct* few = nullptr, bool* few_done = nullptr, int64_t like_M = 0);
 bool tc_bias_rows_mergeable(const float* a_lo, const float* a_up, const float* b_lo, const float* b_up, const float* W,
                             const float* cb_lo, const float* cb_up, int64_t Mb, int N, int K, bool with_norms);
 int launch_split_sign_ffma(const float* a_lo, const float* a_up, const float* W, const float* bias, float* c_lo,
@@ -37,7 +37,8 @@ static int split_sign_gemm(const float* a_lo, const float* a_up, const float* W,
                            int64_t rows_before = 0) {
   if (use_tensor_cores() && tc_gemm_supported(a_lo, a_up, W, c_lo, c_up, M, N, K) &&
       (split_rows == 0 || tc_split_supported(M, N, split_rows, split_d)))
-    return launch_split_sign_tc(a_lo, a_up, W, bias, c_lo, c_up, M, N, K, st, split_rows, split_d);
+    return launch_split_sign_tc(a_lo, a_up, W, bias, c_lo, c_up, M, N, K, st, split_rows, split_d, nullptr, nullptr, 1, nullptr, nullptr, 0,
+                                nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, rows_before);
   return launch_split_sign_ffma(a_lo, a_up, W, bias, c_lo, c_up, M, N, K, st, split_rows, split_d, rows_before);
 }
 
@@ -194,7 +195,7 @@ extern "C" int fb_matmul_coef_f32(const float* x_lw, const float* x_uw, const fl
   int rc = fb::launch_split_sign_tc(x_lw, x_uw, W, nullptr, y_lw, y_uw, M, Dy, Do, st, 0, 0, c_l, c_u, Di, nullptr, nullptr, 0,
                                     nullptr, nullptr, merged ? &br : nullptr, nullptr, takes ? &few : nullptr, &few_done);
   if (rc != FB_OK || merged || few_done) return rc;
-  return fb::split_sign_gemm(x_lb, x_ub, W, bias, y_lb, y_ub, rows, Dy, Do, st);
+  return fb::split_sign_gemm(x_lb, x_ub, W, bias, y_lb, y_ub, rows, Dy, Do, st, 0, 0, M);
 }
 
 // fb_matmul_heads_f32 that also returns the concretised range of its result, y_l / y_u in the layout of
@@ -249,7 +250,8 @@ int fb::matmul_ranges_ex(const float* x_lw, const float* x_uw, const float* x_lb
   } else if (heads > 1 && fb::tc_gemm_supported(x_lb, x_ub, W, norm_ws, norm_ws, rows, Dy, Do)) {
     plain_lb = b_lo;
     plain_ub = b_up;
-    rc = fb::launch_split_sign_tc(x_lb, x_ub, W, bias, plain_lb, plain_ub, rows, Dy, Do, st, 0, 0);
+    rc = fb::launch_split_sign_tc(x_lb, x_ub, W, bias, plain_lb, plain_ub, rows, Dy, Do, st, 0, 0, nullptr, nullptr, 1, nullptr, nullptr, 0,
+                                  nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, M);
   } else if (!fb::tc_gemm_supported(x_lb, x_ub, W, y_lb, y_ub, rows, Dy, Do) && fb::small_product(rows, Dy, Do)) {
     fb::RangeEpilogue rg = {norm_lo, norm_up, y_l, y_u, words, eps, 0, -1, nullptr, nullptr, nullptr, nullptr, nullptr};
     bool split = heads > 1;
@@ -262,7 +264,7 @@ int fb::matmul_ranges_ex(const float* x_lw, const float* x_uw, const float* x_lb
     }
     return fb::launch_split_sign_small(x_lb, x_ub, W, bias, y_lb, y_ub, rows, Dy, Do, st, split ? L : 0, split ? d : 0, &rg);
   } else {
-    rc = fb::split_sign_gemm(x_lb, x_ub, W, bias, y_lb, y_ub, rows, Dy, Do, st, heads > 1 ? L : 0, heads > 1 ? d : 0);
+    rc = fb::split_sign_gemm(x_lb, x_ub, W, bias, y_lb, y_ub, rows, Dy, Do, st, heads > 1 ? L : 0, heads > 1 ? d : 0, M);
   }
   if (rc != FB_OK) return rc;
   const int64_t total = rows * Dy;
@@ -314,7 +316,7 @@ extern "C" int fb_matmul_residual_f32(const float* x_lw, const float* x_uw, cons
                                     r_lw, r_uw, merged ? &br : nullptr);
   if (rc != FB_OK || merged) return rc;
   return fb::launch_split_sign_tc(x_lb, x_ub, W, bias, y_lb, y_ub, rows, Dy, Do, st, 0, 0, nullptr, nullptr, 1, nullptr,
-                                  nullptr, 0, r_lb, r_ub);
+                                  nullptr, 0, r_lb, r_ub, nullptr, nullptr, nullptr, nullptr, M);
 }
 
 // fb_matmul_residual_f32 followed by the layer norm of the encoder blocks (mode no_var, Bounds.layer_norm,

@@ -926,11 +926,24 @@ bool tc_gemm_supported(const float* a_lo, const float* a_up, const float* W, con
          aligned16(a_up) && aligned16(W) && aligned16(c_lo) && aligned16(c_up) && encode_fn() != nullptr;
 }
 
+// Whether a product goes to the fp16-split kernels (matmul_tc_f16.cuh): more than 64 columns (their tile has 128 and costs the same for
+// 64: 128 -> 64 took 1.2 times as long), and work enough for their longer prologue.  K <= 128: two rounds of tiles; us before and with
+// them, 128 -> 128 at 200 / 300 / 1500 row tiles 31 and 31, 35 and 29, 112 and 83; 128 -> 512 61 and 51, 77 and 61, 329 and 223.
+// K >= 320: 512 -> 128 at 300 / 600 / 1000 / 4096 row tiles 81 and 88, 135 and 136, 205 and 186, 810 and 725, with slopes and residual
+// at 1000 / 4096 256 and 224, 1080 and 871; 320 -> 128 at 1000 / 1920 160 and 159, 291 and 272.  Between 128 and 320 the start and
+// the end of every 64 rows weigh too much (256 -> 256 at 1024 row tiles 244 and 268).
+bool f16_applies(int64_t M, int N, int K) {
+  const int64_t tiles = ceil_div(M, 128) * ceil_div(N, 128);
+  if (N <= 64) return false;
+  return K <= 128 ? tiles >= 296 : K >= 320 && tiles * K >= 900 * 512;
+}
+
+// like_M: the number of weight rows where these are their bias rows, so that both take the same kernel.
 int launch_split_sign_tc(const float* a_lo, const float* a_up, const float* W, const float* bias, float* c_lo,
                          float* c_up, int64_t M, int N, int K, cudaStream_t st, int split_rows, int split_d,
                          const float* coef_l, const float* coef_u, int coef_di, float* norm_lo, float* norm_up,
                          int norm_p, const float* res_lo, const float* res_up, const TcBiasRows* br, const TcLnArgs* ln,
-                         const SmallProduct* few, bool* few_done) {
+                         const SmallProduct* few, bool* few_done, int64_t like_M) {
   // Bias rows in the same grid (br != nullptr): they must take the same instantiation as the weight rows (zero
   // radius or not, residual or not); the caller checks tc_bias_rows_mergeable first.
   if (br != nullptr && ((br->res_lo != nullptr) != (res_lo != nullptr) || (br->res_lo != nullptr) != (br->res_up != nullptr) ||
@@ -943,6 +956,17 @@ int launch_split_sign_tc(const float* a_lo, const float* a_up, const float* W, c
   if (norm_lo != nullptr && (coef_l != nullptr || norm_up == nullptr || M % BM != 0)) return FB_ERR_ARG;
   if (res_lo != nullptr && (res_up == nullptr || norm_lo != nullptr || split_rows > 0 || !aligned16(res_lo) || !aligned16(res_up)))
     return FB_ERR_ARG;
+  // zero row blocks: only for the zero-radius products of the operand the hint was set for (weight rows, no bias)
+  const LiveRows no_live = {0, 0, 0, {0, 0, 0, 0}, nullptr, 0};
+  LiveRows live = no_live;
+  if (t_live_rows.L > 0 && t_live_rows.M == M && bias == nullptr && t_live_rows.Di > 0 && t_live_rows.Di % BM == 0 &&
+      t_live_rows.words >= 1 && t_live_rows.words <= 4 && M % ((int64_t)t_live_rows.Di * t_live_rows.L) == 0)
+    live = t_live_rows;
+  if (ln == nullptr && f16_applies(like_M > 0 ? like_M : M, N, K)) {
+    const F16Product q = {a_lo, a_up, W, bias, c_lo, c_up, M, N, K, split_rows, split_d, coef_l, coef_u, coef_di, norm_lo, norm_up, norm_p,
+                          res_lo, res_up, br, t_status_sink, g_wait_tries, g_skip_it, live};
+    return K <= 128 ? launch_split_sign_f16(q, st) : launch_split_sign_f16_stream(q, st);
+  }
   CUtensorMap tm_lo, tm_up, tm_w, tm_out_lo, tm_out_up, tm_res_lo, tm_res_up;
   if (!make_map(&tm_lo, a_lo, (uint64_t)M, (uint64_t)K, BM) || !make_map(&tm_up, a_up, (uint64_t)M, (uint64_t)K, BM) ||
       !make_map(&tm_w, W, (uint64_t)N, (uint64_t)K, BN) ||
@@ -1024,12 +1048,6 @@ int launch_split_sign_tc(const float* a_lo, const float* a_up, const float* W, c
   int* status = t_status_sink;
   const uint32_t tries = g_wait_tries;
   const int skip = g_skip_it;
-  // zero row blocks: only for the zero-radius products of the operand the hint was set for (weight rows, no bias)
-  LiveRows no_live = {0, 0, 0, {0, 0, 0, 0}, nullptr, 0};
-  LiveRows live = no_live;
-  if (t_live_rows.L > 0 && t_live_rows.M == M && bias == nullptr && t_live_rows.Di > 0 && t_live_rows.Di % BM == 0 &&
-      t_live_rows.words >= 1 && t_live_rows.words <= 4 && M % ((int64_t)t_live_rows.Di * t_live_rows.L) == 0)
-    live = t_live_rows;
   TcLnArgs ln_args = {nullptr, nullptr, nullptr, nullptr, nullptr, 0};
   if (ln != nullptr) {
     ln_args = *ln;
@@ -1086,7 +1104,12 @@ extern "C" int fb_tc_error_flag(int* flag) {
   int v3 = 0;
   const int rc3 = fb::dot_tc_any_error_flag(&v3);
   if (rc3 != FB_OK) return rc3;
-  *flag = (v != 0 || v2 != 0 || v3 != 0) ? 1 : 0;
+  int v4 = 0, v5 = 0;   // as do the fp16-split products
+  const int rc4 = fb::f16_error_flag(&v4);
+  if (rc4 != FB_OK) return rc4;
+  const int rc5 = fb::f16_stream_error_flag(&v5);
+  if (rc5 != FB_OK) return rc5;
+  *flag = (v != 0 || v2 != 0 || v3 != 0 || v4 != 0 || v5 != 0) ? 1 : 0;
   return FB_OK;
 }
 
@@ -1193,7 +1216,7 @@ extern "C" int fb_tc_selftest_timeout(const float* x_lw, const float* x_uw, cons
   int* const saved_sink = fb::t_status_sink;
   fb::t_status_sink = status;
   rc = fb::launch_split_sign_tc(x_lw, x_uw, W, nullptr, y_lw, y_uw, M, N, K, (cudaStream_t)stream, 0, 0, nullptr, nullptr, 1,
-                                nullptr, nullptr, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
+                                nullptr, nullptr, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0);
   fb::t_status_sink = saved_sink;
   fb::g_wait_tries = fb::kMaxTries;
   fb::g_skip_it = -1;

@@ -1,0 +1,28 @@
+// Instantiations of the fp16-split product of matmul_tc_f16.cuh, K <= 128: the parts of W stay in shared memory.
+#include <cuda.h>
+
+#include <mutex>
+#include <type_traits>
+#include <unordered_map>
+
+#include "common.cuh"
+
+namespace fb {
+namespace {
+#include "tc_common.cuh"
+#include "matmul_tc_f16.cuh"
+}  // namespace
+
+int launch_split_sign_f16(const F16Product& q, cudaStream_t st) { return hg::launch<false>(q, st); }
+
+int f16_error_flag(int* flag) {
+  int v = 0;
+  FB_CUDA_OK(cudaMemcpyFromSymbol(&v, g_tc_error, sizeof(int)));
+  if (v != 0) {
+    const int zero = 0;
+    FB_CUDA_OK(cudaMemcpyToSymbol(g_tc_error, &zero, sizeof(int)));
+  }
+  *flag = v;
+  return FB_OK;
+}
+}  // namespace fb
