@@ -13,10 +13,12 @@
 //
 // Launches: one that concretises both operands, then one kernel for the bias part and one for the weight part (a single one
 // for both in the transposed layout).
-#include <mutex>
+#include <cuda.h>
 
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
+#include <unordered_map>
 
 #include "common.cuh"
 #include "dot_bias.cuh"
@@ -132,7 +134,7 @@ dot_weight_native(const float* __restrict__ x_lw, const float* __restrict__ x_uw
                   const float* __restrict__ y_u, float* __restrict__ z_lw, float* __restrict__ z_uw,
                   int Lx, int Ly, int Di, int K, int n_it, int n_jt, int n_mt, float out_scale) {
   pdl_sync();
-  extern __shared__ __align__(16) float smem[];
+  extern __shared__ __align__(128) float smem[];
   float* s_xl = smem;
   float* s_xu = s_xl + XT;
   float* s_yl = s_xu + XT;
@@ -306,9 +308,24 @@ int launch_dot_bias(DotBias q, int B, cudaStream_t st) {
   return FB_OK;
 }
 
+namespace tma {   // (a namespace of its own: the packing helpers there take words, those of this file take floats)
+#include "tc_common.cuh"
+}
 #include "dot_product_transposed.cuh"
 
 }  // namespace
+
+// Reads (and clears) this file's copy of the flag raised by an expired bounded wait.
+int dot_transposed_error_flag(int* flag) {
+  int v = 0;
+  FB_CUDA_OK(cudaMemcpyFromSymbol(&v, tma::g_tc_error, sizeof(int)));
+  if (v != 0) {
+    const int zero = 0;
+    FB_CUDA_OK(cudaMemcpyToSymbol(tma::g_tc_error, &zero, sizeof(int)));
+  }
+  *flag = v;
+  return FB_OK;
+}
 }  // namespace fb
 
 namespace fb {

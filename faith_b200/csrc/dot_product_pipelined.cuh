@@ -67,7 +67,7 @@ dot_weight_native_pipelined(const float* __restrict__ x_lw, const float* __restr
                             int Lx, int Ly, int Di, int K, int n_it, int n_jt, int n_mt, int n_kc, int64_t n_items,
                             float out_scale, int heads) {
   pdl_sync();
-  extern __shared__ __align__(16) float smem[];
+  extern __shared__ __align__(128) float smem[];
   const int tid = threadIdx.x;
   const int tj = tid & 7, ti = (tid >> 3) & 7, tm = tid >> 6;
 

@@ -1087,6 +1087,7 @@ int launch_split_sign_tc(const float* a_lo, const float* a_up, const float* W, c
 namespace fb {
 int dot_tc_error_flag(int* flag);
 int dot_tc_any_error_flag(int* flag);
+int dot_transposed_error_flag(int* flag);
 }  // namespace fb
 
 extern "C" int fb_tc_error_flag(int* flag) {
@@ -1104,12 +1105,14 @@ extern "C" int fb_tc_error_flag(int* flag) {
   int v3 = 0;
   const int rc3 = fb::dot_tc_any_error_flag(&v3);
   if (rc3 != FB_OK) return rc3;
-  int v4 = 0, v5 = 0;   // as do the fp16-split products
+  int v4 = 0, v5 = 0, v6 = 0;   // as do the fp16-split products
   const int rc4 = fb::f16_error_flag(&v4);
   if (rc4 != FB_OK) return rc4;
   const int rc5 = fb::f16_stream_error_flag(&v5);
   if (rc5 != FB_OK) return rc5;
-  *flag = (v != 0 || v2 != 0 || v3 != 0 || v4 != 0 || v5 != 0) ? 1 : 0;
+  const int rc6 = fb::dot_transposed_error_flag(&v6);
+  if (rc6 != FB_OK) return rc6;
+  *flag = (v != 0 || v2 != 0 || v3 != 0 || v4 != 0 || v5 != 0 || v6 != 0) ? 1 : 0;
   return FB_OK;
 }
 

@@ -310,8 +310,9 @@ struct MapKey {
   const void* ptr;
   uint64_t dim[5], stride[4];   // extents innermost first; byte strides of dimensions 1 .. rank-1
   uint32_t box[5], rank;
+  bool plain;                   // no swizzle
   bool operator==(const MapKey& o) const {
-    if (ptr != o.ptr || rank != o.rank) return false;
+    if (ptr != o.ptr || rank != o.rank || plain != o.plain) return false;
     for (uint32_t i = 0; i < 5; ++i)
       if (dim[i] != o.dim[i] || box[i] != o.box[i] || (i < 4 && stride[i] != o.stride[i])) return false;
     return true;
@@ -327,7 +328,7 @@ struct MapKeyHash {
 std::mutex g_map_mu;
 std::unordered_map<MapKey, CUtensorMap, MapKeyHash> g_maps;
 
-// fp32 tensor of `rank` dimensions, 128-byte swizzle, zero fill.  dim and box as in MapKey, 1 beyond the rank; stride 0
+// fp32 tensor of `rank` dimensions, 128-byte swizzle unless `plain`, zero fill.  dim and box as in MapKey, 1 beyond the rank; stride 0
 // beyond it.
 bool get_map(CUtensorMap* out, const MapKey& key) {
   {
@@ -346,7 +347,7 @@ bool get_map(CUtensorMap* out, const MapKey& key) {
     if (i < 4) strides[i] = key.stride[i];
   }
   if (fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, key.rank, const_cast<void*>(key.ptr), dims, strides, box, estr,
-         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+         CU_TENSOR_MAP_INTERLEAVE_NONE, key.plain ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return false;
   std::lock_guard<std::mutex> lk(g_map_mu);

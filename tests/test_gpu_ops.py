@@ -1127,6 +1127,14 @@ def test_dot_product_transposed_edges(B, Lx, Ly, Di, K):
         helpers.assert_arbitrated(got, getattr(o, name), getattr(o64, name), "transposed dot %s %s" % (name, (B, Lx, Ly, Di, K)))
 
 
+# (TMA-addressable rows: each block shape with 64, 32 and 16 coordinates to a warp, ragged in every direction, K past the ring and past
+# the values of the ranges staged at a time or shorter than one stage)
+@pytest.mark.parametrize("B,Lx,Ly,Di,K", [(4, 63, 62, 124, 66), (5, 33, 49, 68, 5), (3, 63, 62, 252, 40), (5, 65, 9, 68, 70), (5, 5, 49, 196, 70),
+                                          (4, 23, 21, 100, 30), (5, 17, 49, 4, 150), (3, 9, 9, 196, 70), (3, 5, 49, 20, 70), (1, 5, 6, 4, 270)])
+def test_dot_product_transposed_lane_shares(B, Lx, Ly, Di, K):
+    test_dot_product_transposed_edges(B, Lx, Ly, Di, K)
+
+
 # (few rows against any number in a large batch: a tile of one row and of four, k past the 128 values staged at a time, odd dim_in)
 @pytest.mark.parametrize("B,Lx,Ly,Di,K", [(300, 9, 4, 5, 7), (256, 1, 33, 66, 12), (160, 40, 1, 2, 150), (700, 3, 2, 129, 6)])
 def test_dot_product_transposed_of_many_thin_products(B, Lx, Ly, Di, K):
