@@ -105,7 +105,6 @@ dot_weight_tc(const __grid_constant__ CUtensorMap tm_xl, const __grid_constant__
   const uint32_t bar_ops_ready = bar0 + 32;    // operands of the tile converted
   const uint32_t bar_mma_done = bar0 + 40;     // all MMAs of the tile complete (operands free, accumulators ready)
   const uint32_t bar_acc_free = bar0 + 48;     // accumulators read out
-  const uint32_t bar_epi = bar0 + 56;          // rendezvous of the epilogue warps
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(base_ptr + kDtOffBars + 64);
   volatile int* cta_abort = reinterpret_cast<volatile int*>(base_ptr + kDtOffBars + 72);
 
@@ -120,7 +119,6 @@ dot_weight_tc(const __grid_constant__ CUtensorMap tm_xl, const __grid_constant__
     mbar_init(bar_ops_ready, kDtConvWarps);
     mbar_init(bar_mma_done, kDtIssuers);
     mbar_init(bar_acc_free, kDtEpiWarps);
-    mbar_init(bar_epi, kDtEpiWarps);
     *cta_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -216,23 +214,15 @@ dot_weight_tc(const __grid_constant__ CUtensorMap tm_xl, const __grid_constant__
     const bool leader = threadIdx.x == 32 * kDtFirstEpiWarp;
     float* T = reinterpret_cast<float*>(base_ptr + kDtOffT);   // [2][128][kDtTStride]
     bool ok = true;
-    uint32_t epi_phase = 0;
-    auto epi_sync = [&]() -> bool {
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_epi);
-      const bool r = mbar_wait_warp(bar_epi, epi_phase & 1u, cta_abort);
-      ++epi_phase;
-      return r;
-    };
+    auto epi_sync = [&](bool fine) { return meet_all<1, 32 * kDtEpiWarps>(fine); };
     for (int t = 0; t < my_tiles && ok; ++t) {
       ok = mbar_wait_warp(bar_mma_done, (uint32_t)(t & 1), cta_abort);
-      if (!ok) break;
-      tc_fence_after();
       int b, i0, m0;
       tile_coords(t, b, i0, m0);
       if (leader) tma_store_wait_read();      // the previous tile's stores have read the staging buffer
-      ok = epi_sync();
+      ok = epi_sync(ok);
       if (!ok) break;
+      tc_fence_after();
       // ---- P -/+ Q of row (j, m), columns i  ->  T[side][(i, m)][j]
       {
         const int j = row >> 2, m = row & 3;
@@ -254,8 +244,7 @@ dot_weight_tc(const __grid_constant__ CUtensorMap tm_xl, const __grid_constant__
           }
         }
       }
-      ok = epi_sync();
-      if (!ok) break;
+      epi_sync(true);
       // ---- X_c -/+ X_r of row (i, m), columns j, plus the transposed term; lower side, then upper side.
       // The store staging of a side takes the place of that side's transposition buffer, so it is
       // written only after every thread has read its row of the buffer.
@@ -289,17 +278,14 @@ dot_weight_tc(const __grid_constant__ CUtensorMap tm_xl, const __grid_constant__
             }
           }
         }
-        ok = epi_sync();
-        if (!ok) break;
+        epi_sync(true);
         uint8_t* so = base_ptr + kDtOffT + side * kDtTBytes;
 #pragma unroll
         for (int q = 0; q < 8; ++q)
           *reinterpret_cast<ulonglong2*>(so + swz(row, q)) = make_ulonglong2(z2[2 * q], z2[2 * q + 1]);
       }
-      if (!ok) break;
       fence_async_smem();
-      ok = epi_sync();
-      if (!ok) break;
+      epi_sync(true);
       if (leader) {
         // output [S, Lx, Di, heads * Ly] with b = s * heads + h: box (32 j, 4 m, 32 i) at (h * Ly, m0, s * Lx + i0)
         const int sb = b / heads, hb = b % heads;

@@ -223,7 +223,6 @@ split_sign_gemm_tc(const __grid_constant__ CUtensorMap tm_lo, const __grid_const
   const uint32_t bar_mma_done = bar0 + 80;       // [2]    an array: that would live in local memory)
   const uint32_t bar_acc_ready = bar0 + 96;
   const uint32_t bar_acc_free = bar0 + 104;
-  const uint32_t bar_conv = bar0 + 128;          // rendezvous of the converter warps in the epilogue (bounded, unlike bar.sync)
   const uint32_t bar_res = bar0 + 136;           // residual tile has landed in the staging buffer (kResid)
   const uint32_t bar_mu = bar0 + 144;            // [2] row means of a tile are in shared memory (kLN)
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(base_ptr + SharedLayout::bars() + 112);
@@ -248,7 +247,6 @@ split_sign_gemm_tc(const __grid_constant__ CUtensorMap tm_lo, const __grid_const
     }
     mbar_init(bar_acc_ready, kIssuers);
     mbar_init(bar_acc_free, kEpiWarps);
-    mbar_init(bar_conv, kEpiWarps);
     mbar_init(bar_res, 1);
     mbar_init(bar_mu, kConvWarps);
     mbar_init(bar_mu + 8, kConvWarps);
@@ -427,15 +425,8 @@ split_sign_gemm_tc(const __grid_constant__ CUtensorMap tm_lo, const __grid_const
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const bool leader = threadIdx.x == 32 * kCtrlWarps;
     bool ok = true;
-    uint32_t epi_phase = 0;
-    // rendezvous of the epilogue warps through an mbarrier, so that the wait is bounded
-    auto epi_sync = [&]() -> bool {
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_conv);
-      const bool r = mbar_wait_warp(bar_conv, epi_phase & 1u, wc);
-      ++epi_phase;
-      return r;
-    };
+    // rendezvous of the epilogue warps; the waits between two of them leave their outcome in ok, and all warps leave together
+    auto epi_sync = [&](bool fine) { return meet_all<1, 32 * kEpiWarps>(fine); };
     const int chalf = (warp - kCtrlWarps) >> 2;   // which 32 of the 64 tile columns (= which output box)
     bool staging_zero = false;   // the staging buffer holds zeros (left there by a tile of a zero row block)
     int le = 0;                  // tiles read out of tensor memory so far (the issuers count the same tiles)
@@ -457,13 +448,13 @@ split_sign_gemm_tc(const __grid_constant__ CUtensorMap tm_lo, const __grid_const
         // little else.
         if (!staging_zero) {
           if (leader) tma_store_wait_read();
-          ok = epi_sync();
+          ok = epi_sync(ok);
           if (!ok) break;
           float4* sz = reinterpret_cast<float4*>(base_ptr + SharedLayout::out());
           for (uint32_t i = threadIdx.x - 32 * kCtrlWarps; i < kOutStageBytes / 16; i += 32 * kEpiWarps)
             sz[i] = make_float4(0.f, 0.f, 0.f, 0.f);
           fence_async_smem();
-          ok = epi_sync();
+          ok = epi_sync(ok);
           if (!ok) break;
           staging_zero = true;
         }
@@ -495,7 +486,7 @@ split_sign_gemm_tc(const __grid_constant__ CUtensorMap tm_lo, const __grid_const
       // the staging buffer is free once the previous tile's stores have read it: settle that before
       // the accumulators become ready, so that nothing stands between "ready" and the read-out
       if (leader) tma_store_wait_read();
-      ok = epi_sync();
+      ok = epi_sync(ok);
       if (!ok) break;
       if (kResid && leader) {
         // the staging buffer is free now: fetch the residual tile into it (same boxes as the store below)
@@ -523,18 +514,13 @@ split_sign_gemm_tc(const __grid_constant__ CUtensorMap tm_lo, const __grid_const
         }
       }
       ok = mbar_wait_warp(bar_acc_ready, (uint32_t)(le & 1), wc);
-      if (!ok) break;
       ++le;
       tc_fence_after();
-      if (kResid) {
-        ok = mbar_wait_warp(bar_res, (uint32_t)(e & 1), wc);
-        if (!ok) break;
-      }
+      if (kResid && ok) ok = mbar_wait_warp(bar_res, (uint32_t)(e & 1), wc);
       // kLN: the means over all 128 features of this thread's row of y_lw and of y_uw (product + bias + residual)
       uint64_t mlo2 = 0, mup2 = 0, sl2 = 0, su2 = 0;   // the means as pairs; running sums of the normalised row
       if (kLN) {
-        ok = mbar_wait_warp(bar_mu + 8 * (e & 1), (uint32_t)((e >> 1) & 1), wc);
-        if (!ok) break;
+        if (ok) ok = mbar_wait_warp(bar_mu + 8 * (e & 1), (uint32_t)((e >> 1) & 1), wc);
         const float2* mu = reinterpret_cast<const float2*>(ln_smem + kLnOffMu / 4) + ((e & 1) * 4) * 128 + row;
         const float2 p0 = mu[0], p1 = mu[128], p2 = mu[256], p3 = mu[384];
         const float mc = fadd(fadd(fadd(p0.x, p1.x), p2.x), p3.x), mr = fadd(fadd(fadd(p0.y, p1.y), p2.y), p3.y);
@@ -630,7 +616,7 @@ split_sign_gemm_tc(const __grid_constant__ CUtensorMap tm_lo, const __grid_const
             fadd(__uint_as_float((uint32_t)su2), __uint_as_float((uint32_t)(su2 >> 32)));
       }
       fence_async_smem();
-      ok = epi_sync();
+      ok = epi_sync(ok);
       if (!ok) break;
       if (leader) {
         // The output tensor map is 3-D.  Plain store: (column, row, 0).  Head-split store

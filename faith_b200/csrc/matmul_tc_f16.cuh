@@ -230,7 +230,7 @@ split_sign_gemm_f16(const __grid_constant__ CUtensorMap tm_lo, const __grid_cons
   const uint32_t bar_acc_ready = bar0 + 208, bar_acc_free = bar0 + 216;
   const uint32_t bar_max = bar0 + 224;                               // [row_warps]: largest values of the rows
   const uint32_t bar_scale = bar0 + 256;                             // [4]: scales for the epilogue
-  const uint32_t bar_epi = bar0 + 288, bar_w = bar0 + 296;           // epilogue rendezvous; [2] slices of W
+  const uint32_t bar_w = bar0 + 296;                                 // [2] slices of W
   const uint32_t bar_all = bar0 + 312, bar_scan = bar0 + 320;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + SM::bars + 400);
   volatile int* cta_abort = reinterpret_cast<volatile int*>(smem + SM::bars + 404);
@@ -276,7 +276,6 @@ split_sign_gemm_f16(const __grid_constant__ CUtensorMap tm_lo, const __grid_cons
     }
     mbar_init(bar_acc_ready, 2);
     mbar_init(bar_acc_free, kEpiWarps);
-    mbar_init(bar_epi, kEpiWarps);
     mbar_init(bar_all, kWarps);
     mbar_init(bar_scan, kConvWarps);
     *cta_abort = 0;
@@ -485,14 +484,8 @@ split_sign_gemm_f16(const __grid_constant__ CUtensorMap tm_lo, const __grid_cons
     const bool valid = n < ncols;
     const float wv = winv[n];
     const bool rare_w = *winv_max > 7.0e19f;
-    uint32_t epi_phase = 0;
-    auto epi_sync = [&]() -> bool {
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_epi);
-      const bool r = wait_warp(bar_epi, epi_phase & 1u, wc);
-      ++epi_phase;
-      return r;
-    };
+    // (with norms the epilogue's warps meet once a tile, and whether one has given up is settled there: a meeting has no limit)
+    auto agree = [&](bool fine) { return kNorm ? meet_all<1, 32 * kEpiWarps>(fine) : fine; };
     bool ok = true;
     int lt = 0;
     // kStream: these warps also convert W, the two of a lane quarter a k-block in turn: they wait for the accumulators most of the time.
@@ -512,7 +505,7 @@ split_sign_gemm_f16(const __grid_constant__ CUtensorMap tm_lo, const __grid_cons
       }
       return true;
     };
-    if (kStream) ok = give_w(0, 0, 2);
+    if (kStream) ok = agree(give_w(0, 0, 2));
     for (int pass = 0; pass < kPasses && ok; ++pass) {
       for (int ti = 0; ti < my_tiles && ok; ++ti) {
         const bool live = takes(pass, ti);
@@ -671,15 +664,17 @@ split_sign_gemm_f16(const __grid_constant__ CUtensorMap tm_lo, const __grid_cons
           if (!ok) break;
           ++lt;
         }
-        if (!ok) break;
-        if (kNorm && !bseg) {
+        if (kNorm && !bseg && ok) {
           // the norms over the tile's 128 rows: the two halves' parts in order (two tiles' parts alternate: nobody overwrites what
           // another warp still reads, since it meets that warp again before)
           float* part = reinterpret_cast<float*>(smem + SM::part) + (lt / kSubs & 1) * 512;
           part[h * 256 + n] = norm_combine(p.norm_p, nl[0], nl[1]);
           part[h * 256 + 128 + n] = kPoint ? norm_combine(p.norm_p, nl[0], nl[1]) : norm_combine(p.norm_p, nu[0], nu[1]);
-          ok = epi_sync();
-          if (!ok) break;
+        }
+        ok = agree(ok);
+        if (!ok) break;
+        if (kNorm && !bseg) {
+          const float* part = reinterpret_cast<const float*>(smem + SM::part) + (lt / kSubs & 1) * 512;
           const int line = et >> 7, col = et & 127;
           if (col < ncols)
             (line == 0 ? p.norm_lo : p.norm_up)[(int64_t)(my / BM) * N + n0 + col] =
@@ -688,7 +683,7 @@ split_sign_gemm_f16(const __grid_constant__ CUtensorMap tm_lo, const __grid_cons
       }
       if (kStream && ok && pass == 0) {
         __threadfence();   // a marked tile is stored again
-        ok = meet();
+        ok = agree(meet());
       }
     }
   } else {
