@@ -135,9 +135,6 @@ dot_weight_tc_any(const __grid_constant__ CUtensorMap tm_xl, const __grid_consta
   const uint32_t bar_mma_done = bar0 + 48;     // [2] MMAs of X, Y of the item complete
   const uint32_t bar_acc_ready = bar0 + 64;    // accumulators of the tile complete
   const uint32_t bar_acc_free = bar0 + 72;     // accumulators read out
-  const uint32_t bar_t_ready = bar0 + 80;      // [2] Y^T of a side is in the staging buffer
-  const uint32_t bar_t_free = bar0 + 96;       // [2] the transposition buffer of a side has been read
-  const uint32_t bar_z_ready = bar0 + 112;     // [2] the result of a side is in the buffer
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(base_ptr + kDaOffBars + 128);
   volatile int* cta_abort = reinterpret_cast<volatile int*>(base_ptr + kDaOffBars + 136);
 
@@ -154,9 +151,6 @@ dot_weight_tc_any(const __grid_constant__ CUtensorMap tm_xl, const __grid_consta
       mbar_init(bar_raw_empty + 8 * s, kDaConvWarps);
       mbar_init(bar_ops_ready + 8 * s, kDaConvWarps / 2);
       mbar_init(bar_mma_done + 8 * s, 2);
-      mbar_init(bar_t_ready + 8 * s, kDaEpiWarps / 2);
-      mbar_init(bar_t_free + 8 * s, kDaEpiWarps / 2);
-      mbar_init(bar_z_ready + 8 * s, kDaEpiWarps / 2);
     }
     mbar_init(bar_acc_ready, 4);
     mbar_init(bar_acc_free, kDaEpiWarps);
@@ -258,9 +252,10 @@ dot_weight_tc_any(const __grid_constant__ CUtensorMap tm_xl, const __grid_consta
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const uint64_t scale2 = pack2(__float_as_uint(A.out_scale), __float_as_uint(A.out_scale));
     uint8_t* const Z = base_ptr + kDaOffZ + side * kDaTile;
+    auto meet = [&](bool fine) { return side == 0 ? meet_all<1, 128>(fine) : meet_all<2, 128>(fine); };
     for (int t = 0; t < my_tiles; ++t) {
-      if (t > 0 && !mbar_wait_warp(bar_t_free + 8 * side, (uint32_t)((t - 1) & 1), cta_abort)) break;
-      if (!mbar_wait_warp(bar_acc_ready, (uint32_t)(t & 1), cta_abort)) break;
+      // (the warps of a side meet here, having stored the tile before, and settle whether one has given up)
+      if (!meet(mbar_wait_warp(bar_acc_ready, (uint32_t)(t & 1), cta_abort))) break;
       tc_fence_after();
       {
         const int j = row >> 2, m = row & 3;   // row of Y
@@ -278,11 +273,8 @@ dot_weight_tc_any(const __grid_constant__ CUtensorMap tm_xl, const __grid_consta
       load_acc(tmem_base + lane_addr + kDaX + 32 * side + 16, x[1]);
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(bar_acc_free);
-        mbar_arrive(bar_t_ready + 8 * side);
-      }
-      if (!mbar_wait_warp(bar_t_ready + 8 * side, (uint32_t)(t & 1), cta_abort)) break;
+      if (lane == 0) mbar_arrive(bar_acc_free);
+      meet(true);
       // this thread's row (i, m) of the transposition buffer holds Y^T: the result takes its place
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
@@ -293,14 +285,12 @@ dot_weight_tc_any(const __grid_constant__ CUtensorMap tm_xl, const __grid_consta
         tv.y = mul2(add2(pack2(v[2], v[3]), tv.y), scale2);
         *reinterpret_cast<ulonglong2*>(z) = tv;
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_z_ready + 8 * side);
       int b, i0, j0, m0;
       tile_coords(t, b, i0, j0, m0);
       float* const z0 = (side == 0 ? A.z_lw : A.z_uw) + (((int64_t)(b / A.heads) * A.Lx + i0) * A.Di + m0) * A.ldz +
                         (b % A.heads) * A.Ly + j0;
       const int ni = min(32, A.Lx - i0), nm = min(4, A.Di - m0), nj = min(32, A.Ly - j0);
-      if (!mbar_wait_warp(bar_z_ready + 8 * side, (uint32_t)(t & 1), cta_abort)) break;
+      meet(true);
       // coalesced stores: eight lanes per row (i, m), so a warp writes the four (mostly adjacent) rows of one i; or, for rows
       // that are not 16-byte aligned, a lane per value
       if (kVecOut) {
@@ -327,8 +317,6 @@ dot_weight_tc_any(const __grid_constant__ CUtensorMap tm_xl, const __grid_consta
                   *reinterpret_cast<const float*>(Z + swz(4 * i + m, lane >> 2) + (uint32_t)(lane & 3) * 4u);
         }
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_t_free + 8 * side);
     }
   } else {
     // ------------------------------------------------------------------ converters
