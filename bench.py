@@ -686,14 +686,14 @@ def main():
         # larger of the two fractions.  Both are measured figures (TF32 rate in this run, HBM copy bandwidth of this pool).
         frac_t, frac_h = dom["tflops"] / tf32_alg, dom["gbs"] / pk["hbm_gbs"]
         tensor_side = {"achieved": dom["tflops"], "peak": tf32_alg, "unit": "TFLOP/s", "frac": frac_t,
-                       "peak_source": "measured in this run: tcgen05 kind::tf32 rate %.0f TFLOP/s x 8/12 (the kernel executes "
+                       "peak_source": "measured in this run: tcgen05 kind::tf32 rate %.0f TFLOP/s x 8/12 (the TF32 kernel executes "
                                       "three TF32 products per fp32 product on two GEMMs instead of four: 12 tensor flops per 8 "
-                                      "algorithmic ones)" % pipes["tf32"],
+                                      "algorithmic ones; the fp16-split kernel as many at the fp16 rate)" % pipes["tf32"],
                        "frac_of_bf16_sustained": dom["tflops"] / pk["bf16_sustained"]}
         hbm_side = {"achieved": dom["gbs"], "peak": pk["hbm_gbs"], "unit": "GB/s", "frac": frac_h,
                     "peak_source": "%s HBM copy bandwidth" % pk["source"]}
         binding = hbm_side if frac_h >= frac_t else tensor_side
-        roofline = {"kernel": "split_sign_gemm_tc (all products of the pass)", "bound": "hbm" if frac_h >= frac_t else "tensor",
+        roofline = {"kernel": "split_sign_gemm_f16, split_sign_gemm_tc (all products of the pass)", "bound": "hbm" if frac_h >= frac_t else "tensor",
                     "achieved": binding["achieved"], "peak": binding["peak"], "unit": binding["unit"], "frac": binding["frac"],
                     "peak_source": binding["peak_source"], "tensor": tensor_side, "hbm": hbm_side,
                     "avg_ms_per_call": dom["ms"] / dom["calls"], "share_of_step": dom["share"],
