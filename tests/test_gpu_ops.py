@@ -1127,6 +1127,26 @@ def test_dot_product_transposed_edges(B, Lx, Ly, Di, K):
         helpers.assert_arbitrated(got, getattr(o, name), getattr(o64, name), "transposed dot %s %s" % (name, (B, Lx, Ly, Di, K)))
 
 
+# Short transposed columns, many of them (four to a warp): a last warp with fewer columns, lanes without a value.
+# Sums of at most 128 terms in fp32: within 128 roundings of their size.
+@pytest.mark.parametrize("p", [1.0, 2.0, float("inf")])
+@pytest.mark.parametrize("rows,Do,Di", [(601, 33, 128), (331, 61, 4), (97, 213, 60)])
+def test_concretize_of_short_transposed_columns(rows, Do, Di, p):
+    from faith_b200 import ops
+    from faith_b200._lib import FB_TRANSPOSED
+    g = torch.Generator(device=DEV).manual_seed(5)
+    lw = torch.randn(1, rows, Do, Di, generator=g, device=DEV)
+    uw = lw + torch.rand(1, rows, Do, Di, generator=g, device=DEV)
+    lb = torch.randn(1, rows, Do, generator=g, device=DEV)
+    ub = lb + 0.5
+    l, u = ops.concretize(lw, uw, lb, ub, p, 0.25, 1, FB_TRANSPOSED)
+    dual = {1.0: float("inf"), 2.0: 2.0, float("inf"): 1.0}[p]
+    for got, w, b, sign in ((l, lw, lb, -1.0), (u, uw, ub, 1.0)):
+        norm = torch.linalg.vector_norm(w.double(), dual, dim=-1)
+        tol = 128 * 2.0 ** -24 * (b.double().abs() + 0.25 * norm)
+        assert bool(((got.double() - (b.double() + sign * 0.25 * norm)).abs() <= tol).all())
+
+
 # (TMA-addressable rows: each block shape with 64, 32 and 16 coordinates to a warp, ragged in every direction, K past the ring and past
 # the values of the ranges staged at a time or shorter than one stage)
 @pytest.mark.parametrize("B,Lx,Ly,Di,K", [(4, 63, 62, 124, 66), (5, 33, 49, 68, 5), (3, 63, 62, 252, 40), (5, 65, 9, 68, 70), (5, 5, 49, 196, 70),
